@@ -52,6 +52,7 @@ struct PlanSlot {
     std::vector<ft_path_desc> paths;
     std::vector<ftk::WorkItem> h_items, h_items_w;
     DevBuf items, items_w;
+    ftk::TilePlan tile;
     int smem = -1, stroke = -1, wside = -1;
     uint64_t split = 0;
     void release() {
@@ -160,10 +161,10 @@ int build_smem(const ft_ctx* c, int n_bands) {
     return (int)std::min<size_t>(std::max<size_t>(48 * 1024, need), (size_t)c->max_smem);
 }
 
-// Largest canvas side the warp rasteriser takes (0 disables it).
-int warp_max_side(const ft_ctx* c) {
-    const int v = c->tuned ? c->tune.warp_max_side : ftk::WARP_MAX_SIDE;
-    return std::max(0, std::min(v, ftk::WARP_MAX_SIDE));
+// Largest canvas side of a batch's path that the tile rasteriser takes (0 disables it).
+int tile_max_side(const ft_ctx* c) {
+    const int v = c->tuned ? c->tune.warp_max_side : ftk::TILE_MAX_SIDE;
+    return std::max(0, std::min(v, ftk::TILE_MAX_SIDE));
 }
 
 // Paths of at least this many pixels are split into row ranges.
@@ -178,29 +179,35 @@ int grid_cap(const ft_ctx* c, int per_sm) {
     return c->sm_count * per_sm;
 }
 
-// Work items of the device queues: small paths go whole to the warp rasteriser,
-// large paths are split into row ranges of whole bands for the CTA rasteriser.
+// Most cells of a tile band when there are few paths (96 KB: a row range is one band).
+constexpr int TILE_AREA_FEW = 24576;
+
+// Work items of the device queues: fills of small canvases go to the tile rasteriser
+// (out_w), whole in a batch and by row ranges when there are few paths; large canvases and
+// strokes go to the CTA rasteriser, split into row ranges of whole bands from split_px.
 // Both lists are ordered longest first.
 void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem, std::vector<ftk::WorkItem>& out,
-                std::vector<ftk::WorkItem>& out_w, bool stroke) {
+                std::vector<ftk::WorkItem>& out_w, ftk::TilePlan& tile, bool stroke) {
     out.clear();
     out_w.clear();
     const int area_bytes = smem - ftk::RASTER_FIXED_SMEM;
     const uint64_t big_px = split_px(c);
-    // few paths cannot fill the GPU one warp or one CTA each: split their rows instead
+    // few paths cannot fill the GPU one CTA each: split their rows instead
     const bool few = n_paths < (uint32_t)std::max(2 * c->sm_count, 1);
-    const uint32_t wside = (stroke || few) ? 0u : (uint32_t)warp_max_side(c);  // strokes use the CTA kernel
+    const uint32_t wside = stroke ? 0u : (uint32_t)tile_max_side(c);  // strokes use the CTA kernel
+    tile = ftk::TilePlan{few ? ftk::TILE_THREADS_FEW : ftk::TILE_THREADS, few ? ftk::TILE_CAP_FEW : ftk::TILE_CAP, 8};
     for (uint32_t i = 0; i < n_paths; i++) {
         const ft_path_desc& d = paths[i];
         const uint32_t wp = (d.width + 3) & ~3u;
         uint32_t R = wp ? (uint32_t)(area_bytes / (int)(wp * 4)) : 1;
         R = std::max(1u, std::min(R, std::max(d.height, 1u)));
-        if (d.width <= wside && d.height <= wside) {
+        const bool big = (uint64_t)d.width * d.height >= big_px;
+        uint32_t rows_per_item = std::max(d.height, 1u);
+        if (!few && d.width <= wside && d.height <= wside) {
             out_w.push_back(ftk::WorkItem{i, 0, d.height, R});
             continue;
         }
-        uint32_t rows_per_item = std::max(d.height, 1u);
-        if ((uint64_t)d.width * d.height >= big_px && c->sm_count > 0) {
+        if (big && c->sm_count > 0) {
             uint32_t target = (d.height + (uint32_t)c->sm_count - 1) / (uint32_t)c->sm_count;
             rows_per_item = std::max(R, ((target + R - 1) / R) * R);
         } else if (few && c->sm_count > 0) {
@@ -208,8 +215,14 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
             const uint32_t parts = std::max(1u, (uint32_t)(2 * c->sm_count) / std::max(n_paths, 1u));
             rows_per_item = std::max(16u, (d.height + parts - 1) / parts);
         }
+        const bool tiled = few && !big && wside > 0;
+        if (tiled) {
+            const int pitch = ftk::tile_pitch((int)d.width);
+            const uint64_t want = (uint64_t)pitch * std::min(rows_per_item, std::max(d.height, 1u));
+            tile.few_area = std::max(tile.few_area, std::max(pitch, (int)std::min<uint64_t>(want, TILE_AREA_FEW)));
+        }
         for (uint32_t r = 0; r < std::max(d.height, 1u); r += rows_per_item)
-            out.push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
+            (tiled ? out_w : out).push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
     }
     auto order = [&](std::vector<ftk::WorkItem>& v) {
         std::vector<std::pair<uint64_t, uint32_t>> key(v.size());
@@ -262,20 +275,45 @@ int grid_for(ft_ctx* c, int smem, uint32_t n_items, bool stroke) {
     return std::max(1, std::min(grid, (int)std::max(n_items, 1u)));
 }
 
-// Grid of the warp rasteriser.
-int grid_for_warp(ft_ctx* c, uint32_t n_items_w) {
-    const int grid = grid_cap(c, ftk::raster_warp_blocks_per_sm());
-    const int need = (int)((n_items_w + ftk::NWARP - 1) / ftk::NWARP);
-    return std::max(1, std::min(grid, std::max(need, 1)));
+// Grid of the tile rasteriser.
+int grid_for_tile(ft_ctx* c, const ftk::TilePlan& t, uint32_t n_items_w, int tile_smem) {
+    const int grid = grid_cap(c, ftk::tile_blocks_per_sm(t.threads, tile_smem));
+    return std::max(1, std::min(grid, (int)std::max(n_items_w, 1u)));
 }
 
-// Enqueue the two rasterisers for prepared parameters: warps for small paths,
-// then CTAs for large paths and for small ones a warp could not hold.
-cudaError_t enqueue(const ftk::KParams& p, int grid_b, int grid_w, int smem, cudaStream_t st, uint64_t* launches,
-                    int sm_count) {
+// Scratch of the two rasterisers (they run one after the other and share it).
+size_t raster_scratch(const ftk::TilePlan& t, int grid, int grid_w, uint32_t n_items_w) {
+    return std::max(ftk::SCRATCH_BYTES_PER_CTA * (size_t)grid,
+                    n_items_w ? ftk::tile_scratch(t.cap) * (size_t)grid_w : (size_t)0);
+}
+
+// Enqueue the two rasterisers for prepared parameters: the tile rasteriser for small fills,
+// then the CTA rasteriser for large paths, strokes and what the tile rasteriser handed over.
+cudaError_t enqueue(const ftk::KParams& p, const ftk::TilePlan& t, int grid_b, int grid_w, int smem, cudaStream_t st,
+                    uint64_t* launches, int sm_count) {
     cudaError_t e = cudaSuccess;
     if (p.n_items_w) {
-        e = ftk::launch_raster_warp(p, grid_w, st);
+        ftk::TileParams q{};
+        q.ops = p.ops;
+        q.paths = p.paths;
+        q.items = p.items_w;
+        q.n_items = p.n_items_w;
+        q.overflow = p.overflow;
+        q.queue = p.queue;
+        q.rasters = p.rasters;
+        q.status = p.status;
+        q.sw_out = p.sw_out;
+        q.sw_chain = p.sw_chain;
+        q.scratch = p.scratch;
+        q.cap = t.cap;
+        q.area_ints = t.area(p.fmt, p.host_rasters != 0);
+        q.host_rasters = p.host_rasters;
+        q.rule = p.rule;
+        q.fmt = p.fmt;
+        for (int i = 0; i < 6; i++) q.xf[i] = p.xf[i];
+        q.tol_sq = p.tol_sq;
+        q.tol = std::sqrt(p.tol_sq);
+        e = ftk::launch_tile(q, t.threads, grid_w, t.smem(p.fmt, p.host_rasters != 0), st);
         if (e != cudaSuccess) return e;
         (*launches)++;
     }
@@ -297,12 +335,12 @@ int run_plan(ft_ctx* c, PlanSlot& slot, int stroke, int rule, const ft_op* ops_d
     const int smem = choose_smem(c, max_w);
     // a batch that comes back unchanged (same descriptors and plan knobs) keeps its
     // planned and uploaded work items
-    const bool same_plan = slot.smem == smem && slot.stroke == stroke && slot.wside == warp_max_side(c) &&
+    const bool same_plan = slot.smem == smem && slot.stroke == stroke && slot.wside == tile_max_side(c) &&
                            slot.split == split_px(c) && slot.paths.size() == n_paths &&
                            (n_paths == 0 || memcmp(slot.paths.data(), paths, sizeof(ft_path_desc) * n_paths) == 0);
     if (!same_plan) {
         slot.smem = -1;  // invalid until the new items are on the device
-        plan_items(c, paths, n_paths, smem, slot.h_items, slot.h_items_w, stroke != 0);
+        plan_items(c, paths, n_paths, smem, slot.h_items, slot.h_items_w, slot.tile, stroke != 0);
     }
     const uint32_t n_items = (uint32_t)slot.h_items.size(), n_items_w = (uint32_t)slot.h_items_w.size();
     FT_CU(c->paths.ensure(sizeof(ft_path_desc) * std::max(n_paths, 1u)), "alloc paths");
@@ -314,8 +352,8 @@ int run_plan(ft_ctx* c, PlanSlot& slot, int stroke, int rule, const ft_op* ops_d
     FT_CU(c->queue.ensure(256), "alloc queue");
     const int grid = n_items_w ? std::max(grid_for(c, smem, n_items, stroke), c->sm_count)
                                : grid_for(c, smem, n_items, stroke);
-    const int grid_w = grid_for_warp(c, n_items_w);
-    FT_CU(c->scratch.ensure(ftk::SCRATCH_BYTES_PER_CTA * (size_t)std::max(grid, grid_w)), "alloc scratch");
+    const int grid_w = grid_for_tile(c, slot.tile, n_items_w, slot.tile.smem(fmt, host_rasters));
+    FT_CU(c->scratch.ensure(raster_scratch(slot.tile, grid, grid_w, n_items_w)), "alloc scratch");
     FT_CU(cudaMemcpyAsync(c->paths.p, paths, sizeof(ft_path_desc) * n_paths, cudaMemcpyHostToDevice, c->stream),
           "upload paths");
     if (!same_plan) {
@@ -330,7 +368,7 @@ int run_plan(ft_ctx* c, PlanSlot& slot, int stroke, int rule, const ft_op* ops_d
         slot.paths.assign(paths, paths + n_paths);
         slot.smem = smem;
         slot.stroke = stroke;
-        slot.wside = warp_max_side(c);
+        slot.wside = tile_max_side(c);
         slot.split = split_px(c);
     }
     FT_CU(cudaMemsetAsync(c->queue.p, 0, 256, c->stream), "reset queue");
@@ -355,7 +393,7 @@ int run_plan(ft_ctx* c, PlanSlot& slot, int stroke, int rule, const ft_op* ops_d
     p.scratch = static_cast<unsigned char*>(c->scratch.p);
     c->comp_timed = false;
     if (events) FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
-    FT_CU(enqueue(p, grid, grid_w, smem, c->stream, &c->launches, c->sm_count), "launch rasteriser");
+    FT_CU(enqueue(p, slot.tile, grid, grid_w, smem, c->stream, &c->launches, c->sm_count), "launch rasteriser");
     if (events) {
         FT_CU(cudaEventRecord(c->ev1, c->stream), "event");
         c->timed = true;
@@ -460,6 +498,7 @@ struct ft_batch {
     uint32_t n_paths = 0, n_items = 0, n_items_w = 0;
     uint64_t ops_needed = 0, bytes_needed = 0;
     DevBuf paths, items, items_w, overflow, status, queue, scratch;
+    ftk::TilePlan tile;
     ftk::KParams params;
     const void* g_ops = nullptr;
     void* g_ras = nullptr;
@@ -511,12 +550,12 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
     }
     b->smem = choose_smem(c, max_w);
     std::vector<ftk::WorkItem> items, items_w;
-    plan_items(c, paths, n_paths, b->smem, items, items_w, stroke != 0);
+    plan_items(c, paths, n_paths, b->smem, items, items_w, b->tile, stroke != 0);
     b->n_items = (uint32_t)items.size();
     b->n_items_w = (uint32_t)items_w.size();
     b->grid = b->n_items_w ? std::max(grid_for(c, b->smem, b->n_items, stroke), c->sm_count)
                            : grid_for(c, b->smem, b->n_items, stroke);
-    b->grid_w = grid_for_warp(c, b->n_items_w);
+    b->grid_w = grid_for_tile(c, b->tile, b->n_items_w, b->tile.smem(fmt, false));
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = b->paths.ensure(sizeof(ft_path_desc) * std::max(n_paths, 1u));
     if (e == cudaSuccess) e = b->items.ensure(sizeof(ftk::WorkItem) * std::max(b->n_items, 1u));
@@ -524,7 +563,7 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
     if (e == cudaSuccess) e = b->overflow.ensure(sizeof(uint32_t) * std::max(b->n_items_w, 1u));
     if (e == cudaSuccess) e = b->status.ensure(sizeof(int32_t) * std::max(n_paths, 1u));
     if (e == cudaSuccess) e = b->queue.ensure(256);
-    if (e == cudaSuccess) e = b->scratch.ensure(ftk::SCRATCH_BYTES_PER_CTA * (size_t)std::max(b->grid, b->grid_w));
+    if (e == cudaSuccess) e = b->scratch.ensure(raster_scratch(b->tile, b->grid, b->grid_w, b->n_items_w));
     if (e == cudaSuccess && n_paths)
         e = cudaMemcpyAsync(b->paths.p, paths, sizeof(ft_path_desc) * n_paths, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess && b->n_items)
@@ -550,7 +589,6 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
     b->params.status = static_cast<int32_t*>(b->status.p);
     b->params.scratch = static_cast<unsigned char*>(b->scratch.p);
     ftk::raster_blocks_per_sm(b->smem, stroke != 0);  // sets the kernels' shared-memory attributes outside capture
-    ftk::raster_warp_blocks_per_sm();
     *out = b;
     return FT_OK;
 }
@@ -572,7 +610,7 @@ FT_API int ft_batch_launch(ft_ctx* c, ft_batch* b, const ft_op* ops, uint32_t n_
         FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
         FT_CU(cudaMemsetAsync(b->queue.p, 0, 256, c->stream), "reset queue");
         FT_CU(cudaMemsetAsync(b->status.p, 0, sizeof(int32_t) * std::max(b->n_paths, 1u), c->stream), "reset status");
-        FT_CU(enqueue(b->params, b->grid, b->grid_w, b->smem, c->stream, &c->launches, c->sm_count),
+        FT_CU(enqueue(b->params, b->tile, b->grid, b->grid_w, b->smem, c->stream, &c->launches, c->sm_count),
               "launch rasteriser");
         FT_CU(cudaEventRecord(c->ev1, c->stream), "event");
         c->timed = true;
@@ -586,7 +624,7 @@ FT_API int ft_batch_launch(ft_ctx* c, ft_batch* b, const ft_op* ops, uint32_t n_
         cudaError_t e1 = cudaMemsetAsync(b->queue.p, 0, 256, c->stream);
         cudaError_t e2 = cudaMemsetAsync(b->status.p, 0, sizeof(int32_t) * std::max(b->n_paths, 1u), c->stream);
         uint64_t nl = 0;
-        cudaError_t e3 = enqueue(b->params, b->grid, b->grid_w, b->smem, c->stream, &nl, c->sm_count);
+        cudaError_t e3 = enqueue(b->params, b->tile, b->grid, b->grid_w, b->smem, c->stream, &nl, c->sm_count);
         cudaError_t e4 = cudaStreamEndCapture(c->stream, &g);
         if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
@@ -632,7 +670,7 @@ FT_API int ft_set_tuning(ft_ctx* c, const ft_tuning* t) {
         c->tuned = false;
         return FT_OK;
     }
-    if (t->warp_max_side < 0 || t->warp_max_side > ftk::WARP_MAX_SIDE || t->cta_smem_bytes < 0 ||
+    if (t->warp_max_side < 0 || t->warp_max_side > ftk::TILE_MAX_SIDE || t->cta_smem_bytes < 0 ||
         (t->cta_smem_bytes && t->cta_smem_bytes < 40 * 1024) || t->cta_smem_bytes > c->max_smem ||
         t->split_px < 0 || t->grid_per_sm < 0 || t->band_rows < 0 || t->band_rows > ftk::NWARP ||
         t->pool_edges < 0 || t->host_chunks < 0 || t->host_chunks > 16 || t->host_mapped < 0 || t->host_mapped > 2 ||
@@ -649,7 +687,7 @@ FT_API int ft_get_tuning(ft_ctx* c, ft_tuning* t) {
     if (c->tuned) {
         *t = c->tune;
     } else {
-        *t = ft_tuning{ftk::WARP_MAX_SIDE, 0, 1 << 20, 0, 0, 0, 0, 0, 0, 0, 0};
+        *t = ft_tuning{ftk::TILE_MAX_SIDE, 0, 1 << 20, 0, 0, 0, 0, 0, 0, 0, 0};
     }
     return FT_OK;
 }
@@ -2006,12 +2044,12 @@ FT_API int ft_autotune_batch(ft_ctx* c, int32_t stroke, int32_t rule, const ft_o
     }
     const ft_tuning saved = c->tune;
     const bool saved_tuned = c->tuned;
-    // candidate plans: the built-in plan first, then canvas side of the warp/CTA split x
+    // candidate plans: the built-in plan first, then canvas side of the tile/CTA split x
     // CTA tile height (shared memory) x resident CTAs per SM.  A candidate replaces the
     // plan in hand only when it is faster by more than the timing noise (1 %): a knob the
-    // batch never exercises (the CTA tile of a batch that only the warp rasteriser draws)
+    // batch never exercises (the CTA tile of a batch that only the tile rasteriser draws)
     // keeps its built-in value.
-    const int sides[] = {ftk::WARP_MAX_SIDE, 0, 64, 128, 256, 512};
+    const int sides[] = {ftk::TILE_MAX_SIDE, 0, 64, 128, 256, 512};
     const int smems[] = {0, 40 * 1024, 48 * 1024, 64 * 1024, 96 * 1024};
     const int grids[] = {0, 2};
     float best_ms = 0.0f;

@@ -105,6 +105,11 @@ __device__ __forceinline__ bool pline_x(P2 a0, P2 a1, P2 b0, P2 b1, P2* out) {
     return true;
 }
 
+// min (y, x, id)
+__device__ __forceinline__ bool top_less(int ay, int ax, int ai, int by, int bx, int bi) {
+    return ay < by || (ay == by && (ax < bx || (ax == bx && ai < bi)));
+}
+
 // ------------------------------------------------------- pix 0.14 Ch8 / SrcOver
 __device__ __forceinline__ unsigned ch8_mul(unsigned a, unsigned b) {
     unsigned l = (a << 4) | (a >> 4);

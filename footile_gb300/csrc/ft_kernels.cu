@@ -55,11 +55,8 @@ __device__ __forceinline__ bool ck(bool ok, int site) {
     return !FT_CHECK || ok;
 }
 // Curve leaves of an op kept (in local memory) from the count pass for the emit pass;
-// ops with more leaves are walked again.  Warp builds (small glyphs) keep 64; CTA builds
-// (large figures, few CTAs, L1 to spare) keep more.
-constexpr int LEAF_CACHE = 64;
+// ops with more leaves are walked again.
 constexpr int LEAF_CACHE_CTA = 256;
-constexpr bool BLOCK_COMPACT = true;  // figure building by the whole CTA (false: warp 0)
 constexpr int SRAW = 1024;            // stroke points per window (float4 in the raw window's bytes)
 
 // ------------------------------------------------------------ block scans
@@ -143,8 +140,7 @@ __device__ void block_max_scan(int v, int* tmp, int& incl, int& excl) {
     __syncthreads();
 }
 
-// Thread-group policies: the figure builder runs either on a whole CTA (large
-// paths) or on one warp (small paths, many per CTA, no block barriers).
+// The thread group of the figure builder: a whole CTA.
 struct BlockG {
     static constexpr int N = BLOCK;
     static constexpr int RAW = RAW_CAP;
@@ -154,29 +150,6 @@ struct BlockG {
     __device__ static int incl_max(int v, int* tmp) { return block_incl_max(v, tmp); }
     __device__ static void max_scan(int v, int* tmp, int& incl, int& excl) { block_max_scan(v, tmp, incl, excl); }
 };
-struct WarpG {
-    static constexpr int N = 32;
-    static constexpr int RAW = 256;
-    __device__ static int rank() { return threadIdx.x & 31; }
-    __device__ static void sync() { __syncwarp(); }
-    __device__ static int excl_sum(int v, int*, int& total) {
-        __syncwarp();
-        const int inc = warp_incl_sum(v);
-        total = __shfl_sync(FULL, inc, 31);
-        return inc - v;
-    }
-    __device__ static int incl_max(int v, int*) {
-        __syncwarp();
-        return warp_incl_max(v);
-    }
-    __device__ static void max_scan(int v, int*, int& incl, int& excl) {
-        __syncwarp();
-        incl = warp_incl_max(v);
-        excl = __shfl_up_sync(FULL, incl, 1);
-        if ((threadIdx.x & 31) == 0) excl = -1;
-    }
-};
-
 // ------------------------------------------------- De Casteljau flattening
 // Stack frames of the walks: the right half of a subdivided curve.  A frame keeps no
 // start point: the right half starts where the last leaf of the left half ends (that
@@ -333,7 +306,6 @@ struct CState {
     int has_prev, prev_x, prev_y;  // previous raw vertex
     int rf_x, rf_y, rf_pos;        // first vertex of the current sub-figure and its id
     int capped;
-    int overflow;  // the figure outgrew the warp's scratch: hand the path to a CTA
     int flags;     // 1: depth cap reached, 2: bad argument
     // figure summary
     int top_row;
@@ -356,7 +328,6 @@ struct BuildSmemT {
     unsigned char rs[RAW];
 };
 using BuildSmem = BuildSmemT<BLOCK, RAW_CAP>;
-using WarpBuildSmem = BuildSmemT<32, 256>;
 
 constexpr int MAP_CAP = 4096;  // (edge, row) items mapped per round
 
@@ -370,7 +341,6 @@ struct RasterSmem {
 static_assert(((sizeof(RasterSmem) + 15) & ~(size_t)15) <= (size_t)RASTER_FIXED_SMEM, "raster smem layout");
 static_assert(sizeof(int2) * RAW_CAP >= sizeof(float4) * SRAW && RAW_CAP >= 2 * SRAW, "stroke window layout");
 static_assert(offsetof(BuildSmem, raw) % 16 == 0 && sizeof(BuildSmem) % 16 == 0, "build smem alignment");
-static_assert(offsetof(WarpBuildSmem, raw) % 8 == 0, "warp build smem alignment");
 
 // ------------------------------------------------------------ figure builder
 // Sequential restatement of Fig::add_point / Fig::close (fig.rs:373-461) for one
@@ -418,95 +388,9 @@ __device__ void seq_group(CState& S, const int2* raw, const unsigned char* rsf, 
     S.rf_pos = rf_pos;
 }
 
-// Warp 0: append one window of raw vertices to the figure.  A vertex is kept when
-// it starts a sub-figure or differs from the previous raw vertex; a sub-figure
-// whose last vertex equals its first loses that vertex when it is closed.
-__device__ void compact_window(CState& S, const int2* raw, const unsigned char* rsf, int m, int2* pts, int* ss,
-                               int limit) {
-    int lane = threadIdx.x & 31;
-    for (int base = 0; base < m; base += 32) {
-        int k = base + lane;
-        bool valid = k < m;
-        int2 p = valid ? raw[k] : make_int2(0, 0);
-        int rs = valid ? rsf[k] : 0;
-        int count = S.count, has_prev = S.has_prev;
-        int prevx = S.prev_x, prevy = S.prev_y;
-        int rfx0 = S.rf_x, rfy0 = S.rf_y, rf_pos0 = S.rf_pos;
-        unsigned vmask = __ballot_sync(FULL, valid);
-        unsigned RS = __ballot_sync(FULL, valid && rs);
-        // close of the run that ended with the previous group
-        int count_g = count;
-        if ((RS & 1u) && has_prev && rfx0 == prevx && rfy0 == prevy) count_g -= 1;
-        int qx = __shfl_up_sync(FULL, p.x, 1), qy = __shfl_up_sync(FULL, p.y, 1);
-        if (lane == 0) {
-            qx = prevx;
-            qy = prevy;
-        }
-        bool keep = valid && (rs || p.x != qx || p.y != qy);
-        unsigned K = __ballot_sync(FULL, keep);
-        unsigned E = (RS >> 1) & vmask;  // lane l ends its run when lane l+1 starts one
-        unsigned le = (lane == 31) ? FULL : ((2u << lane) - 1u);
-        unsigned rsl = RS & le;
-        int jf = rsl ? 31 - __clz(rsl) : -1;
-        int src = jf < 0 ? 0 : jf;
-        int rfx = __shfl_sync(FULL, p.x, src), rfy = __shfl_sync(FULL, p.y, src);
-        if (jf < 0) {
-            rfx = rfx0;
-            rfy = rfy0;
-        }
-        bool pop = ((E >> lane) & 1u) && p.x == rfx && p.y == rfy;
-        unsigned PM = __ballot_sync(FULL, pop);
-        unsigned below = (1u << lane) - 1u;
-        int pos = count_g + __popc(K & below) - __popc(PM & below);
-        if (__any_sync(FULL, keep && pos >= limit)) {
-            // more vertices than this warp's scratch holds
-            if (lane == 0) S.overflow = 1;
-            __syncwarp();
-            return;
-        }
-        unsigned capm = __ballot_sync(FULL, keep && pos >= PT_CAP);
-        if (capm) {
-            if (lane == 0) seq_group(S, raw + base, rsf + base, min(32, m - base), pts, ss);
-            __syncwarp();
-            return;
-        }
-        bool write = keep;
-        unsigned Ege = E & ~below;
-        if (keep && Ege) {
-            int e = __ffs(Ege) - 1;
-            if ((PM >> e) & 1u) {
-                unsigned upto_e = (e == 31) ? FULL : ((2u << e) - 1u);
-                if ((K & upto_e & ~le) == 0) write = false;  // the popped vertex
-            }
-        }
-        int posj = __shfl_sync(FULL, pos, src);
-        int ssv = jf < 0 ? rf_pos0 : posj;
-        if (write) {
-            pts[pos] = p;
-            ss[pos] = ssv;
-        }
-        int last = 31 - __clz(vmask);
-        int nprevx = __shfl_sync(FULL, p.x, last), nprevy = __shfl_sync(FULL, p.y, last);
-        int lrs = RS ? 31 - __clz(RS) : 0;
-        int nrfx = __shfl_sync(FULL, p.x, lrs), nrfy = __shfl_sync(FULL, p.y, lrs);
-        int nrfpos = __shfl_sync(FULL, pos, lrs);
-        __syncwarp();
-        if (lane == 0) {
-            S.count = count_g + __popc(K) - __popc(PM);
-            S.prev_x = nprevx;
-            S.prev_y = nprevy;
-            S.has_prev = 1;
-            if (RS) {
-                S.rf_x = nrfx;
-                S.rf_y = nrfy;
-                S.rf_pos = nrfpos;
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// Block-wide variant of compact_window: 256 raw vertices per step, one per thread.
+// Append one window of raw vertices to the figure, 256 per step, one per thread.  A vertex is
+// kept when it starts a sub-figure or differs from the previous raw vertex; a sub-figure whose
+// last vertex equals its first loses that vertex when it is closed.
 // Cross-lane questions (latest sub-figure start at or before a vertex, next kept
 // vertex, next run end) are answered from per-warp ballot masks in shared memory.
 struct CompactSmem {
@@ -892,7 +776,7 @@ __device__ void build_outline(const KParams& P, CState& S, const float4* spts, c
 
 // Path walk + flattening by the thread group G.
 // Fill (Plotter::fill, plotter.rs:339-350): builds the figure in pts[0..S.count) / ss[];
-// `limit` is the vertex capacity of pts/ss (a warp stops with S.overflow set beyond it).
+// `limit` is the figure's vertex cap.
 // STROKE (Plotter::stroke, plotter.rs:356-365, first half): collects the stroke points
 // with their widths in spts[0..S.s_count) and the sub-strokes in subs[0..S.s_nsubs).
 // Global raw store of a CTA figure build (SCR_RAWG ...); null: windows of raw
@@ -930,7 +814,6 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
         S.rf_x = S.rf_y = 0;
         S.rf_pos = 0;
         S.capped = 0;
-        S.overflow = 0;
         S.flags = 0;
         S.s_count = S.s_nsubs = S.s_capped = S.s_has_prev = 0;
         S.s_last_op = -1;
@@ -1023,7 +906,7 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
         int n = 0;
         int depth_hit = 0;
         bool nonfinite = false;
-        constexpr int LC = G::N == 32 ? LEAF_CACHE : LEAF_CACHE_CTA;
+        constexpr int LC = LEAF_CACHE_CTA;
         int2 cache[LC];  // leaves of the count pass, reused by the emit pass
         auto keep_leaf = [&](int k, P2 q, float) {
             if (k < LC) cache[k] = make_int2(f2fx(q.x), f2fx(q.y));
@@ -1075,7 +958,7 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
                 S.last_pc_kind = B.kind[last_pc];
             }
         }
-        if (G::N != 32 && rg.p4 && total > WIN) {
+        if (rg.p4 && total > WIN) {
             // ---- a chunk of several windows: emit every op's vertices once into the raw
             //      store (super-windows of RAWG when the chunk has more), then compact the
             //      store window by window
@@ -1137,9 +1020,9 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
                         compact_window_block(S, reinterpret_cast<const int2*>(rg.p4) + o, rg.rs + o, w1 - w0, pts, ss,
                                              *Cs, limit);
                     G::sync();
-                    if (S.capped || S.overflow || S.s_capped) break;
+                    if (S.capped || S.s_capped) break;
                 }
-                if (S.capped || S.overflow || S.s_capped) break;
+                if (S.capped || S.s_capped) break;
             }
         } else {
             // ---- emit and compact window by window
@@ -1198,26 +1081,22 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
                 if constexpr (STROKE) {
                     compact_stroke_block(S, reinterpret_cast<const float4*>(B.raw), B.rs, B.rs + SRAW, opi, w1 - w0,
                                          spts, subs, *Cs);
-                } else if (N == 32) {
-                    compact_window(S, B.raw, B.rs, w1 - w0, pts, ss, limit);
-                } else if (BLOCK_COMPACT) {
+                } else {
                     compact_window_block(S, B.raw, B.rs, w1 - w0, pts, ss, *Cs, limit);
-                } else if (tid < 32) {
-                    compact_window(S, B.raw, B.rs, w1 - w0, pts, ss, limit);
                 }
                 G::sync();
-                if (S.capped || S.overflow || S.s_capped) break;
+                if (S.capped || S.s_capped) break;
             }
         }
         G::sync();
-        if (S.capped || S.overflow || S.s_capped) break;
+        if (S.capped || S.s_capped) break;
     }
     if (STROKE) {
         G::sync();
         return;
     }
     // Plotter::fill ends with fig.close() (plotter.rs:347)
-    if (tid == 0 && !S.capped && !S.overflow && S.has_prev && S.rf_x == S.prev_x && S.rf_y == S.prev_y)
+    if (tid == 0 && !S.capped && S.has_prev && S.rf_x == S.prev_x && S.rf_y == S.prev_y)
         S.count -= 1;
     G::sync();
 }
@@ -1247,11 +1126,6 @@ __device__ int fig_dir(int top, int count, const int2* pts, const int* ss) {
     int cx = wsub(p0.x, p.x), cy = wsub(p0.y, p.y);
     // (p1 - p).widdershins(p0 - p) -> Forward   (fig.rs:116-119)
     return (fxmul(ax, cy) > fxmul(cx, ay)) ? 0 : 1;
-}
-
-// min (y, x, id)
-__device__ __forceinline__ bool top_less(int ay, int ax, int ai, int by, int bx, int bi) {
-    return ay < by || (ay == by && (ax < bx || (ax == bx && ai < bi)));
 }
 
 // Top vertex (min (y, x, id)) and figure direction (fig.rs:402-411, 493-496).
@@ -1347,22 +1221,6 @@ __device__ void build_edges(const CState& S, const int2* pts, const int* ss, Edg
     for (int i = G::rank(); i < count; i += G::N) edges[i] = edge_rec(i, count, figdir, pts, ss);
 }
 
-// Count one warp's edges by first scan row into hist[0 .. nrows) (zeroed by the
-// caller) for raster_sweep_warp's buckets: the rows of edge_rec's non-horizontal
-// edges, from the vertices alone (the records are built once, into their buckets).
-__device__ void count_edges_warp(const CState& S, const int2* pts, const int* ss, int* hist, int nrows) {
-    const int count = S.count, top_row = S.top_row;
-    for (int i = threadIdx.x & 31; i < count; i += 32) {
-        const int s = ss[i];
-        const int nx = (i + 1 < count && ss[i + 1] == s) ? i + 1 : s;
-        if (nx == i) continue;
-        const int ay = pts[i].y, by = pts[nx].y;
-        if (ay == by) continue;
-        const long long b = (long long)(min(ay, by) >> 16) - top_row;
-        if (b < nrows) atomicAdd(&hist[b], 1);
-    }
-}
-
 // Signed cell areas of one edge on one scan row (fig.rs:238-321), added into
 // `area` (the band row of width W).  The edge on this row: x_bot where it leaves the
 // row, its inverse slope, whether the row is its first (st) or last (en), the 16.16
@@ -1428,48 +1286,15 @@ __device__ __forceinline__ void scan_item(const EdgeRec& E, int y, int* area, in
              cell_step(E), E.ed, area, W, spans);
 }
 
-// Edge record of the warp sweep, 16 bytes, relative to the figure's top row t (rows
-// t .. t + 511 at most): x where the edge would leave row t (wrapping, like the row
-// steps), the inverse slope, the two y fractions, and the cell step with the end row
-// and the direction.  The first row is the bucket the record sits in.
-__device__ __forceinline__ int4 sweep_rec(const EdgeRec& E, int t) {
-    int4 R;
-    R.x = wsub(E.x_bot0, wmul(E.start_row - t, E.inv_slope));
-    R.y = E.inv_slope;
-    R.z = fxfract(E.y_upper) | (fxfract(E.y_lower) << 16);
-    R.w = (cell_step(E) - 1) | (min(E.end_row - t, SWEEP_END_FAR) << 16) | ((E.ed < 0) << 26);
-    return R;
-}
-__device__ __forceinline__ int sweep_end(int4 R) { return (R.w >> 16) & 1023; }
-
-// scan_item for a sweep record on row t + s; st: s is its first row.
-__device__ __forceinline__ void scan_sweep(int4 R, int s, bool st, int* row, int W) {
-    scan_row(wadd(R.x, wmul(s, R.y)), R.y, st, s == sweep_end(R), R.z & FX_MASK, (int)((unsigned)R.z >> 16),
-             (R.w & FX_MASK) + 1, (R.w >> 26) & 1 ? -1 : 1, row, W, nullptr);
-}
-
-// Resolve one band row and write it (fig.rs:621-665, imgbuf.rs:38-199).  With WORDS
-// (rasters in mapped host memory), Matte8 rows are written as aligned 4-byte words
-// whatever the row's alignment: lane L of a step stores the word at row position x - a
-// (a = the row's misalignment), made of the last a bytes of the previous lane's four
-// pixels and the first 4 - a of its own; the words at the row's ends are written byte by
-// byte inside the row — no partial words cross the host link.  In device memory the byte
-// stores of a misaligned row cost less than the shuffles.
-template <bool ZERO, bool WORDS>
-__device__ __forceinline__ void resolve_row(int* arow, int W, int Wp, uint8_t* drow, int rule, int fmt,
+// Resolve one band row and write it (fig.rs:621-665, imgbuf.rs:38-199).
+__device__ __forceinline__ void resolve_row(const int* arow, int W, int Wp, uint8_t* drow, int rule, int fmt,
                                             unsigned clr) {
     const int lane = threadIdx.x & 31;
     unsigned carry = 0;
-    const int mis = WORDS ? (int)(reinterpret_cast<uintptr_t>(drow) & 3) : 0;
-    const int xend = (WORDS && fmt == FT_MATTE8) ? W + mis : W;
-    unsigned pcarry = 0;  // Matte8: the previous step's last four pixels
-    for (int x0 = 0; x0 < xend; x0 += 128) {
+    for (int x0 = 0; x0 < W; x0 += 128) {
         const int x = x0 + lane * 4;
         int4 a = make_int4(0, 0, 0, 0);
-        if (x < Wp) {
-            a = *reinterpret_cast<const int4*>(arow + x);
-            if (ZERO) *reinterpret_cast<int4*>(arow + x) = make_int4(0, 0, 0, 0);
-        }
+        if (x < Wp) a = *reinterpret_cast<const int4*>(arow + x);
         const unsigned s0 = (unsigned)a.x;
         const unsigned s1 = s0 + (unsigned)a.y;
         const unsigned s2 = s1 + (unsigned)a.z;
@@ -1479,17 +1304,13 @@ __device__ __forceinline__ void resolve_row(int* arow, int W, int Wp, uint8_t* d
         carry += __shfl_sync(FULL, inc, 31);
         const unsigned v0 = resolve_cov(s0 + ex, rule), v1 = resolve_cov(s1 + ex, rule);
         const unsigned v2 = resolve_cov(s2 + ex, rule), v3 = resolve_cov(s3 + ex, rule);
-        if (fmt == FT_MATTE8 && !WORDS) {
-            if (x >= W) continue;
+        if (x >= W) continue;
+        if (fmt == FT_MATTE8) {
             uint8_t* dp = drow + x;
             if (x + 3 < W && ((reinterpret_cast<uintptr_t>(dp) & 3) == 0)) {
                 // masks are written once and not read back: stream them past L2 (evict first),
                 // leaving L2 to the rasterisers' figure scratch
-                const unsigned px4 = v0 | (v1 << 8) | (v2 << 16) | (v3 << 24);
-                if (__isGlobal(dp))
-                    __stcs(reinterpret_cast<unsigned*>(dp), px4);
-                else
-                    *reinterpret_cast<unsigned*>(dp) = px4;
+                __stcs(reinterpret_cast<unsigned*>(dp), v0 | (v1 << 8) | (v2 << 16) | (v3 << 24));
             } else {
                 dp[0] = (uint8_t)v0;
                 if (x + 1 < W) dp[1] = (uint8_t)v1;
@@ -1498,31 +1319,11 @@ __device__ __forceinline__ void resolve_row(int* arow, int W, int Wp, uint8_t* d
             }
             continue;
         }
-        if (WORDS && fmt == FT_MATTE8) {
-            const unsigned px4 = v0 | (v1 << 8) | (v2 << 16) | (v3 << 24);  // pixels x .. x + 3
-            unsigned prev = __shfl_up_sync(FULL, px4, 1);
-            if (lane == 0) prev = pcarry;
-            pcarry = __shfl_sync(FULL, px4, 31);
-            const unsigned word = mis ? (px4 << (8 * mis)) | (prev >> (32 - 8 * mis)) : px4;
-            const int lo = x - mis;  // row position of the word's first byte (4-byte aligned address)
-            uint8_t* wp = drow + lo;
-            if (lo >= 0 && lo + 3 < W) {
-                *reinterpret_cast<unsigned*>(wp) = word;
-            } else {
+        unsigned* dp = reinterpret_cast<unsigned*>(drow) + x;
+        const unsigned vv[4] = {v0, v1, v2, v3};
 #pragma unroll
-                for (int b = 0; b < 4; b++)
-                    if (lo + b >= 0 && lo + b < W) wp[b] = (uint8_t)(word >> (8 * b));
-            }
-            continue;
-        }
-        if (x >= W) continue;
-        {
-            unsigned* dp = reinterpret_cast<unsigned*>(drow) + x;
-            const unsigned vv[4] = {v0, v1, v2, v3};
-#pragma unroll
-            for (int c = 0; c < 4; c++)
-                if (x + c < W) dp[c] = srcover_rgba(dp[c], clr, vv[c]);
-        }
+        for (int c = 0; c < 4; c++)
+            if (x + c < W) dp[c] = srcover_rgba(dp[c], clr, vv[c]);
     }
 }
 
@@ -1580,200 +1381,8 @@ __device__ void raster_rows(const KParams& P, const ft_path_desc& d, const CStat
             }
         }
         for (int rr = r0 + warp; rr < r1; rr += NWARP)
-            resolve_row<false, false>(area + (size_t)(rr - r0) * Wp, W, Wp, base + (size_t)rr * d.stride, P.rule,
-                                      P.fmt, clr);
+            resolve_row(area + (size_t)(rr - r0) * Wp, W, Wp, base + (size_t)rr * d.stride, P.rule, P.fmt, clr);
         __syncthreads();
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Warp rasteriser: one warp per small path.  After building the figure, the warp
-// sweeps the scan rows top to bottom like footile's Scanner (fig.rs:536-617):
-// edges are bucketed by their first row, each row processes the active edges one
-// per lane into a one-row i32 buffer, then resolves and writes the row.
-struct WarpSmem {
-    CState S;
-    int tmp3[4];
-    union __align__(16) {
-        WarpBuildSmem B;
-        int hist[WARP_MAX_SIDE];
-    } u;
-    __align__(16) int row[WARP_MAX_SIDE];  // read and cleared as int4 by resolve_row
-};
-static_assert(offsetof(WarpSmem, row) % 16 == 0 && sizeof(WarpSmem) % 16 == 0, "warp smem alignment");
-
-// Rows of a mapped host raster staged in shared memory so that whole 128-byte lines cross
-// the host link: a raster whose rows are contiguous (stride == width) is one byte range
-// [lo, end); rows are resolved into `stg` (which holds the bytes from the line address L0
-// on), then every complete line is stored with one aligned word per lane, and the partial
-// line left over moves to the front of the buffer.  Bytes outside [lo, end) are never
-// stored (the rows above the figure and other rasters keep theirs).
-constexpr int STAGE_BYTES = 768;  // a partial line (< 128 B) and one row (<= WARP_MAX_SIDE B)
-static_assert(127 + WARP_MAX_SIDE < STAGE_BYTES && STAGE_BYTES % 128 == 0, "staging holds a line and a row");
-static_assert(sizeof(int) * WARP_MAX_SIDE + STAGE_BYTES <= sizeof(WarpBuildSmem), "row staging fits the build window");
-
-__device__ __forceinline__ void stage_flush(unsigned char* stg, uint8_t*& L0, const uint8_t* lo, const uint8_t* end,
-                                            bool final) {
-    const int lane = threadIdx.x & 31;
-    const int fill = (int)(end - L0);
-    const int nfull = final ? (fill + 127) >> 7 : fill >> 7;
-    for (int li = 0; li < nfull; li++) {
-        const int o = (li << 7) + 4 * lane;
-        uint8_t* a = L0 + o;
-        const unsigned wv = *reinterpret_cast<const unsigned*>(stg + o);
-        if (a >= lo && a + 4 <= end) {
-            *reinterpret_cast<unsigned*>(a) = wv;
-        } else {
-#pragma unroll
-            for (int b = 0; b < 4; b++)
-                if (a + b >= lo && a + b < end) a[b] = (uint8_t)(wv >> (8 * b));
-        }
-    }
-    if (final) return;
-    const int rest = fill - (nfull << 7);  // < 128: the partial line moves to the front
-    if (nfull > 0) {
-        const unsigned v = *reinterpret_cast<const unsigned*>(stg + (nfull << 7) + 4 * lane);
-        __syncwarp();
-        if (4 * lane < rest) *reinterpret_cast<unsigned*>(stg + 4 * lane) = v;
-        __syncwarp();
-        L0 += nfull << 7;
-    }
-}
-
-// The edge records (sweep_rec) are built straight into their buckets (`sorted`); the
-// active edge list holds the records themselves (one load per edge and row from a list
-// that stays small and hot, instead of an index and a record of the figure's edges).
-// hist holds every start row's edge count (count_edges_warp).
-template <bool WORDS>
-__device__ void raster_sweep_warp(const KParams& P, const ft_path_desc& d, const CState& S, const int2* pts,
-                                  const int* ss, int4* sorted, int4* active, int* hist, int* row,
-                                  unsigned char* stg) {
-    const int lane = threadIdx.x & 31;
-    const int count = S.count, H = (int)d.height, W = (int)d.width, Wp = (W + 3) & ~3;
-    const int top_row = S.top_row, row_begin = max(top_row, 0);
-    const int nrows = H - row_begin;
-    const unsigned clr = (unsigned)d.clr[0] | ((unsigned)d.clr[1] << 8) | ((unsigned)d.clr[2] << 16) |
-                         ((unsigned)d.clr[3] << 24);
-    uint8_t* base = P.rasters + d.raster_offset;
-    // bucket the edges by their first scan row (edges below the last row never start)
-    int carry = 0;
-    for (int b0 = 0; b0 < nrows; b0 += 32) {
-        const int b = b0 + lane;
-        const int v = b < nrows ? hist[b] : 0;
-        const int inc = warp_incl_sum(v);
-        if (b < nrows) hist[b] = carry + inc - v;
-        carry += __shfl_sync(FULL, inc, 31);
-    }
-    __syncwarp();
-    for (int e = lane; e < count; e += 32) {  // the records themselves, in bucket order
-        const EdgeRec E = edge_rec(e, count, S.dir, pts, ss);
-        if (E.ed) {
-            const long long b = (long long)E.start_row - top_row;
-            if (b < nrows && ck(b >= 0, 3)) {
-                const int k = atomicAdd(&hist[b], 1);
-                if (ck(k >= 0 && k < WARP_CAP, 4)) sorted[k] = sweep_rec(E, top_row);
-            }
-        }
-    }
-    for (int x = lane; x < Wp; x += 32) row[x] = 0;
-    __syncwarp();
-    // mapped host rasters with contiguous rows go out in whole lines (stage_flush)
-    const bool staged = WORDS && d.stride == d.width;
-    uint8_t* const lo = base + (size_t)row_begin * d.stride;
-    uint8_t* L0 = reinterpret_cast<uint8_t*>(reinterpret_cast<uintptr_t>(lo) & ~(uintptr_t)127);
-    // hist[b] now ends bucket b
-    int n_act = 0;
-    for (int s = 0; s < nrows; s++) {
-        const int bs = s == 0 ? 0 : hist[s - 1], be = hist[s];
-        for (int k = lane; k < be - bs; k += 32)
-            if (ck(n_act + k < WARP_CAP && bs + k < WARP_CAP, 5)) active[n_act + k] = sorted[bs + k];
-        const int n_old = n_act;  // records from n_old on start on this row
-        n_act += be - bs;
-        __syncwarp();
-        int nn = 0;
-        for (int a0 = 0; a0 < n_act; a0 += 32) {
-            const int idx = a0 + lane;
-            const bool v = idx < n_act;
-            int4 R;
-            int end = -1;
-            if (v) {
-                R = active[idx];
-                end = sweep_end(R);
-                scan_sweep(R, s, idx >= n_old, row, W);
-            }
-            // an edge leaves the active list after its last row (fig.rs:582, 603-617);
-            // records that keep their place are not rewritten
-            const bool keep = v && end > s;
-            const unsigned km = __ballot_sync(FULL, keep);
-            const int dst = nn + __popc(km & ((1u << lane) - 1u));
-            if (keep && dst != idx) active[dst] = R;
-            nn += __popc(km);
-        }
-        n_act = nn;
-        __syncwarp();
-        uint8_t* drow = base + (size_t)(row_begin + s) * d.stride;
-        if (staged) {
-            resolve_row<true, false>(row, W, Wp, stg + (drow - L0), P.rule, P.fmt, clr);
-            __syncwarp();
-            stage_flush(stg, L0, lo, drow + W, false);
-        } else {
-            resolve_row<true, WORDS>(row, W, Wp, drow, P.rule, P.fmt, clr);
-        }
-        __syncwarp();
-    }
-    if (staged) stage_flush(stg, L0, lo, base + (size_t)H * d.stride, true);
-}
-
-// WORDS: the rasters are mapped host memory (Matte8 rows go out as aligned words).
-template <bool WORDS>
-__global__ void __launch_bounds__(BLOCK, 4) k_raster_warp(KParams P) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    WarpSmem& M = reinterpret_cast<WarpSmem*>(smem)[warp];
-    unsigned char* scr = P.scratch + (size_t)blockIdx.x * SCRATCH_BYTES_PER_CTA + (size_t)warp * WS_BYTES;
-    int2* pts = reinterpret_cast<int2*>(scr + WS_PTS);
-    int* ss = reinterpret_cast<int*>(scr + WS_SS);
-    int4* sorted = reinterpret_cast<int4*>(scr + WS_SORT);
-    int4* active = reinterpret_cast<int4*>(scr + WS_ACT);
-    for (;;) {
-        int it = 0;
-        if (lane == 0) it = (int)atomicAdd(&P.queue[1], 1u);
-        it = __shfl_sync(FULL, it, 0);
-        if (it >= (int)P.n_items_w) break;
-        const WorkItem wi = P.items_w[it];
-        const ft_path_desc d = P.paths[wi.path];
-        const float sw0 = P.sw_chain ? *P.sw_chain : d.s_width;
-        build_fill<WarpG>(P, d, sw0, M.u.B, nullptr, M.S, pts, ss, WARP_CAP);
-        if (M.S.overflow) {
-            // too many vertices for a warp: a CTA of the next kernel redoes this path
-            if (lane == 0) P.overflow[atomicAdd(&P.queue[2], 1u)] = wi.path;
-            __syncwarp();
-            continue;
-        }
-        if (M.S.count > 0) {
-            top_and_dir<WarpG>(M.S, pts, ss, M.tmp3);
-            __syncwarp();
-            const int nrows = (int)d.height - max(M.S.top_row, 0);
-            if (nrows > 0 && d.width > 0) {
-                for (int b = lane; b < nrows; b += 32) M.u.hist[b] = 0;  // the build's shared area is free
-                __syncwarp();
-                count_edges_warp(M.S, pts, ss, M.u.hist, nrows);
-                __syncwarp();
-                // the build's window is free during the sweep: its bytes after the
-                // histogram stage the rows of a mapped host raster
-                raster_sweep_warp<WORDS>(P, d, M.S, pts, ss, sorted, active, M.u.hist, M.row,
-                                         reinterpret_cast<unsigned char*>(&M.u) + sizeof(M.u.hist));
-            }
-        }
-        if (P.sw_out) {
-            int lp = -1;
-            for (int i = lane; i < (int)d.n_ops; i += 32)
-                if (P.ops[d.op_begin + i].kind == FT_OP_PEN_WIDTH) lp = max(lp, i);
-            lp = warp_incl_max(lp);
-            if (lane == 31) P.sw_out[wi.path] = lp >= 0 ? P.ops[d.op_begin + lp].v[0] : sw0;
-        }
-        if (lane == 0 && M.S.flags) atomicMax(&P.status[wi.path], (M.S.flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
-        __syncwarp();
     }
 }
 
@@ -1790,7 +1399,7 @@ __global__ void __launch_bounds__(BLOCK) k_raster(KParams P) {
     EdgeRec* edges = reinterpret_cast<EdgeRec*>(scr + SCR_EDGES);
     float4* spts = reinterpret_cast<float4*>(scr + SCR_SPTS);
     SubRec* subs = reinterpret_cast<SubRec*>(scr + SCR_SUBS);
-    // paths the warp rasteriser handed over (it ran before this kernel)
+    // paths the tile rasteriser handed over (it ran before this kernel)
     const int n_over = P.overflow ? (int)*(volatile uint32_t*)&P.queue[2] : 0;
     for (;;) {
         if (tid == 0) s_item = (int)atomicAdd(&P.queue[0], 1u);
@@ -1871,29 +1480,6 @@ int raster_blocks_per_sm(int smem_bytes, bool stroke) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, BLOCK, smem_bytes) != cudaSuccess) return 1;
-    return n > 0 ? n : 1;
-}
-
-cudaError_t launch_raster_warp(const KParams& p, int grid, cudaStream_t s) {
-    const int smem = raster_warp_smem();
-    cudaError_t e = cudaFuncSetAttribute(p.host_rasters ? k_raster_warp<true> : k_raster_warp<false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    if (p.host_rasters)
-        k_raster_warp<true><<<grid, BLOCK, smem, s>>>(p);
-    else
-        k_raster_warp<false><<<grid, BLOCK, smem, s>>>(p);
-    return cudaGetLastError();
-}
-
-int raster_warp_smem() { return (int)(NWARP * sizeof(WarpSmem)); }
-
-int raster_warp_blocks_per_sm() {
-    const int smem = raster_warp_smem();
-    cudaFuncSetAttribute(k_raster_warp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(k_raster_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_raster_warp<false>, BLOCK, smem) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 

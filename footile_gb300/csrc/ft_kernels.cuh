@@ -88,18 +88,6 @@ static_assert(scr_layout(PT_CAP).bytes == SCRATCH_BYTES_PER_CTA && scr_layout(PT
 // Largest figure of the un-capped extension (ft_set_figure_cap).
 constexpr uint32_t FIG_CAP_MAX = 1u << 26;
 
-// Warp rasteriser (one warp per small path): per-warp share of the CTA scratch.
-constexpr int WARP_CAP = 8191;        // vertices a warp holds; larger figures go to a CTA
-constexpr int WARP_MAX_SIDE = 512;    // canvases up to this width and height use the warp rasteriser
-static_assert(WARP_MAX_SIDE <= 1023, "sweep records hold rows below 1023");
-constexpr size_t WS_PTS = 0;
-constexpr size_t WS_SS = align256(WS_PTS + (size_t)WARP_CAP * sizeof(int2));
-constexpr size_t WS_SORT = align256(WS_SS + (size_t)WARP_CAP * sizeof(int));     // sweep records by start row
-constexpr size_t WS_ACT = align256(WS_SORT + (size_t)WARP_CAP * sizeof(int4));
-constexpr size_t WS_BYTES = align256(WS_ACT + (size_t)WARP_CAP * sizeof(int4));  // active sweep records
-constexpr int SWEEP_END_FAR = 1023;  // sweep record end row: beyond the warp's last row
-static_assert(NWARP * WS_BYTES <= SCRATCH_BYTES_PER_CTA, "warp scratch layout");
-
 // Grid-wide figure build of one fill path (launch_grid_build): per-op and per-raw-vertex
 // arrays in one device buffer laid out by gb_layout.
 constexpr int GB_PER = 4;                      // raw vertices per thread of the tile kernels
@@ -193,10 +181,10 @@ struct KParams {
     const ft_path_desc* paths;
     const WorkItem* items;   // CTA work items (large paths, row ranges)
     uint32_t n_items;
-    const WorkItem* items_w; // warp work items (small paths, whole rasters)
+    const WorkItem* items_w; // tile rasteriser's work items
     uint32_t n_items_w;
-    uint32_t* overflow;      // paths a warp handed over to the CTA kernel
-    uint32_t* queue;         // [0]: next CTA item, [1]: next warp item, [2]: overflow count
+    uint32_t* overflow;      // paths the tile rasteriser handed over to the CTA kernel
+    uint32_t* queue;         // [0]: next CTA item, [1]: next tile item, [2]: overflow count
     uint8_t* rasters;
     int32_t* status;         // per path, atomicMax of FT_ERR_* codes
     float* sw_out;           // per path pen width after the call (nullable)
@@ -237,6 +225,52 @@ struct KParams {
     GridBuildBufs gb;
     GridStrokeBufs gs;  // and the stroker's part of one stroke path (launch_grid_stroke)
 };
+
+// The tile rasteriser (ft_tile.cu): fills of small canvases, one CTA of TILE_THREADS per
+// path, or of TILE_THREADS_FEW per row range of a path when there are few paths.
+constexpr int TILE_THREADS = 128, TILE_THREADS_FEW = 512;
+constexpr int TILE_MAX_SIDE = 512;                      // canvases up to this width and height (batches)
+constexpr int TILE_CAP = 32768, TILE_CAP_FEW = 65504;   // segment slots per CTA (at most the vertex cap)
+static_assert(TILE_CAP % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");
+// Cells from one row of a band to the next: three spare cells (a walk of four cells may run
+// past the raster's last), a multiple of eight.
+__host__ __device__ constexpr int tile_pitch(int w) { return (w + 3 + 7) & ~7; }
+constexpr size_t tile_scratch(int cap) { return align256((size_t)cap * 16 + (size_t)cap / 8); }
+struct TileParams {
+    const ft_op* ops;
+    const ft_path_desc* paths;
+    const WorkItem* items;
+    uint32_t n_items;
+    uint32_t* overflow;      // paths handed to k_raster
+    uint32_t* queue;         // [1]: next item, [2]: overflow count
+    uint8_t* rasters;
+    int32_t* status;         // per path, atomicMax of FT_ERR_* codes
+    float* sw_out;           // per path pen width after the call (nullable)
+    const float* sw_chain;   // nullable: initial pen width of every path
+    unsigned char* scratch;  // gridDim.x * tile_scratch(cap) bytes
+    int cap;                 // segment slots per CTA
+    int area_ints;           // cells of a band (a multiple of 8, at least one row of every item)
+    int host_rasters;        // rasters are mapped host memory
+    int rule, fmt;
+    float xf[6];
+    float tol, tol_sq;
+};
+int tile_smem(int threads, int area_ints, bool staged);
+// What one launch of the tile rasteriser runs with.
+struct TilePlan {
+    int threads = TILE_THREADS, cap = TILE_CAP;
+    int few_area = 8;  // with TILE_THREADS_FEW: the largest item's cells, up to 96 KB
+    // Rgba8p and host rows are staged as bytes
+    static bool staged(int fmt, bool host) { return host || fmt == FT_RGBA8P; }
+    // Batches: the cells that leave room for eight CTAs per SM.  65,536 glyphs with 2,560 /
+    // 3,328 / 4,096 / 4,992 cells (the last seven CTAs): 4.75 / 4.46 / 4.29 / 4.34 ms.
+    int area(int fmt, bool host) const {
+        return threads == TILE_THREADS_FEW ? few_area : (staged(fmt, host) ? 3712 : 4736);
+    }
+    int smem(int fmt, bool host) const { return tile_smem(threads, area(fmt, host), staged(fmt, host)); }
+};
+int tile_blocks_per_sm(int threads, int smem);
+cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cudaStream_t s);
 
 // Ordered composite: per-path figure build and edge binning, then one CTA per band.
 // `few_ctas`: at most one CTA per SM — prefer L1 over shared memory (the curve walks'
@@ -283,11 +317,6 @@ constexpr int RASTER_FIXED_SMEM = BLOCK * (int)sizeof(EdgeRec) + 3 * BLOCK * 4 +
 
 // Launch the persistent rasteriser.  Returns the CUDA error of the launch.
 cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas);
-// Launch the warp rasteriser (small paths).  Its dynamic shared memory is fixed.
-cudaError_t launch_raster_warp(const KParams& p, int grid, cudaStream_t s);
-int raster_warp_smem();
-int raster_warp_blocks_per_sm();
-
 // Resident CTAs per SM for `smem_bytes` of dynamic shared memory.
 int raster_blocks_per_sm(int smem_bytes, bool stroke);
 

@@ -1,0 +1,952 @@
+// ft_tile.cu — the tile rasteriser: fills of small canvases, one CTA per path (or per row
+// range of a path), the figure never sorted or compacted.
+//
+// footile builds a figure vertex by vertex (fig.rs:373-461): coincident vertices are
+// dropped, a closing vertex equal to the sub-figure's first is popped, the vertices are
+// sorted and an active-edge list is swept (fig.rs:493-617).  None of that order reaches the
+// mask: the cell areas are wrapping sums, a zero-length segment gives no edge whether its
+// vertex was kept or not, and only two things depend on the vertex list, both functions of
+// the non-zero segments alone:
+//   - the top row, the least y of a vertex that starts a non-zero segment (a sub-figure
+//     whose points all coincide is popped whole, and has no such segment);
+//   - the direction of the figure (fig.rs:402-411): the top vertex is the start of the
+//     first non-zero segment with the least (y, x); the vertex after it is that segment's
+//     end, the vertex before it is the start of the non-zero segment before it in its
+//     sub-figure, cyclically.
+// The direction only flips the sign of every cell sum, so it is applied at the resolve.
+//
+// So every leaf of a curve's subdivision is an edge by itself: the subdivision node's start
+// and end points (the start is the end of the leaf before, bit for bit).  A leaf's address is
+// its path from the root, so the leaves of an op take 2^D consecutive slots, D the depth at
+// which the whole curve is flat (estimated from its second differences, then checked by every
+// leaf), and one thread per slot walks straight down D levels — no stack, no count pass, every
+// lane a leaf of its own.  A node that is flat above depth D belongs to the first slot of its
+// range; the other slots of the range stay empty (zero-length).
+//
+// The segments (16 bytes: both end points in 16.16) go to the CTA's scratch in order.  Bands
+// of raster rows are then accumulated in shared memory: each warp takes 32 segments at a time
+// that reach the band, works out slope and step once per segment, and spreads the (edge, row)
+// items over its lanes.  The rows are resolved 8 pixels per lane, as many rows per warp as
+// fit, and written once.
+//
+// A path whose slots exceed the scratch, or whose curves subdivide deeper than TILE_DEPTH or
+// not as estimated, is handed to k_raster through the overflow list.
+#include <climits>
+#include <cstddef>
+
+#include "ft_device.cuh"
+#include "ft_kernels.cuh"
+
+namespace ftk {
+namespace {
+
+constexpr unsigned ALL = 0xFFFFFFFFu;
+constexpr int TILE_DEPTH = 12;  // deepest subdivision a slot walks
+
+// ---------------------------------------------------------------- arithmetic
+// Low 32 bits of n * 65536 / d (truncated), d != 0: Fixed division (fixed.rs:49-56) of
+// magnitudes without the 64-bit divide.  The quotient is estimated in float (relative error
+// below 2^-21), the remainder corrects it: a second estimate of what is missing leaves less
+// than one unit, which the last comparisons settle.  With n and d below 2^28 (4,096 pixels)
+// the remainder stays below 2^23 + d, so 32-bit wrapping arithmetic holds it.  Larger
+// operands and quotients of 2^31 and above (slopes of 32,768 and more) take the 64-bit divide.
+__device__ __forceinline__ unsigned fx_quot(unsigned n, unsigned d) {
+    float f;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)d));
+    const float est = (float)n * f * 65536.0f;
+    if (((n | d) >> 28) || est >= 2147483000.0f) return (unsigned)(((unsigned long long)n << 16) / d);
+    unsigned q = (unsigned)est;
+    int r = (int)((n << 16) - q * d);
+    const int q2 = __float2int_rn((float)r * f);
+    r = (int)((unsigned)r - (unsigned)q2 * d);
+    return q + (unsigned)q2 - (r < 0 ? 1u : 0u) + (r >= (int)d ? 1u : 0u);
+}
+__device__ __forceinline__ unsigned uabs(int v) { return v < 0 ? 0u - (unsigned)v : (unsigned)v; }
+// fxdiv for any operands (b != 0)
+__device__ __forceinline__ int fx_div(int a, int b) {
+    const unsigned q = fx_quot(uabs(a), uabs(b));
+    return (a ^ b) < 0 ? (int)(0u - q) : (int)q;
+}
+
+// Fixed::from(f32) (fixed.rs:88-93): the conversion instruction saturates and takes NaN to 0
+__device__ __forceinline__ int to_fx(float f) { return __float2int_rz(__fmul_rn(f, 65536.0f)); }
+
+// Depth at which every node of the curve's subdivision is flat (more than TILE_DEPTH: none
+// found), and the depth `safe` above which no node is.  At depth k a node centred at
+// t has its flatness vector 4^-k * p''(t) / 8 (quads: p'' constant; cubics: p'' linear, so the
+// two outermost nodes of a level have the longest).  `safe` and `sure` (every node at the depth
+// is flat) leave room for the rounding of the midpoints, 2^-16 of the largest coordinate (three
+// roundings a level of half an ulp in each of two coordinates and two points), so that the
+// nodes they speak for need no check; the depth itself is taken with 2^-19, and checked by
+// every leaf where it is not sure.
+__device__ __forceinline__ int curve_depth(P2 a, P2 b, P2 c, P2 d, bool cubic, float tol, int& safe, bool& sure) {
+    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
+                          fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
+    const float te = tol * 0.99998f - m * 1.9073486e-6f, th = tol * 1.00002f + m * 1.5258789e-5f;
+    const float ts = tol * 0.99998f - m * 1.5258789e-5f;
+    const float te2 = te * te, th2 = th * th, ts2 = ts > 0.0f ? ts * ts : -1.0f;
+    safe = 0;
+    sure = false;
+    if (!(te > 0.25f * tol)) return TILE_DEPTH + 1;
+    int k = 0;
+    if (!cubic) {
+        const float x = a.x - 2.0f * b.x + c.x, y = a.y - 2.0f * b.y + c.y;
+        float f = (x * x + y * y) * 0.0625f;
+        while (f > te2 && k <= TILE_DEPTH) {
+            if (f > th2) safe = k + 1;
+            f *= 0.0625f;
+            k++;
+        }
+        sure = f <= ts2;
+        return k;
+    }
+    const float x0 = 0.75f * (a.x - 2.0f * b.x + c.x), y0 = 0.75f * (a.y - 2.0f * b.y + c.y);
+    const float x1 = 0.75f * (b.x - 2.0f * c.x + d.x) - x0, y1 = 0.75f * (b.y - 2.0f * c.y + d.y) - y0;
+    // the shortest vector over the curve, for `safe`
+    const float n2 = x1 * x1 + y1 * y1, t = fminf(fmaxf(__fdividef(-(x0 * x1 + y0 * y1), n2), 0.0f), 1.0f);
+    const float wx = x0 + t * x1, wy = y0 + t * y1, w2 = n2 > 0.0f ? (wx * wx + wy * wy) * 0.999f : 0.0f;
+    float h = 0.5f, s = 1.0f;
+    for (; k <= TILE_DEPTH; k++) {
+        const float ux = x0 + h * x1, uy = y0 + h * y1, vx = x0 + (1.0f - h) * x1, vy = y0 + (1.0f - h) * y1;
+        const float f = fmaxf(ux * ux + uy * uy, vx * vx + vy * vy) * s;
+        sure = f <= ts2;
+        if (f <= te2) break;
+        if (w2 * s > th2) safe = k + 1;
+        h *= 0.5f;
+        s *= 0.0625f;
+    }
+    return k;
+}
+
+// The leaf at slot `idx` of a quad (plotter.rs:248-265) of depth D: its end points in a and
+// c.  False when the slot owns no leaf; `ok` is cleared when the node at depth D is not flat.
+__device__ __forceinline__ bool quad_slot(P2& a, P2 b, P2& c, int idx, int D, int safe, bool sure, float tol_sq,
+                                          bool& ok) {
+    for (int k = 0;; k++) {
+        if (sure && k >= D) return true;
+        const P2 ab = pmid(a, b), bc = pmid(b, c), m = pmid(ab, bc);
+        if (k >= safe) {
+            const bool within = pdist_sq(m, pmid(a, c)) <= tol_sq;
+            if (within || k >= D) {
+                if (!within) ok = false;
+                return (idx & ((1 << (D - k)) - 1)) == 0;
+            }
+        }
+        if ((idx >> (D - 1 - k)) & 1) {
+            a = m;
+            b = bc;
+        } else {
+            b = ab;
+            c = m;
+        }
+    }
+}
+// The same for a cubic (plotter.rs:311-332): end points in a and e.
+__device__ __forceinline__ bool cubic_slot(P2& a, P2 b, P2 c, P2& e, int idx, int D, int safe, bool sure, float tol_sq,
+                                           bool& ok) {
+    for (int k = 0;; k++) {
+        if (sure && k >= D) return true;
+        const P2 ab = pmid(a, b), bc = pmid(b, c), cd = pmid(c, e);
+        const P2 abbc = pmid(ab, bc), bccd = pmid(bc, cd);
+        const P2 m = pmid(abbc, bccd);
+        if (k >= safe) {
+            const bool within = pdist_sq(m, pmid(a, e)) <= tol_sq;
+            if (within || k >= D) {
+                if (!within) ok = false;
+                return (idx & ((1 << (D - k)) - 1)) == 0;
+            }
+        }
+        if ((idx >> (D - 1 - k)) & 1) {
+            a = m;
+            b = bccd;
+            c = cd;
+        } else {
+            b = ab;
+            c = abbc;
+            e = m;
+        }
+    }
+}
+
+static_assert(TILE_THREADS_FEW * ((1 << TILE_DEPTH) + 1) < (1 << 22) && TILE_THREADS_FEW <= 512,
+              "slots and listed ops of a chunk fit one word");
+
+// ------------------------------------------------------------------- state
+template <int NT>
+struct TileBuild {  // one chunk of NT ops; g0, g1, off and info of the ops that have slots
+    float4 g0[NT], g1[NT];  // transformed control points (a, b), (c, end)
+    float2 endp[NT];        // the pen after the op
+    int off[NT + 33];       // first slot; past the last op: INT_MAX
+    int info[NT];           // depth | safe << 4 | type << 8 | closing slot << 10 | starts a sub-figure << 11 | sure << 12
+    int kind[NT];
+};
+enum { TY_POINT = 0, TY_QUAD = 1, TY_CUBIC = 2 };
+constexpr int TILE_END = 16;  // kind of the virtual op after the last one
+
+struct TileWarp {  // one warp's segments while a band is accumulated
+    int4 q[64];    // segments that reach the band
+    int4 rec[64];  // two records per segment in work
+};
+
+template <int NT>
+struct TileState {
+    static constexpr int NW = NT / 32;
+    unsigned pcm[NW], vom[NW], rsm[NW];
+    unsigned wsum[NW];
+    // the walk, carried from chunk to chunk
+    int c_kind, c_vo, c_rs;  // kind of the last Move/Line/Quad/Cubic/Close op; last vertex op; last sub-figure start
+    float c_px, c_py;        // pen after the last Move/Line/Quad/Cubic/Close op
+    int flags, item, last_pw;
+    unsigned long long top;  // least (y, x) a non-zero segment starts from
+    int top_slot;            // the first slot of such a segment
+};
+
+template <int NW>
+__device__ __forceinline__ int prev_bit(const unsigned* m, int i) {  // last set bit at or below i, or -1
+    if (i < 0) return -1;
+    int w = i >> 5;
+    unsigned v = m[w] & (ALL >> (31 - (i & 31)));
+    while (!v) {
+        if (--w < 0) return -1;
+        v = m[w];
+    }
+    return (w << 5) + 31 - __clz(v);
+}
+
+__device__ __forceinline__ ft_op tile_op(const ft_op* ops, int i) {
+    const int4* src = reinterpret_cast<const int4*>(ops + i);
+    const int4 q0 = __ldg(src), q1 = __ldg(src + 1);
+    ft_op o;
+    o.kind = q0.x;
+    o.v[0] = __int_as_float(q0.y);
+    o.v[1] = __int_as_float(q0.z);
+    o.v[2] = __int_as_float(q0.w);
+    o.v[3] = __int_as_float(q1.x);
+    o.v[4] = __int_as_float(q1.y);
+    o.v[5] = __int_as_float(q1.z);
+    o.reserved = 0;
+    return o;
+}
+__device__ __forceinline__ P2 op_end(const ft_op& o) {
+    if (o.kind == FT_OP_QUAD) return p2(o.v[2], o.v[3]);
+    if (o.kind == FT_OP_CUBIC) return p2(o.v[4], o.v[5]);
+    return p2(o.v[0], o.v[1]);
+}
+// The first vertex of the sub-figure that op j starts: its point, or for a curve right
+// after a Close (or at the path's start), whose pen is the origin, its first leaf.
+__device__ P2 first_vertex(const TileParams& P, const ft_op* ops, int j) {
+    const ft_op o = tile_op(ops, j);
+    const P2 end = xform(P.xf, op_end(o));
+    if (o.kind != FT_OP_QUAD && o.kind != FT_OP_CUBIC) return end;
+    P2 a = xform(P.xf, p2(0.f, 0.f)), b = xform(P.xf, p2(o.v[0], o.v[1])), c = xform(P.xf, p2(o.v[2], o.v[3]));
+    if (!pfinite(a) || !pfinite(b) || !pfinite(c) || !pfinite(end)) return end;
+    bool ok = true;
+    if (o.kind == FT_OP_QUAD) {
+        quad_slot(a, b, c, 0, TILE_DEPTH, 0, false, P.tol_sq, ok);
+        return c;
+    }
+    P2 e = end;
+    cubic_slot(a, b, c, e, 0, TILE_DEPTH, 0, false, P.tol_sq, ok);
+    return e;
+}
+__device__ __forceinline__ unsigned long long top_key(int x, int y) {
+    return ((unsigned long long)((unsigned)y ^ 0x80000000u) << 32) | ((unsigned)x ^ 0x80000000u);
+}
+
+// -------------------------------------------------------------------- build
+// Segments of the path into E (slots in order, 32-slot groups; empty slots are zero-length)
+// and `ends` (per group the slots that close a sub-figure).  Returns the slots, a multiple of
+// 32, or -1: the path is not for this kernel.  S.top and S.top_slot are set.
+template <int NT>
+__device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& d, TileState<NT>& S, TileBuild<NT>& B, int4* E,
+                          unsigned* ends, float sw0) {
+    constexpr int NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const ft_op* ops = P.ops + d.op_begin;
+    const int n = (int)d.n_ops;
+    const float tol_sq = P.tol_sq;
+    if (tid == 0) {
+        S.c_kind = -1;
+        S.c_vo = S.c_rs = -1;
+        S.c_px = S.c_py = 0.f;
+        S.flags = 0;
+        S.top = ~0ull;
+        S.top_slot = INT_MAX;
+        S.last_pw = -1;
+    }
+    __syncthreads();
+    // the top vertex so far: least (y, x), then the first slot
+    int by = INT_MAX, bx = INT_MAX, best_slot = INT_MAX;
+    auto consider = [&](int4 e, int slot) {
+        if ((e.x != e.z || e.y != e.w) && top_less(e.y, e.x, slot, by, bx, best_slot)) {
+            by = e.y;
+            bx = e.x;
+            best_slot = slot;
+        }
+    };
+    int base = 0, bad = 0;
+    for (int c0 = 0; c0 <= n; c0 += NT) {
+        const int i = c0 + tid;
+        ft_op o;
+        o.kind = -1;
+        if (i < n) {
+            o = tile_op(ops, i);
+            if (o.kind < 0 || o.kind > FT_OP_PEN_WIDTH) {
+                atomicOr(&S.flags, 2);
+                o.kind = -1;
+            }
+        } else if (i == n) {
+            o.kind = TILE_END;
+        }
+        const int kind = o.kind;
+        const bool vo = kind >= FT_OP_MOVE && kind <= FT_OP_CUBIC;
+        const bool pc = vo || kind == FT_OP_CLOSE;
+        if (P.sw_out && kind == FT_OP_PEN_WIDTH) atomicMax(&S.last_pw, i);
+        const unsigned pcb = __ballot_sync(ALL, pc), vob = __ballot_sync(ALL, vo);
+        if (lane == 0) {
+            S.pcm[w] = pcb;
+            S.vom[w] = vob;
+        }
+        B.kind[tid] = kind;
+        const P2 end = vo ? op_end(o) : p2(0.f, 0.f);  // Close puts the pen at the origin (plotter.rs:200-203)
+        if (pc) B.endp[tid] = make_float2(end.x, end.y);
+        __syncthreads();
+        // the pen before this op
+        const int lpc = prev_bit<NW>(S.pcm, tid - 1);
+        const int pk = lpc >= 0 ? B.kind[lpc] : S.c_kind;
+        const P2 pen = lpc >= 0 ? p2(B.endp[lpc].x, B.endp[lpc].y) : p2(S.c_px, S.c_py);
+        const bool rs = vo && (kind == FT_OP_MOVE || pk == FT_OP_CLOSE || pk == -1);
+        const unsigned rsb = __ballot_sync(ALL, rs);
+        if (lane == 0) S.rsm[w] = rsb;
+        const int lvo = prev_bit<NW>(S.vom, tid - 1);
+        const int lvo_op = lvo >= 0 ? c0 + lvo : S.c_vo;
+        const bool closes = (rs || kind == TILE_END) && lvo_op >= 0;  // closes the sub-figure before
+        __syncthreads();
+        const int lrs = prev_bit<NW>(S.rsm, tid - 1);
+        const int lrs_op = lrs >= 0 ? c0 + lrs : S.c_rs;
+        // slots of this op
+        int slots = closes ? 1 : 0, D = 0, safe = 0, type = TY_POINT;
+        bool sure = false;
+        float4 ga = make_float4(0.f, 0.f, 0.f, 0.f), gb = ga;
+        if (vo) {
+            const P2 a = xform(P.xf, pen), e = xform(P.xf, end);
+            P2 b = a, c = e;
+            if (kind == FT_OP_QUAD || kind == FT_OP_CUBIC) {
+                b = xform(P.xf, p2(o.v[0], o.v[1]));
+                c = xform(P.xf, p2(o.v[2], o.v[3]));
+                if (!pfinite(a) || !pfinite(b) || !pfinite(c) || !pfinite(e)) {
+                    atomicOr(&S.flags, 2);
+                } else {
+                    type = kind == FT_OP_QUAD ? TY_QUAD : TY_CUBIC;
+                    D = curve_depth(a, b, c, e, type == TY_CUBIC, P.tol, safe, sure);
+                    if (D > TILE_DEPTH) {
+                        bad = 1;
+                        D = safe = 0;
+                    }
+                }
+            }
+            ga = make_float4(a.x, a.y, b.x, b.y);
+            gb = make_float4(c.x, c.y, e.x, e.y);
+            slots += 1 << D;
+        }
+        // slot offsets and places in the list of ops with slots, in one scan
+        const unsigned mine = (unsigned)slots | ((slots ? 1u : 0u) << 22);
+        unsigned inc = mine;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            const unsigned t = __shfl_up_sync(ALL, inc, s);
+            if (lane >= s) inc += t;
+        }
+        if (lane == 31) S.wsum[w] = inc;
+        __syncthreads();
+        unsigned pre = 0, sum = 0;
+#pragma unroll
+        for (int k = 0; k < NW; k++) {
+            const unsigned v = S.wsum[k];
+            if (k < w) pre += v;
+            sum += v;
+        }
+        const int listed = (int)(sum >> 22), total = (int)(sum & ((1u << 22) - 1));
+        const unsigned excl = pre + inc - mine;
+        const int off = (int)(excl & ((1u << 22) - 1));
+        if (slots) {
+            const int at = (int)(excl >> 22);
+            B.g0[at] = ga;
+            B.g1[at] = gb;
+            B.off[at] = off;
+            B.info[at] = D | (safe << 4) | (type << 8) | ((closes ? 1 : 0) << 10) | ((rs ? 1 : 0) << 11) |
+                        ((sure ? 1 : 0) << 12);
+        }
+        if (tid < 32) B.off[listed + tid] = INT_MAX;
+        const int padded = (total + 31) & ~31;
+        if (base + padded > P.cap) bad = 1;
+        if (__syncthreads_or(bad)) break;
+        if (closes) {  // last vertex -> first vertex of the sub-figure that ends here
+            const P2 l = xform(P.xf, lvo >= 0 ? p2(B.endp[lvo].x, B.endp[lvo].y) : op_end(tile_op(ops, S.c_vo)));
+            const P2 f = first_vertex(P, ops, lrs_op);
+            const int4 e = make_int4(to_fx(l.x), to_fx(l.y), to_fx(f.x), to_fx(f.y));
+            E[base + off] = e;
+            consider(e, base + off);
+        }
+        __syncthreads();
+        if (tid == NT - 1) {  // carry (the arrays below are read-only until the next chunk)
+            const int p = prev_bit<NW>(S.pcm, NT - 1);
+            if (p >= 0) {
+                S.c_kind = B.kind[p];
+                S.c_px = B.endp[p].x;
+                S.c_py = B.endp[p].y;
+            }
+            const int v = prev_bit<NW>(S.vom, NT - 1);
+            if (v >= 0) S.c_vo = c0 + v;
+            const int r = prev_bit<NW>(S.rsm, NT - 1);
+            if (r >= 0) S.c_rs = c0 + r;
+        }
+        // one slot per thread, 32 slots per warp at a time
+        int j0 = 0;
+        for (int s0 = w * 32; s0 < padded; s0 += NT) {
+            const int s = s0 + lane;
+            // the op of the first slot, then the ops that start in the window
+            for (;;) {
+                const unsigned m = __ballot_sync(ALL, B.off[j0 + 1 + lane] <= s0);
+                j0 += __popc(m);
+                if (m != ALL) break;
+            }
+            const int rel = B.off[j0 + 1 + lane] - s0;
+            const unsigned starts = __reduce_or_sync(ALL, rel < 32 ? 1u << rel : 0u);
+            int4 e = make_int4(0, 0, 0, 0);
+            bool close_slot = false;
+            if (s < total) {
+                const int lo = j0 + __popc(starts & (ALL >> (31 - lane)));
+                const int info = B.info[lo];
+                const int idx = s - B.off[lo] - ((info >> 10) & 1);
+                close_slot = idx < 0;
+                if (!close_slot && !(((info >> 11) & 1) && idx == 0 && ((info >> 8) & 3) == TY_POINT)) {
+                    const float4 g0 = B.g0[lo], g1 = B.g1[lo];
+                    P2 a = p2(g0.x, g0.y), z = p2(g1.z, g1.w);
+                    bool own = true, ok = true;
+                    const int type = (info >> 8) & 3, D = info & 15, safe = (info >> 4) & 15;
+                    if (type == TY_QUAD)
+                        own = quad_slot(a, p2(g0.z, g0.w), z, idx, D, safe, (info >> 12) & 1, tol_sq, ok);
+                    else if (type == TY_CUBIC)
+                        own = cubic_slot(a, p2(g0.z, g0.w), p2(g1.x, g1.y), z, idx, D, safe, (info >> 12) & 1, tol_sq, ok);
+                    if (!ok) bad = 1;
+                    // the first vertex of a sub-figure ends no segment
+                    if (own && !(((info >> 11) & 1) && idx == 0))
+                        e = make_int4(to_fx(a.x), to_fx(a.y), to_fx(z.x), to_fx(z.y));
+                }
+            }
+            const unsigned cm = __ballot_sync(ALL, close_slot);
+            if (lane == 0) ends[(base + s) >> 5] = cm;
+            if (!close_slot) E[base + s] = e;
+            consider(e, base + s);
+        }
+        base += padded;
+        __syncthreads();
+    }
+    if (__syncthreads_or(bad)) return -1;
+    const unsigned long long best = best_slot != INT_MAX ? top_key(bx, by) : ~0ull;
+    unsigned long long k = best;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(ALL, k, s);
+        k = t < k ? t : k;
+    }
+    if (lane == 0 && k != ~0ull) atomicMin(&S.top, k);
+    __syncthreads();
+    if (best != ~0ull && best == S.top) atomicMin(&S.top_slot, best_slot);
+    __syncthreads();
+    return base;
+}
+
+// Direction of the figure (fig.rs:402-411, 116-119), by one warp: the non-zero segment out
+// of the top vertex and the one into it.
+__device__ __noinline__ int tile_dir(const int4* E, const unsigned* ends, int n_slots, int top) {
+    const int lane = threadIdx.x & 31;
+    const int4 out = E[top];
+    int4 in = out;
+    bool found = false, edge = false;  // edge: the sub-figure's first slot was passed
+    auto back = [&](int hi, int lo) {  // the last non-zero segment of slots hi, hi - 1, ... lo
+        for (int e = hi; e >= lo && !found && !edge; e -= 32) {
+            const int k = e - lane;
+            int4 v = make_int4(0, 0, 0, 0);
+            bool closing = false;
+            if (k >= lo) {
+                v = E[k];
+                closing = k < top && ((ends[k >> 5] >> (k & 31)) & 1);
+            }
+            const unsigned nz = __ballot_sync(ALL, v.x != v.z || v.y != v.w), cl = __ballot_sync(ALL, closing);
+            const int f = nz ? __ffs(nz) - 1 : 32, c = cl ? __ffs(cl) - 1 : 32;
+            if (f < c) {
+                in.x = __shfl_sync(ALL, v.x, f);
+                in.y = __shfl_sync(ALL, v.y, f);
+                found = true;
+            }
+            edge = c < 32 && !found;
+        }
+    };
+    back(top - 1, 0);
+    if (!found) {
+        // the top is its sub-figure's first vertex: backwards from the sub-figure's closing slot
+        int last = n_slots - 1;
+        for (int g = top >> 5; g < n_slots >> 5; g += 32) {
+            unsigned m = g + lane < n_slots >> 5 ? ends[g + lane] : 0u;
+            if (g + lane == top >> 5) m &= ALL << (top & 31);
+            const unsigned any = __ballot_sync(ALL, m != 0);
+            if (any) {
+                const int f = __ffs(any) - 1;
+                last = ((g + f) << 5) + __ffs(__shfl_sync(ALL, m, f)) - 1;
+                break;
+            }
+        }
+        edge = false;
+        back(last, top);
+    }
+    const int ax = wsub(in.x, out.x), ay = wsub(in.y, out.y), cx = wsub(out.z, out.x), cy = wsub(out.w, out.y);
+    return fxmul(ax, cy) > fxmul(cx, ay) ? 0 : 1;
+}
+
+// ------------------------------------------------------------------- raster
+// Cell areas of the first m segments in Q.q (all reach rows [yb0, yb1)) into `area` (rows of
+// `pitch` cells, the raster W pixels wide), scaled by 2^16: the i16 sums of footile wrap in
+// the upper halves.
+//
+// One lane works out a segment; the (segment, row) items are then spread over the lanes, an
+// item that walks many cells as several lanes of CELLS cells each, so that a window of 32
+// costs the same whatever the slopes in it: the walk is closed (x_cov after j cells is
+// first + j * step), so any lane can start in the middle of it.
+constexpr int CELLS = 4;
+__device__ __forceinline__ void tile_items(TileWarp& Q, int m, int yb0, int yb1, int* area, int pitch, int W) {
+    const int lane = threadIdx.x & 31;
+    int n_items = 0;
+    int4 ra = make_int4(0, 0, 0, 0), rb = ra;
+    if (lane < m) {
+        const int4 e = Q.q[lane];
+        const bool down = e.w > e.y;
+        const int ux = down ? e.x : e.z, uy = down ? e.y : e.w, lx = down ? e.z : e.x, ly = down ? e.w : e.y;
+        const int dx = wsub(lx, ux), dy = wsub(ly, uy);
+        const unsigned ady = uabs(dy), adx = uabs(dx);
+        // fig.rs:187-199; a slope of ONE and above is ONE
+        int step = FX_ONE;
+        if (ady < adx) {
+            step = (int)fx_quot(ady, adx);
+        } else if (adx != 0 && (ady >> 15) >= adx) {  // 32,768 and more: the wrapped low half decides
+            step = min(fxabs(fx_div(dy, dx)), FX_ONE);
+        }
+        if (step <= 0) step = FX_ONE;  // step_cov(ONE) (fig.rs:315-321)
+        const int inv = fx_div(dx, dy);
+        const int fu = fxfract(uy), fl = fxfract(ly);
+        const int start = uy >> 16, end = ly >> 16;
+        const int pu = (fu + 128) >> 8, pl = (fl + 128) >> 8;  // pixel_cov of the fractions
+        const int ya = max(start, yb0), yl = min(fl ? end : end - 1, yb1 - 1);
+        const int nrow = yl - ya + 1;
+        // the longest walk of its rows: cov * 256 / step cells and one, rounded up
+        const int most = start == end ? pl - pu : (end - start > 1 ? 256 : max(256 - pu, pl));
+        const int cells = (int)__fdividef((float)max(most, 0) * 256.0256f, (float)step) + 2;
+        const int ls = cells <= CELLS ? 0 : 32 - __clz((cells - 1) / CELLS);
+        n_items = nrow << ls;
+        ra.x = wadd(wadd(ux, fxmul(inv, FX_ONE - fu)), wmul(ya - start, inv));  // x leaving row ya
+        ra.y = inv;
+        ra.z = ux;                                // x entering the first row
+        ra.w = fl ? fxmul(inv, FX_ONE - fl) : 0;  // from the bottom of the last row back to its end
+        rb.y = step | (ls << 20);
+        rb.z = (ya - yb0) * pitch;
+        rb.w = pl | (pu << 9) | ((ya == start ? 1 : 0) << 18) | ((fl && yl == end ? 1 : 0) << 19) |
+               ((down ? 0 : 1) << 20) | (int)((unsigned)nrow << 21);
+    }
+    int inc = n_items;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const int t = __shfl_up_sync(ALL, inc, s);
+        if (lane >= s) inc += t;
+    }
+    const int off = inc - n_items, tot = __shfl_sync(ALL, inc, 31);
+    rb.x = off;
+    if (lane < m) {
+        Q.rec[2 * lane] = ra;
+        Q.rec[2 * lane + 1] = rb;
+    }
+    __syncwarp();
+    for (int w0 = 0; w0 < tot; w0 += 32) {
+        // the segment of item w0 + lane: segments that start at or before it (each has an item)
+        const int rel = off - w0;
+        const unsigned at = __reduce_or_sync(ALL, (lane < m && rel >= 0 && rel < 32) ? 1u << rel : 0u);
+        const int before = __popc(__ballot_sync(ALL, lane < m && rel < 0));
+        const int item = w0 + lane;
+        if (item >= tot) continue;
+        const int j = before + __popc(at & (ALL >> (31 - lane))) - 1;
+        const int4 A = Q.rec[2 * j], C = Q.rec[2 * j + 1];
+        const int ls = C.y >> 20, step = C.y & 0xFFFFF;
+        const int k = (item - C.x) >> ls, c0 = ((item - C.x) & ((1 << ls) - 1)) * CELLS;
+        const bool st = ((C.w >> 18) & 1) && k == 0, en = ((C.w >> 19) & 1) && k == (int)((unsigned)C.w >> 21) - 1;
+        const int cov = (en ? C.w & 511 : 256) - (st ? (C.w >> 9) & 511 : 0);
+        const int xb = wadd(A.x, wmul(k, A.y));
+        const int x0 = st ? A.z : wsub(xb, A.y), x1 = en ? wsub(xb, A.w) : xb;
+        const int mnx = min(x0, x1), mxx = max(x0, x1);
+        const int minp = mnx >> 16, maxp = mxx >> 16;
+        if (cov <= 0 || minp >= W) continue;
+        // fig.rs:285-321: x_cov runs first, first + step, ...; each cell gets the growth of
+        // min(pixel_cov(x_cov), cov).  pixel_cov(x) is (x + 128) >> 8 for x in [0, ONE], and
+        // cov <= 256 stands in for the cap at ONE.
+        const unsigned r = minp == maxp ? ((unsigned)(FX_ONE - fxfract(fxavg(mxx, mnx))) * (unsigned)cov) >> 8
+                                        : (unsigned)(FX_ONE - fxfract(mnx)) >> 1;
+        unsigned xc = (unsigned)(((unsigned long long)r * (unsigned)step) >> 16) + 128u;
+        int* cell = area + C.z + k * pitch + c0;
+        int left = W - c0;  // cells to the raster's end; the row has CELLS - 1 spare ones after it
+        if (minp < 0) {
+            // cells left of the raster all land in cell 0 (fig.rs:295): their sum telescopes
+            const unsigned long long v = (unsigned long long)xc + (unsigned long long)(unsigned)-minp * (unsigned)step;
+            xc = v > FX_ONE + 128 ? FX_ONE + 128 : (unsigned)v;
+        } else {
+            cell += minp;
+            left -= minp;
+        }
+        if (left <= 0) continue;
+        xc += (unsigned)c0 * (unsigned)step;
+        int prev = c0 ? min((int)((xc - (unsigned)step) >> 8), cov) : 0;
+        const int sgn = (C.w >> 20) & 1 ? -FX_ONE : FX_ONE;
+#pragma unroll
+        for (int u = 0; u < CELLS; u++) {
+            const int v = min((int)(xc >> 8), cov);
+            if (v != prev) atomicAdd(cell + u, (v - prev) * sgn);
+            prev = v;
+            xc += (unsigned)step;
+        }
+    }
+    __syncwarp();
+}
+
+struct TileOut {  // where a band's rows go (in shared memory: it would only hold registers)
+    uint8_t* base;   // the raster
+    unsigned stride, clr;
+    int W, pitch, rule, fmt;
+    int neg;         // the figure runs in reverse: cell sums change sign
+    int lprl;        // log2 of the lanes per row, eight pixels each
+    bool host;       // mapped host memory: Matte8 rows leave as aligned words
+    unsigned char* stg;
+};
+
+// Fill rule on four running sums (i16, in the upper halves; imgbuf.rs:54-61, 157-167),
+// packed into bytes
+template <int RULE>
+__device__ __forceinline__ unsigned resolve4(int a, int b, int c, int d) {
+    if (RULE == FT_NONZERO) {  // clamp to 0 .. 255
+        a = __vimin_s32_relu(a, 0x00FFFFFF);
+        b = __vimin_s32_relu(b, 0x00FFFFFF);
+        c = __vimin_s32_relu(c, 0x00FFFFFF);
+        d = __vimin_s32_relu(d, 0x00FFFFFF);
+    } else {  // |v - odd|: t or 512 - t of the low nine bits t, at most 255
+        a &= 0x01FF0000;
+        b &= 0x01FF0000;
+        c &= 0x01FF0000;
+        d &= 0x01FF0000;
+        a = __vimin3_s32(a, 0x02000000 - a, 0x00FF0000);
+        b = __vimin3_s32(b, 0x02000000 - b, 0x00FF0000);
+        c = __vimin3_s32(c, 0x02000000 - c, 0x00FF0000);
+        d = __vimin3_s32(d, 0x02000000 - d, 0x00FF0000);
+    }
+    return __byte_perm(__byte_perm(a, b, 0x0062), __byte_perm(c, d, 0x0062), 0x5410);
+}
+// The last n (one to three) bytes of a row, from w, to a 4-byte aligned address
+__device__ __forceinline__ void store_tail(uint8_t* dp, unsigned w, int n) {
+    if (n & 2) *reinterpret_cast<unsigned short*>(dp) = (unsigned short)w;
+    if (n & 1) dp[n & 2] = (uint8_t)(w >> (8 * (n & 2)));
+}
+
+// SrcOver of one pixel, skipped when it changes nothing (coverage 0 changes channel values
+// 1..15 only)
+__device__ __forceinline__ void tile_px(unsigned* p, unsigned clr, unsigned av) {
+    const unsigned v = *p;
+    if (!av) {
+        const unsigned nz = (((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) & 0x80808080u;
+        const unsigned hi = (((v & 0x70707070u) + 0x70707070u) | v) & 0x80808080u;
+        if (!(nz & ~hi)) return;
+    }
+    *p = srcover_rgba(v, clr, av);
+}
+
+// A row's eight cells of one lane, cleared, and their running sum in s[0 .. 7]; `inc` gets the
+// inclusive sum over the row's lanes (l: the lane in its row).
+__device__ __forceinline__ void take8(int* ap, bool in, int l, unsigned* s, unsigned& inc) {
+    int4 a = make_int4(0, 0, 0, 0), b = a;
+    if (in) {
+        a = reinterpret_cast<const int4*>(ap)[0];
+        b = reinterpret_cast<const int4*>(ap)[1];
+        reinterpret_cast<int4*>(ap)[0] = make_int4(0, 0, 0, 0);
+        reinterpret_cast<int4*>(ap)[1] = make_int4(0, 0, 0, 0);
+    }
+    s[0] = a.x;
+    s[1] = s[0] + a.y;
+    s[2] = s[1] + a.z;
+    s[3] = s[2] + a.w;
+    s[4] = s[3] + b.x;
+    s[5] = s[4] + b.y;
+    s[6] = s[5] + b.z;
+    s[7] = s[6] + b.w;
+    inc = s[7];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {  // lane l of a row takes from lane l - o of the same row
+        const unsigned t = __shfl_up_sync(ALL, inc, o);
+        if (l >= o) inc += t;
+    }
+}
+// The eight pixels of sums s + ex, the figure's direction (sg: 1 or -1) flipping every sum
+template <int RULE>
+__device__ __forceinline__ uint2 pixels8(const unsigned* s, unsigned ex, int sg) {
+    int u[8];
+    const unsigned exs = ex * (unsigned)sg;
+#pragma unroll
+    for (int k = 0; k < 8; k++) u[k] = (int)(s[k] * (unsigned)sg + exs);
+    return make_uint2(resolve4<RULE>(u[0], u[1], u[2], u[3]), resolve4<RULE>(u[4], u[5], u[6], u[7]));
+}
+
+// Resolve rows r0 .. r0 + nr - 1 (imgbuf.rs:38-199) from `area`, clearing it, and write them
+// (fig.rs:621-665).  Matte8 in device memory, rows of at most 256 pixels on 4-byte
+// boundaries: each lane eight pixels, as many rows a warp as fit, straight-line.
+template <int NT, int RULE>
+__device__ __noinline__ void tile_rows_matte(const TileOut& T, int* area, int r0, int nr) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = lane & ((1 << T.lprl) - 1), rpw = 32 >> T.lprl, first = warp * rpw + (lane >> T.lprl);
+    const int nb = T.W - 8 * l, sg = T.neg ? -1 : 1;
+    int* ap = area + first * T.pitch + 8 * l;
+    uint8_t* dp = T.base + (size_t)(r0 + first) * T.stride + 8 * l;
+    for (int q = warp * rpw; q < nr; q += NW * rpw) {
+        const bool in = nb > 0 && q + (lane >> T.lprl) < nr;
+        unsigned s[8], inc;
+        take8(ap, in, l, s, inc);
+        const uint2 px = pixels8<RULE>(s, inc - s[7], sg);
+        if (in) {  // written once and not read back
+            if (nb >= 4) __stcs(reinterpret_cast<unsigned*>(dp), px.x);
+            if (nb >= 8)
+                __stcs(reinterpret_cast<unsigned*>(dp + 4), px.y);
+            else if (nb & 3)
+                store_tail(dp + (nb & 4), nb < 4 ? px.x : px.y, nb & 3);
+        }
+        ap += NW * rpw * T.pitch;
+        dp += (size_t)(NW * rpw) * T.stride;
+    }
+}
+
+// Every other row: Rgba8p, host rasters, unaligned or wide Matte8; `o0`: with contiguous host
+// rows, the staged byte of row r0's first pixel.
+template <int NT, int RULE>
+__device__ __noinline__ void tile_rows(const TileOut& T, int* area, int r0, int nr, bool contig, int o0) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int W = T.W, lpr = 1 << T.lprl, rpw = 32 >> T.lprl, l = lane & (lpr - 1), sub = lane >> T.lprl;
+    for (int q = warp * rpw; q < nr; q += NW * rpw) {
+        const int rr = q + sub;
+        const bool valid = rr < nr;
+        int* arow = area + rr * T.pitch;
+        uint8_t* drow = T.base + (size_t)(r0 + rr) * T.stride;
+        unsigned carry = 0;
+        for (int x0 = 0; x0 < W; x0 += lpr * 8) {
+            const int x = x0 + l * 8, nb = min(W - x, 8);
+            const bool in = valid && nb > 0;
+            unsigned s[8], inc;
+            take8(arow + x, in, l, s, inc);
+            const uint2 px = pixels8<RULE>(s, inc - s[7] + carry, T.neg ? -1 : 1);
+            carry += __shfl_sync(ALL, inc, lpr - 1, lpr);
+            if (!in) continue;
+            if (contig) {
+                unsigned char* sp = T.stg + o0 + rr * W + x;
+                for (int k = 0; k < nb; k++) sp[k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
+            } else if (T.fmt == FT_MATTE8 && !T.host) {
+                for (int k = 0; k < nb; k++) drow[x + k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
+            } else {
+                *reinterpret_cast<uint2*>(T.stg + rr * T.pitch + x) = px;
+            }
+        }
+        if (contig || (T.fmt == FT_MATTE8 && !T.host)) continue;
+        __syncwarp();
+        if (valid) {
+            const unsigned char* sp = T.stg + rr * T.pitch;
+            if (T.fmt == FT_RGBA8P) {
+                unsigned* dp = reinterpret_cast<unsigned*>(drow);
+                for (int x = l; x < W; x += lpr) tile_px(dp + x, T.clr, sp[x]);
+            } else {  // aligned words of a host row, its ends byte by byte
+                const int mis = (int)(reinterpret_cast<uintptr_t>(drow) & 3);
+                for (int x = 4 * l - mis; x < W; x += 4 * lpr) {
+                    if (x >= 0 && x + 4 <= W) {
+                        *reinterpret_cast<unsigned*>(drow + x) = (unsigned)sp[x] | ((unsigned)sp[x + 1] << 8) |
+                                                                 ((unsigned)sp[x + 2] << 16) | ((unsigned)sp[x + 3] << 24);
+                    } else {
+                        for (int k = max(x, 0); k < min(x + 4, W); k++) drow[k] = sp[k];
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+template <int NT>
+struct TileLayout {
+    static constexpr int build = (int)((sizeof(TileBuild<NT>) + 15) & ~(size_t)15);
+    static constexpr int warps = (int)sizeof(TileWarp) * (NT / 32);
+    // the build's arrays and the raster's queues, cells and staged bytes share the space
+    static int bytes(int area_ints, bool staged) {
+        const int raster = warps + area_ints * 4 + (staged ? area_ints + 256 : 0);
+        return raster > build ? raster : build;
+    }
+};
+
+template <int NT>
+__global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ TileState<NT> S;
+    __shared__ TileOut T;
+    constexpr int NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned char* scr = P.scratch + (size_t)blockIdx.x * tile_scratch(P.cap);
+    int4* E = reinterpret_cast<int4*>(scr);
+    unsigned* ends = reinterpret_cast<unsigned*>(scr + (size_t)P.cap * sizeof(int4));
+    TileBuild<NT>& B = *reinterpret_cast<TileBuild<NT>*>(smem);
+    TileWarp& Q = reinterpret_cast<TileWarp*>(smem)[warp];
+    int* area = reinterpret_cast<int*>(smem + TileLayout<NT>::warps);
+    for (;;) {
+        if (tid == 0) S.item = (int)atomicAdd(&P.queue[1], 1u);
+        __syncthreads();
+        const int it = S.item;
+        if (it >= (int)P.n_items) break;
+        const WorkItem wi = P.items[it];
+        const ft_path_desc d = P.paths[wi.path];
+        const float sw0 = P.sw_chain ? *P.sw_chain : d.s_width;
+        const int n_slots = tile_build<NT>(P, d, S, B, E, ends, sw0);
+        if (n_slots < 0) {  // the path goes to k_raster, once
+            if (tid == 0 && wi.row_begin == 0) P.overflow[atomicAdd(&P.queue[2], 1u)] = wi.path;
+            __syncthreads();
+            continue;
+        }
+        if (tid == 0 && wi.row_begin == 0) {
+            if (S.flags) atomicMax(&P.status[wi.path], FT_ERR_ARG);
+            if (P.sw_out) P.sw_out[wi.path] = S.last_pw >= 0 ? P.ops[d.op_begin + S.last_pw].v[0] : sw0;
+        }
+        const int W = (int)d.width, H = (int)d.height;
+        if (S.top != ~0ull && W > 0) {
+            const int top_row = (int)((unsigned)(S.top >> 32) ^ 0x80000000u) >> 16;
+            const int tmin = min(top_row, 0);
+            const int lo = max((int)wi.row_begin, max(top_row, 0)), hi = min((int)wi.row_end, H);
+            const int pitch = tile_pitch(W);
+            const int R = max(1, min(P.area_ints / pitch, 1024));
+            uint8_t* const base = P.rasters + d.raster_offset;
+            const bool host = P.host_rasters != 0;
+            if (tid == 0) {
+                T.base = base;
+                T.stride = d.stride;
+                T.clr = (unsigned)d.clr[0] | ((unsigned)d.clr[1] << 8) | ((unsigned)d.clr[2] << 16) |
+                        ((unsigned)d.clr[3] << 24);
+                T.W = W;
+                T.pitch = pitch;
+                T.rule = P.rule;
+                T.fmt = P.fmt;
+                T.host = host;
+                T.stg = smem + TileLayout<NT>::warps + P.area_ints * 4;
+                T.lprl = W <= 8 ? 0 : min(32 - __clz((W - 1) >> 3), 5);
+            }
+            const bool quick = P.fmt == FT_MATTE8 && !host && W <= 256 &&
+                               (((unsigned)reinterpret_cast<uintptr_t>(base) | d.stride) & 3) == 0;
+            // contiguous host rows: whole 128-byte lines leave from the staging bytes
+            const bool contig = host && P.fmt == FT_MATTE8 && d.stride == d.width;
+            uint8_t* const g0 = base + (size_t)lo * d.stride;
+            uint8_t* const g1 = base + (size_t)hi * d.stride;
+            uint8_t* L0 = reinterpret_cast<uint8_t*>(reinterpret_cast<uintptr_t>(g0) & ~(uintptr_t)127);
+            if (lo < hi) {
+                const int cells = min(R, hi - lo) * pitch;
+                for (int x = tid * 4; x < cells; x += NT * 4) *reinterpret_cast<int4*>(area + x) = make_int4(0, 0, 0, 0);
+                __syncthreads();
+                if (warp == 0) {
+                    const int dir = tile_dir(E, ends, n_slots, S.top_slot);
+                    if (lane == 0) T.neg = dir;
+                }
+                for (int r0 = lo; r0 < hi; r0 += R) {
+                    const int nr = min(R, hi - r0), yb0 = r0 + tmin, yb1 = yb0 + nr;
+                    int cnt = 0;
+                    for (int g = warp;; g += NW) {
+                        const bool more = g < n_slots >> 5;
+                        if (more) {
+                            const int4 e = E[g * 32 + lane];
+                            const int y0 = min(e.y, e.w), y1 = max(e.y, e.w);
+                            const bool on = y0 != y1 && (y0 >> 16) < yb1 && ((y1 - 1) >> 16) >= yb0;
+                            const unsigned m = __ballot_sync(ALL, on);
+                            if (on) Q.q[cnt + __popc(m & ((1u << lane) - 1u))] = e;
+                            cnt += __popc(m);
+                            __syncwarp();
+                        }
+                        if (cnt >= 32 || (!more && cnt > 0)) {
+                            tile_items(Q, min(cnt, 32), yb0, yb1, area, pitch, W);
+                            cnt -= 32;
+                            if (lane < cnt) Q.q[lane] = Q.q[32 + lane];
+                            __syncwarp();
+                        }
+                        if (!more) break;
+                    }
+                    __syncthreads();
+                    const int o0 = contig ? (int)(base + (size_t)r0 * d.stride - L0) : 0;
+                    if (quick && P.rule == FT_NONZERO)
+                        tile_rows_matte<NT, FT_NONZERO>(T, area, r0, nr);
+                    else if (quick)
+                        tile_rows_matte<NT, FT_EVENODD>(T, area, r0, nr);
+                    else if (P.rule == FT_NONZERO)
+                        tile_rows<NT, FT_NONZERO>(T, area, r0, nr, contig, o0);
+                    else
+                        tile_rows<NT, FT_EVENODD>(T, area, r0, nr, contig, o0);
+                    __syncthreads();
+                    if (contig) {
+                        const bool last = r0 + nr >= hi;
+                        const int fill = o0 + nr * W, lines = last ? (fill + 127) >> 7 : fill >> 7;
+                        for (int x = tid * 16; x < lines * 128; x += NT * 16) {
+                            uint8_t* a = L0 + x;
+                            const uint4 v = *reinterpret_cast<const uint4*>(T.stg + x);
+                            if (a >= g0 && a + 16 <= g1) {
+                                *reinterpret_cast<uint4*>(a) = v;
+                            } else {
+                                for (int k = 0; k < 16; k++)
+                                    if (a + k >= g0 && a + k < g1) a[k] = T.stg[x + k];
+                            }
+                        }
+                        if (!last && lines > 0) {  // the partial line moves to the front
+                            const int rest = fill - lines * 128;
+                            __syncthreads();
+                            if (tid * 16 < rest)
+                                *reinterpret_cast<uint4*>(T.stg + tid * 16) =
+                                    *reinterpret_cast<const uint4*>(T.stg + lines * 128 + tid * 16);
+                            L0 += lines * 128;
+                        }
+                        __syncthreads();
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+}  // namespace
+
+int tile_smem(int threads, int area_ints, bool staged) {
+    return threads == 128 ? TileLayout<128>::bytes(area_ints, staged) : TileLayout<512>::bytes(area_ints, staged);
+}
+
+int tile_blocks_per_sm(int threads, int smem) {
+    int n = 0;
+    cudaError_t e;
+    if (threads == 128) {
+        cudaFuncSetAttribute(k_tile<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<128>, 128, smem);
+    } else {
+        cudaFuncSetAttribute(k_tile<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<512>, 512, smem);
+    }
+    return e == cudaSuccess && n > 0 ? n : 1;
+}
+
+cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cudaStream_t s) {
+    auto kern = threads == 128 ? k_tile<128> : k_tile<512>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, threads, smem, s>>>(p);
+    return cudaGetLastError();
+}
+
+}  // namespace ftk

@@ -195,8 +195,9 @@ FT_API int ft_batch_launch_status(ft_ctx* ctx, ft_batch* batch, int32_t* status,
 FT_API void ft_batch_destroy(ft_batch* batch);
 
 /* Plan tuning — no counterpart in footile (its CPU plotter has nothing to tune).
- * The knobs of a batch plan: `warp_max_side`, the largest canvas side given whole to
- * one warp (0..512, 0 sends every path to the CTA rasteriser); `cta_smem_bytes`, the
+ * The knobs of a batch plan: `warp_max_side`, the largest canvas side of a fill given whole
+ * to one CTA of the tile rasteriser (0..512, 0 sends every path to the CTA rasteriser, few
+ * paths included); `cta_smem_bytes`, the
  * CTA rasteriser's shared memory, which sets its tile: bands of as many full-width rows
  * as fit (0 = built-in choice; the ordered composite's figure builds keep their own
  * 48 KB); `split_px`, paths of at least this many pixels are
@@ -404,7 +405,7 @@ FT_API int ft_last_composite_ms(ft_ctx* ctx, float* ms);
 
 /* Bounds-check build (the library compiled with -DFT_CHECK=1) — no counterpart in
  * footile; it stands in for a memory checker.  Device code checks the indices of its
- * shared-memory cell buffers, warp scratch, edge pool, compositor queues and the grid-wide
+ * shared-memory cell buffers, edge pool, compositor queues and the grid-wide
  * figure build's raw vertices and figure writes; a failed check
  * skips the access and keeps the first failing site's number.  `site` (may be NULL)
  * receives that number since the last call (0: none) and is reset; `compiled_in` (may be
