@@ -258,6 +258,7 @@ void fill_params(ft_ctx* c, ftk::KParams& p, int stroke, int rule, int fmt, int 
     memset(&p, 0, sizeof(p));
     for (int i = 0; i < 6; i++) p.xf[i] = c->xf[i];
     const float t = std::max(c->tolerance, 0.01f);
+    p.tol = t;
     p.tol_sq = t * t;
     p.join = c->join;
     p.miter_limit = c->miter_limit;
@@ -311,8 +312,8 @@ cudaError_t enqueue(const ftk::KParams& p, const ftk::TilePlan& t, int grid_b, i
         q.rule = p.rule;
         q.fmt = p.fmt;
         for (int i = 0; i < 6; i++) q.xf[i] = p.xf[i];
+        q.tol = p.tol;
         q.tol_sq = p.tol_sq;
-        q.tol = std::sqrt(p.tol_sq);
         e = ftk::launch_tile(q, t.threads, grid_w, t.smem(p.fmt, p.host_rasters != 0), st);
         if (e != cudaSuccess) return e;
         (*launches)++;

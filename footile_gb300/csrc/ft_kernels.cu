@@ -38,6 +38,7 @@
 
 #include "ft_device.cuh"
 #include "ft_kernels.cuh"
+#include "ft_slots.cuh"
 
 namespace ftk {
 
@@ -317,15 +318,33 @@ struct CState {
     int s_items;  // outline items of all sub-strokes
 };
 
+// One chunk of ops whose curves are taken by slots (ft_slots.cuh), in place of the raw window:
+// the ops that have slots, and one round of BLOCK leaves.
+struct SlotSmem {
+    float4 g0[BLOCK], g1[BLOCK];  // transformed control points (a, b), (c, end)
+    float2 w[BLOCK];              // strokes: the widths of the pen and of the op
+    int off[BLOCK + 32];          // first slot; past the last op INT_MAX
+    int info[BLOCK];              // depth | safe << 4 | type << 8 | starts a sub-figure << 10 | Move << 11 | op << 12
+    __align__(16) float4 raw[BLOCK];  // leaves: int2 16.16 vertices (fills), or points and widths (strokes)
+    int opi[BLOCK];
+    unsigned char rs[BLOCK], jp[BLOCK];
+};
+enum { SLOT_POINT = 0, SLOT_QUAD = 1, SLOT_CUBIC = 2 };
+
 template <int N, int RAW>
 struct BuildSmemT {
     int kind[N];
     float pwval[N];
     float penx[N], peny[N], penw[N];
     int scan[2 * NWARP + 2];
-    // 16-byte aligned: stroke points are stored here as float4
-    __align__(16) int2 raw[RAW];
-    unsigned char rs[RAW];
+    union {
+        struct {
+            // 16-byte aligned: stroke points are stored here as float4
+            __align__(16) int2 raw[RAW];
+            unsigned char rs[RAW];
+        };
+        SlotSmem slots;
+    };
 };
 using BuildSmem = BuildSmemT<BLOCK, RAW_CAP>;
 
@@ -911,40 +930,141 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
         auto keep_leaf = [&](int k, P2 q, float) {
             if (k < LC) cache[k] = make_int2(f2fx(q.x), f2fx(q.y));
         };
+        int D_slots = 0, safe = 0;  // the curve's slots: 2^D_slots
         P2 A = p2(0, 0), Bq = p2(0, 0), C = p2(0, 0), D = p2(0, 0);
         if (kind == FT_OP_MOVE || kind == FT_OP_LINE) {
             A = xform(P.xf, p2(op.v[0], op.v[1]));
             n = 1;
-        } else if (kind == FT_OP_QUAD) {
+        } else if (kind == FT_OP_QUAD || kind == FT_OP_CUBIC) {
             A = xform(P.xf, p2(pen_x, pen_y));
             Bq = xform(P.xf, p2(op.v[0], op.v[1]));
             C = xform(P.xf, p2(op.v[2], op.v[3]));
-            if (!pfinite(A) || !pfinite(Bq) || !pfinite(C)) {
-                nonfinite = true;
-                n = 1;
-            } else if (STROKE) {
-                n = quad_walk<true>(A, Bq, C, wa, wb, wc, tol_sq, 0, INT_MAX, &depth_hit, [](int, P2, float) {});
-            } else {
-                n = quad_walk<false>(A, Bq, C, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &depth_hit, keep_leaf);
+            D = kind == FT_OP_CUBIC ? xform(P.xf, p2(op.v[4], op.v[5])) : C;
+            nonfinite = !pfinite(A) || !pfinite(Bq) || !pfinite(C) || !pfinite(D);
+            n = 1;
+            if (!nonfinite) D_slots = curve_depth(A, Bq, C, D, kind == FT_OP_CUBIC, P.tol, safe);
+        }
+        if (nonfinite) atomicOr(&S.flags, 2);
+        if (!__syncthreads_or(D_slots > SLOT_DEPTH)) {
+            // ---- the chunk's leaves by slots, BLOCK at a time
+            SlotSmem& Q = B.slots;
+            const unsigned slots = n ? 1u << D_slots : 0u;
+            unsigned inc = slots | ((slots ? 1u : 0u) << 22);
+            const unsigned own = inc;
+#pragma unroll
+            for (int s = 1; s < 32; s <<= 1) {
+                const unsigned t = __shfl_up_sync(FULL, inc, s);
+                if ((tid & 31) >= s) inc += t;
             }
-        } else if (kind == FT_OP_CUBIC) {
-            A = xform(P.xf, p2(pen_x, pen_y));
-            Bq = xform(P.xf, p2(op.v[0], op.v[1]));
-            C = xform(P.xf, p2(op.v[2], op.v[3]));
-            D = xform(P.xf, p2(op.v[4], op.v[5]));
-            if (!pfinite(A) || !pfinite(Bq) || !pfinite(C) || !pfinite(D)) {
-                nonfinite = true;
-                n = 1;
-            } else if (STROKE) {
+            if ((tid & 31) == 31) B.scan[tid >> 5] = (int)inc;
+            __syncthreads();
+            unsigned pre = 0, sum = 0;
+#pragma unroll
+            for (int k = 0; k < NWARP; k++) {
+                const unsigned v = (unsigned)B.scan[k];
+                if (k < tid >> 5) pre += v;
+                sum += v;
+            }
+            const int listed = (int)(sum >> 22), total = (int)(sum & ((1u << 22) - 1));
+            if (slots) {
+                const unsigned ex = pre + inc - own;
+                const int at = (int)(ex >> 22);
+                const bool curve = (kind == FT_OP_QUAD || kind == FT_OP_CUBIC) && !nonfinite;
+                if (curve) Q.g0[at] = make_float4(A.x, A.y, Bq.x, Bq.y);
+                const P2 end = kind == FT_OP_MOVE || kind == FT_OP_LINE ? A : D;
+                Q.g1[at] = make_float4(C.x, C.y, end.x, end.y);
+                if (STROKE) Q.w[at] = make_float2(pen_w, sw_i);
+                Q.off[at] = (int)(ex & ((1u << 22) - 1));
+                Q.info[at] = (curve ? D_slots : 0) | (safe << 4) |
+                             ((!curve ? SLOT_POINT : kind == FT_OP_QUAD ? SLOT_QUAD : SLOT_CUBIC) << 8) | (rs << 10) |
+                             ((kind == FT_OP_MOVE ? 1 : 0) << 11) | (tid << 12);
+            }
+            if (tid < 32) Q.off[listed + tid] = INT_MAX;
+            // carry the path-walk state to the next chunk (everyone has read S by now)
+            if (tid == N - 1) {
+                S.sw = sw_i;
+                const int last_pc = isPC ? tid : lpc;
+                if (last_pc >= 0) {
+                    S.pen_x = B.penx[last_pc];
+                    S.pen_y = B.peny[last_pc];
+                    S.pen_w = B.penw[last_pc];
+                    S.last_pc_kind = B.kind[last_pc];
+                }
+            }
+            __syncthreads();
+            int j0 = 0;
+            for (int w0 = 0; w0 < total; w0 += N) {
+                const int s = w0 + tid;
+                int at = -1, info = 0, idx = 0;
+                P2 z = p2(0, 0);
+                float zw = 0.f;
+                if (w0 + (tid & ~31) < total) {
+                    const int j = slot_op(Q.off, w0 + (tid & ~31), j0);
+                    if (s < total) {
+                        info = Q.info[j];
+                        idx = s - Q.off[j];
+                        const float4 g1 = Q.g1[j];
+                        const int depth = info & 15, sf = (info >> 4) & 15, type = (info >> 8) & 3;
+                        z = p2(g1.z, g1.w);
+                        float2 w = make_float2(0.f, 0.f);
+                        if (STROKE) w = Q.w[j];
+                        zw = w.y;
+                        if (type == SLOT_POINT) {
+                            at = 0;
+                        } else {
+                            const float4 g0 = Q.g0[j];
+                            P2 a = p2(g0.x, g0.y);
+                            float w0v = w.x;
+                            // widths of a curve's control points (plotter.rs:235-236, 294-298)
+                            if (type == SLOT_QUAD)
+                                at = quad_slot<STROKE>(a, p2(g0.z, g0.w), z, w0v, __fmul_rn(__fadd_rn(w.x, w.y), 0.5f), zw,
+                                                       idx, depth, sf, tol_sq);
+                            else
+                                at = cubic_slot<STROKE>(a, p2(g0.z, g0.w), p2(g1.x, g1.y), z, w0v,
+                                                        __fadd_rn(w.y, __fmul_rn(__fsub_rn(w.x, w.y), 1.0f / 3.0f)),
+                                                        __fadd_rn(w.y, __fmul_rn(__fsub_rn(w.x, w.y), 2.0f / 3.0f)), zw,
+                                                        idx, depth, sf, tol_sq);
+                        }
+                    }
+                }
+                int m;
+                const int pos = block_excl_sum(at >= 0 ? 1 : 0, B.scan, m);
+                if (at >= 0) {
+                    Q.rs[pos] = (unsigned char)(idx == 0 ? (info >> 10) & 1 : 0);
+                    if (STROKE) {
+                        Q.raw[pos] = make_float4(z.x, z.y, zw, 0.f);
+                        Q.jp[pos] = (unsigned char)(((info >> 11) & 1) ^ 1);
+                        Q.opi[pos] = c0 + (info >> 12);
+                    } else {
+                        reinterpret_cast<int2*>(Q.raw)[pos] = make_int2(f2fx(z.x), f2fx(z.y));
+                    }
+                }
+                __syncthreads();
+                if (STROKE)
+                    compact_stroke_block(S, Q.raw, Q.rs, Q.jp, Q.opi, m, spts, subs, *Cs);
+                else
+                    compact_window_block(S, reinterpret_cast<const int2*>(Q.raw), Q.rs, m, pts, ss, *Cs, limit);
+                __syncthreads();
+                if (S.capped || S.s_capped) break;
+            }
+            __syncthreads();
+            if (S.capped || S.s_capped) break;
+            continue;
+        }
+        // ---- a curve deeper than a slot walk: the whole chunk depth first
+        if (kind == FT_OP_QUAD && !nonfinite) {
+            if (STROKE)
+                n = quad_walk<true>(A, Bq, C, wa, wb, wc, tol_sq, 0, INT_MAX, &depth_hit, [](int, P2, float) {});
+            else
+                n = quad_walk<false>(A, Bq, C, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &depth_hit, keep_leaf);
+        } else if (kind == FT_OP_CUBIC && !nonfinite) {
+            if (STROKE)
                 n = cubic_walk<true>(A, Bq, C, D, wa, wb, wc, wd, tol_sq, 0, INT_MAX, &depth_hit,
                                      [](int, P2, float) {});
-            } else {
-                n = cubic_walk<false>(A, Bq, C, D, 0.f, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &depth_hit,
-                                      keep_leaf);
-            }
+            else
+                n = cubic_walk<false>(A, Bq, C, D, 0.f, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &depth_hit, keep_leaf);
         }
         if (depth_hit) atomicOr(&S.flags, 1);
-        if (nonfinite) atomicOr(&S.flags, 2);
         int total;
         const int off = G::excl_sum(n, B.scan, total);
         // carry the path-walk state to the next chunk (everyone has read S by now)
@@ -3819,6 +3939,7 @@ extern "C" FT_API int ft_fill_noalloc(int32_t rule, const ft_op* ops, uint32_t n
     static const float ident[6] = {1, 0, 0, 0, 1, 0};
     for (int i = 0; i < 6; i++) p.xf[i] = transform ? transform[i] : ident[i];
     const float t = tolerance > 0.01f ? tolerance : 0.01f;
+    p.tol = t;
     p.tol_sq = t * t;
     const int wp = (int)((w + 3) & ~3u);
     int smem = std::max(ftk::RASTER_FIXED_SMEM + 16 * wp * 4, 40 * 1024);

@@ -192,7 +192,7 @@ struct KParams {
     const float* sw_chain;   // nullable: initial pen width of every path
     unsigned char* scratch;  // gridDim.x * SCRATCH_BYTES_PER_CTA bytes
     float xf[6];
-    float tol_sq;
+    float tol, tol_sq;
     int join;
     float miter_limit;
     float miter_g;           // ft_miter_angle(miter_limit): the miter decision's threshold on |th/2|

@@ -16,12 +16,9 @@
 // The direction only flips the sign of every cell sum, so it is applied at the resolve.
 //
 // So every leaf of a curve's subdivision is an edge by itself: the subdivision node's start
-// and end points (the start is the end of the leaf before, bit for bit).  A leaf's address is
-// its path from the root, so the leaves of an op take 2^D consecutive slots, D the depth at
-// which the whole curve is flat (estimated from its second differences, then checked by every
-// leaf), and one thread per slot walks straight down D levels — no stack, no count pass, every
-// lane a leaf of its own.  A node that is flat above depth D belongs to the first slot of its
-// range; the other slots of the range stay empty (zero-length).
+// and end points (the start is the end of the leaf before, bit for bit).  Leaves are taken by
+// address (ft_slots.cuh): 2^D slots per curve, one thread each; slots that own no leaf stay
+// empty (zero-length segments).
 //
 // The segments (16 bytes: both end points in 16.16) go to the CTA's scratch in order.  Bands
 // of raster rows are then accumulated in shared memory: each warp takes 32 segments at a time
@@ -29,19 +26,18 @@
 // items over its lanes.  The rows are resolved 8 pixels per lane, as many rows per warp as
 // fit, and written once.
 //
-// A path whose slots exceed the scratch, or whose curves subdivide deeper than TILE_DEPTH or
-// not as estimated, is handed to k_raster through the overflow list.
+// A path whose slots exceed the scratch, or with a curve not known to be flat at SLOT_DEPTH, is
+// handed to k_raster through the overflow list.
 #include <climits>
 #include <cstddef>
 
-#include "ft_device.cuh"
 #include "ft_kernels.cuh"
+#include "ft_slots.cuh"
 
 namespace ftk {
 namespace {
 
 constexpr unsigned ALL = 0xFFFFFFFFu;
-constexpr int TILE_DEPTH = 12;  // deepest subdivision a slot walks
 
 // ---------------------------------------------------------------- arithmetic
 // Low 32 bits of n * 65536 / d (truncated), d != 0: Fixed division (fixed.rs:49-56) of
@@ -71,104 +67,7 @@ __device__ __forceinline__ int fx_div(int a, int b) {
 // Fixed::from(f32) (fixed.rs:88-93): the conversion instruction saturates and takes NaN to 0
 __device__ __forceinline__ int to_fx(float f) { return __float2int_rz(__fmul_rn(f, 65536.0f)); }
 
-// Depth at which every node of the curve's subdivision is flat (more than TILE_DEPTH: none
-// found), and the depth `safe` above which no node is.  At depth k a node centred at
-// t has its flatness vector 4^-k * p''(t) / 8 (quads: p'' constant; cubics: p'' linear, so the
-// two outermost nodes of a level have the longest).  `safe` and `sure` (every node at the depth
-// is flat) leave room for the rounding of the midpoints, 2^-16 of the largest coordinate (three
-// roundings a level of half an ulp in each of two coordinates and two points), so that the
-// nodes they speak for need no check; the depth itself is taken with 2^-19, and checked by
-// every leaf where it is not sure.
-__device__ __forceinline__ int curve_depth(P2 a, P2 b, P2 c, P2 d, bool cubic, float tol, int& safe, bool& sure) {
-    const float m = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
-                          fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
-    const float te = tol * 0.99998f - m * 1.9073486e-6f, th = tol * 1.00002f + m * 1.5258789e-5f;
-    const float ts = tol * 0.99998f - m * 1.5258789e-5f;
-    const float te2 = te * te, th2 = th * th, ts2 = ts > 0.0f ? ts * ts : -1.0f;
-    safe = 0;
-    sure = false;
-    if (!(te > 0.25f * tol)) return TILE_DEPTH + 1;
-    int k = 0;
-    if (!cubic) {
-        const float x = a.x - 2.0f * b.x + c.x, y = a.y - 2.0f * b.y + c.y;
-        float f = (x * x + y * y) * 0.0625f;
-        while (f > te2 && k <= TILE_DEPTH) {
-            if (f > th2) safe = k + 1;
-            f *= 0.0625f;
-            k++;
-        }
-        sure = f <= ts2;
-        return k;
-    }
-    const float x0 = 0.75f * (a.x - 2.0f * b.x + c.x), y0 = 0.75f * (a.y - 2.0f * b.y + c.y);
-    const float x1 = 0.75f * (b.x - 2.0f * c.x + d.x) - x0, y1 = 0.75f * (b.y - 2.0f * c.y + d.y) - y0;
-    // the shortest vector over the curve, for `safe`
-    const float n2 = x1 * x1 + y1 * y1, t = fminf(fmaxf(__fdividef(-(x0 * x1 + y0 * y1), n2), 0.0f), 1.0f);
-    const float wx = x0 + t * x1, wy = y0 + t * y1, w2 = n2 > 0.0f ? (wx * wx + wy * wy) * 0.999f : 0.0f;
-    float h = 0.5f, s = 1.0f;
-    for (; k <= TILE_DEPTH; k++) {
-        const float ux = x0 + h * x1, uy = y0 + h * y1, vx = x0 + (1.0f - h) * x1, vy = y0 + (1.0f - h) * y1;
-        const float f = fmaxf(ux * ux + uy * uy, vx * vx + vy * vy) * s;
-        sure = f <= ts2;
-        if (f <= te2) break;
-        if (w2 * s > th2) safe = k + 1;
-        h *= 0.5f;
-        s *= 0.0625f;
-    }
-    return k;
-}
-
-// The leaf at slot `idx` of a quad (plotter.rs:248-265) of depth D: its end points in a and
-// c.  False when the slot owns no leaf; `ok` is cleared when the node at depth D is not flat.
-__device__ __forceinline__ bool quad_slot(P2& a, P2 b, P2& c, int idx, int D, int safe, bool sure, float tol_sq,
-                                          bool& ok) {
-    for (int k = 0;; k++) {
-        if (sure && k >= D) return true;
-        const P2 ab = pmid(a, b), bc = pmid(b, c), m = pmid(ab, bc);
-        if (k >= safe) {
-            const bool within = pdist_sq(m, pmid(a, c)) <= tol_sq;
-            if (within || k >= D) {
-                if (!within) ok = false;
-                return (idx & ((1 << (D - k)) - 1)) == 0;
-            }
-        }
-        if ((idx >> (D - 1 - k)) & 1) {
-            a = m;
-            b = bc;
-        } else {
-            b = ab;
-            c = m;
-        }
-    }
-}
-// The same for a cubic (plotter.rs:311-332): end points in a and e.
-__device__ __forceinline__ bool cubic_slot(P2& a, P2 b, P2 c, P2& e, int idx, int D, int safe, bool sure, float tol_sq,
-                                           bool& ok) {
-    for (int k = 0;; k++) {
-        if (sure && k >= D) return true;
-        const P2 ab = pmid(a, b), bc = pmid(b, c), cd = pmid(c, e);
-        const P2 abbc = pmid(ab, bc), bccd = pmid(bc, cd);
-        const P2 m = pmid(abbc, bccd);
-        if (k >= safe) {
-            const bool within = pdist_sq(m, pmid(a, e)) <= tol_sq;
-            if (within || k >= D) {
-                if (!within) ok = false;
-                return (idx & ((1 << (D - k)) - 1)) == 0;
-            }
-        }
-        if ((idx >> (D - 1 - k)) & 1) {
-            a = m;
-            b = bccd;
-            c = cd;
-        } else {
-            b = ab;
-            c = abbc;
-            e = m;
-        }
-    }
-}
-
-static_assert(TILE_THREADS_FEW * ((1 << TILE_DEPTH) + 1) < (1 << 22) && TILE_THREADS_FEW <= 512,
+static_assert(TILE_THREADS_FEW * ((1 << SLOT_DEPTH) + 1) < (1 << 22) && TILE_THREADS_FEW <= 512,
               "slots and listed ops of a chunk fit one word");
 
 // ------------------------------------------------------------------- state
@@ -177,7 +76,7 @@ struct TileBuild {  // one chunk of NT ops; g0, g1, off and info of the ops that
     float4 g0[NT], g1[NT];  // transformed control points (a, b), (c, end)
     float2 endp[NT];        // the pen after the op
     int off[NT + 33];       // first slot; past the last op: INT_MAX
-    int info[NT];           // depth | safe << 4 | type << 8 | closing slot << 10 | starts a sub-figure << 11 | sure << 12
+    int info[NT];           // depth | safe << 4 | type << 8 | closing slot << 10 | starts a sub-figure << 11
     int kind[NT];
 };
 enum { TY_POINT = 0, TY_QUAD = 1, TY_CUBIC = 2 };
@@ -240,13 +139,13 @@ __device__ P2 first_vertex(const TileParams& P, const ft_op* ops, int j) {
     if (o.kind != FT_OP_QUAD && o.kind != FT_OP_CUBIC) return end;
     P2 a = xform(P.xf, p2(0.f, 0.f)), b = xform(P.xf, p2(o.v[0], o.v[1])), c = xform(P.xf, p2(o.v[2], o.v[3]));
     if (!pfinite(a) || !pfinite(b) || !pfinite(c) || !pfinite(end)) return end;
-    bool ok = true;
+    float w = 0.f;
     if (o.kind == FT_OP_QUAD) {
-        quad_slot(a, b, c, 0, TILE_DEPTH, 0, false, P.tol_sq, ok);
+        quad_slot(a, b, c, w, w, w, 0, SLOT_DEPTH, 0, P.tol_sq);
         return c;
     }
     P2 e = end;
-    cubic_slot(a, b, c, e, 0, TILE_DEPTH, 0, false, P.tol_sq, ok);
+    cubic_slot(a, b, c, e, w, w, w, w, 0, SLOT_DEPTH, 0, P.tol_sq);
     return e;
 }
 __device__ __forceinline__ unsigned long long top_key(int x, int y) {
@@ -326,7 +225,6 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
         const int lrs_op = lrs >= 0 ? c0 + lrs : S.c_rs;
         // slots of this op
         int slots = closes ? 1 : 0, D = 0, safe = 0, type = TY_POINT;
-        bool sure = false;
         float4 ga = make_float4(0.f, 0.f, 0.f, 0.f), gb = ga;
         if (vo) {
             const P2 a = xform(P.xf, pen), e = xform(P.xf, end);
@@ -338,8 +236,8 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
                     atomicOr(&S.flags, 2);
                 } else {
                     type = kind == FT_OP_QUAD ? TY_QUAD : TY_CUBIC;
-                    D = curve_depth(a, b, c, e, type == TY_CUBIC, P.tol, safe, sure);
-                    if (D > TILE_DEPTH) {
+                    D = curve_depth(a, b, c, e, type == TY_CUBIC, P.tol, safe);
+                    if (D > SLOT_DEPTH) {
                         bad = 1;
                         D = safe = 0;
                     }
@@ -374,8 +272,7 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
             B.g0[at] = ga;
             B.g1[at] = gb;
             B.off[at] = off;
-            B.info[at] = D | (safe << 4) | (type << 8) | ((closes ? 1 : 0) << 10) | ((rs ? 1 : 0) << 11) |
-                        ((sure ? 1 : 0) << 12);
+            B.info[at] = D | (safe << 4) | (type << 8) | ((closes ? 1 : 0) << 10) | ((rs ? 1 : 0) << 11);
         }
         if (tid < 32) B.off[listed + tid] = INT_MAX;
         const int padded = (total + 31) & ~31;
@@ -405,33 +302,25 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
         int j0 = 0;
         for (int s0 = w * 32; s0 < padded; s0 += NT) {
             const int s = s0 + lane;
-            // the op of the first slot, then the ops that start in the window
-            for (;;) {
-                const unsigned m = __ballot_sync(ALL, B.off[j0 + 1 + lane] <= s0);
-                j0 += __popc(m);
-                if (m != ALL) break;
-            }
-            const int rel = B.off[j0 + 1 + lane] - s0;
-            const unsigned starts = __reduce_or_sync(ALL, rel < 32 ? 1u << rel : 0u);
+            const int lo = slot_op(B.off, s0, j0);
             int4 e = make_int4(0, 0, 0, 0);
             bool close_slot = false;
             if (s < total) {
-                const int lo = j0 + __popc(starts & (ALL >> (31 - lane)));
                 const int info = B.info[lo];
                 const int idx = s - B.off[lo] - ((info >> 10) & 1);
                 close_slot = idx < 0;
                 if (!close_slot && !(((info >> 11) & 1) && idx == 0 && ((info >> 8) & 3) == TY_POINT)) {
                     const float4 g0 = B.g0[lo], g1 = B.g1[lo];
                     P2 a = p2(g0.x, g0.y), z = p2(g1.z, g1.w);
-                    bool own = true, ok = true;
                     const int type = (info >> 8) & 3, D = info & 15, safe = (info >> 4) & 15;
+                    float w = 0.f;
+                    int at = 0;  // the leaf's depth, -1: none
                     if (type == TY_QUAD)
-                        own = quad_slot(a, p2(g0.z, g0.w), z, idx, D, safe, (info >> 12) & 1, tol_sq, ok);
+                        at = quad_slot(a, p2(g0.z, g0.w), z, w, w, w, idx, D, safe, tol_sq);
                     else if (type == TY_CUBIC)
-                        own = cubic_slot(a, p2(g0.z, g0.w), p2(g1.x, g1.y), z, idx, D, safe, (info >> 12) & 1, tol_sq, ok);
-                    if (!ok) bad = 1;
+                        at = cubic_slot(a, p2(g0.z, g0.w), p2(g1.x, g1.y), z, w, w, w, w, idx, D, safe, tol_sq);
                     // the first vertex of a sub-figure ends no segment
-                    if (own && !(((info >> 11) & 1) && idx == 0))
+                    if (at >= 0 && !(((info >> 11) & 1) && idx == 0))
                         e = make_int4(to_fx(a.x), to_fx(a.y), to_fx(z.x), to_fx(z.y));
                 }
             }
