@@ -18,8 +18,8 @@ OUT = os.path.join(HERE, "_build")
 LIB = os.path.join(OUT, "libfootile_gpu.so")
 STATIC_LIB = os.path.join(OUT, "libfootile_gpu.a")
 
-SOURCES = ["ft_kernels.cu", "ft_tile.cu", "ft_adjoint.cu", "ft_convert.cu", "ft_capi.cu"]
-HEADERS = ["ft_device.cuh", "ft_slots.cuh", "ft_kernels.cuh", "ft_adjoint.cuh"]
+SOURCES = ["ft_kernels.cu", "ft_tile.cu", "ft_bands.cu", "ft_adjoint.cu", "ft_convert.cu", "ft_capi.cu"]
+HEADERS = ["ft_device.cuh", "ft_slots.cuh", "ft_items.cuh", "ft_kernels.cuh", "ft_adjoint.cuh"]
 GENCODE = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Bit-exact float stages: no FMA contraction, IEEE division and square root.
 NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "--fmad=false", "-prec-div=true", "-prec-sqrt=true",

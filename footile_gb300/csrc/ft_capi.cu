@@ -1339,27 +1339,35 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             bool streamed = false;
             if (mask_route && smem_m <= c->max_smem) {
                 FT_CU(c->mask.ensure((size_t)mstride * h), "alloc mask");
+                ftk::KParams pm = p;
+                pm.rasters = static_cast<uint8_t*>(c->mask.p);
+                pm.canvas_stride = mstride;
+                pm.fmt = FT_MATTE8;
+                FT_CU(ftk::launch_band_single(pm, c->max_smem, c->stream), "launch band compositor");
+                const uint8_t* k = paths[0].clr;
+                const unsigned clr = (unsigned)k[0] | ((unsigned)k[1] << 8) | ((unsigned)k[2] << 16) |
+                                     ((unsigned)k[3] << 24);
+                const int top = std::min(cr0.x, (int)h);
+                FT_CU(cudaEventRecord(c->ev_comp, c->stream), "event");
+                // streamed by TMA where the canvas allows a tensor map (16-byte rows).  Canvases
+                // of other strides (1531 x 1117: 63 us in the tile compositor, which walks the
+                // edges again per tile) take the mask row by row.
                 CUtensorMap tc, tmk;
                 if (canvas_tensor_map(&tc, ras_d, w, h, stride, ftk::SO_COLS, ftk::SO_ROWS) &&
-                    canvas_tensor_map(&tmk, c->mask.p, w, h, mstride, ftk::SO_COLS, ftk::SO_ROWS, true)) {
-                    ftk::KParams pm = p;
-                    pm.rasters = static_cast<uint8_t*>(c->mask.p);
-                    pm.canvas_stride = mstride;
-                    pm.fmt = FT_MATTE8;
-                    FT_CU(ftk::launch_composite_bands(pm, smem_m, c->stream), "launch band compositor");
-                    const uint8_t* k = paths[0].clr;
-                    const unsigned clr = (unsigned)k[0] | ((unsigned)k[1] << 8) | ((unsigned)k[2] << 16) |
-                                         ((unsigned)k[3] << 24);
-                    FT_CU(cudaEventRecord(c->ev_comp, c->stream), "event");
-                    FT_CU(ftk::launch_srcover_mask(tc, tmk, (int)w, (int)h, std::min(cr0.x, (int)h), clr, p.status,
-                                                   c->sm_count, c->stream),
+                    canvas_tensor_map(&tmk, c->mask.p, w, h, mstride, ftk::SO_COLS, ftk::SO_ROWS, true))
+                    FT_CU(ftk::launch_srcover_mask(tc, tmk, (int)w, (int)h, top, clr, p.status, c->sm_count, c->stream),
                           "launch mask compositor");
-                    c->comp_timed = true;
-                    c->launches++;
-                    streamed = true;
-                }
+                else
+                    FT_CU(ftk::launch_srcover_rows(ras_d, stride, static_cast<const uint8_t*>(c->mask.p), mstride, (int)w,
+                                                   (int)h, top, clr, c->stream),
+                          "launch mask compositor");
+                c->comp_timed = true;
+                c->launches++;
+                streamed = true;
             }
             if (streamed) {
+            } else if (fmt == FT_MATTE8 && n_paths == 1) {
+                FT_CU(ftk::launch_band_single(p, c->max_smem, c->stream), "launch band compositor");
             } else if (fmt == FT_MATTE8) {
                 FT_CU(ftk::launch_composite_bands(p, smem_b, c->stream), "launch band compositor");
             } else {

@@ -131,6 +131,14 @@ __device__ __forceinline__ unsigned srcover_rgba(unsigned d, unsigned clr, unsig
     return out;
 }
 
+// Whether an alpha-0 SrcOver changes the pixel: it maps each channel d to ch8_mul(d, 255),
+// which leaves all but 1..15 as they are (non-zero bytes whose high nibble is zero).
+__device__ __forceinline__ unsigned low_channels(unsigned v) {
+    const unsigned nz = (((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) & 0x80808080u;
+    const unsigned hi = (((v & 0x70707070u) + 0x70707070u) | v) & 0x80808080u;
+    return nz & ~hi;
+}
+
 // fill rule on the wrapped i16 running sum (imgbuf.rs:54-61, 157-167)
 __device__ __forceinline__ unsigned resolve_cov(unsigned sum32, int rule) {
     int s = (int)(short)(sum32 & 0xFFFF);

@@ -309,7 +309,14 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
 // done and final_flag, the full build's skip): when the point cap is reached there the
 // points are complete and the full build's point kernels do nothing.
 cudaError_t launch_grid_stroke(const KParams& p, int sm_count, cudaStream_t s, const KParams* probe = nullptr);
+// Shared memory either band compositor needs for rows of `width` pixels.
 int composite_bands_smem(int band_rows, int width);
+// A single call's rows from its binned edges (Matte8, or the coverage mask of an Rgba8p call).
+cudaError_t launch_band_single(const KParams& p, int max_smem, cudaStream_t s);
+int band_single_smem(int band_rows, int width);
+// SrcOver of one call's colour from its mask, for canvases that no tensor map fits.
+cudaError_t launch_srcover_rows(uint8_t* canvas, uint32_t stride, const uint8_t* mask, uint32_t mstride, int W, int H,
+                                int r0, unsigned clr, cudaStream_t s);
 int composite_build_blocks_per_sm(int smem_bytes, bool stroke);
 
 // Static shared memory of the kernel besides the dynamic area buffer.
