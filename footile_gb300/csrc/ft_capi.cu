@@ -2,6 +2,7 @@
 // Plotter settings), device buffers, work-item planning and kernel launches.
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -104,7 +105,7 @@ struct ft_ctx {
 
 static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* ops, uint32_t n_ops_total,
                           const ft_path_desc* paths, uint32_t n_paths, int32_t fmt, uint8_t* raster, uint32_t w,
-                          uint32_t h, uint32_t stride, int32_t where, float* sw_out);
+                          uint32_t h, uint32_t stride, int32_t where, float* sw_out, const float* sw_in);
 
 namespace {
 
@@ -468,11 +469,7 @@ int single(ft_ctx* c, int stroke, int32_t rule, const ft_op* ops, uint32_t n_ops
     if ((uncapped || (uint64_t)w * h >= split_px(c)) && ftk::composite_bands_smem(1, (int)w) <= c->max_smem) {
         // a large canvas, or an un-capped fill: build the figure once and bin its edges,
         // then one CTA per band of rows (the ordered compositor with a single call)
-        float sw0 = c->s_width;
-        FT_CU(cudaMemcpyAsync(&sw0, sw_in, sizeof(float), cudaMemcpyDeviceToHost, c->stream), "pen width");
-        FT_CU(cudaStreamSynchronize(c->stream), "synchronize");
-        d.s_width = sw0;
-        st = composite_impl(c, stroke, rule, ops_d, n_ops, &d, 1, fmt, ras_d, w, h, stride, FT_DEVICE, sw_next);
+        st = composite_impl(c, stroke, rule, ops_d, n_ops, &d, 1, fmt, ras_d, w, h, stride, FT_DEVICE, sw_next, sw_in);
     } else {
         st = run(c, stroke, rule, ops_d, &d, 1, fmt, ras_d, sw_in, sw_next);
     }
@@ -1061,14 +1058,14 @@ FT_API int ft_composite_batch(ft_ctx* c, int32_t stroke, int32_t rule, const ft_
                               uint32_t h, uint32_t stride, int32_t where) {
     Stage stage_("ft_composite_batch");
     return composite_impl(c, stroke, rule, ops, n_ops_total, paths, n_paths, fmt, raster, w, h, stride, where,
-                          nullptr);
+                          nullptr, nullptr);
 }
 
 }  // extern "C"
 
 static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* ops, uint32_t n_ops_total,
                           const ft_path_desc* paths, uint32_t n_paths, int32_t fmt, uint8_t* raster, uint32_t w,
-                          uint32_t h, uint32_t stride, int32_t where, float* sw_out) {
+                          uint32_t h, uint32_t stride, int32_t where, float* sw_out, const float* sw_in) {
     if (!c) return FT_ERR_ARG;
     if ((rule != FT_NONZERO && rule != FT_EVENODD) || (fmt != FT_MATTE8 && fmt != FT_RGBA8P) ||
         (where != FT_HOST && where != FT_DEVICE))
@@ -1181,6 +1178,7 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
         p.bandoff = static_cast<int*>(c->bandoff.p);
         p.crec = static_cast<int4*>(c->crec.p);
         p.sw_out = sw_out;
+        p.sw_chain = sw_in;  // a single call's pen width on the device (nullable: the descriptors')
         p.pt_cap = uncapped ? (int)c->fig_cap : ftk::PT_CAP;
         p.L = L;
         if (split) {
@@ -1200,7 +1198,9 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             ftk::GridBuildBufs& g = p.gb;
             g.ops = ops_d + paths[0].op_begin;
             g.n_ops = (int)paths[0].n_ops;
-            g.s_width = paths[0].s_width;
+            g.s_width = sw_in ? sw_in
+                              : reinterpret_cast<const float*>(static_cast<char*>(c->paths.p) +
+                                                               offsetof(ft_path_desc, s_width));
             g.raw_cap = (int)raw_cap;
             g.done = reinterpret_cast<unsigned*>(gb);
             g.n_raw = reinterpret_cast<long long*>(gb + 32);

@@ -60,6 +60,28 @@ __device__ __forceinline__ bool ck(bool ok, int site) {
 constexpr int LEAF_CACHE_CTA = 256;
 constexpr int SRAW = 1024;            // stroke points per window (float4 in the raw window's bytes)
 
+// Kernels launched one after another on small data (the grid-wide builds): each waits for the
+// one before (programmatic dependent launch) and lets the next be set up meanwhile, so that
+// a launch's latency is spent while its predecessor still runs.
+__device__ __forceinline__ void chain_link() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <class... A>
+cudaError_t launch_chain(void (*kern)(A...), int grid, int threads, int smem, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // ------------------------------------------------------------ block scans
 __device__ __forceinline__ int warp_incl_sum(int v) {
     int lane = threadIdx.x & 31;
@@ -1741,13 +1763,14 @@ __global__ void __launch_bounds__(BLOCK, 4) k_cbuild(KParams P) {
         __syncthreads();
         if (it >= (int)P.n_items) break;
         const ft_path_desc d = P.paths[it];
+        const float sw0 = P.sw_chain ? *P.sw_chain : d.s_width;
         if (STROKE) {
             int* opi = reinterpret_cast<int*>(smem + cs_off + ((sizeof(CompactSmem) + 15) & ~(size_t)15));
-            build_fill<BlockG, true>(P, d, d.s_width, B, Cs, S, pts, ss, PT_CAP, spts, subs, opi, raw_store(scr, L));
+            build_fill<BlockG, true>(P, d, sw0, B, Cs, S, pts, ss, PT_CAP, spts, subs, opi, raw_store(scr, L));
             finish_subs(P, d, S, subs, B.scan);
             build_outline(P, S, spts, subs, B, *Cs, pts, ss);
         } else {
-            build_fill<BlockG>(P, d, d.s_width, B, Cs, S, pts, ss, P.pt_cap, nullptr, nullptr, nullptr,
+            build_fill<BlockG>(P, d, sw0, B, Cs, S, pts, ss, P.pt_cap, nullptr, nullptr, nullptr,
                                raw_store(scr, L));
         }
         if (P.split_bin) {
@@ -1768,7 +1791,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_cbuild(KParams P) {
             for (int i = tid; i < (int)d.n_ops; i += BLOCK)
                 if (P.ops[d.op_begin + i].kind == FT_OP_PEN_WIDTH) lp = max(lp, i);
             lp = block_incl_max(lp, s_tmp3);
-            if (tid == BLOCK - 1) P.sw_out[it] = lp >= 0 ? P.ops[d.op_begin + lp].v[0] : d.s_width;
+            if (tid == BLOCK - 1) P.sw_out[it] = lp >= 0 ? P.ops[d.op_begin + lp].v[0] : sw0;
         }
         if (tid == 0 && S.flags) atomicMax(&P.status[it], (S.flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
         __syncthreads();
@@ -2458,6 +2481,7 @@ __device__ void fig_bin_prefix(int* sh, int nb, int* tmp) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_fig_edges(KParams P) {
+    chain_link();
     extern __shared__ int sh_bins[];  // n_bands + 1 differences (when n_bands <= BIN_SMEM_BANDS)
     __shared__ int tmp[2 * NWARP + 2];
     const FigBins f = fig_bins(P);
@@ -2491,6 +2515,7 @@ __global__ void __launch_bounds__(BLOCK) k_fig_edges(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_fig_bin_scan(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ unsigned long long s_base;
     const FigBins f = fig_bins(P);
@@ -2526,6 +2551,7 @@ struct BinStage {
 };
 
 __global__ void __launch_bounds__(BLOCK) k_fig_bin_fill(KParams P) {
+    chain_link();
     // n_bands + 1 counts, then n_bands cursors (n_bands <= BIN_SMEM_BANDS), then the stage
     extern __shared__ __align__(16) int sh_bins[];
     const FigBins f = fig_bins(P);
@@ -2621,14 +2647,9 @@ cudaError_t launch_figure_bins(const KParams& p, int grid, cudaStream_t s) {
     e = cudaFuncSetAttribute(k_fig_edges, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (BIN_SMEM_BANDS + 1) * (int)sizeof(int));
     if (e != cudaSuccess) return e;
-    k_fig_edges<<<grid, BLOCK, sm_e, s>>>(p);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_fig_bin_scan<<<1, BLOCK, 0, s>>>(p);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_fig_bin_fill<<<grid, BLOCK, sm_f, s>>>(p);
-    return cudaGetLastError();
+    if ((e = launch_chain(k_fig_edges, grid, BLOCK, sm_e, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_fig_bin_scan, 1, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    return launch_chain(k_fig_bin_fill, grid, BLOCK, sm_f, s, p);
 }
 
 // ---- grid-wide figure build of one fill path
@@ -2852,6 +2873,7 @@ __device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, fl
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_ops(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ int s_tot[3];
     const GridBuildBufs& G = P.gb;
@@ -2889,7 +2911,7 @@ __global__ void __launch_bounds__(BLOCK) k_gb_ops(KParams P) {
     }
     if (tid == 0) {
         // pen width after the call: the last PenWidth op of the path
-        if (P.sw_out) P.sw_out[0] = cpw >= 0 ? G.ops[cpw].v[0] : G.s_width;
+        if (P.sw_out) P.sw_out[0] = cpw >= 0 ? G.ops[cpw].v[0] : *G.s_width;
         if (P.gs.st) {
             P.gs.st[3] = cpc;
             P.gs.st[4] = ccm;
@@ -2927,6 +2949,7 @@ __device__ __forceinline__ GbOp gb_op_of(const GridBuildBufs& G, int& flags) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_count(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ long long ltmp[NWARP];
     const GridBuildBufs& G = P.gb;
@@ -2984,6 +3007,7 @@ __device__ void gb_scan_tr(const GridBuildBufs& G, long long n_raw, int* tmp, in
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_emit(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ int s_c;
     const GridBuildBufs& G = P.gb;
@@ -3012,6 +3036,7 @@ __global__ void __launch_bounds__(BLOCK) k_gb_emit(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_keep(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ PAgg wt[NWARP];
     const GridBuildBufs& G = P.gb;
@@ -3087,6 +3112,7 @@ __global__ void __launch_bounds__(BLOCK) k_gb_keep(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_write(KParams P) {
+    chain_link();
     __shared__ PAgg wt[NWARP];
     __shared__ int s_l;
     const GridBuildBufs& G = P.gb;
@@ -3159,6 +3185,7 @@ __global__ void __launch_bounds__(BLOCK) k_gb_write(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gb_top(KParams P) {
+    chain_link();
     __shared__ int4 wb[NWARP];
     const GridBuildBufs& G = P.gb;
     if (G.skip && *G.skip) return;  // a probe over a prefix of the ops completed the figure
@@ -3230,17 +3257,18 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
     if (nbo <= 0 || p.gb.raw_cap % GB_TILE || p.gb.raw_cap > GB_RAW_MAX) return cudaErrorInvalidValue;
     if (probe && (probe->gb.n_ops <= 0 || probe->gb.n_ops > p.gb.n_ops)) return cudaErrorInvalidValue;
     const int gt = std::max(1, 4 * sm_count);
-    k_gb_ops<<<nbo, BLOCK, 0, s>>>(p);  // pens of every op (the probe's too) and the pen width after
+    cudaError_t e;
+    if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens of every op (the probe's too) and the pen width after
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
         const int nbw = (q->gb.n_ops + GB_OPB - 1) / GB_OPB;
-        k_gb_count<<<nbw, BLOCK, 0, s>>>(*q);
-        k_gb_emit<<<nbw, BLOCK, 0, s>>>(*q);
-        k_gb_keep<<<gt, BLOCK, 0, s>>>(*q);
-        k_gb_write<<<gt, BLOCK, 0, s>>>(*q);
-        k_gb_top<<<GB_TOP_BLOCKS, BLOCK, 0, s>>>(*q);
+        if ((e = launch_chain(k_gb_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gb_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gb_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gb_write, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gb_top, GB_TOP_BLOCKS, BLOCK, 0, s, *q)) != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // ---- grid-wide build of one stroke path
@@ -3271,9 +3299,9 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
 // width in effect at op j: its path's last PenWidth op at or before it, else the width
 // the path starts with
 __device__ __forceinline__ float gs_width(const GridBuildBufs& G, int j) {
-    if (j < 0) return G.s_width;
+    if (j < 0) return *G.s_width;
     const int lpw = max(G.opw[j], G.opa[j / BLOCK].y);
-    return lpw >= 0 ? __ldg(&G.ops[lpw].v[0]) : G.s_width;
+    return lpw >= 0 ? __ldg(&G.ops[lpw].v[0]) : *G.s_width;
 }
 
 // Raw stroke points of a Move/Line/Quad/Cubic op with the pen at (px, py) and widths
@@ -3370,6 +3398,7 @@ __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, fl
 __device__ __forceinline__ bool gs_over(const GridStrokeBufs& S) { return *S.n_sraw > S.sraw_cap; }
 
 __global__ void __launch_bounds__(BLOCK) k_gs_count(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ long long ltmp[NWARP];
     const GridBuildBufs& G = P.gb;
@@ -3411,6 +3440,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_count(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gs_emit(KParams P) {
+    chain_link();
     const GridBuildBufs& G = P.gb;
     const GridStrokeBufs& S = P.gs;
     if (S.skip && *S.skip) return;  // a probe over a prefix of the ops completed the points
@@ -3440,6 +3470,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_emit(KParams P) {
 
 // Kept raw stroke points and sub-stroke starts per tile, packed (kept << 32 | starts).
 __global__ void __launch_bounds__(BLOCK) k_gs_keep(KParams P) {
+    chain_link();
     __shared__ long long ltmp[NWARP];
     const GridStrokeBufs& S = P.gs;
     if (S.skip && *S.skip) return;  // a probe over a prefix of the ops completed the points
@@ -3490,6 +3521,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_keep(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_gs_write(KParams P) {
+    chain_link();
     __shared__ long long ltmp[NWARP];
     const GridStrokeBufs& S = P.gs;
     if (S.skip && *S.skip) return;  // a probe over a prefix of the ops completed the points
@@ -3547,6 +3579,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_write(KParams P) {
 
 // Sub-strokes (stroker.rs:87-96, 239-262), 256 a CTA step.
 __global__ void __launch_bounds__(BLOCK) k_gs_subs(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     const GridBuildBufs& G = P.gb;
     const GridStrokeBufs& S = P.gs;
@@ -3611,6 +3644,7 @@ __device__ __forceinline__ SubRec go_item(const GridStrokeBufs& S, const SubRec*
 }
 
 __global__ void __launch_bounds__(BLOCK) k_go_count(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ long long ltmp[NWARP];
     const GridBuildBufs& G = P.gb;
@@ -3648,6 +3682,7 @@ __global__ void __launch_bounds__(BLOCK) k_go_count(KParams P) {
 }
 
 __global__ void __launch_bounds__(BLOCK) k_go_emit(KParams P) {
+    chain_link();
     __shared__ int tmp[2 * NWARP + 2];
     __shared__ int s_c;
     const GridBuildBufs& G = P.gb;
@@ -3689,22 +3724,23 @@ cudaError_t launch_grid_stroke(const KParams& p, int sm_count, cudaStream_t s, c
         return cudaErrorInvalidValue;
     if (probe && (probe->gb.n_ops <= 0 || probe->gb.n_ops > p.gb.n_ops)) return cudaErrorInvalidValue;
     const int gt = std::max(1, 4 * sm_count);
-    k_gb_ops<<<nbo, BLOCK, 0, s>>>(p);  // pens and widths of every op (the probe's too)
+    cudaError_t e;
+    if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens and widths of every op (the probe's too)
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
         const int nbw = (q->gb.n_ops + GB_OPB - 1) / GB_OPB;
-        k_gs_count<<<nbw, BLOCK, 0, s>>>(*q);
-        k_gs_emit<<<nbw, BLOCK, 0, s>>>(*q);
-        k_gs_keep<<<gt, BLOCK, 0, s>>>(*q);
-        k_gs_write<<<gt, BLOCK, 0, s>>>(*q);
+        if ((e = launch_chain(k_gs_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gs_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gs_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
+        if ((e = launch_chain(k_gs_write, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
     }
-    k_gs_subs<<<std::max(1, std::min(gt, PT_CAP / BLOCK + 1)), BLOCK, 0, s>>>(p);
-    k_go_count<<<gt, BLOCK, 0, s>>>(p);
-    k_go_emit<<<gt, BLOCK, 0, s>>>(p);
-    k_gb_keep<<<gt, BLOCK, 0, s>>>(p);
-    k_gb_write<<<gt, BLOCK, 0, s>>>(p);
-    k_gb_top<<<GB_TOP_BLOCKS, BLOCK, 0, s>>>(p);
-    return cudaGetLastError();
+    if ((e = launch_chain(k_gs_subs, std::max(1, std::min(gt, PT_CAP / BLOCK + 1)), BLOCK, 0, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_go_count, gt, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_go_emit, gt, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_gb_keep, gt, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_gb_write, gt, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    if ((e = launch_chain(k_gb_top, GB_TOP_BLOCKS, BLOCK, 0, s, p)) != cudaSuccess) return e;
+    return cudaSuccess;
 }
 
 cudaError_t launch_composite_build(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas) {

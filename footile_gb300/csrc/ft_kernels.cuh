@@ -100,7 +100,7 @@ constexpr long long GB_RAW_MAX = 1ll << 29;    // raw vertices the grid build ta
 struct GridBuildBufs {
     const ft_op* ops;   // the path's ops
     int n_ops;
-    float s_width;      // pen width before the path
+    const float* s_width;  // pen width before the path (device)
     int raw_cap;        // raw vertices the arrays hold (a multiple of GB_TILE)
     unsigned* done;     // [8] tickets: the last CTA of a kernel to finish runs its scan
     long long* n_raw;   // raw vertices of the path
