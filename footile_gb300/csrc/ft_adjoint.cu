@@ -25,6 +25,7 @@
 
 #include "ft_adjoint.cuh"
 #include "ft_device.cuh"
+#include "ft_slots.cuh"
 
 namespace fta {
 
@@ -237,15 +238,99 @@ __device__ __forceinline__ ft_op load_op(const ft_op* ops, int i) {
     return o;
 }
 
-enum { WALK_EMIT = 0, WALK_GRAD = 1 };
+// The curves of one chunk of ops, for leaves by slots (ft_slots.cuh); in the dynamic shared
+// memory, which is free during the walks.
+struct SlotBuf {
+    float4 g0[ABLOCK], g1[ABLOCK];  // transformed control points (a, b), (c, end)
+    float2 w[ABLOCK];               // strokes: the widths of the pen and of the op
+    int off[ABLOCK + 32];           // first slot; past the last op INT_MAX
+    int info[ABLOCK];               // depth | safe << 4 | form << 8 | starts a sub-figure << 10 | op in the chunk << 11
+    int src[ABLOCK];                // op the pen was set by, -1
+};
+enum { F_POINT = 0, F_QUAD = 1, F_CUBIC = 2 };
 
-// The path walk of plotter.rs:175-224 over ops [0, n) in chunks of ABLOCK ops.
-// WALK_EMIT writes vertex positions and sub-figure starts (and zeroes vertex gradients
-// when `zero_grad`); WALK_GRAD chains vertex gradients to the op floats.  Returns the
-// vertex count.
-template <int MODE>
-__device__ int path_walk(const AParams& p, ASmem& sm, const ft_op* ops, int n, float2* vpos, int* vsub,
-                         float2* vgrad, bool zero_grad, float* gops) {
+// Lists the chunk's ops that have slots; returns the chunk's slots.  Every thread must call.
+__device__ int list_slots(ASmem& sm, SlotBuf& Q, int slots, P2 A, P2 B, P2 C, P2 end, float2 w, int info, int src) {
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const unsigned own = (unsigned)slots | ((slots ? 1u : 0u) << 22);
+    unsigned inc = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) sm.wsum[wp] = (int)inc;
+    __syncthreads();
+    unsigned pre = 0, sum = 0;
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+        const unsigned v = (unsigned)sm.wsum[k];
+        if (k < wp) pre += v;
+        sum += v;
+    }
+    if (slots) {
+        const unsigned ex = pre + inc - own;
+        const int at = (int)(ex >> 22);
+        Q.g0[at] = make_float4(A.x, A.y, B.x, B.y);
+        Q.g1[at] = make_float4(C.x, C.y, end.x, end.y);
+        Q.w[at] = w;
+        Q.off[at] = (int)(ex & ((1u << 22) - 1));
+        Q.info[at] = info;
+        Q.src[at] = src;
+    }
+    if (tid < 32) Q.off[(int)(sum >> 22) + tid] = INT_MAX;
+    __syncthreads();
+    return (int)(sum & ((1u << 22) - 1));
+}
+
+// The leaf of slot `s`: its op's entry in Q, end point q, end parameter t and (W) width w.
+// False when the slot owns none.  Every thread must call; j0: 0 before the first window.
+template <bool W>
+__device__ __forceinline__ bool slot_leaf(const SlotBuf& Q, int s, int total, float tol_sq, int& j0, int& j, int& idx,
+                                          P2& q, float& t, float& w) {
+    const int s0 = s & ~31;
+    if (s0 >= total) return false;  // the whole warp
+    j = ftk::slot_op(Q.off, s0, j0);
+    if (s >= total) return false;
+    const int info = Q.info[j], D = info & 15, safe = (info >> 4) & 15, form = (info >> 8) & 3;
+    idx = s - Q.off[j];
+    const float4 g1 = Q.g1[j];
+    q = p2(g1.z, g1.w);
+    t = 1.0f;
+    float2 ws = make_float2(0.0f, 0.0f);
+    if (W) ws = Q.w[j];
+    w = ws.y;
+    if (form == F_POINT) return true;
+    const float4 g0 = Q.g0[j];
+    P2 a = p2(g0.x, g0.y);
+    float wa = ws.x;
+    int k;
+    if (form == F_QUAD)
+        k = ftk::quad_slot<W>(a, p2(g0.z, g0.w), q, wa, ftk::fmid(ws.x, ws.y), w, idx, D, safe, tol_sq);
+    else  // float_lerp (geom.rs:14-16)
+        k = ftk::cubic_slot<W>(a, p2(g0.z, g0.w), p2(g1.x, g1.y), q, wa,
+                               __fadd_rn(ws.y, __fmul_rn(__fsub_rn(ws.x, ws.y), 1.0f / 3.0f)),
+                               __fadd_rn(ws.y, __fmul_rn(__fsub_rn(ws.x, ws.y), 2.0f / 3.0f)), w, idx, D, safe, tol_sq);
+    if (k < 0) return false;
+    t = __fmul_rn((float)(idx + (1 << (D - k))), pow2neg(D));  // dyadic, exact
+    return true;
+}
+
+// Where a vertex came from (backward): its op, the op its curve's pen was set by, its end
+// parameter and its form, with bit 2 / 3 set where x / y takes a gradient (fx_pass).
+struct VProv {
+    int op, pen;
+    float t;
+    int form;
+};
+static_assert(sizeof(VProv) == VPROV_BYTES, "layout");
+
+// The path walk of plotter.rs:175-224 over ops [0, n) in chunks of ABLOCK ops: vertex
+// positions and sub-figure starts, and with `prov` the vertices' provenance and zeroed vertex
+// gradients.  Returns the vertex count.  Curves are taken by slots; a chunk with a curve not
+// known to be flat at depth 12 is walked depth first.
+__device__ int path_walk(const AParams& p, ASmem& sm, SlotBuf& Q, const ft_op* ops, int n, float2* vpos, int* vsub,
+                         float2* vgrad, VProv* prov) {
     const int tid = threadIdx.x;
     if (tid == 0) {
         sm.carry_pen = -1;
@@ -269,12 +354,12 @@ __device__ int path_walk(const AParams& p, ASmem& sm, const ft_op* ops, int n, f
         exc_pen = max(exc_pen, carry_pen);
         exc_close = max(exc_close, carry_close);
         const int prev_pen = exc_pen > exc_close ? exc_pen : -1;
-        // curve geometry (transformed) and leaf count
+        // curve geometry (transformed)
         P2 A = p2(0.f, 0.f), B = A, C = A, D = A;
-        int cnt = 0, depth_hit = 0;
-        bool curve = false;
+        int cnt = 0, depth = 0, safe = 0, form = F_POINT;
         if (kind == FT_OP_MOVE || kind == FT_OP_LINE) {
             cnt = 1;
+            D = xform(m, op_pt(o, 0));
         } else if (kind == FT_OP_QUAD || kind == FT_OP_CUBIC) {
             P2 pen = p2(0.f, 0.f);
             if (prev_pen >= 0) {
@@ -285,93 +370,75 @@ __device__ int path_walk(const AParams& p, ASmem& sm, const ft_op* ops, int n, f
             B = xform(m, op_pt(o, 0));
             C = xform(m, op_pt(o, 1));
             D = kind == FT_OP_CUBIC ? xform(m, op_pt(o, 2)) : C;
+            cnt = 1;
             if (!pfinite(A) || !pfinite(B) || !pfinite(C) || !pfinite(D)) {
-                cnt = 1;
                 atomicMax(&sm.status, (int)FT_ERR_ARG);
             } else {
-                curve = true;
-                auto none = [](int, P2, float) {};
-                cnt = kind == FT_OP_CUBIC ? curve_walk<true>(A, B, C, D, p.tol_sq, &depth_hit, none)
-                                          : curve_walk<false>(A, B, C, D, p.tol_sq, &depth_hit, none);
-                if (depth_hit) atomicMax(&sm.status, (int)FT_ERR_DEPTH);
+                form = kind == FT_OP_CUBIC ? F_CUBIC : F_QUAD;
+                depth = ftk::curve_depth(A, B, C, D, form == F_CUBIC, __fsqrt_rn(p.tol_sq), safe);
             }
+        }
+        const bool starts = cnt > 0 && (kind == FT_OP_MOVE || prev_pen < 0);
+        auto put = [&](int k, P2 q, float t, int sub, int op, int pen, int form_) {
+            if (k >= VCAP) return;
+            const float x = fx_range(q.x), y = fx_range(q.y);
+            vpos[k] = make_float2(x, y);
+            vsub[k] = sub;
+            if (prov) {
+                vgrad[k] = make_float2(0.f, 0.f);
+                *reinterpret_cast<int4*>(prov + k) =
+                    make_int4(op, pen, __float_as_int(t), form_ | (x == q.x ? 4 : 0) | (y == q.y ? 8 : 0));
+            }
+        };
+        if (!__syncthreads_or(depth > ftk::SLOT_DEPTH)) {
+            const int total = list_slots(sm, Q, cnt << depth, A, B, C, D, make_float2(0.f, 0.f),
+                                         depth | (safe << 4) | (form << 8) | ((starts ? 1 : 0) << 10) | (tid << 11),
+                                         prev_pen);
+            if (tid == ABLOCK - 1) {
+                sm.carry_pen = max(inc_pen, carry_pen);
+                sm.carry_close = max(inc_close, carry_close);
+            }
+            int j0 = 0;
+            for (int s0 = 0; s0 < total; s0 += ABLOCK) {
+                int j = 0, idx = 0;
+                P2 q = p2(0.f, 0.f);
+                float t = 0.f, w;
+                const bool own = slot_leaf<false>(Q, s0 + tid, total, p.tol_sq, j0, j, idx, q, t, w);
+                int kept;
+                const int k = sm.carry_base + block_excl_sum(own ? 1 : 0, sm.wsum, kept);
+                const int info = own ? Q.info[j] : 0;
+                int inc_sub, exc_sub;
+                block_max_scan(own && idx == 0 && ((info >> 10) & 1) ? k : -1, sm.wmax3, inc_sub, exc_sub);
+                const int sub = max(inc_sub, sm.carry_sub);
+                if (own) put(k, q, t, sub, c0 + (info >> 11), Q.src[j], (info >> 8) & 3);
+                __syncthreads();
+                if (tid == ABLOCK - 1) {
+                    sm.carry_base += kept;
+                    sm.carry_sub = sub;
+                }
+                __syncthreads();
+            }
+            continue;
+        }
+        int depth_hit = 0;
+        if (form != F_POINT) {
+            auto none = [](int, P2, float) {};
+            cnt = form == F_CUBIC ? curve_walk<true>(A, B, C, D, p.tol_sq, &depth_hit, none)
+                                  : curve_walk<false>(A, B, C, D, p.tol_sq, &depth_hit, none);
+            if (depth_hit) atomicMax(&sm.status, (int)FT_ERR_DEPTH);
         }
         int chunk_total;
         const int base = sm.carry_base + block_excl_sum(cnt, sm.wsum, chunk_total);
-        const bool starts = cnt > 0 && (kind == FT_OP_MOVE || prev_pen < 0);
         int inc_sub, exc_sub;
         block_max_scan(starts ? base : -1, sm.wmax3, inc_sub, exc_sub);
         const int sub = max(inc_sub, sm.carry_sub);
-        if (MODE == WALK_EMIT) {
-            auto put = [&](int j, P2 q, float) {
-                const int k = base + j;
-                if (k < VCAP) {
-                    vpos[k] = make_float2(fx_range(q.x), fx_range(q.y));
-                    vsub[k] = sub;
-                    if (zero_grad) vgrad[k] = make_float2(0.f, 0.f);
-                }
-            };
-            if (curve) {
-                if (kind == FT_OP_CUBIC)
-                    curve_walk<true>(A, B, C, D, p.tol_sq, &depth_hit, put);
-                else
-                    curve_walk<false>(A, B, C, D, p.tol_sq, &depth_hit, put);
-            } else if (cnt == 1) {
-                put(0, xform(m, op_pt(o, end_slot(kind))), 1.0f);
-            }
-        } else if (cnt > 0) {
-            // back through the transform: d(m*p)/dp = [[m0, m1], [m3, m4]]
-            float* g = gops + (size_t)i * 6;
-            if (!curve) {
-                const float2 gv = fx_pass(xform(m, op_pt(o, end_slot(kind))), __ldcg(&vgrad[base]));  // L2 atomics
-                const int s = end_slot(kind);
-                atomicAdd(g + 2 * s, __fadd_rn(__fmul_rn(m[0], gv.x), __fmul_rn(m[3], gv.y)));
-                atomicAdd(g + 2 * s + 1, __fadd_rn(__fmul_rn(m[1], gv.x), __fmul_rn(m[4], gv.y)));
-            } else {
-                float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // pen, b, c, d
-                auto chain = [&](int j, P2 q, float t) {
-                    const float2 gv = fx_pass(q, __ldcg(&vgrad[base + j]));
-                    const float gx = __fadd_rn(__fmul_rn(m[0], gv.x), __fmul_rn(m[3], gv.y));
-                    const float gy = __fadd_rn(__fmul_rn(m[1], gv.x), __fmul_rn(m[4], gv.y));
-                    const float u = __fsub_rn(1.0f, t);
-                    float w0, w1, w2, w3;
-                    if (kind == FT_OP_CUBIC) {
-                        w0 = __fmul_rn(__fmul_rn(u, u), u);
-                        w1 = __fmul_rn(__fmul_rn(3.0f, t), __fmul_rn(u, u));
-                        w2 = __fmul_rn(__fmul_rn(3.0f, t), __fmul_rn(t, u));
-                        w3 = __fmul_rn(__fmul_rn(t, t), t);
-                    } else {
-                        w0 = __fmul_rn(u, u);
-                        w1 = __fmul_rn(__fmul_rn(2.0f, t), u);
-                        w2 = __fmul_rn(t, t);
-                        w3 = 0.0f;
-                    }
-                    acc[0] = __fadd_rn(acc[0], __fmul_rn(w0, gx));
-                    acc[1] = __fadd_rn(acc[1], __fmul_rn(w0, gy));
-                    acc[2] = __fadd_rn(acc[2], __fmul_rn(w1, gx));
-                    acc[3] = __fadd_rn(acc[3], __fmul_rn(w1, gy));
-                    acc[4] = __fadd_rn(acc[4], __fmul_rn(w2, gx));
-                    acc[5] = __fadd_rn(acc[5], __fmul_rn(w2, gy));
-                    acc[6] = __fadd_rn(acc[6], __fmul_rn(w3, gx));
-                    acc[7] = __fadd_rn(acc[7], __fmul_rn(w3, gy));
-                };
-                if (kind == FT_OP_CUBIC)
-                    curve_walk<true>(A, B, C, D, p.tol_sq, &depth_hit, chain);
-                else
-                    curve_walk<false>(A, B, C, D, p.tol_sq, &depth_hit, chain);
-                const int nslot = kind == FT_OP_CUBIC ? 3 : 2;
-                for (int s = 0; s < nslot; s++) {
-                    atomicAdd(g + 2 * s, acc[2 + 2 * s]);
-                    atomicAdd(g + 2 * s + 1, acc[3 + 2 * s]);
-                }
-                if (prev_pen >= 0) {
-                    const int s = end_slot(load_op(ops, prev_pen).kind);
-                    float* gp = gops + (size_t)prev_pen * 6;
-                    atomicAdd(gp + 2 * s, acc[0]);
-                    atomicAdd(gp + 2 * s + 1, acc[1]);
-                }
-            }
-        }
+        auto leaf = [&](int k, P2 q, float t) { put(base + k, q, t, sub, i, prev_pen, form); };
+        if (form == F_CUBIC)
+            curve_walk<true>(A, B, C, D, p.tol_sq, &depth_hit, leaf);
+        else if (form == F_QUAD)
+            curve_walk<false>(A, B, C, D, p.tol_sq, &depth_hit, leaf);
+        else if (cnt == 1)
+            leaf(0, D, 1.0f);
         __syncthreads();
         if (tid == ABLOCK - 1) {
             sm.carry_pen = max(inc_pen, carry_pen);
@@ -382,6 +449,89 @@ __device__ int path_walk(const AParams& p, ASmem& sm, const ft_op* ops, int n, f
         __syncthreads();
     }
     return sm.carry_base;
+}
+
+// Sum v over the lanes of this lane's run of equal keys (runs are contiguous), into the run's
+// first lane; `last` is the run's last lane.
+__device__ __forceinline__ float run_sum(float v, int lane, int last) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float t = __shfl_down_sync(FULL, v, o);
+        if (lane + o <= last) v = __fadd_rn(v, t);
+    }
+    return v;
+}
+// First lane of a run of equal keys, and the run's last lane.
+__device__ __forceinline__ bool run_head(int key, int lane, int& last) {
+    const int before = __shfl_up_sync(FULL, key, 1);
+    const unsigned heads = __ballot_sync(FULL, lane == 0 || key != before);
+    const unsigned after = lane == 31 ? 0u : heads & (FULL << (lane + 1));
+    last = after ? __ffs(after) - 2 : 31;
+    return (heads >> lane) & 1;
+}
+
+// Vertex (or stroke point) gradient (gx, gy) to the floats of its op and of the op its pen was
+// set by, by the Bernstein weights of its end parameter (plotter.rs:248-332).  The lanes of
+// one op's vertices are summed before the atomics.  Every lane must call; op < 0: no vertex.
+__device__ __forceinline__ void chain_point(const ft_op* ops, float* gops, int op, int pen, int form, float t, float gx,
+                                            float gy, bool head, int lane, int last) {
+    const float u = __fsub_rn(1.0f, t);
+    float w0 = 0.f, w1 = 0.f, w2 = 0.f, w3 = 0.f;  // pen, and the op's points (the last: its end)
+    if (form == F_CUBIC) {
+        w0 = __fmul_rn(__fmul_rn(u, u), u);
+        w1 = __fmul_rn(__fmul_rn(3.0f, t), __fmul_rn(u, u));
+        w2 = __fmul_rn(__fmul_rn(3.0f, t), __fmul_rn(t, u));
+        w3 = __fmul_rn(__fmul_rn(t, t), t);
+    } else if (form == F_QUAD) {
+        w0 = __fmul_rn(u, u);
+        w1 = __fmul_rn(__fmul_rn(2.0f, t), u);
+        w3 = __fmul_rn(t, t);
+    } else {
+        w3 = 1.0f;
+    }
+    const float px = run_sum(__fmul_rn(w0, gx), lane, last), py = run_sum(__fmul_rn(w0, gy), lane, last);
+    const float bx = run_sum(__fmul_rn(w1, gx), lane, last), by = run_sum(__fmul_rn(w1, gy), lane, last);
+    const float cx = run_sum(__fmul_rn(w2, gx), lane, last), cy = run_sum(__fmul_rn(w2, gy), lane, last);
+    const float ex = run_sum(__fmul_rn(w3, gx), lane, last), ey = run_sum(__fmul_rn(w3, gy), lane, last);
+    if (!head || op < 0) return;
+    float* g = gops + (size_t)op * 6;
+    const int e = end_slot(load_op(ops, op).kind);
+    atomicAdd(g + 2 * e, ex);
+    atomicAdd(g + 2 * e + 1, ey);
+    if (form == F_POINT) return;
+    atomicAdd(g, bx);
+    atomicAdd(g + 1, by);
+    if (form == F_CUBIC) {
+        atomicAdd(g + 2, cx);
+        atomicAdd(g + 3, cy);
+    }
+    if (pen >= 0) {
+        float* gp = gops + (size_t)pen * 6 + 2 * end_slot(load_op(ops, pen).kind);
+        atomicAdd(gp, px);
+        atomicAdd(gp + 1, py);
+    }
+}
+
+// Vertex gradients to the op floats, back through the transform (d(m*p)/dp = [[m0, m1], [m3, m4]]).
+__device__ void chain_vertices(const AParams& p, const ft_op* ops, int V, const VProv* prov, const float2* vgrad,
+                               float* gops) {
+    const float* m = p.xf;
+    const int lane = threadIdx.x & 31;
+    for (int k0 = threadIdx.x & ~31; k0 < V; k0 += ABLOCK) {
+        const int k = k0 + lane;
+        int4 r = make_int4(-1, -1, 0, 0);
+        float2 g = make_float2(0.f, 0.f);
+        if (k < V) {
+            r = *reinterpret_cast<const int4*>(prov + k);
+            g = __ldcg(&vgrad[k]);  // L2 atomics
+        }
+        const float vx = (r.w & 4) ? g.x : 0.0f, vy = (r.w & 8) ? g.y : 0.0f;
+        int last;
+        const bool head = run_head(r.x, lane, last);
+        chain_point(ops, gops, r.x, r.y, r.w & 3, __int_as_float(r.z),
+                    __fadd_rn(__fmul_rn(m[0], vx), __fmul_rn(m[3], vy)),
+                    __fadd_rn(__fmul_rn(m[1], vx), __fmul_rn(m[4], vy)), head, lane, last);
+    }
 }
 
 __device__ __forceinline__ int2 fxp(const float2* vpos, int k) {
@@ -759,7 +909,6 @@ struct SSub {
 };
 static_assert(sizeof(SPt) == SPT_BYTES && sizeof(SNd) == SND_BYTES && sizeof(SSub) == SSUB_BYTES, "layout");
 enum { N_OFF = 0, N_MITER = 1, N_ARC = 2 };
-enum { F_POINT = 0, F_QUAD = 1, F_CUBIC = 2 };
 
 // The De Casteljau walk carrying widths (geom.rs:31-35): leaf(index, point, width, t).
 template <bool CUBIC, class Leaf>
@@ -862,13 +1011,15 @@ __device__ __forceinline__ StrokeScr stroke_scr(unsigned char* scr) {
 // Every thread must call.
 constexpr int SP_RAW = 65536;  // raw points per window
 static_assert((size_t)SP_RAW * SPT_BYTES <= (size_t)NODE_CAP * SND_BYTES, "raw window fits the node area");
-__device__ int stroke_points_block(const AParams& p, ASmem& sm, const ft_op* ops, int n, float sw0,
+__device__ int stroke_points_block(const AParams& p, ASmem& sm, SlotBuf& Q, const ft_op* ops, int n, float sw0,
                                    const StrokeScr& S, int* n_sub) {
     const int tid = threadIdx.x;
     const float* m = p.xf;
     SPCarry& C = sm.spc;
     SPt* raw = reinterpret_cast<SPt*>(S.nd);
-    int* lpw_of = sm.off;  // per op of the chunk: the last PenWidth op before it
+    // per op of the chunk: the last PenWidth op before it, that of its pen, its close events
+    int *lpw_of = sm.off, *lps_of = sm.off + ABLOCK, *lce_of = sm.off + 2 * ABLOCK;
+    static_assert(ECHUNK >= 3 * ABLOCK, "per-op arrays");
     if (tid == 0) {
         C.pw = C.pc = C.pc_pw = C.ce = -1;
         C.kept = C.nsub = C.have_prev = 0;
@@ -913,14 +1064,16 @@ __device__ int stroke_points_block(const AParams& p, ASmem& sm, const ft_op* ops
         }
         const float sw = sw_at(lpw);
         const int cur_pw = lpw;
+        lps_of[tid] = pen_wsrc;
         // this op's points
         const bool cubic = kind == FT_OP_CUBIC;
         P2 A = p2(0.0f, 0.0f), B = A, Cc = A, D = A;
         float wb = 0.0f, wc = 0.0f, wd = 0.0f;
         bool curve = false;
-        int cnt = 0;
+        int cnt = 0, depth = 0, safe = 0;
         if (kind == FT_OP_MOVE || kind == FT_OP_LINE) {
             cnt = 1;
+            D = xform(m, op_pt(o, 0));
         } else if (kind == FT_OP_QUAD || cubic) {
             A = xform(m, penp);
             B = xform(m, op_pt(o, 0));
@@ -940,19 +1093,53 @@ __device__ int stroke_points_block(const AParams& p, ASmem& sm, const ft_op* ops
                 atomicMax(&sm.status, (int)FT_ERR_ARG);
             } else {
                 curve = true;
-                int dh = 0;
-                auto none = [](int, P2, float, float) {};
-                cnt = cubic ? curve_walk_w<true>(A, B, Cc, D, penw, wb, wc, wd, p.tol_sq, &dh, none)
-                            : curve_walk_w<false>(A, B, Cc, D, penw, wb, wc, wd, p.tol_sq, &dh, none);
-                if (dh) atomicMax(&sm.status, (int)FT_ERR_DEPTH);
+                depth = ftk::curve_depth(A, B, Cc, D, cubic, __fsqrt_rn(p.tol_sq), safe);
             }
         }
-        int total;
-        const int base = block_excl_sum(cnt, sm.wsum, total);
+        // leaves by slots, unless a curve is not known to be flat at depth 12 or the chunk's
+        // slots exceed the raw window
+        const bool deep = __syncthreads_or(depth > ftk::SLOT_DEPTH) != 0;
+        int total = 0, base = 0;
+        bool by_slots = false;
+        if (!deep) {
+            lce_of[tid] = ce;
+            const int form = !curve ? F_POINT : (cubic ? F_CUBIC : F_QUAD);
+            const int slots = list_slots(sm, Q, cnt << depth, A, B, Cc, D, make_float2(penw, sw),
+                                         depth | (safe << 4) | (form << 8) | (tid << 11), pen);
+            by_slots = slots <= SP_RAW;
+            if (by_slots) {
+                int j0 = 0;
+                for (int s0 = 0; s0 < slots; s0 += ABLOCK) {
+                    int j = 0, idx = 0;
+                    P2 q = p2(0.f, 0.f);
+                    float t = 0.f, w = 0.f;
+                    const bool own = slot_leaf<true>(Q, s0 + tid, slots, p.tol_sq, j0, j, idx, q, t, w);
+                    int kept;
+                    const int k = total + block_excl_sum(own ? 1 : 0, sm.wsum, kept);
+                    if (own) {
+                        // the op's PenWidth and close events, and the PenWidth of its pen
+                        const int info = Q.info[j], lt = info >> 11, f = (info >> 8) & 3, pn = Q.src[j];
+                        const int lp = lpw_of[lt];
+                        raw[k] = SPt{q.x, q.y, w, t, c0 + lt, f, f == F_POINT ? -1 : pn,
+                                     f == F_POINT ? lp : lps_of[lt], lp, lce_of[lt]};
+                    }
+                    total += kept;
+                }
+                __syncthreads();
+            }
+        }
+        if (!by_slots && curve) {
+            int dh = 0;
+            auto none = [](int, P2, float, float) {};
+            cnt = cubic ? curve_walk_w<true>(A, B, Cc, D, penw, wb, wc, wd, p.tol_sq, &dh, none)
+                        : curve_walk_w<false>(A, B, Cc, D, penw, wb, wc, wd, p.tol_sq, &dh, none);
+            if (dh) atomicMax(&sm.status, (int)FT_ERR_DEPTH);
+        }
+        if (!by_slots) base = block_excl_sum(cnt, sm.wsum, total);
         for (int w0 = 0; w0 < total; w0 += SP_RAW) {
             const int w1 = min(w0 + SP_RAW, total);
             // ---- this window's raw points; `pad` holds the op's close events
-            if (cnt > 0 && base < w1 && base + cnt > w0) {
+            if (!by_slots && cnt > 0 && base < w1 && base + cnt > w0) {
                 auto put = [&](int k, P2 q, float w, float t, int form, int pn, int ws0) {
                     const int r = base + k;
                     if (r >= w0 && r < w1) raw[r - w0] = SPt{q.x, q.y, w, t, i, form, pn, ws0, cur_pw, ce};
@@ -1048,6 +1235,13 @@ __device__ int stroke_points_block(const AParams& p, ASmem& sm, const ft_op* ops
     __syncthreads();
     *n_sub = nsub;
     return ns;
+}
+
+// The same with slots of its own.
+[[maybe_unused]] __device__ int stroke_points_block(const AParams& p, ASmem& sm, const ft_op* ops, int n, float sw0,
+                                                    const StrokeScr& S, int* n_sub) {
+    __shared__ SlotBuf Q;
+    return stroke_points_block(p, sm, Q, ops, n, sw0, S, n_sub);
 }
 
 // All threads: the outline of every sub-stroke (stroker.rs:239-416) and the polygon
@@ -1362,39 +1556,28 @@ __device__ void stroke_backward_block(const AParams& p, const ft_op* ops, float*
         atomicAdd(&S.spg[nd.b].y, gt.y);
     }
     __syncthreads();
-    auto gw = [&](int src, float v) {
-        if (src < 0)
-            atomicAdd(gwidth, v);
-        else
-            atomicAdd(gops + (size_t)src * 6, v);
-    };
-    for (int k = tid; k < ns; k += ABLOCK) {
-        const SPt q = S.sp[k];
-        const float4 g = __ldcg(&S.spg[k]);
-        const float gx = m[0] * g.x + m[3] * g.y, gy = m[1] * g.x + m[4] * g.y;
-        const int kind = load_op(ops, q.op).kind;
-        auto add = [&](int j, int slot, float wgt) {
-            atomicAdd(gops + (size_t)j * 6 + 2 * slot, wgt * gx);
-            atomicAdd(gops + (size_t)j * 6 + 2 * slot + 1, wgt * gy);
-        };
-        if (q.form == F_POINT) {
-            add(q.op, end_slot(kind), 1.0f);
-            gw(q.w1, g.z);
-            continue;
+    const int lane = tid & 31;
+    for (int k0 = tid & ~31; k0 < ns; k0 += ABLOCK) {
+        const int k = k0 + lane;
+        SPt q{};
+        q.op = -1;
+        float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (k < ns) {
+            q = S.sp[k];
+            g = __ldcg(&S.spg[k]);
         }
-        const float t = q.t, u = 1.0f - t;
-        if (q.form == F_QUAD) {
-            if (q.pen >= 0) add(q.pen, end_slot(load_op(ops, q.pen).kind), u * u);
-            add(q.op, 0, 2.0f * t * u);
-            add(q.op, 1, t * t);
-        } else {
-            if (q.pen >= 0) add(q.pen, end_slot(load_op(ops, q.pen).kind), u * u * u);
-            add(q.op, 0, 3.0f * t * u * u);
-            add(q.op, 1, 3.0f * t * t * u);
-            add(q.op, 2, t * t * t);
+        int last;
+        const bool head = run_head(q.op, lane, last);
+        chain_point(ops, gops, q.op, q.pen, q.form, q.t, m[0] * g.x + m[3] * g.y, m[1] * g.x + m[4] * g.y, head, lane,
+                    last);
+        // widths: linear in t between the pen's and the op's
+        const float t = q.form == F_POINT ? 1.0f : q.t;
+        const float g0 = run_sum((1.0f - t) * g.z, lane, last), g1 = run_sum(t * g.z, lane, last);
+        if (head && q.op >= 0) {
+            auto gw = [&](int src, float v) { atomicAdd(src < 0 ? gwidth : gops + (size_t)src * 6, v); };
+            if (q.form != F_POINT) gw(q.w0, g0);
+            gw(q.w1, g1);
         }
-        gw(q.w0, u * g.z);
-        gw(q.w1, t * g.z);
     }
 }
 
@@ -1443,10 +1626,12 @@ __device__ __forceinline__ float GradAt::operator()(int r, int c) const {
     return __fmul_rn(__fmul_rn(sign, gg), cov_d(rule, *reinterpret_cast<const float*>(ar + o)));
 }
 
+static_assert(sizeof(SlotBuf) <= BAND_FLOATS * sizeof(float), "the slots fit the band");
 template <bool BWD>
 __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
-    extern __shared__ float band[];
+    extern __shared__ __align__(16) float band[];
     __shared__ ASmem sm;
+    SlotBuf& Q = *reinterpret_cast<SlotBuf*>(band);
     unsigned char* scr = p.scratch + (size_t)blockIdx.x * (p.stroke ? A_SCRATCH_STROKE : A_SCRATCH_PER_CTA);
     const StrokeScr S = stroke_scr(scr);
     __shared__ int s_counts[4];
@@ -1454,6 +1639,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
     int* vsub = reinterpret_cast<int*>(scr + AS_SUB);
     float2* vgrad = reinterpret_cast<float2*>(scr + AS_GRAD);
     int* vflag = reinterpret_cast<int*>(scr + AS_FLAG);
+    VProv* prov = reinterpret_cast<VProv*>(scr + AS_PROV);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (uint32_t path = blockIdx.x; path < p.n_paths; path += gridDim.x) {
         const ft_path_desc d = p.paths[path];
@@ -1464,7 +1650,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
         int V;
         if (p.stroke) {
             int nsub = 0;
-            const int ns = stroke_points_block(p, sm, ops, (int)d.n_ops, d.s_width, S, &nsub);
+            const int ns = stroke_points_block(p, sm, Q, ops, (int)d.n_ops, d.s_width, S, &nsub);
             if (tid == 0) {
                 s_counts[2] = ns;
                 s_counts[0] = nsub;
@@ -1484,7 +1670,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
                 for (int k = tid; k < min(V, VCAP); k += ABLOCK) vgrad[k] = make_float2(0.0f, 0.0f);
             __syncthreads();
         } else {
-            V = path_walk<WALK_EMIT>(p, sm, ops, (int)d.n_ops, vpos, vsub, vgrad, BWD, nullptr);
+            V = path_walk(p, sm, Q, ops, (int)d.n_ops, vpos, vsub, vgrad, BWD ? prov : nullptr);
         }
         const bool cap = V > VCAP || (p.stroke && sm.status == FT_ERR_CAP);
         if (cap && tid == 0) atomicMax(&sm.status, (int)FT_ERR_CAP);
@@ -1577,8 +1763,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
                 stroke_backward_block(p, ops, p.grad_ops + (size_t)d.op_begin * 6, p.grad_width + path, V,
                                       s_counts[1], s_counts[2], s_counts[3], S, vgrad);
             } else {
-                path_walk<WALK_GRAD>(p, sm, ops, (int)d.n_ops, vpos, vsub, vgrad, false,
-                                     p.grad_ops + (size_t)d.op_begin * 6);
+                chain_vertices(p, ops, V, prov, vgrad, p.grad_ops + (size_t)d.op_begin * 6);
             }
         }
         if (tid == 0) p.status[path] = sm.status;
@@ -1593,7 +1778,7 @@ int adjoint_blocks_per_sm(bool backward) {
     const int smem = BAND_FLOATS * (int)sizeof(float);
     int n = 0;
     if (backward) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adjoint<true>, ABLOCK, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adjoint<true>, ABLOCK, (int)sizeof(SlotBuf));
     } else {
         cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adjoint<false>, ABLOCK, smem);
@@ -1604,7 +1789,7 @@ int adjoint_blocks_per_sm(bool backward) {
 cudaError_t launch_adjoint(bool backward, const AParams& p, int grid, cudaStream_t s) {
     const int smem = BAND_FLOATS * (int)sizeof(float);
     if (backward) {
-        k_adjoint<true><<<grid, ABLOCK, 0, s>>>(p);
+        k_adjoint<true><<<grid, ABLOCK, sizeof(SlotBuf), s>>>(p);
     } else {
         cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         k_adjoint<false><<<grid, ABLOCK, smem, s>>>(p);
