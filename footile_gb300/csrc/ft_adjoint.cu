@@ -617,9 +617,8 @@ __device__ float fig_sign(ASmem& sm, int V, const float2* vpos, const int* vsub,
 // One edge, top end a, bottom end b (a.y < b.y).
 struct EdgeG {
     P2 a, b;
-    float dy, dxdy, xlo, xhi;
+    float dxdy;
     float dir;   // +1 when the edge runs down (P0 on top), -1 up
-    P2 perp;     // (-dy, dx) of P1 - P0
     int e, nxt;
     bool ok;
 };
@@ -639,11 +638,7 @@ __device__ __forceinline__ EdgeG make_edge(const float2* vpos, const int* vsub, 
     E.a = down ? p0 : p1;
     E.b = down ? p1 : p0;
     E.dir = down ? 1.0f : -1.0f;
-    E.dy = __fsub_rn(E.b.y, E.a.y);
-    E.dxdy = __fdiv_rn(__fsub_rn(E.b.x, E.a.x), E.dy);
-    E.xlo = fminf(E.a.x, E.b.x);
-    E.xhi = fmaxf(E.a.x, E.b.x);
-    E.perp = p2(-__fsub_rn(p1.y, p0.y), __fsub_rn(p1.x, p0.x));
+    E.dxdy = __fdiv_rn(__fsub_rn(E.b.x, E.a.x), __fsub_rn(E.b.y, E.a.y));
     return E;
 }
 
@@ -657,55 +652,24 @@ __device__ __forceinline__ int edge_rows(const EdgeG& E, int b0, int b1, int* r0
     return (int)f1 - (int)f0 + 1;
 }
 
-// Pieces of the edge in raster row r, cell by cell: cb(cell, h, xmid, u0, u1); cell -1
-// is everything left of the raster; cells at or right of W are dropped.
-template <class CB>
-__device__ __forceinline__ void row_pieces(const EdgeG& E, int r, int W, CB cb) {
-    const float yt = fmaxf(E.a.y, (float)r), yb = fminf(E.b.y, (float)(r + 1));
-    if (!(yb > yt)) return;
-    const float xt = yt == E.a.y ? E.a.x
-                                 : fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(yt, E.a.y), E.dxdy)), E.xlo), E.xhi);
-    const float xb = yb == E.b.y ? E.b.x
-                                 : fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(yb, E.a.y), E.dxdy)), E.xlo), E.xhi);
-    const float ut = __fdiv_rn(__fsub_rn(yt, E.a.y), E.dy), ub = __fdiv_rn(__fsub_rn(yb, E.a.y), E.dy);
-    const float h = __fsub_rn(yb, yt);
-    const float xl = fminf(xt, xb), xr = fmaxf(xt, xb);
-    const bool rising = xt <= xb;
-    const float cl = floorf(xl), cr = floorf(xr);
-    if (cl == cr || xr == xl) {
-        if (cl < (float)W) cb(cl < 0.0f ? -1 : (int)cl, h, __fmul_rn(__fadd_rn(xl, xr), 0.5f), ut, ub);
-        return;
-    }
-    const float span = __fsub_rn(xr, xl), du = __fsub_rn(ub, ut);
-    auto piece = [&](float x0, float x1, int c) {
-        const float f0 = __fdiv_rn(__fsub_rn(x0, xl), span), f1 = __fdiv_rn(__fsub_rn(x1, xl), span);
-        const float u0 = rising ? __fadd_rn(ut, __fmul_rn(f0, du)) : __fsub_rn(ub, __fmul_rn(f1, du));
-        const float u1 = rising ? __fadd_rn(ut, __fmul_rn(f1, du)) : __fsub_rn(ub, __fmul_rn(f0, du));
-        cb(c, __fmul_rn(__fsub_rn(f1, f0), h), __fmul_rn(__fadd_rn(x0, x1), 0.5f), u0, u1);
-    };
-    float c = cl;
-    if (c < 0.0f) {
-        const float x1 = fminf(xr, 0.0f);
-        if (x1 > xl) piece(xl, x1, -1);
-        c = 0.0f;
-    }
-    const float cend = fminf(cr, (float)(W - 1));
-    for (; c <= cend; c = __fadd_rn(c, 1.0f)) {
-        const float x0 = fmaxf(xl, c), x1 = fminf(xr, __fadd_rn(c, 1.0f));
-        if (x1 > x0) piece(x0, x1, (int)c);
-    }
+// The part of an edge in raster row r: its y range [yt, yb] and the x it has there (xt at yt,
+// xb at yb, inside the edge's own x range).  False when the row has none of it.
+__device__ __forceinline__ bool row_span(P2 a, P2 b, float dxdy, int r, float& yt, float& yb, float& xt, float& xb) {
+    yt = fmaxf(a.y, (float)r);
+    yb = fminf(b.y, (float)(r + 1));
+    if (!(yb > yt)) return false;
+    const float xlo = fminf(a.x, b.x), xhi = fmaxf(a.x, b.x);
+    xt = yt == a.y ? a.x : fminf(fmaxf(__fadd_rn(a.x, __fmul_rn(__fsub_rn(yt, a.y), dxdy)), xlo), xhi);
+    xb = yb == b.y ? b.x : fminf(fmaxf(__fadd_rn(a.x, __fmul_rn(__fsub_rn(yb, a.y), dxdy)), xlo), xhi);
+    return true;
 }
 
-// Forward pieces of the edge in raster row r: cb(cell, h, xmid) as row_pieces gives
-// them, with one division per row (the height per unit of x) instead of two per piece.
+// Pieces of the edge in raster row r, cell by cell: cb(cell, h, xmid); cell -1 is everything
+// left of the raster; cells at or right of W are dropped.
 template <class CB>
 __device__ __forceinline__ void row_cells(const EdgeG& E, int r, int W, CB cb) {
-    const float yt = fmaxf(E.a.y, (float)r), yb = fminf(E.b.y, (float)(r + 1));
-    if (!(yb > yt)) return;
-    const float xt = yt == E.a.y ? E.a.x
-                                 : fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(yt, E.a.y), E.dxdy)), E.xlo), E.xhi);
-    const float xb = yb == E.b.y ? E.b.x
-                                 : fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(yb, E.a.y), E.dxdy)), E.xlo), E.xhi);
+    float yt, yb, xt, xb;
+    if (!row_span(E.a, E.b, E.dxdy, r, yt, yb, xt, xb)) return;
     const float h = __fsub_rn(yb, yt);
     const float xl = fminf(xt, xb), xr = fmaxf(xt, xb);
     const float cl = floorf(xl), cr = floorf(xr);
@@ -730,17 +694,13 @@ __device__ __forceinline__ void row_cells(const EdgeG& E, int r, int W, CB cb) {
     }
 }
 
-// All (edge, row) items of rows [b0, b0 + nb) of the path: forward adds cell areas to
-// the band, backward accumulates the edge integrals against g = gv(row, cell) (the
-// loss gradient times dcov/dS at that cell).  The edges visited are elist[0 .. n_e)
-// (the band's binned edges), or 0 .. n_e - 1 when elist is null.
-struct NoG {
-    __device__ float operator()(int, int) const { return 0.0f; }
-    __device__ void prefetch(int, int) const {}
-};
-template <bool BWD, class GV = NoG>
-__device__ void band_edges(ASmem& sm, float* band, int W, int b0, int nb, int V, const float2* vpos,
-                           const int* vsub, float2* vgrad, const int* elist, int n_e, GV gv = GV()) {
+// Forward: the (edge, row) items of rows [b0, b0 + nb) add their cell areas to the band.  The
+// edges visited are elist[0 .. n_e) (the band's binned edges), or 0 .. n_e - 1 when elist is
+// null.  Items go to threads in contiguous ranges: a cell's areas are float sums, and an order
+// of its own decides on which side of a kink of the fill rule a pixel of no area falls (spread
+// as the backward's, the forward gains 20 %, but such pixels of earlier results move).
+__device__ void band_areas(ASmem& sm, float* band, int W, int b0, int nb, int V, const float2* vpos, const int* vsub,
+                           const int* elist, int n_e) {
     const int tid = threadIdx.x;
     const int b1 = b0 + nb - 1;
     auto edge_at = [&](int i) { return elist ? elist[i] : i; };
@@ -778,16 +738,8 @@ __device__ void band_edges(ASmem& sm, float* band, int W, int b0, int nb, int V,
             EdgeG E = make_edge(vpos, vsub, V, edge_at(e0 + slot));
             int r0 = 0;
             edge_rows(E, b0, b1, &r0);
-            float ga = 0.0f, gb = 0.0f;
             for (int it = beg; it < end; it++) {
                 if (sm.off[slot + 1] <= it) {
-                    if (BWD) {
-                        atomicAdd(&vgrad[E.e].x, __fmul_rn(E.perp.x, ga));
-                        atomicAdd(&vgrad[E.e].y, __fmul_rn(E.perp.y, ga));
-                        atomicAdd(&vgrad[E.nxt].x, __fmul_rn(E.perp.x, gb));
-                        atomicAdd(&vgrad[E.nxt].y, __fmul_rn(E.perp.y, gb));
-                        ga = gb = 0.0f;
-                    }
                     do {
                         slot++;
                     } while (sm.off[slot + 1] <= it);
@@ -795,50 +747,119 @@ __device__ void band_edges(ASmem& sm, float* band, int W, int b0, int nb, int V,
                     edge_rows(E, b0, b1, &r0);
                 }
                 const int r = r0 + (it - sm.off[slot]);
-                if (!BWD) {
-                    float* row = band + (size_t)(r - b0) * W;
-                    row_cells(E, r, W, [&](int c, float h, float xm) {
-                        const float dh = __fmul_rn(E.dir, h);
-                        if (c < 0) {
-                            atomicAdd(row, dh);
-                        } else {
-                            atomicAdd(row + c, __fmul_rn(dh, __fsub_rn((float)(c + 1), xm)));
-                            if (c + 1 < W) atomicAdd(row + c + 1, __fmul_rn(dh, __fsub_rn(xm, (float)c)));
-                        }
-                    });
-                } else {
-                    // the next item is usually this edge one row down: ask L1 for its cells now
-                    if (r + 1 <= b1 && (float)(r + 1) < E.b.y) {
-                        const float y0 = (float)(r + 1), y1 = fminf(E.b.y, (float)(r + 2));
-                        const float xa = fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(y0, E.a.y), E.dxdy)), E.xlo), E.xhi);
-                        const float xb = fminf(fmaxf(__fadd_rn(E.a.x, __fmul_rn(__fsub_rn(y1, E.a.y), E.dxdy)), E.xlo), E.xhi);
-                        const float lo = fminf(xa, xb), hi = fmaxf(xa, xb);
-                        if (hi >= 0.0f && lo < (float)W) {
-                            const int c0 = max((int)floorf(lo), 0), c1 = min((int)floorf(hi), W - 1);
-                            gv.prefetch(r + 1, c0);
-                            if ((c1 >> 5) != (c0 >> 5)) gv.prefetch(r + 1, c1);
-                        }
+                float* row = band + (size_t)(r - b0) * W;
+                row_cells(E, r, W, [&](int c, float h, float xm) {
+                    const float dh = __fmul_rn(E.dir, h);
+                    if (c < 0) {
+                        atomicAdd(row, dh);
+                    } else {
+                        atomicAdd(row + c, __fmul_rn(dh, __fsub_rn((float)(c + 1), xm)));
+                        if (c + 1 < W) atomicAdd(row + c + 1, __fmul_rn(dh, __fsub_rn(xm, (float)c)));
                     }
-                    const bool down = E.dir > 0.0f;
-                    row_pieces(E, r, W, [&](int c, float, float, float u0, float u1) {
-                        if (c < 0) return;
-                        const float g = gv(r, c);
-                        const float i1 = __fsub_rn(u1, u0);
-                        const float iu = __fmul_rn(__fmul_rn(0.5f, i1), __fadd_rn(u1, u0));
-                        const float i0 = __fsub_rn(i1, iu);
-                        ga = __fadd_rn(ga, __fmul_rn(g, down ? i0 : iu));
-                        gb = __fadd_rn(gb, __fmul_rn(g, down ? iu : i0));
-                    });
-                }
-            }
-            if (BWD) {
-                atomicAdd(&vgrad[E.e].x, __fmul_rn(E.perp.x, ga));
-                atomicAdd(&vgrad[E.e].y, __fmul_rn(E.perp.y, ga));
-                atomicAdd(&vgrad[E.nxt].x, __fmul_rn(E.perp.x, gb));
-                atomicAdd(&vgrad[E.nxt].y, __fmul_rn(E.perp.y, gb));
+                });
             }
         }
         __syncthreads();
+    }
+}
+
+// Backward: the edge integrals of every (edge, row) item of the path against g = gv(row, cell)
+// (the loss gradient times dcov/dS at that cell), into the vertex gradients.
+//
+// A warp takes 32 edges at a time: each lane works one out, then the (edge, row) items are
+// spread over the lanes, a row that crosses many cells as several items of PIECES cells, so
+// that no lane waits for a shallow edge's walk; an item takes its edge's values by shuffles,
+// loads g for all of its cells before using any, divides once per row, and its integrals are
+// summed over the items of its edge in the warp before the four atomics per edge.
+constexpr int PIECES = 4;
+template <class GV>
+__device__ void edge_integrals(int W, int H, int V, const float2* vpos, const int* vsub, float2* vgrad, GV gv) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int g = warp * 32; g < V; g += ABLOCK) {
+        EdgeG E;
+        E.e = E.nxt = 0;
+        E.a = E.b = p2(0.f, 0.f);
+        E.dxdy = E.dir = 0.f;
+        E.ok = false;
+        int r0 = 0, ls = 0, n = 0;
+        if (g + lane < V) {
+            E = make_edge(vpos, vsub, V, g + lane);
+            n = edge_rows(E, 0, H - 1, &r0);
+            // cells a row can cross: the slope's run and two, or the edge's own width
+            const float run = fminf(fminf(fabsf(E.dxdy), fabsf(__fsub_rn(E.b.x, E.a.x))), (float)W);
+            const int cells = (int)run + 3;
+            ls = cells <= PIECES ? 0 : 32 - __clz((cells - 1) / PIECES);
+            if (n == 0) E.a = E.b = p2(0.f, 0.f);  // one item without a row: every edge has some
+        }
+        const int items = g + lane < V ? max(n << ls, 1) : 0;
+        const int packed = r0 | (ls << 24);
+        int inc = warp_incl_sum(items);
+        const int off = inc - items, tot = __shfl_sync(FULL, inc, 31);
+        for (int w0 = 0; w0 < tot; w0 += 32) {
+            // the edge of item w0 + lane: the last that starts at or before it
+            const int rel = off - w0;
+            const unsigned at = __reduce_or_sync(FULL, (items > 0 && rel >= 0 && rel < 32) ? 1u << rel : 0u);
+            const int before = __popc(__ballot_sync(FULL, items > 0 && rel < 0));
+            const int j = before + __popc(at & (FULL >> (31 - lane))) - 1;
+            const P2 a = p2(__shfl_sync(FULL, E.a.x, j), __shfl_sync(FULL, E.a.y, j));
+            const P2 b = p2(__shfl_sync(FULL, E.b.x, j), __shfl_sync(FULL, E.b.y, j));
+            const float dxdy = __shfl_sync(FULL, E.dxdy, j), dir = __shfl_sync(FULL, E.dir, j);
+            const int pk = __shfl_sync(FULL, packed, j), oj = __shfl_sync(FULL, off, j);
+            const int it = w0 + lane - oj, lj = pk >> 24, r = (pk & 0xFFFFFF) + (it >> lj);
+            const int c0 = (it & ((1 << lj) - 1)) * PIECES;  // first of this item's cells in the row
+            float yt, yb, xt, xb;
+            const bool on = w0 + lane < tot && row_span(a, b, dxdy, r, yt, yb, xt, xb);
+            float ga = 0.0f, gb = 0.0f;
+            if (on) {
+                const float xl = fminf(xt, xb), xr = fmaxf(xt, xb);
+                const float cl = floorf(xl), cr = floorf(xr);
+                const bool one = cl == cr || xr == xl;  // one cell
+                const int first = cl < 0.0f ? 0 : (cl < (float)W ? (int)cl : W);  // cells from the raster's left on
+                const int end = one ? (cl < 0.0f ? -1 : first) : (int)fminf(cr, (float)(W - 1));
+                // the edge's parameter along x: u(x) = ut or ub at xl, du / span per pixel
+                const float dy = __fsub_rn(b.y, a.y);
+                const float ut = __fdiv_rn(__fsub_rn(yt, a.y), dy), ub = __fdiv_rn(__fsub_rn(yb, a.y), dy);
+                const float du = __fsub_rn(ub, ut);
+                const bool rising = xt <= xb, down = dir > 0.0f;
+                const float k = one ? 0.0f : __fdiv_rn(du, __fsub_rn(xr, xl));
+                float gs[PIECES];
+#pragma unroll
+                for (int u = 0; u < PIECES; u++) {
+                    const int c = first + c0 + u;
+                    gs[u] = c <= end && c < W ? gv(r, c) : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < PIECES; u++) {
+                    const float c = (float)(first + c0 + u);
+                    const float x0 = fmaxf(xl, c), x1 = fminf(xr, __fadd_rn(c, 1.0f));
+                    const float i1 = one ? du : __fmul_rn(fmaxf(__fsub_rn(x1, x0), 0.0f), k);
+                    // (differences from xl first: they are exact, a midpoint of x0 and x1 is not)
+                    const float d = __fmul_rn(__fmul_rn(0.5f, __fadd_rn(__fsub_rn(x0, xl), __fsub_rn(x1, xl))), k);
+                    const float um = one ? __fmul_rn(0.5f, __fadd_rn(ut, ub))
+                                         : (rising ? __fadd_rn(ut, d) : __fsub_rn(ub, d));
+                    const float iu = __fmul_rn(i1, um), i0 = __fsub_rn(i1, iu);
+                    if (gs[u] != 0.0f) {
+                        ga = __fadd_rn(ga, __fmul_rn(gs[u], down ? i0 : iu));
+                        gb = __fadd_rn(gb, __fmul_rn(gs[u], down ? iu : i0));
+                    }
+                }
+            }
+            const int key = w0 + lane < tot ? j : 32;
+            int last;
+            const bool head = run_head(key, lane, last);
+            ga = run_sum(ga, lane, last);
+            gb = run_sum(gb, lane, last);
+            const int e = __shfl_sync(FULL, E.e, j), nxt = __shfl_sync(FULL, E.nxt, j);
+            if (head && key < 32 && (ga != 0.0f || gb != 0.0f)) {
+                // (-dy, dx) of the edge as it runs
+                const float px = dir > 0.0f ? -__fsub_rn(b.y, a.y) : __fsub_rn(b.y, a.y);
+                const float py = dir > 0.0f ? __fsub_rn(b.x, a.x) : -__fsub_rn(b.x, a.x);
+                atomicAdd(&vgrad[e].x, __fmul_rn(px, ga));
+                atomicAdd(&vgrad[e].y, __fmul_rn(py, ga));
+                atomicAdd(&vgrad[nxt].x, __fmul_rn(px, gb));
+                atomicAdd(&vgrad[nxt].y, __fmul_rn(py, gb));
+            }
+        }
     }
 }
 
@@ -1019,7 +1040,6 @@ __device__ int stroke_points_block(const AParams& p, ASmem& sm, SlotBuf& Q, cons
     SPt* raw = reinterpret_cast<SPt*>(S.nd);
     // per op of the chunk: the last PenWidth op before it, that of its pen, its close events
     int *lpw_of = sm.off, *lps_of = sm.off + ABLOCK, *lce_of = sm.off + 2 * ABLOCK;
-    static_assert(ECHUNK >= 3 * ABLOCK, "per-op arrays");
     if (tid == 0) {
         C.pw = C.pc = C.pc_pw = C.ce = -1;
         C.kept = C.nsub = C.have_prev = 0;
@@ -1605,11 +1625,6 @@ struct GradAt {
     bool no_area;
     __device__ size_t at(int r, int c) const { return off + (size_t)r * stride + 4 * (size_t)c; }
     __device__ float operator()(int r, int c) const;
-    __device__ void prefetch(int r, int c) const {
-        const size_t o = at(r, c);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(g + o));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"((no_area ? cv : ar) + o));
-    }
 };
 
 __device__ __forceinline__ float* px_at(float* base, const ft_path_desc& d, int r) {
@@ -1685,7 +1700,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
                 GradAt gv{reinterpret_cast<const char*>(p.grad_cov), reinterpret_cast<const char*>(p.cov),
                           reinterpret_cast<const char*>(p.area), d.raster_offset, d.stride, sign, p.rule,
                           p.no_area != 0};
-                band_edges<true>(sm, nullptr, W, 0, H, V, vpos, vsub, vgrad, nullptr, V, gv);
+                edge_integrals(W, H, V, vpos, vsub, vgrad, gv);
             }
             __syncthreads();
         }
@@ -1716,7 +1731,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
             }
             for (int i = tid; i < nc; i += ABLOCK) band[i] = 0.0f;
             __syncthreads();
-            if (!cap) band_edges<false>(sm, band, W, b0, nb, V, vpos, vsub, vgrad, binned ? blist + e_lo : nullptr, n_e);
+            if (!cap) band_areas(sm, band, W, b0, nb, V, vpos, vsub, binned ? blist + e_lo : nullptr, n_e);
             {
                 __syncthreads();
                 // row prefix sums, four 32-cell chunks scanned side by side; the float
