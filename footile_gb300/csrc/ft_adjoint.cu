@@ -1320,13 +1320,14 @@ __device__ void outline_block(const AParams& p, const StrokeScr& S, int nsub, AS
         g.fwd = u < g.len;
         g.k = g.fwd ? u : u - g.len;
         const int n = sb.n;
-        if (g.fwd) {
-            g.v0 = sb.start + g.k % n;
-            g.v1 = sb.start + (g.k + 1) % n;
-        } else {  // from the last point backwards (stroker.rs:244-246)
-            g.v0 = sb.start + ((n - 1 - g.k) % n + n) % n;
-            g.v1 = sb.start + ((n - 2 - g.k) % n + n) % n;
-        }
+        auto at = [&](int v) {  // v mod n, a turn or two away at most
+            while (v >= n) v -= n;
+            while (v < 0) v += n;
+            return sb.start + v;
+        };
+        // the reverse side runs from the last point backwards (stroker.rs:244-246)
+        g.v0 = at(g.fwd ? g.k : n - 1 - g.k);
+        g.v1 = at(g.fwd ? g.k + 1 : n - 2 - g.k);
         return g;
     };
     auto P = [&](int k) { return p2(S.sp[k].x, S.sp[k].y); };
@@ -1513,15 +1514,18 @@ __device__ void stroke_backward_block(const AParams& p, const ft_op* ops, float*
     // Miter intersections.  Their four offset points are recomputed from the stroke
     // points in double: between very short segments the float offsets' rounding is a
     // large part of the offset lines' directions, and the intersection's Jacobian
-    // amplifies it.
-    auto off64 = [&](int id, double& x, double& y) {
+    // amplifies it.  (a0, a1) and (b0, b1) are the two ends of one segment each, moved along
+    // its one normal: one reciprocal square root per segment and one division per join.
+    struct Off64 {
+        double x0, y0, x1, y1;
+    };
+    auto off64 = [&](int id) {
         const SNd o = S.nd[id];  // an offset node: stroke points a -> b
-        const double fx = S.sp[o.a].x, fy = S.sp[o.a].y, tx = S.sp[o.b].x, ty = S.sp[o.b].y;
-        const double ux = ty - fy, uy = -(tx - fx), len = sqrt(ux * ux + uy * uy);
-        const int ks = o.c ? o.b : o.a;
-        const double hw = 0.5 * (double)S.sp[ks].w;
-        x = (double)S.sp[ks].x + ux / len * hw;
-        y = (double)S.sp[ks].y + uy / len * hw;
+        const SPt f = S.sp[o.a], t = S.sp[o.b];
+        const double ux = (double)t.y - (double)f.y, uy = (double)f.x - (double)t.x;
+        const double inv = 0.5 * rsqrt(ux * ux + uy * uy);
+        const double hx = ux * inv, hy = uy * inv;
+        return Off64{f.x + hx * f.w, f.y + hy * f.w, t.x + hx * t.w, t.y + hy * t.w};
     };
     for (int i = n_off + tid; i < nn; i += ABLOCK) {
         const SNd nd = S.nd[i];
@@ -1531,28 +1535,18 @@ __device__ void stroke_backward_block(const AParams& p, const ft_op* ops, float*
         // intersection of lines a0-a1 and b0-b1 in coordinates relative to a1:
         // x = a1 + (B / D) * (a1 - a0), u = a0 - a1, v3 = b0 - a1, v4 = b1 - a1,
         // D = u x (v3 - v4), B = v3 x v4
-        double a0x, a0y, ax, ay, b0x, b0y, b1x, b1y;
-        off64(nd.a, a0x, a0y);
-        off64(nd.b, ax, ay);
-        off64(nd.c, b0x, b0y);
-        off64(nd.d, b1x, b1y);
+        const Off64 A = off64(nd.a), B = off64(nd.c);
         const double gx = gf.x, gy = gf.y;
-        const double ux = a0x - ax, uy = a0y - ay;
-        const double v3x = b0x - ax, v3y = b0y - ay;
-        const double v4x = b1x - ax, v4y = b1y - ay;
-        const double den = ux * (v3y - v4y) - uy * (v3x - v4x);
-        const double bb = v3x * v4y - v3y * v4x;
-        const double q = bb / den;
-        double gux = -q * gx, guy = -q * gy;
-        const double gq = -(ux * gx + uy * gy);
-        const double gb = gq / den, gden = -gq * q / den;
-        double g3x = gb * v4y, g3y = -gb * v4x, g4x = -gb * v3y, g4y = gb * v3x;
-        gux += gden * (v3y - v4y);
-        guy -= gden * (v3x - v4x);
-        g3y += gden * ux;
-        g4y -= gden * ux;
-        g3x -= gden * uy;
-        g4x += gden * uy;
+        const double ux = A.x0 - A.x1, uy = A.y0 - A.y1;
+        const double v3x = B.x0 - A.x1, v3y = B.y0 - A.y1;
+        const double v4x = B.x1 - A.x1, v4y = B.y1 - A.y1;
+        const double wx = v3x - v4x, wy = v3y - v4y;
+        const double rden = 1.0 / (ux * wy - uy * wx);
+        const double q = (v3x * v4y - v3y * v4x) * rden;
+        const double gb = -(ux * gx + uy * gy) * rden, gden = -gb * q;
+        const double gux = gden * wy - q * gx, guy = -gden * wx - q * gy;
+        const double g3x = gb * v4y - gden * uy, g3y = gden * ux - gb * v4x;
+        const double g4x = gden * uy - gb * v3y, g4y = gb * v3x - gden * ux;
         atomicAdd(&S.ng[nd.a].x, (float)gux);
         atomicAdd(&S.ng[nd.a].y, (float)guy);
         atomicAdd(&S.ng[nd.c].x, (float)g3x);
@@ -1563,17 +1557,37 @@ __device__ void stroke_backward_block(const AParams& p, const ft_op* ops, float*
         atomicAdd(&S.ng[nd.b].y, (float)(gy - guy - g3y - g4y));
     }
     __syncthreads();
-    for (int i = tid; i < min(nn, n_off); i += ABLOCK) {
-        const SNd nd = S.nd[i];
-        if (nd.kind != N_OFF) continue;
-        const float2 g = __ldcg(&S.ng[i]);
-        if (g.x == 0.0f && g.y == 0.0f) continue;
-        float2 gf, gt;
-        offset_back(g, S.sp[nd.a].x, S.sp[nd.a].y, S.sp[nd.b].x, S.sp[nd.b].y, nd.c ? nd.b : nd.a, &gf, &gt);
-        atomicAdd(&S.spg[nd.a].x, gf.x);
-        atomicAdd(&S.spg[nd.a].y, gf.y);
-        atomicAdd(&S.spg[nd.b].x, gt.x);
-        atomicAdd(&S.spg[nd.b].y, gt.y);
+    // offset nodes 2 s and 2 s + 1: the two ends of segment s, one direction, their gradients
+    // summed per stroke point
+    for (int sg = tid; sg < min(nn, n_off) / 2; sg += ABLOCK) {
+        const float2 g0 = __ldcg(&S.ng[2 * sg]), g1 = __ldcg(&S.ng[2 * sg + 1]);
+        if (g0.x == 0.0f && g0.y == 0.0f && g1.x == 0.0f && g1.y == 0.0f) continue;
+        const SNd nd = S.nd[2 * sg];
+        const SPt f = S.sp[nd.a], t = S.sp[nd.b];
+        const float ux = t.y - f.y, uy = -(t.x - f.x);
+        const float len = sqrtf(ux * ux + uy * uy);
+        const float vx = ux / len, vy = uy / len;
+        float gfx = 0.0f, gfy = 0.0f, gtx = 0.0f, gty = 0.0f;
+        auto end = [&](float2 g, float w, float& gx, float& gy) {  // one end's own point and width, and the direction
+            if (g.x == 0.0f && g.y == 0.0f) return 0.0f;
+            gx += g.x;
+            gy += g.y;
+            const float gvx = g.x * w * 0.5f, gvy = g.y * w * 0.5f;
+            const float dv = vx * gvx + vy * gvy;
+            const float gux = (gvx - vx * dv) / len, guy = (gvy - vy * dv) / len;
+            gtx += -guy;  // u = (d.y, -d.x), d = to - from
+            gty += gux;
+            gfx += guy;
+            gfy += -gux;
+            return 0.5f * (vx * g.x + vy * g.y);
+        };
+        const float w0 = end(g0, f.w, gfx, gfy), w1 = end(g1, t.w, gtx, gty);
+        atomicAdd(&S.spg[nd.a].x, gfx);
+        atomicAdd(&S.spg[nd.a].y, gfy);
+        atomicAdd(&S.spg[nd.a].z, w0);
+        atomicAdd(&S.spg[nd.b].x, gtx);
+        atomicAdd(&S.spg[nd.b].y, gty);
+        atomicAdd(&S.spg[nd.b].z, w1);
     }
     __syncthreads();
     const int lane = tid & 31;
@@ -1729,7 +1743,7 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
                 }
                 continue;
             }
-            for (int i = tid; i < nc; i += ABLOCK) band[i] = 0.0f;
+            for (int i = 4 * tid; i < nc; i += 4 * ABLOCK) *reinterpret_cast<float4*>(band + i) = make_float4(0.f, 0.f, 0.f, 0.f);
             __syncthreads();
             if (!cap) band_areas(sm, band, W, b0, nb, V, vpos, vsub, binned ? blist + e_lo : nullptr, n_e);
             {
