@@ -183,6 +183,13 @@ int grid_cap(const ft_ctx* c, int per_sm) {
 // Most cells of a tile band when there are few paths (96 KB: a row range is one band).
 constexpr int TILE_AREA_FEW = 24576;
 
+// Cells of a band for row ranges of `rows` rows: the whole range up to TILE_AREA_FEW, a row at
+// least.
+int few_area(int width, int rows) {
+    const int pitch = ftk::tile_pitch(width);
+    return std::max(pitch, (int)std::min<uint64_t>((uint64_t)pitch * rows, TILE_AREA_FEW));
+}
+
 // Work items of the device queues: fills of small canvases go to the tile rasteriser
 // (out_w), whole in a batch and by row ranges when there are few paths; large canvases and
 // strokes go to the CTA rasteriser, split into row ranges of whole bands from split_px.
@@ -217,11 +224,8 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
             rows_per_item = std::max(16u, (d.height + parts - 1) / parts);
         }
         const bool tiled = few && !big && wside > 0;
-        if (tiled) {
-            const int pitch = ftk::tile_pitch((int)d.width);
-            const uint64_t want = (uint64_t)pitch * std::min(rows_per_item, std::max(d.height, 1u));
-            tile.few_area = std::max(tile.few_area, std::max(pitch, (int)std::min<uint64_t>(want, TILE_AREA_FEW)));
-        }
+        if (tiled)
+            tile.few_area = std::max(tile.few_area, few_area((int)d.width, (int)std::min(rows_per_item, std::max(d.height, 1u))));
         for (uint32_t r = 0; r < std::max(d.height, 1u); r += rows_per_item)
             (tiled ? out_w : out).push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
     }
@@ -312,6 +316,9 @@ cudaError_t enqueue(const ftk::KParams& p, const ftk::TilePlan& t, int grid_b, i
         q.host_rasters = p.host_rasters;
         q.rule = p.rule;
         q.fmt = p.fmt;
+        q.single = p.single;
+        q.rows_per = p.rows_per;
+        q.d = p.d;
         for (int i = 0; i < 6; i++) q.xf[i] = p.xf[i];
         q.tol = p.tol;
         q.tol_sq = p.tol_sq;
@@ -320,7 +327,7 @@ cudaError_t enqueue(const ftk::KParams& p, const ftk::TilePlan& t, int grid_b, i
         (*launches)++;
     }
     if (p.n_items || p.n_items_w) {
-        e = ftk::launch_raster(p, grid_b, smem, st, grid_b <= sm_count);
+        e = ftk::launch_raster(p, grid_b, smem, st, grid_b <= sm_count, p.single && p.n_items_w);
         if (e == cudaSuccess) (*launches)++;
     }
     return e;
@@ -410,6 +417,47 @@ int run(ft_ctx* c, int stroke, int rule, const ft_op* ops_d, const ft_path_desc*
                     static_cast<int32_t*>(c->status.p), true, host_rasters);
 }
 
+// One path (ft_fill, ft_stroke) below split_px: row ranges of it, one CTA each.  A call this
+// small is bound by its launches: the path travels in the launch itself, so nothing is
+// uploaded or reset, and k_raster is set up while k_tile runs.  Every CTA rebuilds the figure,
+// which bounds how low the ranges go.  256 x 256 fill / 97 x 61 stroke, us: planned, uploaded
+// and drawn from the queue in ranges of 16 rows 29.6 / 33.4; this way in ranges of 16 rows
+// 21.4 / 27.8, 8 rows 20.5 / 26.6, 4 rows 20.8 / 29.1.
+int run_single(ft_ctx* c, int stroke, int rule, const ft_op* ops_d, const ft_path_desc& d, int fmt, uint8_t* ras_d,
+               const float* sw_in, float* sw_next) {
+    const int smem = choose_smem(c, std::max(d.width, 1u));
+    const bool tiled = !stroke && tile_max_side(c) > 0;
+    const int parts = std::max(1, grid_cap(c, 2)), h = (int)std::max(d.height, 1u);
+    const int rows = std::max(8, (h + parts - 1) / parts), n = (h + rows - 1) / rows;
+    ftk::TilePlan t{ftk::TILE_THREADS_FEW, ftk::TILE_CAP_FEW, few_area((int)d.width, std::min(rows, h))};
+    FT_CU(c->status.ensure(sizeof(int32_t)), "alloc status");
+    FT_CU(c->overflow.ensure(sizeof(uint32_t) * n), "alloc overflow list");
+    FT_CU(c->scratch.ensure(std::max(ftk::SCRATCH_BYTES_PER_CTA * (size_t)n,
+                                     tiled ? ftk::tile_scratch(t.cap) * (size_t)n : (size_t)0)),
+          "alloc scratch");
+    ftk::KParams p;
+    fill_params(c, p, stroke, rule, fmt, smem);
+    p.ops = ops_d;
+    p.n_items = tiled ? 0 : n;
+    p.n_items_w = tiled ? n : 0;
+    p.overflow = tiled ? static_cast<uint32_t*>(c->overflow.p) : nullptr;
+    p.rasters = ras_d;
+    p.status = static_cast<int32_t*>(c->status.p);
+    p.sw_out = sw_next;
+    p.sw_chain = sw_in;
+    p.scratch = static_cast<unsigned char*>(c->scratch.p);
+    p.single = 1;
+    p.rows_per = rows;
+    p.d = d;
+    c->last_n_paths = 1;
+    c->comp_timed = false;
+    FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
+    FT_CU(enqueue(p, t, n, n, smem, c->stream, &c->launches, c->sm_count), "launch rasteriser");
+    FT_CU(cudaEventRecord(c->ev1, c->stream), "event");
+    c->timed = true;
+    return FT_OK;
+}
+
 bool valid_ops_host(const ft_op* ops, uint64_t n) {
     for (uint64_t i = 0; i < n; i++)
         if (ops[i].kind < FT_OP_CLOSE || ops[i].kind > FT_OP_PEN_WIDTH) return false;
@@ -470,8 +518,10 @@ int single(ft_ctx* c, int stroke, int32_t rule, const ft_op* ops, uint32_t n_ops
         // a large canvas, or an un-capped fill: build the figure once and bin its edges,
         // then one CTA per band of rows (the ordered compositor with a single call)
         st = composite_impl(c, stroke, rule, ops_d, n_ops, &d, 1, fmt, ras_d, w, h, stride, FT_DEVICE, sw_next, sw_in);
-    } else {
+    } else if ((uint64_t)w * h >= split_px(c)) {  // no band of it fits in shared memory
         st = run(c, stroke, rule, ops_d, &d, 1, fmt, ras_d, sw_in, sw_next);
+    } else {
+        st = run_single(c, stroke, rule, ops_d, d, fmt, ras_d, sw_in, sw_next);
     }
     if (st != FT_OK) return st;
     c->sw_cur ^= 1;

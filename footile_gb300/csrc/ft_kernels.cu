@@ -1542,23 +1542,30 @@ __global__ void __launch_bounds__(BLOCK) k_raster(KParams P) {
     float4* spts = reinterpret_cast<float4*>(scr + SCR_SPTS);
     SubRec* subs = reinterpret_cast<SubRec*>(scr + SCR_SUBS);
     // paths the tile rasteriser handed over (it ran before this kernel)
-    const int n_over = P.overflow ? (int)*(volatile uint32_t*)&P.queue[2] : 0;
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(&P.queue[0], 1u);
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();
-        if (it >= (int)P.n_items + n_over) break;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int n_over = P.overflow && !P.single ? (int)*(volatile uint32_t*)&P.queue[2] : 0;
+    for (int round = 0;; round++) {
         WorkItem wi;
-        if (it < (int)P.n_items) {
-            wi = P.items[it];
+        ft_path_desc d;
+        if (P.single) {  // CTA b's rows of the one path, unless the tile rasteriser drew them
+            if (round || (P.overflow && !*(volatile uint32_t*)&P.overflow[blockIdx.x])) break;
+            d = P.d;
+            wi = WorkItem{0, (uint32_t)(blockIdx.x * P.rows_per),
+                          min(d.height, (uint32_t)((blockIdx.x + 1) * P.rows_per)), 0};
         } else {
-            wi.path = P.overflow[it - (int)P.n_items];
-            wi.row_begin = 0;
-            wi.row_end = P.paths[wi.path].height;
-            wi.band_rows = 0;
+            if (tid == 0) s_item = (int)atomicAdd(&P.queue[0], 1u);
+            __syncthreads();
+            const int it = s_item;
+            __syncthreads();
+            if (it >= (int)P.n_items + n_over) break;
+            if (it < (int)P.n_items) {
+                wi = P.items[it];
+            } else {
+                wi = P.items_w[P.overflow[it - (int)P.n_items]];
+                wi.band_rows = 0;
+            }
+            d = P.paths[wi.path];
         }
-        const ft_path_desc d = P.paths[wi.path];
         if (wi.band_rows == 0) {
             const int wp4 = (int)(((d.width + 3) & ~3u) * 4);
             wi.band_rows = (uint32_t)max(1, min((P.smem_bytes - RASTER_FIXED_SMEM) / max(wp4, 4), (int)d.height));
@@ -1593,7 +1600,12 @@ __global__ void __launch_bounds__(BLOCK) k_raster(KParams P) {
             lp = block_incl_max(lp, reinterpret_cast<BuildSmem*>(smem)->scan);
             if (tid == BLOCK - 1) P.sw_out[wi.path] = lp >= 0 ? P.ops[d.op_begin + lp].v[0] : sw0;
         }
-        if (tid == 0 && S.flags) atomicMax(&P.status[wi.path], (S.flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
+        const int st = S.flags ? ((S.flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG) : FT_OK;
+        if (tid == 0 && P.single) {
+            if (wi.row_begin == 0) P.status[0] = st;
+        } else if (tid == 0 && S.flags) {
+            atomicMax(&P.status[wi.path], st);
+        }
         __syncthreads();
     }
 }
@@ -1602,12 +1614,13 @@ __global__ void __launch_bounds__(BLOCK) k_raster(KParams P) {
 // one CTA per SM: the rest stays L1 for the curve walks' local-memory stacks.
 constexpr int FEW_CTAS_CARVEOUT = 25;
 
-cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas) {
+cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas, bool chained) {
     auto kern = p.stroke ? k_raster<true> : k_raster<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                          few_ctas ? FEW_CTAS_CARVEOUT : (int)cudaSharedmemCarveoutDefault);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;
+    if (chained) return launch_chain(kern, grid, BLOCK, smem_bytes, s, p);
     kern<<<grid, BLOCK, smem_bytes, s>>>(p);
     return cudaGetLastError();
 }

@@ -183,12 +183,14 @@ struct KParams {
     uint32_t n_items;
     const WorkItem* items_w; // tile rasteriser's work items
     uint32_t n_items_w;
-    uint32_t* overflow;      // paths the tile rasteriser handed over to the CTA kernel
+    uint32_t* overflow;      // tile items handed over to the CTA kernel (single: a flag per CTA)
     uint32_t* queue;         // [0]: next CTA item, [1]: next tile item, [2]: overflow count
     uint8_t* rasters;
     int32_t* status;         // per path, atomicMax of FT_ERR_* codes
     float* sw_out;           // per path pen width after the call (nullable)
     int host_rasters;        // rasters are mapped host memory: Matte8 rows go out as aligned words
+    int single, rows_per;    // one path, `d`, CTA b drawing rows b * rows_per .. (as TileParams)
+    ft_path_desc d;
     const float* sw_chain;   // nullable: initial pen width of every path
     unsigned char* scratch;  // gridDim.x * SCRATCH_BYTES_PER_CTA bytes
     float xf[6];
@@ -241,8 +243,12 @@ struct TileParams {
     const ft_path_desc* paths;
     const WorkItem* items;
     uint32_t n_items;
-    uint32_t* overflow;      // paths handed to k_raster
+    uint32_t* overflow;      // items handed to k_raster (single: per CTA, whether its rows are)
     uint32_t* queue;         // [1]: next item, [2]: overflow count
+    // one path (ft_fill): CTA b draws rows b * rows_per .. of it; the descriptor is `d`, nothing is
+    // uploaded or reset before the launch
+    int single, rows_per;
+    ft_path_desc d;
     uint8_t* rasters;
     int32_t* status;         // per path, atomicMax of FT_ERR_* codes
     float* sw_out;           // per path pen width after the call (nullable)
@@ -323,7 +329,9 @@ int composite_build_blocks_per_sm(int smem_bytes, bool stroke);
 constexpr int RASTER_FIXED_SMEM = BLOCK * (int)sizeof(EdgeRec) + 3 * BLOCK * 4 + 256 + 4096;
 
 // Launch the persistent rasteriser.  Returns the CUDA error of the launch.
-cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas);
+// `chained`: right behind the tile rasteriser of the same path.
+cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas,
+                          bool chained = false);
 // Resident CTAs per SM for `smem_bytes` of dynamic shared memory.
 int raster_blocks_per_sm(int smem_bytes, bool stroke);
 

@@ -512,22 +512,37 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
     TileBuild<NT>& B = *reinterpret_cast<TileBuild<NT>*>(smem);
     TileWarp& Q = reinterpret_cast<TileWarp*>(smem)[warp];
     int* area = reinterpret_cast<int*>(smem + TileLayout<NT>::warps);
-    for (;;) {
-        if (tid == 0) S.item = (int)atomicAdd(&P.queue[1], 1u);
-        __syncthreads();
-        const int it = S.item;
-        if (it >= (int)P.n_items) break;
-        const WorkItem wi = P.items[it];
-        const ft_path_desc d = P.paths[wi.path];
+    // k_raster, behind this kernel, may be set up (it waits for this kernel's end)
+    if (P.single) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int round = 0;; round++) {
+        int it = blockIdx.x;
+        WorkItem wi;
+        ft_path_desc d;
+        if (P.single) {
+            if (round) break;
+            d = P.d;
+            wi = WorkItem{0, (uint32_t)(it * P.rows_per), min(d.height, (uint32_t)((it + 1) * P.rows_per)), 0};
+        } else {
+            if (tid == 0) S.item = (int)atomicAdd(&P.queue[1], 1u);
+            __syncthreads();
+            it = S.item;
+            if (it >= (int)P.n_items) break;
+            wi = P.items[it];
+            d = P.paths[wi.path];
+        }
         const float sw0 = P.sw_chain ? *P.sw_chain : d.s_width;
         const int n_slots = tile_build<NT>(P, d, S, B, E, ends, sw0);
-        if (n_slots < 0) {  // the path goes to k_raster, once
-            if (tid == 0 && wi.row_begin == 0) P.overflow[atomicAdd(&P.queue[2], 1u)] = wi.path;
+        if (P.single && tid == 0) P.overflow[it] = n_slots < 0;
+        if (n_slots < 0) {  // these rows go to k_raster
+            if (!P.single && tid == 0) P.overflow[atomicAdd(&P.queue[2], 1u)] = (uint32_t)it;
             __syncthreads();
             continue;
         }
         if (tid == 0 && wi.row_begin == 0) {
-            if (S.flags) atomicMax(&P.status[wi.path], FT_ERR_ARG);
+            if (P.single)
+                P.status[0] = S.flags ? FT_ERR_ARG : FT_OK;
+            else if (S.flags)
+                atomicMax(&P.status[wi.path], FT_ERR_ARG);
             if (P.sw_out) P.sw_out[wi.path] = S.last_pw >= 0 ? P.ops[d.op_begin + S.last_pw].v[0] : sw0;
         }
         const int W = (int)d.width, H = (int)d.height;
