@@ -78,6 +78,7 @@ struct ft_ctx {
     // device buffers
     DevBuf ops, paths, overflow, status, sw_out, rasters, queue, scratch, sw_chain;
     DevBuf pool, pool_used, bandoff, crec;  // ordered composite
+    DevBuf tile_done;                       // ordered composite: batches done per tile
     DevBuf figbins;                         // one path's figure state and band counts (split binning)
     DevBuf mask;                            // a single large Rgba8p call's Matte8 coverage
     DevBuf gbuf;                            // one fill path's grid-wide figure build
@@ -782,7 +783,7 @@ FT_API void ft_ctx_destroy(ft_ctx* c) {
     DevBuf* bufs[] = {&c->ops,     &c->paths,   &c->overflow,
                       &c->status,  &c->sw_out,  &c->rasters, &c->queue,   &c->scratch,
                       &c->sw_chain, &c->pool,   &c->pool_used, &c->bandoff, &c->crec,
-                      &c->srgb_lut, &c->conv_src, &c->conv_dst, &c->figbins, &c->mask};
+                      &c->srgb_lut, &c->conv_src, &c->conv_dst, &c->figbins, &c->mask, &c->tile_done};
     for (DevBuf* b : bufs) b->release();
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev_comp) cudaEventDestroy(c->ev_comp);
@@ -1060,8 +1061,8 @@ FT_API int ft_fill_batch(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* o
 }
 
 // Rows per band of the ordered composite = warps of a compositor CTA (one row each):
-// at most eight (built-in: 4 for Rgba8p tiles, measured fastest on 16,384 strokes on
-// 2048x2048; 8 for Matte8, whose compositor keeps whole rows: as many as its shared
+// at most eight (built-in: 4 for Rgba8p tiles: 16,384 strokes on 2048x2048 take
+// 97 / 94 / 95 ms with 2 / 4 / 8; 8 for Matte8, whose compositor keeps whole rows: as many as its shared
 // memory holds).
 static int composite_band_rows(ft_ctx* c, uint32_t w, int fmt) {
     int R = (c->tuned && c->tune.band_rows > 0) ? std::min((int)c->tune.band_rows, ftk::NWARP)
@@ -1071,13 +1072,17 @@ static int composite_band_rows(ft_ctx* c, uint32_t w, int fmt) {
     return R;
 }
 
-// Width of an Rgba8p compositor tile (pixels): built-in the narrowest of 1024, 512, 256
-// and 128 that covers the canvas in as few tiles (every tile re-reads its band's edges).
-static int composite_tile_w(const ft_ctx* c, uint32_t w) {
+// Width of an Rgba8p compositor segment (pixels), a warp's share of a row: built-in the canvas in
+// equal parts of at most 1,024, whole 256-pixel boxes or one of 128; in up to four parts while
+// their warps all find room (24 per SM), since a warp is then bound by the latency of its chain
+// of calls (2,000 strokes, 1,024 / 512 / 256 / 128 pixels: 300 x 300 10.0 / 10.0 / 9.7 / 7.6 ms,
+// 800 x 800 10.9 / 8.9 / 7.6 / 11.6, 2048 x 2048 10.1 / 16.4 / 31.6 / 54.9).
+static int composite_tile_w(const ft_ctx* c, uint32_t w, uint32_t h) {
     if (c->tuned && c->tune.tile_w > 0) return c->tune.tile_w;
-    int tw = 1024;
-    while (tw > 128 && (w + tw / 2 - 1) / (tw / 2) == (w + tw - 1) / tw) tw /= 2;
-    return tw;
+    uint32_t parts = std::max(1u, (w + 1023) / 1024);
+    while (2 * parts <= ftk::CT_MAX_SEGS && (uint64_t)2 * parts * h <= 24ull * c->sm_count && w / parts > 128) parts *= 2;
+    const uint32_t part = (w + parts - 1) / parts;
+    return part <= 128 ? 128 : (int)((part + 255) / 256 * 256);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1163,10 +1168,16 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
                             ftk::composite_bands_smem(composite_band_rows(c, w, FT_MATTE8), (int)w) <= c->max_smem;
     const int R = composite_band_rows(c, w, mask_route ? FT_MATTE8 : fmt);
     const int n_bands = (int)((h + R - 1) / R);
-    const int tile_w = composite_tile_w(c, w);
+    const int tile_w = composite_tile_w(c, w, h);
     const int stage = (c->tuned && c->tune.tile_stage > 0) ? c->tune.tile_stage : 1;
+    // The segments of a row that fit in one tile have their edges binned by segment, while the
+    // build's counters of all bins fit in the shared memory it runs with.
+    const int n_segs = (int)((w + tile_w - 1) / tile_w);
+    const bool by_segs = fmt == FT_RGBA8P && n_paths > 1 && n_segs <= ftk::CT_MAX_SEGS &&
+                         ((size_t)n_bands * n_segs + 1) * sizeof(int) <= (size_t)build_smem(c, 0);
+    const int bin_segs = by_segs ? std::max(n_segs, 1) : 1;
     const int smem_b = fmt == FT_MATTE8 ? ftk::composite_bands_smem(R, (int)w)
-                                        : ftk::composite_tile_smem(R, tile_w, stage == 1);
+                                        : ftk::composite_tile_smem(R, bin_segs, tile_w, stage == 1);
     if (smem_b > c->max_smem) return fail(c, FT_ERR_CAP, "raster too wide for the band compositor");
     const int smem_a = build_smem(c, n_bands);
     if ((size_t)(n_bands + 1) * sizeof(int) > (size_t)smem_a)
@@ -1175,7 +1186,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
     FT_CU(c->status.ensure(sizeof(int32_t) * std::max(n_paths, 1u)), "alloc status");
     FT_CU(c->queue.ensure(256), "alloc queue");
     FT_CU(c->crec.ensure(sizeof(int4) * std::max(n_paths, 1u)), "alloc path records");
-    FT_CU(c->bandoff.ensure(sizeof(int) * (size_t)std::max(n_paths, 1u) * (n_bands + 1)), "alloc band offsets");
+    FT_CU(c->bandoff.ensure(sizeof(int) * (size_t)std::max(n_paths, 1u) * ((size_t)n_bands * bin_segs + 1)),
+          "alloc band offsets");
     FT_CU(c->pool_used.ensure(sizeof(unsigned long long)), "alloc pool counter");
     // un-capped fills: every CTA's scratch holds a figure of fig_cap vertices (8 GB in all at most)
     const bool uncapped = !stroke && c->fig_cap > (uint32_t)ftk::PT_CAP;
@@ -1231,6 +1243,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
         p.canvas_stride = stride;
         p.band_rows = R;
         p.n_bands = n_bands;
+        p.seg_w = tile_w;
+        p.bin_segs = bin_segs;
         p.pool = static_cast<ftk::EdgeRec*>(c->pool.p);
         p.pool_used = static_cast<unsigned long long*>(c->pool_used.p);
         p.pool_cap = c->pool.cap / sizeof(ftk::EdgeRec);
@@ -1432,10 +1446,14 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             } else {
                 CUtensorMap tm;
                 memset(&tm, 0, sizeof(tm));
-                p.seg_w = tile_w;
-                p.use_tma = stage == 1 && canvas_tensor_map(&tm, ras_d, w, h, stride, std::min(tile_w, 256), R) ? 1 : 0;
+                p.use_tma = stage == 1 && canvas_tensor_map(&tm, ras_d, w, h, stride, std::min(tile_w, 256),
+                                                          ftk::composite_tile_rows(R, bin_segs))
+                                ? 1
+                                : 0;
                 FT_CU(cudaEventRecord(c->ev_comp, c->stream), "event");
-                FT_CU(ftk::launch_composite_tiles(p, tm, c->stream), "launch tile compositor");
+                FT_CU(c->tile_done.ensure(sizeof(unsigned) * (size_t)ftk::composite_tiles(p)), "alloc tile counters");
+                p.tile_done = static_cast<unsigned*>(c->tile_done.p);
+                FT_CU(ftk::launch_composite_tiles(p, tm, c->sm_count, c->stream), "launch tile compositor");
                 c->comp_timed = true;
             }
             c->launches++;

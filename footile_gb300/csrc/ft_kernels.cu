@@ -37,6 +37,7 @@
 #include <cuda.h>
 
 #include "ft_device.cuh"
+#include "ft_items.cuh"
 #include "ft_kernels.cuh"
 #include "ft_slots.cuh"
 
@@ -1357,10 +1358,37 @@ __device__ __forceinline__ EdgeRec edge_rec(int i, int count, int figdir, const 
     return e;
 }
 
+// The segments of seg_w pixels that an edge's cells can reach: its x-range between its ends, two
+// pixels more to each side for the rounding of its slope, and the longest walk of a row to the
+// right of it.  Edges whose x could wrap take every segment.
+__device__ __forceinline__ int2 edge_segs(const EdgeRec& e, int segs, int seg_w) {
+    const int inv = e.inv_slope, fu = fxfract(e.y_upper), fl = fxfract(e.y_lower);
+    const long long end = (long long)(e.end_row - e.start_row) * inv + e.x_bot0 - fxmul(inv, FX_ONE - fl);
+    constexpr int FAR = 1 << 29;
+    if (abs(end) >= FAR || abs((long long)e.x_bot0) >= FAR || abs((long long)inv) >= FAR) return make_int2(0, segs - 1);
+    const int a = e.x_bot0 - fxmul(inv, FX_ONE - fu), z = (int)end;
+    const int cells = e.step_pix > 0 ? (int)__fdividef(65536.0f * 1.01f, (float)e.step_pix) + 3 : 4;
+    const int lo = (min(a, z) >> 16) - 2, hi = (max(a, z) >> 16) + 2 + cells;
+    int2 g = make_int2(0, 0);
+    for (int k = 1; k < segs; k++) {
+        g.x += lo >= k * seg_w;
+        g.y += hi >= k * seg_w;
+    }
+    return g;
+}
+
+// `segs` > 1: an edge's direction goes into the low byte of ed, its segments above it.
 template <class G>
-__device__ void build_edges(const CState& S, const int2* pts, const int* ss, EdgeRec* edges) {
+__device__ void build_edges(const CState& S, const int2* pts, const int* ss, EdgeRec* edges, int segs = 1, int seg_w = 0) {
     const int count = S.count, figdir = S.dir;
-    for (int i = G::rank(); i < count; i += G::N) edges[i] = edge_rec(i, count, figdir, pts, ss);
+    for (int i = G::rank(); i < count; i += G::N) {
+        EdgeRec e = edge_rec(i, count, figdir, pts, ss);
+        if (segs > 1 && e.ed) {
+            const int2 g = edge_segs(e, segs, seg_w);
+            e.ed = (e.ed & 0xFF) | (g.x << 8) | (g.y << 12);
+        }
+        edges[i] = e;
+    }
 }
 
 // Signed cell areas of one edge on one scan row (fig.rs:238-321), added into
@@ -1662,16 +1690,17 @@ namespace ftk {
 // resolves its rows and composites.  Every call of footile composites every pixel
 // from its top row down, alpha 0 included, and SrcOver with alpha 0 maps each
 // premultiplied channel d to ch8_mul(d, 255), which changes only d in 1..15 and
-// is the identity after 15 applications.  So a band keeps, per row, the number of
-// calls so far and, per pixel, the call count at its last covering call: a covered
-// pixel first takes the pending alpha-0 maps from a 16-entry table of powers,
-// uncovered pixels are not touched, and the band ends with one pending flush.
+// is the identity after 15 applications.  So a tile keeps, per row, the number of
+// calls so far and, per four pixels, the call count at their last visit: covered
+// pixels first take the alpha-0 maps they missed in one step, uncovered pixels are
+// not touched, and the tile ends with one pending flush.
 
-// Bin the built figure's edges by raster band into the pool (block-wide).
+// Bin the built figure's edges by raster band, and by segment of the row where the compositor's
+// warps share a row (bins of a band one after another), into the pool (block-wide).
 __device__ void bin_edges(const KParams& P, uint32_t path, const CState& S, const EdgeRec* edges, int* hist,
                           int* tmp) {
     const int tid = threadIdx.x;
-    const int count = S.count, H = (int)P.canvas_h, R = P.band_rows, nb = P.n_bands;
+    const int count = S.count, H = (int)P.canvas_h, R = P.band_rows, segs = P.bin_segs, nb = P.n_bands * segs;
     const int tmin = min(S.top_row, 0);
     const int rb = count > 0 ? max(S.top_row, 0) : H;  // first raster row footile writes
     for (int b = tid; b < nb; b += BLOCK) hist[b] = 0;
@@ -1684,6 +1713,13 @@ __device__ void bin_edges(const KParams& P, uint32_t path, const CState& S, cons
         hi = min(q.w - tmin, H - 1);
         return q.y != 0 && lo <= hi;
     };
+    auto each_bin = [&](const int4& q, auto f) {
+        int lo, hi;
+        if (!rows_of(q, lo, hi)) return;
+        const int g0 = segs > 1 ? (q.y >> 8) & 15 : 0, g1 = segs > 1 ? (q.y >> 12) & 15 : 0;
+        for (int b = lo / R; b <= hi / R; b++)
+            for (int k = g0; k <= g1; k++) f(b * segs + k);
+    };
     const int4* erec = reinterpret_cast<const int4*>(edges);
     constexpr int EU = 4;
     for (int e0 = 0; e0 < count; e0 += BLOCK * EU) {
@@ -1694,11 +1730,7 @@ __device__ void bin_edges(const KParams& P, uint32_t path, const CState& S, cons
             q[u] = e < count ? erec[2 * e + 1] : make_int4(0, 0, 0, 0);
         }
 #pragma unroll
-        for (int u = 0; u < EU; u++) {
-            int lo, hi;
-            if (rows_of(q[u], lo, hi))
-                for (int b = lo / R; b <= hi / R; b++) atomicAdd(&hist[b], 1);
-        }
+        for (int u = 0; u < EU; u++) each_bin(q[u], [&](int b) { atomicAdd(&hist[b], 1); });
     }
     __syncthreads();
     int carry = 0;
@@ -1714,8 +1746,8 @@ __device__ void bin_edges(const KParams& P, uint32_t path, const CState& S, cons
     __syncthreads();
     const unsigned long long base = s_base;
     const bool fits = base + (unsigned long long)carry <= P.pool_cap;
-    // band offsets band-major (bandoff[b * n_items + path]): the compositors read 32 calls'
-    // offsets of one band as one coalesced load
+    // bin offsets bin-major (bandoff[b * n_items + path]): the compositors read 32 calls'
+    // offsets of one bin as one coalesced load
     for (int b = tid; b <= nb; b += BLOCK)
         P.bandoff[(size_t)b * P.n_items + path] = fits ? (b < nb ? hist[b] : carry) : 0;
     if (tid == 0) {
@@ -1734,17 +1766,14 @@ __device__ void bin_edges(const KParams& P, uint32_t path, const CState& S, cons
                 q1[u] = e < count ? erec[2 * e + 1] : make_int4(0, 0, 0, 0);
             }
 #pragma unroll
-            for (int u = 0; u < FU; u++) {
-                int lo, hi;
-                if (!rows_of(q1[u], lo, hi)) continue;
-                for (int b = lo / R; b <= hi / R; b++) {
+            for (int u = 0; u < FU; u++)
+                each_bin(q1[u], [&](int b) {
                     const unsigned long long k = base + (unsigned)atomicAdd(&hist[b], 1);
-                    if (!ck(k < P.pool_cap, 11)) continue;
+                    if (!ck(k < P.pool_cap, 11)) return;
                     int4* dst = reinterpret_cast<int4*>(P.pool + k);
                     dst[0] = q0[u];
-                    dst[1] = q1[u];
-                }
-            }
+                    dst[1] = make_int4(q1[u].x, (int)(signed char)q1[u].y, q1[u].z, q1[u].w);
+                });
         }
     }
     __syncthreads();
@@ -1794,7 +1823,7 @@ __global__ void __launch_bounds__(BLOCK, 4) k_cbuild(KParams P) {
         } else {
             if (S.count > 0) {
                 top_and_dir<BlockG>(S, pts, ss, s_tmp3);
-                build_edges<BlockG>(S, pts, ss, edges);
+                build_edges<BlockG>(S, pts, ss, edges, P.bin_segs, P.seg_w);
             }
             __syncthreads();
             bin_edges(P, (uint32_t)it, S, edges, reinterpret_cast<int*>(smem), s_tmp3);
@@ -1809,20 +1838,6 @@ __global__ void __launch_bounds__(BLOCK, 4) k_cbuild(KParams P) {
         if (tid == 0 && S.flags) atomicMax(&P.status[it], (S.flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
         __syncthreads();
     }
-}
-
-// The alpha-0 SrcOver of pix maps a premultiplied channel d to ch8_mul(d, 255), which
-// leaves d >= 16 unchanged: ftab[k][d] (d < 16) is d after k such composites.
-constexpr int FTAB_BYTES = 16 * 16;
-__device__ __forceinline__ unsigned ftab4(const unsigned char* ftab, unsigned d, int k) {
-    const unsigned char* t = ftab + (k << 4);
-    unsigned out = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const unsigned c = (d >> (8 * i)) & 0xFFu;
-        out |= (c < 16u ? (unsigned)t[c] : c) << (8 * i);
-    }
-    return out;
 }
 
 // Per-warp shared memory of the Matte8 band compositor for rows of `width` pixels: the
@@ -1906,49 +1921,78 @@ __global__ void __launch_bounds__(BLOCK) k_cbands(KParams P) {
 }
 
 // ===========================================================================
-// Rgba8p ordered composite on tiles (ft_composite_batch, and single large calls).
+// Rgba8p ordered composite on tiles (ft_composite_batch).
 //
-// One CTA per tile of R band rows x `seg_w` pixels; one warp per tile row.  The tile's
-// canvas pixels are staged in shared memory for the whole call sequence: loaded by TMA
-// (cp.async.bulk.tensor.2d, boxes of at most 256 pixels x R rows, completion on an
-// mbarrier) when the canvas allows a tensor map, stored back by TMA at the end.  Each
-// warp walks the calls in order.  For a call, every band edge crossing the row gives its
-// cells inside the segment (into a shared i32 segment row, atomics) and, from the closed
-// form of the cell walk, the running sum it leaves to the left of the segment (the carry
-// into the segment: the cumulative cell sum through column c of an (edge, row) item is
-// min(pixel_cov(min(first + (c - minp) * step, ONE)), cov), fig.rs:285-321).  The row is
-// then resolved sparsely: only the 8-pixel chunks that received cells are summed and
-// resolved (32 at a time, one per lane, a warp scan placing them), and the untouched gap
-// after each chunk holds that chunk's final running sum, so it is one run of a single
-// alpha.  The covered pixels (alpha > 0) of the chunks and of the runs are composited
-// with all lanes busy; the alpha-0 SrcOver footile applies to every other pixel from the
-// call's top row down is applied lazily, as a pending count per pixel and a table of
-// powers of the alpha-0 map (the map changes only channel values 1..15 and settles after
-// 15 applications).
+// A tile is a few rows of one or more segments of P.seg_w pixels, one warp per row and segment,
+// its canvas pixels in shared memory: loaded by TMA (cp.async.bulk.tensor.2d, boxes of at most
+// 256 pixels wide, completion on an mbarrier) when the canvas allows a tensor map, stored back by
+// TMA at the end.  Each warp walks the calls in order.  For a call, the edges crossing its row
+// are spread over its lanes; an edge's cells go into the segment's i32 areas in shared memory
+// (atomics).  The row is then resolved sparsely: only the 8-pixel chunks that received cells are
+// summed (32 at a time, one per lane, a warp scan placing them), and the untouched gap after a
+// chunk holds that chunk's final running sum, so it is one run of a single alpha.
+//
+// Up to CT_MAX_SEGS segments cover the whole row: the build then bins each edge under the
+// segments that its cells reach (bin_edges), no warp sees another's edges, and the running sum
+// at the end of a segment is handed to the next one's warp through a ring of 64 words, so the
+// warps of a row only follow one another.  Wider rows are cut into tiles of one segment, each
+// walking all the band's edges: the closed form of an edge's walk gives what it leaves to the
+// left of the segment (the cumulative cell sum through column c of an (edge, row) item is
+// min(pixel_cov(min(first + (c - minp) * step, ONE)), cov), fig.rs:285-321).
+//
+// What is composited are quads, four pixels a lane as one 16-byte word, those of the chunks that
+// hold any coverage and those of the runs, queued until all lanes have one.  The alpha-0 SrcOver
+// footile applies to every other pixel from the call's top row down is applied lazily: a quad
+// keeps the number of calls at its last visit (mod 256), and what it missed since is one packed
+// step, because the alpha-0 map takes one from channels 1..15 and leaves the rest.
+//
+// Bound by the instructions issued and by the 24 warps per SM that 9 KB per 1,024 pixels leave
+// room for.  16,384 strokes on 2048 x 2048, 31.5 million (call, row) pairs of 45 edges and 175
+// covered pixels each: every warp walking all the band's edges, a queue of single pixels and a
+// table for the alpha-0 powers 118 ms; quads, two warps sharing the row's edges between barriers
+// 92 ms; one warp resolving a whole row and one compositing behind it 129 ms; this way 81 ms.
 
-constexpr int CT_QN = 256 + 40;  // queued covered pixels of one round (32 chunks of 8) and its runs
+constexpr int CT_QN = 96;       // queued quads of a warp: 31 left over and a round's 64
+constexpr int CT_CHAIN = 64;    // sums under way from a segment's warp to the next one's
 
+// Tile rows (they divide the band's) and segments: four warps where the band has the rows.
+struct CTileShape {
+    int rows, segs;
+};
+__host__ __device__ inline CTileShape ctile_shape(int R, int bin_segs) {
+    const int want = bin_segs == 1 ? 4 : (bin_segs == 2 ? 2 : 1);
+    int rows = want < R ? want : R;
+    while (R % rows) rows--;
+    return {rows, bin_segs};
+}
 struct CTileLayout {
-    int tile, mbar, area, last, queue, bmap, bytes;
+    int tile, area, q, runs, bmap, chain, mbar, qi, clist, last, bytes;
 };
 // Shared memory of a compositor CTA; `staged`: the canvas tile is held in shared memory.
-__host__ __device__ inline CTileLayout ctile_layout(int R, int sw, bool staged) {
+__host__ __device__ inline CTileLayout ctile_layout(CTileShape t, int sw, bool staged) {
     CTileLayout L;
-    int o = FTAB_BYTES;
-    o = (o + 127) & ~127;
-    L.tile = o;  // R x sw canvas pixels, [box][row][box width]
-    if (staged) o += R * sw * 4;
+    const int warps = t.rows * t.segs;
+    int o = 0;
+    L.tile = o;  // canvas pixels, [box][row][box width]
+    if (staged) o += warps * sw * 4;
+    L.area = o;  // per warp: sw i32 cell areas
+    o += warps * sw * 4;
+    L.bmap = o;  // per warp: touched 8-pixel chunks, one bit each
+    o += warps * 16;
     L.mbar = o;
     o += 16;
-    L.area = o;  // per warp: sw i32 cell areas
-    o += R * sw * 4;
-    L.queue = o;  // per warp: CT_QN queued pixels (x << 8 | alpha) and runs
-    o += R * CT_QN * 4;
-    L.bmap = o;  // per warp: touched 8-pixel chunks (one bit each), then the chunk list (a byte each)
-    o += R * (((sw / 8 + 31) / 32) * 4 + sw / 8);
-    o = (o + 15) & ~15;
-    L.last = o;  // per warp: sw u8, calls so far (mod 256) at each pixel's last cover
-    o += R * sw;
+    L.q = o;  // per warp: the alphas of queued quads
+    o += warps * CT_QN * 4;
+    L.runs = o;  // per warp: the gap runs of a round
+    o += warps * 32 * 4;
+    L.chain = o;  // per row and segment but the last: sums handed on, and how many were taken
+    o += t.rows * (t.segs - 1) * (CT_CHAIN + 1) * 4;
+    L.qi = o;  // per warp: which quads are queued
+    o += warps * CT_QN;
+    L.clist = o;  // per warp: touched chunks
+    o += warps * (sw / 8);
+    L.last = o;  // per warp: calls so far (mod 256) at each quad's last visit
+    o += warps * (sw / 4);
     L.bytes = (o + 15) & ~15;
     return L;
 }
@@ -1980,302 +2024,423 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, unsigned parity) {
     return false;
 }
 
-// Cells of one (edge, row) item inside the segment [s0, s0 + sw) of a raster row of W
-// pixels (fig.rs:238-321 restricted to the segment): the cells' growths go into `area`
-// (segment cells), the cumulative sum the item leaves left of s0 into `carry`, and the
-// 8-pixel chunks it touched into the bitmap `bmap`.  The other arguments are scan_row's.
-__device__ __forceinline__ void seg_row(int x_bot, int inv, bool st, bool en, int fu, int fl, int step, int ed,
-                                        int* area, int s0, int sw, int W, unsigned& carry, unsigned* bmap) {
-    const int ccov = en ? pixel_cov(fl) : 256;
-    const int cov = st ? ccov - pixel_cov(fu) : ccov;
-    if (cov <= 0) return;
-    const int s1 = min(s0 + sw, W);
-    {
-        // quick bounds: the item's x-range lies between x_bot and x_bot - inv (when that
-        // does not wrap, neither do the exact ends below)
-        const long long xa = (long long)x_bot - inv;
-        if (xa == (long long)(int)xa) {
-            const int lo = (int)(min((long long)x_bot, xa) >> 16), hi = (int)(max((long long)x_bot, xa) >> 16);
-            if (lo >= s1) return;  // right of the segment: nothing here, nothing carried in
-            // left of it, its walk complete before s0 (first + j * step >= ONE for every
-            // cell left of the segment from any start <= hi): it leaves its whole coverage
-            if (s0 - 1 - hi > 0 && (long long)(s0 - 1 - hi) * step >= FX_ONE) {
-                carry += (unsigned)(ed * cov);
-                return;
-            }
+// Wait until `done(word)` of a word in shared memory that another warp writes; false after ten
+// seconds.
+template <class F>
+__device__ __forceinline__ bool smem_wait(const unsigned* word, unsigned& v, F done) {
+    unsigned long long t0 = 0, t;
+    for (int it = 0; it < (1 << 30); it++) {
+        v = *reinterpret_cast<const volatile unsigned*>(word);
+        if (done(v)) return true;
+        if ((it & 255) == 255) {
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (!t0) t0 = t;
+            if (t - t0 > 10000000000ull) break;
         }
     }
-    const int x0 = st ? wsub(x_bot, fxmul(inv, wsub(FX_ONE, fu))) : wsub(x_bot, inv);
-    const int x1 = en ? wsub(x_bot, fxmul(inv, fl ? FX_ONE - fl : 0)) : x_bot;
+    return false;
+}
+
+// Wait until a tile's `batch` batches are done; false after ten seconds.
+__device__ __forceinline__ bool tile_wait(const unsigned* done, unsigned batch) {
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    for (int it = 0; it < (1 << 28); it++) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
+        if (v >= batch) return true;
+        __nanosleep(200);
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        if (t - t0 > 10000000000ull) break;
+    }
+    return false;
+}
+
+// k (at most 15) alpha-0 composites of a pixel: channels 1..15 each lose one per composite
+// down to 0 (ch8_mul(d, 255)), channels of 16 and more stay.
+__device__ __forceinline__ unsigned alpha0_pow(unsigned d, int k) {
+    // bytes whose high nibble is zero, as 0x00 / 0xFF masks
+    const unsigned hi = (((d & 0x70707070u) + 0x70707070u) | d) & 0x80808080u;
+    unsigned high;  // the top bit of each byte, spread over it
+    asm("prmt.b32 %0, %1, %1, 0xBA98;" : "=r"(high) : "r"(hi));
+    const unsigned low = ~high;
+    const unsigned t = ((d & low) | 0x10101010u) - (unsigned)k * 0x01010101u;  // bit 4: not below 0
+    const unsigned ge = (t >> 4) & 0x01010101u;
+    return (d & ~low) | (t & 0x0F0F0F0Fu & (ge * 15u) & low);
+}
+// srcover_rgba with the colour's channels widened (wide8 of each, c0 .. c3), two channels per word
+__device__ __forceinline__ unsigned wide8(unsigned v) { return (v << 4) | (v >> 4); }
+__device__ __forceinline__ unsigned srcover_wide(unsigned d, unsigned c0, unsigned c1, unsigned c2, unsigned c3,
+                                                 unsigned alpha) {
+    const unsigned ra = wide8(alpha);
+    const unsigned p3 = c3 * ra;
+    const unsigned se = __byte_perm(c0 * ra, c2 * ra, 0x7632), so = __byte_perm(c1 * ra, p3, 0x7632);
+    const unsigned ri = wide8(255u - (p3 >> 16));
+    const unsigned e = d & 0x00FF00FFu, o = (d >> 8) & 0x00FF00FFu;
+    const unsigned le = (e << 4) | ((e >> 4) & 0x000F000Fu), lo = (o << 4) | ((o >> 4) & 0x000F000Fu);
+    const unsigned de = __byte_perm((le & 0xFFFFu) * ri, (le >> 16) * ri, 0x7632);
+    const unsigned dd = __byte_perm((lo & 0xFFFFu) * ri, (lo >> 16) * ri, 0x7632);
+    return __vminu2(se + de, 0x00FF00FFu) | (__vminu2(so + dd, 0x00FF00FFu) << 8);
+}
+
+// Cells of one (edge, row) item inside [s0, s1) of a raster row (fig.rs:238-321): the cells'
+// growths, scaled by 2^16, into `area` (cells from s0 on), the touched 8-pixel chunks into
+// `bmap`, and what the item leaves left of s0 into `left0`.
+__device__ __forceinline__ void row_cells(const int4 ha, const int4 hb, int y, int* area, unsigned* bmap, int s0, int s1,
+                                          unsigned& left0) {
+    const int inv = ha.w;
+    const bool st = y == hb.z, en = y == hb.w;
+    const int fu = fxfract(ha.x), fl = fxfract(ha.y);
+    const int cov = (en ? (fl + 128) >> 8 : 256) - (st ? (fu + 128) >> 8 : 0);
+    const int xb = wadd(ha.z, wmul(y - hb.z, inv));
+    const int x0 = st ? wsub(xb, fxmul(inv, FX_ONE - fu)) : wsub(xb, inv);
+    const int x1 = en && fl ? wsub(xb, fxmul(inv, FX_ONE - fl)) : xb;
     const int mnx = min(x0, x1), mxx = max(x0, x1);
     const int minp = mnx >> 16, maxp = mxx >> 16;
-    if (minp >= W) return;
-    if (minp >= s1) return;  // right of the segment: nothing here, nothing carried in
-    const int full = cov << 8;
-    const int r = (minp == maxp) ? fxmul(wsub(FX_ONE, fxfract(fxavg(mxx, mnx))), full)
-                                 : fxmul(wsub(FX_ONE, fxfract(mnx)), FX_HALF);
-    const int first = fxmul(r, step);
-    int c = max(max(s0, minp), 0);
-    int prev = 0;
-    if (s0 > 0 && minp < s0) {
-        // cumulative sum through cell s0 - 1: min(pixel_cov(min(first + j * step, ONE)), cov)
-        const long long v = (long long)first + (long long)(s0 - 1 - minp) * step;
-        prev = min(pixel_cov(v > FX_ONE ? FX_ONE : (int)v), cov);
-        carry += (unsigned)(ed * prev);
-    }
-    if (prev >= cov) return;
-    const long long xv = (long long)first + (long long)(c - minp) * step;
-    int x_cov = xv > FX_ONE ? FX_ONE : (int)xv;
-    int c_lo = -1, c_hi = -1;
-    for (; c < s1; c++) {
-        const int v = min(pixel_cov(x_cov), cov);
-        if (v != prev) {
-            if (ck(c - s0 >= 0 && c - s0 < sw, 6)) atomicAdd(&area[c - s0], ed * (v - prev));
-            if (c_lo < 0) c_lo = c - s0;
-            c_hi = c - s0;
+    if (cov <= 0 || minp >= s1) return;
+    const unsigned step = hb.x > 0 ? hb.x : FX_ONE;
+    const unsigned r = minp == maxp ? ((unsigned)(FX_ONE - fxfract(fxavg(mxx, mnx))) * (unsigned)cov) >> 8
+                                    : (unsigned)(FX_ONE - fxfract(mnx)) >> 1;
+    const unsigned xc0 = (unsigned)(((unsigned long long)r * step) >> 16) + 128u;
+    // 256 * the cumulative sum left of cell x > minp, before the cap at cov
+    auto upto = [&](int x) {
+        const unsigned long long v = xc0 + (unsigned long long)(unsigned)(x - 1 - minp) * step;
+        return v > FX_ONE + 128 ? (unsigned)FX_ONE + 128u : (unsigned)v;
+    };
+    const unsigned ed = (unsigned)hb.y << 16;
+    unsigned xc = xc0;
+    int prev = 0, c = minp;
+    if (minp < s0) {
+        c = s0;
+        xc = upto(s0);
+        if (s0 > 0) {
+            prev = min((int)(xc >> 8), cov);
+            left0 += ed * (unsigned)prev;
+            if (prev >= cov) return;
         }
-        prev = v;
-        if (v >= cov) break;
-        x_cov = min(x_cov + step, FX_ONE);
+        xc = min(xc + step, (unsigned)FX_ONE + 128u);
     }
-    if (c_lo >= 0) {  // the touched chunks c_lo / 8 .. c_hi / 8
-        const int k0 = c_lo >> 3, k1 = c_hi >> 3;
-        for (int w = k0 >> 5; w <= (k1 >> 5); w++) {
-            const int lo = max(k0 - 32 * w, 0), hi = min(k1 - 32 * w, 31);
-            const unsigned m = (hi == 31 ? 0xFFFFFFFFu : ((1u << (hi + 1)) - 1u)) & ~((1u << lo) - 1u);
-            if (ck(w < (sw / 8 + 31) / 32, 7)) atomicOr(&bmap[w], m);
-        }
-    }
-}
-
-__device__ __forceinline__ unsigned warp_sum_u(unsigned v) {
+    const int k0 = (c - s0) >> 3;
+    int v;
+    do {  // four cells a step
 #pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    return v;
+        for (int u = 0; u < 4; u++) {
+            v = min((int)(xc >> 8), cov);
+            if (v != prev && c + u < s1 && ck(c + u >= s0, 6)) atomicAdd(area + (c + u - s0), (v - prev) * (int)ed);
+            prev = v;
+            xc += step;
+        }
+        c += 4;
+    } while (v < cov && c < s1);
+    const int k1 = (min(c, s1) - 1 - s0) >> 3;
+    for (int w = k0 >> 5; w <= (k1 >> 5); w++) {  // the chunks k0 .. k1
+        const int lo = max(k0 - 32 * w, 0), hi = min(k1 - 32 * w, 31);
+        if (ck(w >= 0 && w < 4, 7)) atomicOr(&bmap[w], (0xFFFFFFFFu >> (31 - hi)) & (0xFFFFFFFFu << lo));
+    }
 }
 
-template <bool STAGED>
-__global__ void __launch_bounds__(BLOCK, 4) k_ctile(KParams P, const __grid_constant__ CUtensorMap tmap) {
+template <bool STAGED, int RULE>
+__global__ void __launch_bounds__(BLOCK, 3) k_ctile(KParams P, const __grid_constant__ CUtensorMap tmap) {
     extern __shared__ __align__(128) unsigned char smem_tma[];  // TMA destinations: 128-byte aligned
     unsigned char* smem = smem_tma;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int W = (int)P.canvas_w, H = (int)P.canvas_h, R = P.band_rows, sw = P.seg_w;
-    const int nseg = (W + sw - 1) / sw;
-    const int b = (int)blockIdx.x / nseg, x0 = ((int)blockIdx.x % nseg) * sw;
-    const int r = b * R + warp;
-    const CTileLayout L = ctile_layout(R, sw, STAGED);
+    const CTileShape T = ctile_shape(R, P.bin_segs);
+    const int span = T.segs * sw, per_row = (W + span - 1) / span;
+    const int n_tiles = (H + T.rows - 1) / T.rows * per_row;
+    const int wrow = warp / T.segs, seg = warp % T.segs;
+    const CTileLayout L = ctile_layout(T, sw, STAGED);
     const int BW = sw < 256 ? sw : 256;  // TMA box width (pixels)
     const int bw_shift = BW == 256 ? 8 : 7;
-    const int nchunks = sw >> 3;             // 8-pixel chunks of the segment
-    const int nwords = (nchunks + 31) >> 5;  // bitmap words
-    unsigned char* ftab = smem;
     unsigned* tile = reinterpret_cast<unsigned*>(smem + L.tile);
     uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + L.mbar);
     int* area = reinterpret_cast<int*>(smem + L.area) + warp * sw;
-    unsigned* q = reinterpret_cast<unsigned*>(smem + L.queue) + warp * CT_QN;
-    unsigned* bmap = reinterpret_cast<unsigned*>(smem + L.bmap + warp * (nwords * 4 + nchunks));
-    unsigned char* clist = reinterpret_cast<unsigned char*>(bmap + nwords);
-    unsigned char* last = smem + L.last + warp * sw;
-    unsigned* crow = reinterpret_cast<unsigned*>(P.rasters + (size_t)r * P.canvas_stride) + x0;
-    // the canvas pixel of this warp's row at segment position x: in the shared tile
-    // (staged by TMA), or in place in global memory
-    auto px = [&](int x) -> unsigned* {
-        return STAGED ? tile + (((x >> bw_shift) * R + warp) << bw_shift) + (x & (BW - 1)) : crow + x;
-    };
-    const bool tma = STAGED;
-    if (tma && threadIdx.x == 0) {
+    unsigned* q = reinterpret_cast<unsigned*>(smem + L.q) + warp * CT_QN;
+    unsigned char* qi = smem + L.qi + warp * CT_QN;
+    unsigned* runs = reinterpret_cast<unsigned*>(smem + L.runs) + warp * 32;
+    uint4* bmap = reinterpret_cast<uint4*>(smem + L.bmap) + warp;
+    unsigned char* clist = smem + L.clist + warp * (sw / 8);
+    unsigned char* last = smem + L.last + warp * (sw / 4);
+    // sums to the next segment's warp, and from the one before
+    unsigned* out = reinterpret_cast<unsigned*>(smem + L.chain) + (wrow * (T.segs - 1) + seg) * (CT_CHAIN + 1);
+    unsigned* in = out - (CT_CHAIN + 1);
+    const bool has_out = seg + 1 < T.segs, has_in = seg > 0;
+    const unsigned lt = (1u << lane) - 1u;
+    const int n = (int)P.n_items;
+    __shared__ int s_unit;
+    if (STAGED && threadIdx.x == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    __syncthreads();
-    if (tma && threadIdx.x == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)),
-                     "r"(R * sw * 4)
-                     : "memory");
-        for (int bx = 0; bx < sw / BW; bx++)
-            asm volatile(
-                "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
-                "%3}], [%4];" ::"r"(smem_u32(tile + bx * R * BW)),
-                "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(x0 + bx * BW), "r"(b * R), "r"(smem_u32(mbar))
-                : "memory");
-    }
-    for (int i = threadIdx.x; i < FTAB_BYTES; i += blockDim.x) {
-        unsigned v = (unsigned)(i & 15);
-        for (int k = 0; k < (i >> 4); k++) v = ch8_mul(v, 255u);
-        ftab[i] = (unsigned char)v;
-    }
     for (int x = lane * 4; x < sw; x += 128) *reinterpret_cast<int4*>(area + x) = make_int4(0, 0, 0, 0);
-    for (int x = lane; x < sw; x += 32) last[x] = 0;
-    if (lane < nwords) bmap[lane] = 0u;
+    if (lane == 0) *bmap = make_uint4(0, 0, 0, 0);
+    if (has_out)
+        for (int k = lane; k <= CT_CHAIN; k += 32) out[k] = 0;
     bool ok = true;
-    if (tma) ok = mbar_wait(mbar, 0);
-    ok = __syncthreads_and(ok) != 0;
-    if (!ok && threadIdx.x == 0) atomicMax(&P.status[0], FT_ERR_TIMEOUT);
-    if (ok && r < H) {
-        const int n = (int)P.n_items, rule = P.rule;
-        const unsigned lt = (1u << lane) - 1u;
-        const int xend = min(sw, W - x0);  // segment pixels on the canvas
-        int G = 0;  // calls so far that reach this row
-        for (int c0 = 0; c0 < n; c0 += 32) {
-            // 32 calls' records at once, one per lane
-            const int i = c0 + lane;
-            const int4 cr = i < n ? P.crec[i] : make_int4(INT_MAX, 0, 0, 0);
-            const bool reach = cr.x <= r;
-            int o0 = 0, o1 = 0;
-            if (i < n) {
-                o0 = P.bandoff[(size_t)b * n + i];
-                o1 = P.bandoff[(size_t)(b + 1) * n + i];
+    unsigned m = 0;  // sums handed on so far
+    for (unsigned phase = 0;; phase ^= 1) {
+        // the next unit: tile `unit % n_tiles`, call batch `unit / n_tiles`, once the tile's batch before
+        // is on the canvas (its CTA took it from the queue earlier, so it is running or done)
+        if (threadIdx.x == 0) {
+            const int u = (int)atomicAdd(&P.queue[3], 1u);
+            s_unit = u;
+            if (u >= n_tiles && u < n_tiles * P.tile_batches &&
+                !tile_wait(P.tile_done + u % n_tiles, (unsigned)(u / n_tiles)))
+                ok = false;
+        }
+        ok = __syncthreads_and(ok) != 0;
+        const int unit = s_unit;
+        if (unit >= n_tiles * P.tile_batches) break;
+        const int tix = unit % n_tiles, batch = unit / n_tiles;
+        const int X0 = tix % per_row * span;  // the tile's pixels: rows y0 .., columns X0 ..
+        const int y0 = tix / per_row * T.rows;
+        const int r = y0 + wrow, x0 = X0 + seg * sw;
+        unsigned* crow = reinterpret_cast<unsigned*>(P.rasters + (size_t)r * P.canvas_stride) + x0;
+        const int xend = min(sw, W - x0);                 // the segment's pixels on the canvas
+        const int qend = xend > 0 ? (xend + 3) >> 2 : 0;  // and quads
+        const int n_box = (min(span, W - X0) + BW - 1) / BW;
+        // a quad of this warp: in the shared tile (staged by TMA; pixels right of the canvas are
+        // never stored), or in place in global memory, pixel by pixel
+        auto quad = [&](int k) {
+            const int x = seg * sw + 4 * k;
+            return reinterpret_cast<uint4*>(tile + (((x >> bw_shift) * T.rows + wrow) << bw_shift) + (x & (BW - 1)));
+        };
+        auto get = [&](int k) {
+            if (STAGED) return *quad(k);
+            const unsigned* p = crow + 4 * k;
+            const int left = xend - 4 * k;
+            return make_uint4(p[0], left > 1 ? p[1] : 0u, left > 2 ? p[2] : 0u, left > 3 ? p[3] : 0u);
+        };
+        auto put = [&](int k, uint4 v) {
+            if (STAGED) {
+                *quad(k) = v;
+                return;
             }
-            const unsigned rmask = __ballot_sync(FULL, reach);
-            unsigned dmask = __ballot_sync(FULL, reach && o1 > o0);
-            const unsigned long long my_first =
-                ((unsigned long long)(unsigned)cr.z | ((unsigned long long)(unsigned)cr.w << 32)) + (unsigned)o0;
-            unsigned my_clr = 0;
-            if (reach && o1 > o0) {
-                const ft_path_desc& d = P.paths[i];
-                my_clr = (unsigned)d.clr[0] | ((unsigned)d.clr[1] << 8) | ((unsigned)d.clr[2] << 16) |
-                         ((unsigned)d.clr[3] << 24);
-            }
-            while (dmask) {
-                const int j = __ffs(dmask) - 1;
-                dmask &= dmask - 1;
-                const int Gj = G + __popc(rmask & ((1u << j) - 1u));
-                const unsigned long long first = __shfl_sync(FULL, my_first, j);
-                const int ne = __shfl_sync(FULL, o1 - o0, j);
-                const int y = r + __shfl_sync(FULL, cr.y, j);
-                const unsigned clr = __shfl_sync(FULL, my_clr, j);
-                // cells of the band edges crossing scan row y, inside the segment
-                unsigned carry = 0;
-                const int4* E = reinterpret_cast<const int4*>(P.pool + first);
-                for (int e = lane; e < ne; e += 32) {
-                    const int4 hb = E[2 * e + 1];  // step_pix, ed, start_row, end_row
-                    const int4 ha = E[2 * e];      // y_upper, y_lower, x_bot0, inv_slope
-                    if (y < hb.z || y > hb.w) continue;
-                    const int x_bot = wadd(ha.z, wmul(y - hb.z, ha.w));
-                    seg_row(x_bot, ha.w, y == hb.z, y == hb.w, fxfract(ha.x), fxfract(ha.y), hb.x > 0 ? hb.x : FX_ONE,
-                            hb.y, area, x0, sw, W, carry, bmap);
+            unsigned* p = crow + 4 * k;
+            const int left = xend - 4 * k;
+            p[0] = v.x;
+            if (left > 1) p[1] = v.y;
+            if (left > 2) p[2] = v.z;
+            if (left > 3) p[3] = v.w;
+        };
+        if (STAGED && ok && threadIdx.x == 0) {
+            asm volatile("fence.proxy.async;" ::: "memory");  // the canvas, acquired, before the copy reads it
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)),
+                         "r"(n_box * T.rows * BW * 4)
+                         : "memory");
+            for (int bx = 0; bx < n_box; bx++)
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+                    "%3}], [%4];" ::"r"(smem_u32(tile + bx * T.rows * BW)),
+                    "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(X0 + bx * BW), "r"(y0), "r"(smem_u32(mbar))
+                    : "memory");
+        }
+        for (int k = lane; k < sw / 4; k += 32) last[k] = 0;
+        if (STAGED && ok) ok = mbar_wait(mbar, phase);
+        ok = __syncthreads_and(ok) != 0;
+        if (ok && r < H) {
+            // the segment's bin of the band, and the band's bins (a call with edges in any of them is
+            // walked by all of the row's warps)
+            const int b = r / R, s1 = x0 + max(xend, 0);
+            const int *bin = P.bandoff + (size_t)(b * T.segs + seg) * n, *bin0 = P.bandoff + (size_t)(b * T.segs) * n;
+            const int call0 = (int)((long long)n * batch / P.tile_batches);
+            const int call1 = (int)((long long)n * (batch + 1) / P.tile_batches);
+            int G = 0;  // calls so far that reach this row
+            for (int c0 = call0; c0 < call1; c0 += 32) {
+                // 32 calls' records at once, one per lane
+                const int i = c0 + lane;
+                const int4 cr = i < call1 ? P.crec[i] : make_int4(INT_MAX, 0, 0, 0);
+                const bool reach = cr.x <= r;
+                int o0 = 0, o1 = 0;
+                bool any = false;
+                if (i < call1) {
+                    o0 = bin[i];
+                    o1 = bin[i + n];
+                    any = T.segs > 1 ? bin0[i] < bin0[i + (size_t)T.segs * n] : o0 < o1;
                 }
-                carry = warp_sum_u(carry);
+                const unsigned rmask = __ballot_sync(FULL, reach);
+                unsigned dmask = __ballot_sync(FULL, reach && any);
+                const unsigned long long my_first =
+                    ((unsigned long long)(unsigned)cr.z | ((unsigned long long)(unsigned)cr.w << 32)) + (unsigned)o0;
+                unsigned my_clr = 0;
+                if (reach && any) my_clr = *reinterpret_cast<const unsigned*>(P.paths[i].clr);
+                if (has_out && ok) {  // room for this round's sums
+                    unsigned v;
+                    ok = __all_sync(FULL, smem_wait(out + CT_CHAIN, v, [&](unsigned d) { return m - d <= CT_CHAIN - 32; }));
+                }
                 __syncwarp();
-                // the touched chunks, in order
-                int T = 0;
-                for (int w = 0; w < nwords; w++) {
-                    const unsigned bw = bmap[w];
-                    if (((bw >> lane) & 1u) && ck(T + __popc(bw & lt) < nchunks, 8))
-                        clist[T + __popc(bw & lt)] = (unsigned char)(32 * w + lane);
-                    T += __popc(bw);
-                }
-                __syncwarp();
-                if (lane < nwords) bmap[lane] = 0u;
-                auto compose = [&](int x, unsigned av) {
-                    if (!ck(x >= 0 && x < xend, 10)) return;
-                    unsigned* p = px(x);
-                    unsigned dv = *p;
-                    const int kk = min((Gj - (int)last[x]) & 255, 15);
-                    if (kk) dv = ftab4(ftab, dv, kk);
-                    *p = srcover_rgba(dv, clr, av);
-                    last[x] = (unsigned char)(Gj + 1);
-                };
-                // the run before the first touched chunk holds the carry
-                {
-                    const unsigned av0 = resolve_cov(carry, rule);
-                    if (av0) {
-                        const int end = min(T ? (int)clist[0] * 8 : sw, xend);
-                        for (int x = lane; x < end; x += 32) compose(x, av0);
+                while (dmask) {
+                    const int j = __ffs(dmask) - 1;
+                    dmask &= dmask - 1;
+                    const unsigned long long first = __shfl_sync(FULL, my_first, j);
+                    const int ne = __shfl_sync(FULL, o1 - o0, j);
+                    const int y = r + __shfl_sync(FULL, cr.y, j);
+                    const int4* E = reinterpret_cast<const int4*>(P.pool + first);
+                    if (dmask) {  // the next call's first edges, on their way meanwhile
+                        const unsigned long long nf = __shfl_sync(FULL, my_first, __ffs(dmask) - 1);
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.pool + nf + lane));
                     }
-                }
-                unsigned base = carry;
-                for (int t0 = 0; t0 < T; t0 += 32) {
-                    const int t = t0 + lane;
-                    const bool valid = t < T;
-                    const int ch = valid ? clist[t] : 0;
-                    int4 a0 = make_int4(0, 0, 0, 0), a1 = a0;
-                    if (valid) {
-                        int4* ap = reinterpret_cast<int4*>(area + ch * 8);
-                        a0 = ap[0];
-                        a1 = ap[1];
-                        ap[0] = make_int4(0, 0, 0, 0);
-                        ap[1] = make_int4(0, 0, 0, 0);
+                    unsigned base = 0;  // the running sum entering the segment
+                    for (int e = lane; e < ne; e += 32) {
+                        const int4 hb = E[2 * e + 1];  // step_pix, ed, start_row, end_row
+                        const int4 ha = E[2 * e];      // y_upper, y_lower, x_bot0, inv_slope
+                        if (hb.z <= y && y <= hb.w) row_cells(ha, hb, y, area, reinterpret_cast<unsigned*>(bmap), x0, s1, base);
                     }
-                    const unsigned csum = (unsigned)a0.x + (unsigned)a0.y + (unsigned)a0.z + (unsigned)a0.w +
-                                          (unsigned)a1.x + (unsigned)a1.y + (unsigned)a1.z + (unsigned)a1.w;
-                    const unsigned inc = warp_incl_sum_u(csum);
-                    unsigned run = base + inc - csum;
-                    base += __shfl_sync(FULL, inc, 31);
-                    const int av_v[8] = {(int)a0.x, (int)a0.y, (int)a0.z, (int)a0.w,
-                                         (int)a1.x, (int)a1.y, (int)a1.z, (int)a1.w};
-                    unsigned w0 = 0, w1 = 0;
+                    base = X0 ? __reduce_add_sync(FULL, base) : 0u;
+                    // a barrier of this warp alone: after the edge loops' divergent ends the lanes went on
+                    // in groups through all that follows, which __syncwarp did not undo (5.9 / 3.7 ms for
+                    // 768 strokes)
+                    asm volatile("bar.sync %0, 32;" ::"r"(1 + warp) : "memory");
+                    // the touched chunks, in order
+                    const uint4 bw = *bmap;
+                    const unsigned bws[4] = {bw.x, bw.y, bw.z, bw.w};
+                    int nt = 0;
 #pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        run += (unsigned)av_v[k];
-                        const unsigned v = (valid && ch * 8 + k < xend) ? resolve_cov(run, rule) : 0u;
-                        if (k < 4)
-                            w0 |= v << (8 * k);
-                        else
-                            w1 |= v << (8 * (k - 4));
-                    }
-                    // the gap after this chunk up to the next touched one holds `run`
-                    const int nxt = t + 1 < T ? (int)clist[t + 1] : nchunks;
-                    const unsigned gav = valid ? resolve_cov(run, rule) : 0u;
-                    const int g0 = ch * 8 + 8, g1 = min(nxt * 8, xend);
-                    const bool has_gap = gav && g0 < g1;
-                    auto nzb = [](unsigned w) { return (((w & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | w) & 0x80808080u; };
-                    const int cnt = __popc(nzb(w0)) + __popc(nzb(w1));
-                    const unsigned cinc = warp_incl_sum_u((unsigned)cnt);
-                    const int tot = (int)__shfl_sync(FULL, cinc, 31);
-                    const unsigned gm = __ballot_sync(FULL, has_gap);
-                    int pos = (int)(cinc - (unsigned)cnt);
-#pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        const unsigned v = ((k < 4 ? w0 : w1) >> (8 * (k & 3))) & 0xFFu;
-                        if (v && ck(pos < 256, 9)) q[pos++] = ((unsigned)(ch * 8 + k) << 8) | v;
-                    }
-                    if (has_gap) q[256 + __popc(gm & lt)] = ((unsigned)g0 << 19) | ((unsigned)(g1 - g0) << 8) | gav;
-                    __syncwarp();
-                    for (int k = lane; k < tot; k += 32) {
-                        const unsigned e = q[k];
-                        compose((int)(e >> 8), e & 255u);
-                    }
-                    for (unsigned m = gm; m; m &= m - 1) {  // the gap runs, all lanes on each
-                        const unsigned e = q[256 + __popc(gm & ((1u << (__ffs(m) - 1)) - 1u))];
-                        const int gs = (int)(e >> 19), gl = (int)((e >> 8) & 0x7FF);
-                        for (int x = gs + lane; x < gs + gl; x += 32) compose(x, e & 255u);
+                    for (int w = 0; w < 4; w++) {
+                        const int at = nt + __popc(bws[w] & lt);
+                        if (((bws[w] >> lane) & 1u) && ck(at < sw / 8, 8)) clist[at] = (unsigned char)(32 * w + lane);
+                        nt += __popc(bws[w]);
                     }
                     __syncwarp();
+                    if (lane == 0) *bmap = make_uint4(0, 0, 0, 0);
+                    __syncwarp();
+                    const unsigned clr = __shfl_sync(FULL, my_clr, j);
+                    const unsigned w0 = wide8(clr & 0xFFu), w1 = wide8((clr >> 8) & 0xFFu),
+                                   w2 = wide8((clr >> 16) & 0xFFu), w3 = wide8(clr >> 24);
+                    const int Gj = G + __popc(rmask & ((1u << j) - 1u));
+                    m++;
+                    if (has_in && ok) {  // sums are multiples of 2^16: the count is in the lower half
+                        unsigned v = 0;
+                        ok = __all_sync(FULL, smem_wait(in + (m & (CT_CHAIN - 1)), v,
+                                                        [&](unsigned d) { return ((d ^ m) & 0xFFFFu) == 0; }));
+                        base = v & 0xFFFF0000u;
+                    }
+                    __syncwarp();
+                    // the run at hand (quads [run_k, run_e) of alpha run_a, in every byte): at first the
+                    // one before the first touched chunk, which holds the sum entering the segment
+                    unsigned run_a = resolve4<RULE>((int)base, (int)base, (int)base, (int)base);
+                    int run_k = 0, run_e = run_a ? min(nt ? (int)clist[0] * 2 : qend, qend) : 0;
+                    unsigned gm = 0;      // runs of the round still to be queued
+                    int t0 = 0, cnt = 0;  // chunks done, quads queued
+                    bool sent = !has_out;
+                    for (;;) {
+                        if (cnt < 32) {
+                            if (run_k >= run_e && gm) {
+                                const unsigned rec = runs[__ffs(gm) - 1];
+                                gm &= gm - 1;
+                                run_k = (int)(rec >> 20);
+                                run_e = (int)((rec >> 8) & 0xFFF);
+                                run_a = (rec & 0xFFu) * 0x01010101u;
+                            }
+                            if (run_k < run_e) {
+                                const int k = run_k + lane, add = min(run_e - run_k, 32);
+                                if (k < run_e && ck(cnt + lane < CT_QN, 9)) {
+                                    q[cnt + lane] = run_a;
+                                    qi[cnt + lane] = (unsigned char)k;
+                                }
+                                run_k += add;
+                                cnt += add;
+                                __syncwarp();
+                                continue;
+                            }
+                            if (t0 < nt) {
+                                const int t = t0 + lane;
+                                const bool valid = t < nt;
+                                const int ch = valid ? clist[t] : 0;
+                                unsigned s[8], inc;
+                                take8(area + ch * 8, valid, lane, s, inc);
+                                const uint2 px = pixels8<RULE>(s, inc - s[7] + base, 1);
+                                base += __shfl_sync(FULL, inc, 31);
+                                // the gap after this chunk up to the next touched one holds its last sum
+                                const int g0 = ch * 2 + 2, g1 = min((t + 1 < nt ? (int)clist[t + 1] : sw / 8) * 2, qend);
+                                const unsigned ga = px.y >> 24;
+                                gm = __ballot_sync(FULL, valid && ga && g0 < g1);
+                                if (valid) runs[lane] = ((unsigned)g0 << 20) | ((unsigned)g1 << 8) | ga;
+                                const bool a0 = valid && px.x && ch * 2 < qend, a1 = valid && px.y && ch * 2 + 1 < qend;
+                                const unsigned m0 = __ballot_sync(FULL, a0), m1 = __ballot_sync(FULL, a1);
+                                const int at = cnt + __popc(m0 & lt) + __popc(m1 & lt), at1 = at + (a0 ? 1 : 0);
+                                if (a0 && ck(at < CT_QN, 9)) {
+                                    q[at] = px.x;
+                                    qi[at] = (unsigned char)(ch * 2);
+                                }
+                                if (a1 && ck(at1 < CT_QN, 9)) {
+                                    q[at1] = px.y;
+                                    qi[at1] = (unsigned char)(ch * 2 + 1);
+                                }
+                                cnt += __popc(m0) + __popc(m1);
+                                t0 += 32;
+                                __syncwarp();
+                                continue;
+                            }
+                            if (!sent) {
+                                if (lane == 0)
+                                    *reinterpret_cast<volatile unsigned*>(out + (m & (CT_CHAIN - 1))) = base | (m & 0xFFFFu);
+                                sent = true;
+                                __syncwarp();
+                            }
+                            if (cnt == 0) break;
+                        }
+                        // composite 32 queued quads (the last of a call: what there is)
+                        const int at = max(cnt - 32, 0) + lane;
+                        if (at < cnt) {
+                            const unsigned a = q[at];
+                            const int k = qi[at];
+                            if (ck(k < qend, 10)) {
+                                uint4 d = get(k);
+                                const int kk = min((Gj - (int)last[k]) & 255, 15);
+                                last[k] = (unsigned char)(Gj + 1);
+                                d.x = srcover_wide(alpha0_pow(d.x, kk), w0, w1, w2, w3, a & 0xFFu);
+                                d.y = srcover_wide(alpha0_pow(d.y, kk), w0, w1, w2, w3, (a >> 8) & 0xFFu);
+                                d.z = srcover_wide(alpha0_pow(d.z, kk), w0, w1, w2, w3, (a >> 16) & 0xFFu);
+                                d.w = srcover_wide(alpha0_pow(d.w, kk), w0, w1, w2, w3, a >> 24);
+                                put(k, d);
+                            }
+                        }
+                        cnt = max(cnt - 32, 0);
+                        __syncwarp();
+                    }
+                }
+                __syncwarp();
+                if (has_in && lane == 0) *reinterpret_cast<volatile unsigned*>(in + CT_CHAIN) = m;
+                const int G0 = G;
+                G += __popc(rmask);
+                if ((G0 >> 6) != (G >> 6)) {
+                    // every 64 calls: pending counts of 15 or more saturate, so a quad's stamp
+                    // moves up to 15 calls behind; the u8 differences then stay below 256
+                    for (int k = lane; k < sw / 4; k += 32)
+                        if (((G - (int)last[k]) & 255) > 15) last[k] = (unsigned char)(G - 15);
+                    __syncwarp();
                 }
             }
-            const int G0 = G;
-            G += __popc(rmask);
-            if ((G0 >> 6) != (G >> 6)) {
-                // every 64 calls: pending counts of 15 or more saturate, so a pixel's stamp
-                // moves up to 15 calls behind; the u8 differences then stay below 256
-                __syncwarp();
-                for (int x = lane; x < sw; x += 32)
-                    if (((G - (int)last[x]) & 255) > 15) last[x] = (unsigned char)(G - 15);
-                __syncwarp();
+            // the alpha-0 composites still pending since each quad's last visit
+            for (int k = lane; k < qend; k += 32) {
+                const int kk = min((G - (int)last[k]) & 255, 15);
+                if (kk) {
+                    uint4 d = get(k);
+                    d.x = alpha0_pow(d.x, kk);
+                    d.y = alpha0_pow(d.y, kk);
+                    d.z = alpha0_pow(d.z, kk);
+                    d.w = alpha0_pow(d.w, kk);
+                    put(k, d);
+                }
             }
         }
-        // the alpha-0 composites still pending since each pixel's last cover
-        __syncwarp();
-        for (int x = lane; x < xend; x += 32) {
-            const int kk = min((G - (int)last[x]) & 255, 15);
-            if (kk) {
-                unsigned* p = px(x);
-                *p = ftab4(ftab, *p, kk);
+        if (STAGED) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        ok = __syncthreads_and(ok) != 0;
+        if (threadIdx.x == 0) {
+            if (!ok) atomicMax(&P.status[0], FT_ERR_TIMEOUT);
+            if (STAGED && ok) {
+                for (int bx = 0; bx < n_box; bx++)
+                    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                                     reinterpret_cast<uint64_t>(&tmap)),
+                                 "r"(X0 + bx * BW), "r"(y0), "r"(smem_u32(tile + bx * T.rows * BW))
+                                 : "memory");
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                asm volatile("fence.proxy.async;" ::: "memory");
             }
-        }
-    }
-    if (tma) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (ok && threadIdx.x == 0) {
-            for (int bx = 0; bx < sw / BW; bx++)
-                asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                                 reinterpret_cast<uint64_t>(&tmap)),
-                             "r"(x0 + bx * BW), "r"(b * R), "r"(smem_u32(tile + bx * R * BW))
-                             : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __threadfence();
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.tile_done + tix), "r"((unsigned)batch + 1u) : "memory");
         }
     }
 }
@@ -2437,16 +2602,39 @@ cudaError_t launch_srcover_mask(const CUtensorMap& canvas, const CUtensorMap& ma
     return cudaGetLastError();
 }
 
-int composite_tile_smem(int band_rows, int seg_w, bool staged) { return ctile_layout(band_rows, seg_w, staged).bytes; }
+int composite_tile_rows(int band_rows, int bin_segs) { return ctile_shape(band_rows, bin_segs).rows; }
+int composite_tile_smem(int band_rows, int bin_segs, int seg_w, bool staged) {
+    return ctile_layout(ctile_shape(band_rows, bin_segs), seg_w, staged).bytes;
+}
+int composite_tiles(const KParams& p) {
+    const CTileShape t = ctile_shape(p.band_rows, p.bin_segs);
+    const int span = t.segs * p.seg_w;
+    return ((int)p.canvas_h + t.rows - 1) / t.rows * (((int)p.canvas_w + span - 1) / span);
+}
 
-cudaError_t launch_composite_tiles(const KParams& p, const CUtensorMap& tmap, cudaStream_t s) {
-    const bool staged = p.use_tma != 0;
-    const int smem = composite_tile_smem(p.band_rows, p.seg_w, staged);
-    auto kern = staged ? k_ctile<true> : k_ctile<false>;
+cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_count, cudaStream_t s) {
+    const bool staged = p.use_tma != 0, odd = p.rule == FT_EVENODD;
+    const CTileShape t = ctile_shape(p.band_rows, p.bin_segs);
+    const int smem = ctile_layout(t, p.seg_w, staged).bytes;
+    auto kern = staged ? (odd ? k_ctile<true, FT_EVENODD> : k_ctile<true, FT_NONZERO>)
+                       : (odd ? k_ctile<false, FT_EVENODD> : k_ctile<false, FT_NONZERO>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const int nseg = ((int)p.canvas_w + p.seg_w - 1) / p.seg_w;
-    kern<<<p.n_bands * nseg, 32 * p.band_rows, smem, s>>>(p, tmap);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    const int threads = 32 * t.rows * t.segs;
+    int per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
+    const int tiles = composite_tiles(p), slots = std::max(1, per_sm) * sm_count;
+    // A tile beyond the resident ones would be composited alone, from the first call to the last
+    // (1,024 tiles on 912 places take twice as long as 912): the calls are cut into batches, every
+    // tile's first batch goes before any second, and the count with the least left over is taken.
+    p.tile_batches = 1;
+    auto rounds = [&](int nb) { return (double)(((long long)tiles * nb + slots - 1) / slots) / nb; };
+    if (tiles > slots)
+        for (int nb = 2; nb <= 16 && (int)p.n_items >= 32 * nb; nb++)
+            if (rounds(nb) < 0.97 * rounds(p.tile_batches)) p.tile_batches = nb;
+    if (p.tile_batches > 1 && (e = cudaMemsetAsync(p.tile_done, 0, sizeof(unsigned) * tiles, s)) != cudaSuccess) return e;
+    kern<<<(int)std::min<long long>((long long)tiles * p.tile_batches, slots), threads, smem, s>>>(p, tmap);
     return cudaGetLastError();
 }
 

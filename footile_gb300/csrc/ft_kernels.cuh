@@ -223,6 +223,9 @@ struct KParams {
     // whether the canvas is staged by TMA through the tensor map passed beside these
     int seg_w;
     int use_tma;
+    int bin_segs;         // segments of seg_w pixels that a band's edges are binned by (1: not)
+    int tile_batches;     // batches the calls are cut into (k_ctile)
+    unsigned* tile_done;  // per tile: batches done
     // one fill path built over the whole GPU (launch_grid_build) instead of by k_cbuild
     GridBuildBufs gb;
     GridStrokeBufs gs;  // and the stroker's part of one stroke path (launch_grid_stroke)
@@ -284,8 +287,12 @@ cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cu
 cudaError_t launch_composite_build(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas);
 cudaError_t launch_composite_bands(const KParams& p, int smem_bytes, cudaStream_t s);
 // Rgba8p: tiles of band_rows x seg_w pixels, canvas staged through `tmap` when use_tma.
-cudaError_t launch_composite_tiles(const KParams& p, const CUtensorMap& tmap, cudaStream_t s);
-int composite_tile_smem(int band_rows, int seg_w, bool staged);
+// p.tile_done: composite_tiles(p) words, p.queue[3] zero.
+cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_count, cudaStream_t s);
+int composite_tiles(const KParams& p);
+constexpr int CT_MAX_SEGS = 4;  // segments of a row in one tile
+int composite_tile_smem(int band_rows, int bin_segs, int seg_w, bool staged);
+int composite_tile_rows(int band_rows, int bin_segs);  // rows of a tile (and of its tensor-map boxes)
 // SrcOver of one call's colour onto the canvas rows r0.. from its Matte8 coverage `mask`
 // (both as 2-D tensor maps with boxes of SO_COLS x SO_ROWS elements: the kernel's stage
 // size and its expected transaction bytes derive from the same two constants), streamed
