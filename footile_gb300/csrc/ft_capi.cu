@@ -1476,7 +1476,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
 namespace ftc {
 cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride, uint8_t* dst, uint32_t dst_stride,
                            uint32_t w, uint32_t h, const uint8_t* lut, int grid, cudaStream_t s);
-int convert_blocks_per_sm();
+int convert_block();
+int convert_blocks_per_sm(int src_fmt);
 cudaError_t launch_srcover(bool backward, const float* cov, uint32_t n_layers, uint64_t plane, const float4* clr,
                            const float4* init, float4* out, const float4* grad_out, float* grad_cov,
                            float4* grad_init, uint32_t n_px, int grid, cudaStream_t s, bool partial = false);
@@ -1824,9 +1825,10 @@ FT_API int ft_convert(ft_ctx* c, int32_t src_fmt, const uint8_t* src, uint32_t s
         s_d = static_cast<const uint8_t*>(c->conv_src.p);
         d_d = static_cast<uint8_t*>(c->conv_dst.p);
     }
-    const uint64_t work = (row / 16 + row % 16) * h;
+    const uint64_t work = (row * h + 15) / 16;  // 16 bytes a thread
     const int grid = (int)std::max<uint64_t>(
-        1, std::min<uint64_t>((work + 255) / 256, (uint64_t)c->sm_count * ftc::convert_blocks_per_sm()));
+        1, std::min<uint64_t>((work + ftc::convert_block() - 1) / ftc::convert_block(),
+                              (uint64_t)c->sm_count * ftc::convert_blocks_per_sm(src_fmt)));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     FT_CU(ftc::launch_convert(src_fmt, s_d, src_stride, d_d, dst_stride, w, h,

@@ -6,8 +6,7 @@
 // examples/drop.rs:22): straight alpha (channel / alpha) and the sRGB transfer
 // function.  The conversion of one channel depends only on (alpha, channel), so it is a
 // 256 x 256 byte table the host builds once (correctly rounded sRGB encoding of
-// channel / alpha, IEC 61966-2-1) and every thread reads from shared memory.  The
-// kernel streams 16-byte vectors: 4 Rgba8p or 16 Matte8 pixels per thread and step.
+// channel / alpha, IEC 61966-2-1) and every thread reads from shared memory.
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -15,89 +14,108 @@
 
 namespace ftc {
 
-constexpr int CBLOCK = 256;
+// A memory stream (8192 x 8192 Rgba8p: 537 MB, 79 us at the copy rate) held back by its lookups,
+// three bytes from random words per pixel (3.4 accesses of the 32 banks each): what helps is
+// warps, 64 per SM on two tables.  Matte8 reads only the row of alpha 255, which is held with a
+// column of words per lane, so that lanes never meet.  Rasters without padding between the rows
+// are one row.  24 warps per SM, three tables and a 64-bit divide per 16 bytes: 110.8 us; this way
+// 90.6 us (two loads of a thread in flight 99 us; the alpha 255 row in columns for Rgba8p too,
+// beside the table, 120 us).  Matte8 45 / 35 us.  1531 x 1117, whose rows start at any word, byte
+// by byte 53 us, as one row 18 us.
+constexpr int CBLOCK = 1024;
+constexpr int FULL_ROW = 64 * 32 * 4;  // the columns
+__host__ __device__ constexpr int convert_smem(bool rgba) { return rgba ? 256 * 256 : FULL_ROW; }
 
-__device__ __forceinline__ uint4 convert16(uint4 v, int src_fmt, const uint8_t* lut) {
-    unsigned* u = reinterpret_cast<unsigned*>(&v);
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const unsigned p = u[j];
-        if (src_fmt == FT_RGBA8P) {
-            const unsigned a = p >> 24, row = a << 8;
-            u[j] = (unsigned)lut[row | (p & 0xFF)] | ((unsigned)lut[row | ((p >> 8) & 0xFF)] << 8) |
-                   ((unsigned)lut[row | ((p >> 16) & 0xFF)] << 16) | (a << 24);
-        } else {  // Matte8: the mask byte is linear gray at full alpha
-            u[j] = (unsigned)lut[0xFF00 | (p & 0xFF)] | ((unsigned)lut[0xFF00 | ((p >> 8) & 0xFF)] << 8) |
-                   ((unsigned)lut[0xFF00 | ((p >> 16) & 0xFF)] << 16) | ((unsigned)lut[0xFF00 | (p >> 24)] << 24);
-        }
-    }
+__device__ __forceinline__ unsigned byte_at(unsigned addr) {  // of shared memory
+    unsigned v;
+    asm("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-
-// Persistent grid (one CTA per resident slot, each loads the table once).  Rows are
-// cut into 16-byte groups; a thread takes UNROLL groups per step and issues all their
-// loads before converting, which keeps enough bytes in flight for HBM.  Row tails
-// (and rows that are not 16-byte aligned) go byte by byte.  `lut[a * 256 + c]`:
-// straight, sRGB-encoded channel.
-constexpr int UNROLL = 4;
-__global__ void __launch_bounds__(CBLOCK) k_convert(int src_fmt, const uint8_t* __restrict__ src, uint32_t src_stride,
-                                                    uint8_t* __restrict__ dst, uint32_t dst_stride, uint32_t w,
-                                                    uint32_t h, const uint8_t* __restrict__ lut_g) {
-    __shared__ __align__(16) uint8_t lut[256 * 256];
-    for (int i = threadIdx.x; i < 256 * 256 / 16; i += CBLOCK)
-        reinterpret_cast<uint4*>(lut)[i] = reinterpret_cast<const uint4*>(lut_g)[i];
-    __syncthreads();
-    const uint32_t row_bytes = src_fmt == FT_RGBA8P ? 4 * w : w;
-    const bool vec = ((src_stride | dst_stride) & 15) == 0 &&
-                     ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
-    const uint32_t groups = vec ? row_bytes / 16 : 0;  // 16-byte groups per row
-    const uint64_t n_groups = (uint64_t)groups * h;
-    const uint64_t nthreads = (uint64_t)gridDim.x * CBLOCK;
-    for (uint64_t t0 = (uint64_t)blockIdx.x * CBLOCK + threadIdx.x; t0 < n_groups; t0 += nthreads * UNROLL) {
-        uint4 v[UNROLL];
-        uint64_t g[UNROLL];
-#pragma unroll
-        for (int j = 0; j < UNROLL; j++) {
-            g[j] = t0 + (uint64_t)j * nthreads;
-            if (g[j] < n_groups) {
-                const uint32_t y = (uint32_t)(g[j] / groups), k = (uint32_t)(g[j] - (uint64_t)y * groups);
-                v[j] = reinterpret_cast<const uint4*>(src + (size_t)y * src_stride)[k];
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < UNROLL; j++) {
-            if (g[j] < n_groups) {
-                const uint32_t y = (uint32_t)(g[j] / groups), k = (uint32_t)(g[j] - (uint64_t)y * groups);
-                reinterpret_cast<uint4*>(dst + (size_t)y * dst_stride)[k] = convert16(v[j], src_fmt, lut);
-            }
-        }
+// lut: the table (a * 256 + c), for Matte8 the lane's column, as a shared address
+template <bool RGBA>
+__device__ __forceinline__ unsigned convert_e(unsigned p, unsigned lut) {
+    const unsigned c0 = p & 0xFFu, c1 = (p >> 8) & 0xFFu, c2 = (p >> 16) & 0xFFu, c3 = p >> 24;
+    if (RGBA) {
+        const unsigned row = lut + (c3 << 8);
+        return byte_at(row + c0) | (byte_at(row + c1) << 8) | (byte_at(row + c2) << 16) | (p & 0xFF000000u);
     }
-    // row tails
-    const uint32_t tail = row_bytes - groups * 16;
-    const uint64_t n_tail = (uint64_t)tail * h;
-    for (uint64_t t = (uint64_t)blockIdx.x * CBLOCK + threadIdx.x; t < n_tail; t += nthreads) {
-        const uint32_t y = (uint32_t)(t / tail), b = groups * 16 + (uint32_t)(t - (uint64_t)y * tail);
-        const uint8_t* s = src + (size_t)y * src_stride;
-        uint8_t* d = dst + (size_t)y * dst_stride;
-        if (src_fmt == FT_RGBA8P) {
-            const uint32_t px = b >> 2, ch = b & 3;
-            const unsigned a = s[4 * px + 3];
-            d[b] = ch == 3 ? (uint8_t)a : lut[(a << 8) | s[b]];
+    auto at = [&](unsigned c) { return byte_at(lut + (((c & 0xFCu) << 5) | (c & 3u))); };
+    return at(c0) | (at(c1) << 8) | (at(c2) << 16) | (at(c3) << 24);
+}
+template <bool RGBA>
+__device__ __forceinline__ uint4 convert_e(uint4 v, unsigned lut) {
+    return make_uint4(convert_e<RGBA>(v.x, lut), convert_e<RGBA>(v.y, lut), convert_e<RGBA>(v.z, lut),
+                      convert_e<RGBA>(v.w, lut));
+}
+
+// `n` elements of T per row, from byte `off` of each
+template <bool RGBA, class T>
+__device__ __forceinline__ void convert_rows(const uint8_t* src, uint64_t src_stride, uint8_t* dst, uint64_t dst_stride,
+                                             uint64_t off, uint64_t n, uint32_t h, unsigned lut) {
+    const uint64_t total = n * h;
+    for (uint64_t i = (uint64_t)blockIdx.x * CBLOCK + threadIdx.x; i < total; i += (uint64_t)gridDim.x * CBLOCK) {
+        uint64_t y = 0;
+        if (h > 1) y = total >> 32 ? i / n : (uint32_t)i / (uint32_t)n;
+        const uint64_t at = off + (i - y * n) * sizeof(T);
+        *reinterpret_cast<T*>(dst + y * dst_stride + at) =
+            convert_e<RGBA>(*reinterpret_cast<const T*>(src + y * src_stride + at), lut);
+    }
+}
+
+template <bool RGBA>
+__global__ void __launch_bounds__(CBLOCK, 2) k_convert(const uint8_t* src, uint32_t src_stride, uint8_t* dst,
+                                                       uint32_t dst_stride, uint32_t w, uint32_t h,
+                                                       const uint8_t* __restrict__ lut_g) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    if (RGBA) {
+        for (int i = threadIdx.x; i < 256 * 256 / 16; i += CBLOCK)
+            reinterpret_cast<uint4*>(smem)[i] = reinterpret_cast<const uint4*>(lut_g)[i];
+    } else {
+        for (int i = threadIdx.x; i < FULL_ROW / 4; i += CBLOCK)
+            reinterpret_cast<unsigned*>(smem)[i] = reinterpret_cast<const unsigned*>(lut_g + 0xFF00)[i >> 5];
+    }
+    __syncthreads();
+    const unsigned lut = (unsigned)__cvta_generic_to_shared(smem) + (RGBA ? 0 : 4 * (threadIdx.x & 31));
+    uint64_t row_bytes = RGBA ? 4ull * w : w;
+    if (src_stride == row_bytes && dst_stride == row_bytes) {
+        row_bytes *= h;
+        h = 1;
+    }
+    const uintptr_t align = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) |
+                            (h > 1 ? (uintptr_t)(src_stride | dst_stride) : 0);
+    const uint64_t vec = align & 15 ? 0 : row_bytes / 16, words = align & 3 ? 0 : (row_bytes - vec * 16) / 4;
+    if (vec) convert_rows<RGBA, uint4>(src, src_stride, dst, dst_stride, 0, vec, h, lut);
+    if (words) convert_rows<RGBA, unsigned>(src, src_stride, dst, dst_stride, vec * 16, words, h, lut);
+    // the last bytes of Matte8 rows; all of rows that start at any byte
+    const uint64_t done = vec * 16 + words * 4, tail = row_bytes - done, n_tail = tail * h;
+    for (uint64_t t = (uint64_t)blockIdx.x * CBLOCK + threadIdx.x; t < n_tail; t += (uint64_t)gridDim.x * CBLOCK) {
+        const uint64_t y = t / tail, b = done + (t - y * tail);
+        const uint8_t* s = src + y * src_stride;
+        uint8_t* d = dst + y * dst_stride;
+        if (!RGBA) {
+            d[b] = lut_g[0xFF00 | s[b]];
         } else {
-            d[b] = lut[0xFF00 | s[b]];
+            const unsigned a = s[b | 3];
+            d[b] = (b & 3) == 3 ? (uint8_t)a : smem[(a << 8) | s[b]];
         }
     }
 }
 
-int convert_blocks_per_sm() {
+int convert_block() { return CBLOCK; }
+int convert_blocks_per_sm(int src_fmt) {
+    const bool rgba = src_fmt == FT_RGBA8P;
+    auto kern = rgba ? k_convert<true> : k_convert<false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, convert_smem(rgba));
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_convert, CBLOCK, 0) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, CBLOCK, convert_smem(rgba)) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
 cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride, uint8_t* dst, uint32_t dst_stride,
                            uint32_t w, uint32_t h, const uint8_t* lut, int grid, cudaStream_t s) {
-    k_convert<<<grid, CBLOCK, 0, s>>>(src_fmt, src, src_stride, dst, dst_stride, w, h, lut);
+    const bool rgba = src_fmt == FT_RGBA8P;
+    auto kern = rgba ? k_convert<true> : k_convert<false>;
+    kern<<<grid, CBLOCK, convert_smem(rgba), s>>>(src, src_stride, dst, dst_stride, w, h, lut);
     return cudaGetLastError();
 }
 

@@ -56,3 +56,29 @@ def test_bad_formats(ctx):
     rc = ctx.L.ft_convert(ctx.h, _abi.MATTE8, ctypes.c_void_p(src.ctypes.data), 4, _abi.SRGBA8,
                           ctypes.c_void_p(src.ctypes.data), 4, 4, 4, _abi.HOST)
     assert rc == _abi.ERR_ARG
+
+
+@pytest.mark.parametrize("w", [1, 2, 3, 5, 15, 16, 17, 33, 257])
+@pytest.mark.parametrize("pad,off", [(0, 0), (0, 4), (0, 1), (1, 0), (3, 2), (4, 0), (12, 4), (16, 16)])
+def test_device_rows(ctx, w, pad, off):
+    """Rows by 16 bytes, words and bytes: any stride and first byte, padding untouched; one row
+    when nothing lies between them."""
+    import ctypes
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(w)
+    h = 21
+    for img, fmt, out_fmt in ((premul(rng, h, w), _abi.RGBA8P, _abi.SRGBA8),
+                              (rng.integers(0, 256, (h, w)).astype(np.uint8), _abi.MATTE8, _abi.SGRAY8)):
+        row = img.nbytes // h
+        src = np.zeros(off + h * (row + pad), np.uint8)
+        rows = src[off:].reshape(h, row + pad)
+        rows[:, :row] = img.reshape(h, row)
+        want = np.full_like(src, 7)
+        want[off:].reshape(h, row + pad)[:, :row] = oracle.convert(img).reshape(h, row)
+        s, d = torch.from_numpy(src).cuda(), torch.full((len(src),), 7, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        rc = ctx.L.ft_convert(ctx.h, fmt, ctypes.c_void_p(s.data_ptr() + off), row + pad, out_fmt,
+                              ctypes.c_void_p(d.data_ptr() + off), row + pad, w, h, _abi.DEVICE)
+        assert rc == 0
+        ctx.sync()
+        assert np.array_equal(d.cpu().numpy(), want)
