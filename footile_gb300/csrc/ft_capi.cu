@@ -1478,6 +1478,7 @@ cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride,
                            uint32_t w, uint32_t h, const uint8_t* lut, int grid, cudaStream_t s);
 int convert_block();
 int convert_blocks_per_sm(int src_fmt);
+int srcover_block();
 cudaError_t launch_srcover(bool backward, const float* cov, uint32_t n_layers, uint64_t plane, const float4* clr,
                            const float4* init, float4* out, const float4* grad_out, float* grad_cov,
                            float4* grad_init, uint32_t n_px, int grid, cudaStream_t s, bool partial = false);
@@ -1857,7 +1858,8 @@ static int srcover_call(ft_ctx* c, bool backward, const float* cov, uint32_t n_l
                          reinterpret_cast<uintptr_t>(grad_init);
     if (v4 & 15) return fail(c, FT_ERR_ARG, "colour and canvas buffers need 16-byte alignment");
     FT_CU(cudaSetDevice(c->device), "set device");
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n_px + 255) / 256, (uint64_t)c->sm_count * 16));
+    const int sob = ftc::srcover_block();
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     FT_CU(ftc::launch_srcover(backward, cov, n_layers, plane, reinterpret_cast<const float4*>(clr),
@@ -1998,7 +2000,8 @@ FT_API int ft_stroke_composite_forward(ft_ctx* c, const ft_op* ops, uint32_t n_o
         FT_CU(cudaMemcpyAsync(s->prefix.p, init, 16ull * n_px, in, c->stream), "copy initial canvas");
     else
         FT_CU(cudaMemsetAsync(s->prefix.p, 0, 16ull * n_px, c->stream), "clear initial canvas");
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n_px + 255) / 256, (uint64_t)c->sm_count * 16));
+    const int sob = ftc::srcover_block();
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     for (uint32_t ch = 0; ch < s->n_chunks; ch++) {
@@ -2059,7 +2062,8 @@ FT_API int ft_stroke_composite_backward(ft_ctx* c, ft_composite_adjoint* s, cons
           "copy canvas gradient");
     if (gops_bytes) FT_CU(cudaMemsetAsync(gops_d, 0, gops_bytes, c->stream), "reset op gradient");
     if (s->n_paths) FT_CU(cudaMemsetAsync(gw_d, 0, 4ull * s->n_paths, c->stream), "reset width gradient");
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((n_px + 255) / 256, (uint64_t)c->sm_count * 16));
+    const int sob = ftc::srcover_block();
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     for (uint32_t ch = s->n_chunks; ch-- > 0;) {

@@ -130,9 +130,39 @@ cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride,
 // one pass forward for E (recomputed, nothing kept from the forward call), written
 // into the gradient planes, then one pass backward for P.  No division, so opaque
 // layers (factor 0) are exact.  One thread per pixel; planes are n_layers x n_px floats.
-// Layers are read SB at a time (independent streaming loads, then the recurrence), so
-// that each thread keeps SB coverage loads in flight.
+// Bound by the planes' stream from memory: the recurrence goes SB layers at a time, the
+// loads of the next SB in flight meanwhile, in CTAs of 128 threads (400 layers of 480 x 360
+// are 5 CTAs of 256 on some SMs and 4 on the others).  400 layers, 276 MB, forward / backward:
+// loads and recurrence in turn 114 / 268 us, next loads in flight 69 / 274 us (4 layers at a
+// time 93 / 234 us), in CTAs of 128 64 / 277 us, nine of the backward's per SM instead of eight
+// (all 1,350 resident; ten, with fewer registers, 234 us) 64 / 194 us.
 constexpr int SB = 8;
+constexpr int SO_BLOCK = 128;
+
+// `step(k, v)` for k = 0 .. n - 1 in turn, v[u] = the SB coverages from layer(k) on (layer(k) +
+// dir * u), loaded a step ahead
+template <class Step>
+__device__ __forceinline__ void stream_layers(const float* cov, uint64_t plane, uint32_t n, uint32_t first, int dir,
+                                              Step step) {
+    const float* at = cov + (uint64_t)first * plane;
+    const int64_t inc = dir < 0 ? -(int64_t)plane : (int64_t)plane;
+    float nx[SB];
+    if (n) {
+#pragma unroll
+        for (int u = 0; u < SB; u++) nx[u] = __ldcs(at + u * inc);
+    }
+    for (uint32_t k = 0; k < n; k++) {
+        float v[SB];
+#pragma unroll
+        for (int u = 0; u < SB; u++) v[u] = nx[u];
+        at += SB * inc;
+        if (k + 1 < n) {
+#pragma unroll
+            for (int u = 0; u < SB; u++) nx[u] = __ldcs(at + u * inc);
+        }
+        step(k, v);
+    }
+}
 
 __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
                               const float4* __restrict__ clr, const float4* __restrict__ init,
@@ -146,15 +176,11 @@ __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, 
             const float f = 1.0f - k.w * v;
             c = make_float4(k.x * v + c.x * f, k.y * v + c.y * f, k.z * v + c.z * f, k.w * v + c.w * f);
         };
-        uint32_t n = 0;
-        for (; n + SB <= n_layers; n += SB) {
-            float v[SB];
+        stream_layers(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
 #pragma unroll
-            for (int u = 0; u < SB; u++) v[u] = __ldcs(cov + (uint64_t)(n + u) * plane + p);
-#pragma unroll
-            for (int u = 0; u < SB; u++) layer(n + u, v[u]);
-        }
-        for (; n < n_layers; n++) layer(n, __ldcs(cov + (uint64_t)n * plane + p));
+            for (int u = 0; u < SB; u++) layer(k * SB + u, v[u]);
+        });
+        for (uint32_t n = n_layers / SB * SB; n < n_layers; n++) layer(n, __ldcs(cov + (uint64_t)n * plane + p));
         out[p] = c;
     }
 }
@@ -162,7 +188,7 @@ __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, 
 // PARTIAL: dLoss/dcov only where 0 < cov < 1 (elsewhere the plane is neither read nor
 // written) — all a NonZero coverage adjoint needs, since dcov/dS is 0 at cov 0 and 1.
 template <bool PARTIAL>
-__global__ void k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
+__global__ void __launch_bounds__(SO_BLOCK, 9) k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
                               const float4* __restrict__ clr, const float4* __restrict__ init,
                               const float4* __restrict__ grad_out, float* __restrict__ grad_cov,
                               float4* __restrict__ grad_init, uint32_t n_px) {
@@ -179,15 +205,11 @@ __global__ void k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, 
             const float4 k = clr[n];
             e = (g.x * k.x + g.y * k.y + g.z * k.z + g.w * k.w) * v + e * (1.0f - k.w * v);
         };
-        uint32_t n = 0;
-        for (; n + SB <= n_layers; n += SB) {
-            float v[SB];
+        stream_layers(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
 #pragma unroll
-            for (int u = 0; u < SB; u++) v[u] = __ldcs(cov + (uint64_t)(n + u) * plane + p);
-#pragma unroll
-            for (int u = 0; u < SB; u++) up(n + u, v[u]);
-        }
-        for (; n < n_layers; n++) up(n, __ldcs(cov + (uint64_t)n * plane + p));
+            for (int u = 0; u < SB; u++) up(k * SB + u, v[u]);
+        });
+        for (uint32_t n = n_layers / SB * SB; n < n_layers; n++) up(n, __ldcs(cov + (uint64_t)n * plane + p));
         // then the suffix products P, last layer first
         float P = 1.0f;
         auto down = [&](uint32_t n, float v, float en) {
@@ -195,17 +217,15 @@ __global__ void k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, 
             if (keep(v)) grad_cov[(uint64_t)n * plane + p] = P * ((g.x * k.x + g.y * k.y + g.z * k.z + g.w * k.w) - k.w * en);
             P *= 1.0f - k.w * v;
         };
-        uint32_t m = n_layers;
-        for (; m >= SB; m -= SB) {
-            float v[SB], en[SB];
-#pragma unroll
-            for (int u = 0; u < SB; u++) v[u] = __ldcs(cov + (uint64_t)(m - 1 - u) * plane + p);
+        stream_layers(cov + p, plane, n_layers / SB, n_layers - 1, -1, [&](uint32_t k, const float* v) {
+            const uint32_t m = n_layers - k * SB;
+            float en[SB];
 #pragma unroll
             for (int u = 0; u < SB; u++) en[u] = keep(v[u]) ? grad_cov[(uint64_t)(m - 1 - u) * plane + p] : 0.0f;
 #pragma unroll
             for (int u = 0; u < SB; u++) down(m - 1 - u, v[u], en[u]);
-        }
-        for (; m > 0; m--) {
+        });
+        for (uint32_t m = n_layers % SB; m > 0; m--) {
             const float v = __ldcs(cov + (uint64_t)(m - 1) * plane + p);
             down(m - 1, v, keep(v) ? grad_cov[(uint64_t)(m - 1) * plane + p] : 0.0f);
         }
@@ -213,15 +233,17 @@ __global__ void k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, 
     }
 }
 
+int srcover_block() { return SO_BLOCK; }
+
 cudaError_t launch_srcover(bool backward, const float* cov, uint32_t n_layers, uint64_t plane, const float4* clr,
                            const float4* init, float4* out, const float4* grad_out, float* grad_cov,
                            float4* grad_init, uint32_t n_px, int grid, cudaStream_t s, bool partial) {
     if (backward && partial)
-        k_srcover_bwd<true><<<grid, 256, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
+        k_srcover_bwd<true><<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
     else if (backward)
-        k_srcover_bwd<false><<<grid, 256, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
+        k_srcover_bwd<false><<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
     else
-        k_srcover_fwd<<<grid, 256, 0, s>>>(cov, n_layers, plane, clr, init, out, n_px);
+        k_srcover_fwd<<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, out, n_px);
     return cudaGetLastError();
 }
 
