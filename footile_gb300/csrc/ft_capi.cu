@@ -1074,7 +1074,7 @@ static int composite_band_rows(ft_ctx* c, uint32_t w, int fmt) {
 
 // Width of an Rgba8p compositor segment (pixels), a warp's share of a row: built-in the canvas in
 // equal parts of at most 1,024, whole 256-pixel boxes or one of 128; in up to four parts while
-// their warps all find room (24 per SM), since a warp is then bound by the latency of its chain
+// there are at most 24 of their warps per SM, since a warp is then bound by the latency of its chain
 // of calls (2,000 strokes, 1,024 / 512 / 256 / 128 pixels: 300 x 300 10.0 / 10.0 / 9.7 / 7.6 ms,
 // 800 x 800 10.9 / 8.9 / 7.6 / 11.6, 2048 x 2048 10.1 / 16.4 / 31.6 / 54.9).
 static int composite_tile_w(const ft_ctx* c, uint32_t w, uint32_t h) {

@@ -1946,16 +1946,17 @@ __global__ void __launch_bounds__(BLOCK) k_cbands(KParams P) {
 // keeps the number of calls at its last visit (mod 256), and what it missed since is one packed
 // step, because the alpha-0 map takes one from channels 1..15 and leaves the rest.
 //
-// Bound by the instructions issued and by the 24 warps per SM that 9 KB per 1,024 pixels leave
-// room for.  16,384 strokes on 2048 x 2048, 31.5 million (call, row) pairs of 45 edges and 175
+// Bound by the instructions issued, at 20 warps per SM (9 KB of shared memory per 1,024 pixels
+// would hold 24).  16,384 strokes on 2048 x 2048, 31.5 million (call, row) pairs of 45 edges and 175
 // covered pixels each: every warp walking all the band's edges, a queue of single pixels and a
 // table for the alpha-0 powers 118 ms; quads, two warps sharing the row's edges between barriers
-// 92 ms; one warp resolving a whole row and one compositing behind it 129 ms; this way 81 ms.
+// 92 ms; one warp resolving a whole row and one compositing behind it 129 ms; this way 80 ms.
 
 constexpr int CT_QN = 96;       // queued quads of a warp: 31 left over and a round's 64
 constexpr int CT_CHAIN = 64;    // sums under way from a segment's warp to the next one's
 
-// Tile rows (they divide the band's) and segments: four warps where the band has the rows.
+// Tile rows (they divide the band's) and segments: four warps where the band has the rows, never
+// more.
 struct CTileShape {
     int rows, segs;
 };
@@ -2139,8 +2140,22 @@ __device__ __forceinline__ void row_cells(const int4 ha, const int4 hb, int y, i
     }
 }
 
+// A barrier of warp `warp` (0 .. 3) alone.  Written out: a barrier number in a register reserves
+// all 16, and the SM's 64 then hold four CTAs (81.4 ms; five, with 96 registers, 79.6; six, with
+// 80, 85.8).
+__device__ __forceinline__ void warp_barrier(int warp) {
+    if (warp == 0)
+        asm volatile("bar.sync 1, 32;" ::: "memory");
+    else if (warp == 1)
+        asm volatile("bar.sync 2, 32;" ::: "memory");
+    else if (warp == 2)
+        asm volatile("bar.sync 3, 32;" ::: "memory");
+    else
+        asm volatile("bar.sync 4, 32;" ::: "memory");
+}
+
 template <bool STAGED, int RULE>
-__global__ void __launch_bounds__(BLOCK, 3) k_ctile(KParams P, const __grid_constant__ CUtensorMap tmap) {
+__global__ void __launch_bounds__(128, 5) k_ctile(KParams P, const __grid_constant__ CUtensorMap tmap) {
     extern __shared__ __align__(128) unsigned char smem_tma[];  // TMA destinations: 128-byte aligned
     unsigned char* smem = smem_tma;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2290,7 +2305,7 @@ __global__ void __launch_bounds__(BLOCK, 3) k_ctile(KParams P, const __grid_cons
                     // a barrier of this warp alone: after the edge loops' divergent ends the lanes went on
                     // in groups through all that follows, which __syncwarp did not undo (5.9 / 3.7 ms for
                     // 768 strokes)
-                    asm volatile("bar.sync %0, 32;" ::"r"(1 + warp) : "memory");
+                    warp_barrier(warp);
                     // the touched chunks, in order
                     const uint4 bw = *bmap;
                     const unsigned bws[4] = {bw.x, bw.y, bw.z, bw.w};
