@@ -1271,6 +1271,7 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             ftk::GridBuildBufs& g = p.gb;
             g.ops = ops_d + paths[0].op_begin;
             g.n_ops = (int)paths[0].n_ops;
+            g.d0 = ftk::gb_d0(paths[0].n_ops);
             g.s_width = sw_in ? sw_in
                               : reinterpret_cast<const float*>(static_cast<char*>(c->paths.p) +
                                                                offsetof(ft_path_desc, s_width));
@@ -1315,7 +1316,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             if (use_probe && stroke) {
                 // the stroke points over the first ops: the 65,535-point cap is usually reached there
                 pp = p;
-                pp.gb.n_ops = probe_ops;
+                pp.gb.n_ops = probe_ops;  // its walks' arrays fit: 2^5 lanes of n_ops / 8 ops at most
+                pp.gb.d0 = ftk::gb_d0(probe_ops);
                 ftk::GridStrokeBufs& q = pp.gs;
                 q.n_sraw = reinterpret_cast<long long*>(gb + 256);
                 q.done = reinterpret_cast<unsigned*>(gb + 288);
@@ -1324,7 +1326,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
             } else if (use_probe) {
                 pp = p;
                 ftk::GridBuildBufs& q = pp.gb;
-                q.n_ops = probe_ops;
+                q.n_ops = probe_ops;  // its walks' arrays fit: 2^5 lanes of n_ops / 8 ops at most
+                q.d0 = ftk::gb_d0(probe_ops);
                 q.done = reinterpret_cast<unsigned*>(gb + 128);
                 q.n_raw = reinterpret_cast<long long*>(gb + 160);
                 q.count = reinterpret_cast<int*>(gb + 168);

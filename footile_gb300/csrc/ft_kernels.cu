@@ -2894,7 +2894,7 @@ cudaError_t launch_figure_bins(const KParams& p, int grid, cudaStream_t s) {
 // last CTA of its kernel to finish):
 //   k_gb_ops    per 256 ops: the last Move/Line/Quad/Cubic/Close op and the last PenWidth op
 //   k_gb_count  every op's pen (the end point of the last such op before it) and raw
-//               vertex count (the count walk, GB_LANES lanes per op); scan of the counts
+//               vertex count (the count walk, 2^d0 lanes per op); scan of the counts
 //   k_gb_emit   every op's raw vertices at its offset (the emit walk); per tile of 1,024
 //               raw vertices its last sub-figure start, scanned
 //   k_gb_keep   keep, pop and R per raw vertex; tile aggregates, scanned
@@ -3008,15 +3008,15 @@ __device__ __forceinline__ void gb_pen(const ft_op* ops, int j, float& x, float&
     }
 }
 // Raw vertices of a Move/Line/Quad/Cubic op with the pen at (px, py), as build_fill
-// flattens them for a fill, split over GB_LANES lanes: lane s takes the subtree of the
-// curve's subdivision whose path from the root is the GB_D0 bits of s (left half 0, in
+// flattens them for a fill, split over 2^d0 lanes: lane s takes the subtree of the
+// curve's subdivision whose path from the root is the d0 bits of s (left half 0, in
 // the depth-first order of the walk); a leaf above that depth goes to the first lane of
 // its range, a Move or Line to lane 0.  Each subtree is the walk's own arithmetic, so the
 // lanes' leaves in lane order are the walk's leaves.  emit(k, vertex) for the lane's k-th
 // leaf; returns the lane's leaf count.  flags: 1 depth cap reached, 2 non-finite control
 // point.
 template <class Emit>
-__device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, float py, int lane, int& flags,
+__device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, float py, int lane, int d0, int& flags,
                        Emit emit) {
     if (kind == FT_OP_MOVE || kind == FT_OP_LINE) {
         if (lane) return 0;
@@ -3035,16 +3035,16 @@ __device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, fl
             emit(0, make_int2(f2fx(c.x), f2fx(c.y)));
             return 1;
         }
-        for (int d = 0; d < GB_D0; d++) {
+        for (int d = 0; d < d0; d++) {
             const P2 ab = pmid(a, b), bc = pmid(b, c), abbc = pmid(ab, bc), ac = pmid(a, c);
             const bool within = pdist_sq(abbc, ac) <= tol_sq;
             if (within || d >= FT_MAX_DEPTH) {
-                if (lane & ((1 << (GB_D0 - d)) - 1)) return 0;
+                if (lane & ((1 << (d0 - d)) - 1)) return 0;
                 if (!within) flags |= 1;
                 emit(0, make_int2(f2fx(c.x), f2fx(c.y)));
                 return 1;
             }
-            if ((lane >> (GB_D0 - 1 - d)) & 1) {
+            if ((lane >> (d0 - 1 - d)) & 1) {
                 a = abbc;
                 b = bc;
             } else {
@@ -3052,7 +3052,7 @@ __device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, fl
                 c = abbc;
             }
         }
-        n = quad_walk<false>(a, b, c, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &dh, leaf, GB_D0);
+        n = quad_walk<false>(a, b, c, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &dh, leaf, d0);
     } else {
         P2 e = xform(P.xf, p2(op.v[4], op.v[5]));
         if (!pfinite(a) || !pfinite(b) || !pfinite(c) || !pfinite(e)) {
@@ -3061,18 +3061,18 @@ __device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, fl
             emit(0, make_int2(f2fx(e.x), f2fx(e.y)));
             return 1;
         }
-        for (int d = 0; d < GB_D0; d++) {
+        for (int d = 0; d < d0; d++) {
             const P2 ab = pmid(a, b), bc = pmid(b, c), cd = pmid(c, e);
             const P2 abbc = pmid(ab, bc), bccd = pmid(bc, cd);
             const P2 pe = pmid(abbc, bccd), ad = pmid(a, e);
             const bool within = pdist_sq(pe, ad) <= tol_sq;
             if (within || d >= FT_MAX_DEPTH) {
-                if (lane & ((1 << (GB_D0 - d)) - 1)) return 0;
+                if (lane & ((1 << (d0 - d)) - 1)) return 0;
                 if (!within) flags |= 1;
                 emit(0, make_int2(f2fx(e.x), f2fx(e.y)));
                 return 1;
             }
-            if ((lane >> (GB_D0 - 1 - d)) & 1) {
+            if ((lane >> (d0 - 1 - d)) & 1) {
                 a = pe;
                 b = bccd;
                 c = cd;
@@ -3082,7 +3082,7 @@ __device__ int gb_walk(const KParams& P, const ft_op& op, int kind, float px, fl
                 e = pe;
             }
         }
-        n = cubic_walk<false>(a, b, c, e, 0.f, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &dh, leaf, GB_D0);
+        n = cubic_walk<false>(a, b, c, e, 0.f, 0.f, 0.f, 0.f, tol_sq, 0, INT_MAX, &dh, leaf, d0);
     }
     if (dh) flags |= 1;
     return n;
@@ -3135,7 +3135,7 @@ __global__ void __launch_bounds__(BLOCK) k_gb_ops(KParams P) {
     }
 }
 
-// Op i of a CTA of k_gb_count / k_gb_emit (GB_OPB ops, GB_LANES lanes each) and its pen.
+// Op i of a CTA of k_gb_count / k_gb_emit (2^d0 lanes each) and its pen.
 struct GbOp {
     int i, lane, kind, lpc, rs;
     float px, py;
@@ -3143,8 +3143,8 @@ struct GbOp {
 };
 __device__ __forceinline__ GbOp gb_op_of(const GridBuildBufs& G, int& flags) {
     GbOp o;
-    o.i = blockIdx.x * GB_OPB + (int)(threadIdx.x / GB_LANES);
-    o.lane = (int)(threadIdx.x % GB_LANES);
+    o.i = (int)((blockIdx.x * BLOCK + threadIdx.x) >> G.d0);
+    o.lane = (int)(threadIdx.x & ((1u << G.d0) - 1u));
     o.kind = -1;
     o.lpc = -1;
     o.rs = 0;
@@ -3175,20 +3175,20 @@ __global__ void __launch_bounds__(BLOCK) k_gb_count(KParams P) {
     const GbOp o = gb_op_of(G, flags);
     int n = 0;
     if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
-        n = gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, flags, [](int, int2) {});
+        n = gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [](int, int2) {});
     if (flags) atomicMax(&P.status[0], (flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
     // the lanes' offsets within the op, the ops' offsets within the CTA
     int inc = n;
-#pragma unroll
-    for (int d = 1; d < GB_LANES; d <<= 1) {
-        const int t = __shfl_up_sync(FULL, inc, d, GB_LANES);
+    const int lanes = 1 << G.d0;
+    for (int d = 1; d < lanes; d <<= 1) {
+        const int t = __shfl_up_sync(FULL, inc, d, lanes);
         if (o.lane >= d) inc += t;
     }
-    const int n_op = __shfl_sync(FULL, inc, GB_LANES - 1, GB_LANES);
+    const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
     int tot;
     const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
     if (o.i < G.n_ops) {
-        G.opl[o.i * GB_LANES + o.lane] = inc - n;
+        G.opl[(o.i << G.d0) + o.lane] = inc - n;
         if (o.lane == 0) G.opi[o.i].y = ex;
     }
     if (tid == 0) G.opn[blockIdx.x] = tot;
@@ -3234,12 +3234,12 @@ __global__ void __launch_bounds__(BLOCK) k_gb_emit(KParams P) {
     const GbOp o = gb_op_of(G, flags);
     if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC) {
         const long long off0 = G.opn[blockIdx.x] + G.opi[o.i].y;
-        const int off = (int)(off0 + G.opl[o.i * GB_LANES + o.lane]);
+        const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
         int2* raw = G.raw;
         unsigned char* fl = G.fl;
         const int cap = G.raw_cap;
         const unsigned char rs0 = (o.lane == 0 && o.rs) ? 1 : 0;
-        gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, flags, [&](int k, int2 q) {
+        gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [&](int k, int2 q) {
             if (ck(off + k < cap, 13) && off + k < cap) {
                 raw[off + k] = q;
                 fl[off + k] = k == 0 ? rs0 : (unsigned char)0;
@@ -3477,7 +3477,7 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
     if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens of every op (the probe's too) and the pen width after
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
-        const int nbw = (q->gb.n_ops + GB_OPB - 1) / GB_OPB;
+        const int nbw = gb_ctas(q->gb.n_ops);
         if ((e = launch_chain(k_gb_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gb_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gb_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
@@ -3493,7 +3493,7 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
 // close, stroker.rs:204-236), makes every sub-stroke's outline (stroker.rs:239-416) and
 // fills it NonZero.  Over the whole GPU, in stream order:
 //   k_gb_ops    pens, the last PenWidth op at or before each op, the last Close/Move op
-//   k_gs_count  every op's raw stroke points (the walk carrying widths, GB_LANES lanes
+//   k_gs_count  every op's raw stroke points (the walk carrying widths, 2^d0 lanes
 //               per op), scanned
 //   k_gs_emit   the raw points (x, y, width), whether each starts a sub-stroke, its op
 //   k_gs_keep   per raw point: kept when it starts a sub-stroke or its f32 position
@@ -3522,11 +3522,11 @@ __device__ __forceinline__ float gs_width(const GridBuildBufs& G, int j) {
 
 // Raw stroke points of a Move/Line/Quad/Cubic op with the pen at (px, py) and widths
 // pen_w (at the pen) and sw (at the op), as build_fill's STROKE walk makes them
-// (plotter.rs:233-236, 294-298), split over GB_LANES lanes as gb_walk splits a fill's:
+// (plotter.rs:233-236, 294-298), split over 2^d0 lanes as gb_walk splits a fill's:
 // emit(k, point, width) for the lane's k-th leaf; returns the lane's leaf count.
 template <class Emit>
 __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, float py, float pen_w, float sw,
-                       int lane, int& flags, Emit emit) {
+                       int lane, int d0, int& flags, Emit emit) {
     if (kind == FT_OP_MOVE || kind == FT_OP_LINE) {
         if (lane) return 0;
         emit(0, xform(P.xf, p2(op.v[0], op.v[1])), sw);
@@ -3543,17 +3543,17 @@ __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, fl
             emit(0, c, wc);
             return 1;
         }
-        for (int d = 0; d < GB_D0; d++) {
+        for (int d = 0; d < d0; d++) {
             const P2 ab = pmid(a, b), bc = pmid(b, c), abbc = pmid(ab, bc), ac = pmid(a, c);
             const bool within = pdist_sq(abbc, ac) <= tol_sq;
             if (within || d >= FT_MAX_DEPTH) {
-                if (lane & ((1 << (GB_D0 - d)) - 1)) return 0;
+                if (lane & ((1 << (d0 - d)) - 1)) return 0;
                 if (!within) flags |= 1;
                 emit(0, c, wc);
                 return 1;
             }
             const float wab = fmid(wa, wb), wbc = fmid(wb, wc), wabbc = fmid(wab, wbc);
-            if ((lane >> (GB_D0 - 1 - d)) & 1) {
+            if ((lane >> (d0 - 1 - d)) & 1) {
                 a = abbc;
                 b = bc;
                 wa = wabbc;
@@ -3565,7 +3565,7 @@ __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, fl
                 wc = wabbc;
             }
         }
-        n = quad_walk<true>(a, b, c, wa, wb, wc, tol_sq, 0, INT_MAX, &dh, emit, GB_D0);
+        n = quad_walk<true>(a, b, c, wa, wb, wc, tol_sq, 0, INT_MAX, &dh, emit, d0);
     } else {
         P2 e = xform(P.xf, p2(op.v[4], op.v[5]));
         float wa = pen_w, wb = __fadd_rn(sw, __fmul_rn(__fsub_rn(pen_w, sw), 1.0f / 3.0f)),
@@ -3576,20 +3576,20 @@ __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, fl
             emit(0, e, we);
             return 1;
         }
-        for (int d = 0; d < GB_D0; d++) {
+        for (int d = 0; d < d0; d++) {
             const P2 ab = pmid(a, b), bc = pmid(b, c), cd = pmid(c, e);
             const P2 abbc = pmid(ab, bc), bccd = pmid(bc, cd);
             const P2 pe = pmid(abbc, bccd), ad = pmid(a, e);
             const bool within = pdist_sq(pe, ad) <= tol_sq;
             if (within || d >= FT_MAX_DEPTH) {
-                if (lane & ((1 << (GB_D0 - d)) - 1)) return 0;
+                if (lane & ((1 << (d0 - d)) - 1)) return 0;
                 if (!within) flags |= 1;
                 emit(0, e, we);
                 return 1;
             }
             const float wab = fmid(wa, wb), wbc = fmid(wb, wc), wcd = fmid(wc, we);
             const float wabbc = fmid(wab, wbc), wbccd = fmid(wbc, wcd), wpe = fmid(wabbc, wbccd);
-            if ((lane >> (GB_D0 - 1 - d)) & 1) {
+            if ((lane >> (d0 - 1 - d)) & 1) {
                 a = pe;
                 b = bccd;
                 c = cd;
@@ -3605,7 +3605,7 @@ __device__ int gs_walk(const KParams& P, const ft_op& op, int kind, float px, fl
                 we = wpe;
             }
         }
-        n = cubic_walk<true>(a, b, c, e, wa, wb, wc, we, tol_sq, 0, INT_MAX, &dh, emit, GB_D0);
+        n = cubic_walk<true>(a, b, c, e, wa, wb, wc, we, tol_sq, 0, INT_MAX, &dh, emit, d0);
     }
     if (dh) flags |= 1;
     return n;
@@ -3625,20 +3625,20 @@ __global__ void __launch_bounds__(BLOCK) k_gs_count(KParams P) {
     const GbOp o = gb_op_of(G, flags);
     int n = 0;
     if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
-        n = gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, flags,
+        n = gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
                     [](int, P2, float) {});
     if (flags) atomicMax(&P.status[0], (flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
     int inc = n;
-#pragma unroll
-    for (int d = 1; d < GB_LANES; d <<= 1) {
-        const int t = __shfl_up_sync(FULL, inc, d, GB_LANES);
+    const int lanes = 1 << G.d0;
+    for (int d = 1; d < lanes; d <<= 1) {
+        const int t = __shfl_up_sync(FULL, inc, d, lanes);
         if (o.lane >= d) inc += t;
     }
-    const int n_op = __shfl_sync(FULL, inc, GB_LANES - 1, GB_LANES);
+    const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
     int tot;
     const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
     if (o.i < G.n_ops) {
-        G.opl[o.i * GB_LANES + o.lane] = inc - n;
+        G.opl[(o.i << G.d0) + o.lane] = inc - n;
         if (o.lane == 0) G.opi[o.i].y = ex;
     }
     if (tid == 0) G.opn[blockIdx.x] = tot;
@@ -3665,7 +3665,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_emit(KParams P) {
     const GbOp o = gb_op_of(G, flags);
     if (o.kind < FT_OP_MOVE || o.kind > FT_OP_CUBIC) return;
     const long long off0 = G.opn[blockIdx.x] + G.opi[o.i].y;
-    const int off = (int)(off0 + G.opl[o.i * GB_LANES + o.lane]);
+    const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
     const int cap = S.sraw_cap;
     // a Move ends the sub-stroke before it open, a Close joined (stroker.rs:87-96)
     const unsigned char f0 = (unsigned char)(((o.lane == 0 && o.rs) ? 1 : 0) | (o.kind != FT_OP_MOVE ? 2 : 0));
@@ -3674,7 +3674,7 @@ __global__ void __launch_bounds__(BLOCK) k_gs_emit(KParams P) {
     unsigned char* sfl = S.sfl;
     int* sopi = S.sopi;
     const int i = o.i;
-    gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, flags,
+    gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
             [&](int k, P2 q, float w) {
                 if (ck(off + k < cap, 13) && off + k < cap) {
                     raw4[off + k] = make_float4(q.x, q.y, w, 0.f);
@@ -3944,7 +3944,7 @@ cudaError_t launch_grid_stroke(const KParams& p, int sm_count, cudaStream_t s, c
     if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens and widths of every op (the probe's too)
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
-        const int nbw = (q->gb.n_ops + GB_OPB - 1) / GB_OPB;
+        const int nbw = gb_ctas(q->gb.n_ops);
         if ((e = launch_chain(k_gs_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gs_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gs_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;

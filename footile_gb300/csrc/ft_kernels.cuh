@@ -93,9 +93,13 @@ constexpr uint32_t FIG_CAP_MAX = 1u << 26;
 constexpr int GB_PER = 4;                      // raw vertices per thread of the tile kernels
 constexpr int GB_TILE = GB_PER * BLOCK;        // raw vertices per tile
 constexpr int GB_TOP_BLOCKS = 512;             // CTAs of the top-vertex search
-constexpr int GB_D0 = 3;                       // an op's curve walk is split at this depth
-constexpr int GB_LANES = 1 << GB_D0;           // threads per op of the count and emit walks
-constexpr int GB_OPB = BLOCK / GB_LANES;       // ops per CTA of the count and emit walks
+// An op's curve walk is split at depth d0 over 2^d0 threads: 8, or a warp while the ops are few
+// enough for all warps to be resident (GB_WIDE_OPS).  8 / 16 / 32 threads on the 2,048 ops that
+// complete a capped figure: 4096 x 4096 scene 188 / 178 / 168 us, its stroke 288 / 280 / 268;
+// on 3,780 ops, poster of 1531 x 1117 119 / 116 / 116 us.
+constexpr int GB_WIDE_OPS = 8192;
+constexpr int gb_d0(size_t n_ops) { return n_ops <= (size_t)GB_WIDE_OPS ? 5 : 3; }
+constexpr int gb_ctas(size_t n_ops) { return (int)(((n_ops << gb_d0(n_ops)) + BLOCK - 1) / BLOCK); }
 constexpr long long GB_RAW_MAX = 1ll << 29;    // raw vertices the grid build takes at most
 struct GridBuildBufs {
     const ft_op* ops;   // the path's ops
@@ -107,8 +111,9 @@ struct GridBuildBufs {
     int* count;         // vertices kept
     int4* opa;          // per 256 ops: last Move/Line/Quad/Cubic/Close op, last PenWidth op, last Close/Move op
     int* opw;           // per op: last PenWidth op at or before it in its 256 (strokes)
-    long long* opn;     // per GB_OPB ops: raw vertices
-    int2* opi;          // per op: last Move/Line/Quad/Cubic/Close op before it in its 256, raw offset in its GB_OPB
+    int d0;             // gb_d0(n_ops)
+    long long* opn;     // per CTA of the walks: raw vertices
+    int2* opi;          // per op: last Move/Line/Quad/Cubic/Close op before it in its 256, raw offset in its CTA
     int* opl;           // per op and lane: the lane's raw offset in the op
     int2* raw;          // raw vertices, 16.16
     unsigned char* fl;  // per raw vertex: 1 = starts a sub-figure
@@ -146,7 +151,7 @@ struct GbLayout {
 };
 constexpr GbLayout gb_layout(size_t n_ops, size_t raw_cap, size_t sraw_cap = 0) {
     GbLayout g{};
-    const size_t nbo = (n_ops + BLOCK - 1) / BLOCK, nbw = (n_ops + GB_OPB - 1) / GB_OPB,
+    const size_t nbo = (n_ops + BLOCK - 1) / BLOCK, nbw = (size_t)gb_ctas(n_ops),
                  ntiles = raw_cap / GB_TILE;
     // two builds' done[8] at 0 / 128, n_raw at 32 / 160, count at 40 / 168, final at 44 / 172;
     // a stroke build's st[] at 128, n_sraw at 160, done[] at 192, its probe's n_sraw at 256,
@@ -157,7 +162,7 @@ constexpr GbLayout gb_layout(size_t n_ops, size_t raw_cap, size_t sraw_cap = 0) 
     g.opn = align256(g.opw + n_ops * 4);
     g.opi = align256(g.opn + nbw * 8);
     g.opl = align256(g.opi + n_ops * 8);
-    g.raw = align256(g.opl + n_ops * GB_LANES * 4);
+    g.raw = align256(g.opl + (n_ops << gb_d0(n_ops)) * 4);
     g.fl = align256(g.raw + raw_cap * 8);
     g.kp = align256(g.fl + raw_cap);
     g.rk = align256(g.kp + raw_cap);
