@@ -1304,7 +1304,8 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
                 q.sopi = reinterpret_cast<int*>(gb + G.sopi);
                 q.stile = reinterpret_cast<int2*>(gb + G.stile);
                 q.subt = reinterpret_cast<int*>(gb + G.subt);
-                q.itoff = reinterpret_cast<int*>(gb + G.itoff);
+                q.itoff = reinterpret_cast<int2*>(gb + G.itoff);
+                q.itp = reinterpret_cast<float4*>(gb + G.itp);
                 q.itc = reinterpret_cast<int*>(gb + G.itc);
                 q.final_flag = nullptr;
                 q.skip = nullptr;

@@ -692,8 +692,13 @@ __device__ int outline_item(const KParams& P, const float4* spts, const SubRec& 
     const bool joined = sr.joined != 0;
     const bool rev = u > len;
     const int j = rev ? u - len - 1 : u;  // iteration on this side; j == len is the end item
-    auto v0 = [&](int jj) { return rev ? s + ((n - 1 - jj) % n + n) % n : s + (jj % n); };
-    auto v1 = [&](int jj) { return rev ? s + ((n - 2 - jj) % n + n) % n : s + ((jj + 1) % n); };
+    // point k modulo n (k - n .. k + n without a division: all there is unless len wrapped)
+    auto at = [&](int k) {
+        k = k < 0 ? k + n : (k >= n ? k - n : k);
+        return s + ((unsigned)k < (unsigned)n ? k : (k % n + n) % n);
+    };
+    auto v0 = [&](int jj) { return at(rev ? n - 1 - jj : jj); };
+    auto v1 = [&](int jj) { return at(rev ? n - 2 - jj : jj + 1); };
     auto seg = [&](int jj, P2* r0, P2* r1) { seg_offset(spts[v0(jj)], spts[v1(jj)], r0, r1); };
     if (j == len) {  // end of an open side: the last offset point
         if (joined) return 0;
@@ -3507,7 +3512,9 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
 //               Move op after its last point when the cap stopped the points, else the
 //               path's last Move/Line/Quad/Cubic/Close op), SubStroke::len in u16
 //               arithmetic and 2 len + 2 outline items, scanned
-//   k_go_count  every outline item's points (outline_item), scanned
+//   k_go_count  every outline item's points (outline_item), their number scanned, the first
+//               two kept (all there are but for arcs; computed again for the emit: 23 / 26 us
+//               on the 65,535 points of a capped stroke from a cold cache, kept 21 / 17 us)
 //   k_go_emit   the outline's raw vertices through the second transform (plotter.rs:
 //               219-224), the figure runs' starts per tile, scanned
 // then k_gb_keep, k_gb_write and k_gb_top build the outline's figure as they do a fill's.
@@ -3874,14 +3881,26 @@ __global__ void __launch_bounds__(BLOCK) k_go_count(KParams P) {
     for (int c = blockIdx.x; c < nc; c += gridDim.x) {
         const int t = c * BLOCK + tid;
         int n = 0;
+        bool starts = false;
         if (t < n_items) {
             int u;
             const SubRec sr = go_item(S, subs, nsub, t, u);
-            n = outline_item(P, spts, sr, u, INT_MAX, INT_MAX, &depth_hit, [](int, P2) {});
+            float4 two = make_float4(0.f, 0.f, 0.f, 0.f);
+            n = outline_item(P, spts, sr, u, 0, INT_MAX, &depth_hit, [&](int k, P2 q) {
+                if (k == 0) two.x = q.x, two.y = q.y;
+                if (k == 1) two.z = q.x, two.w = q.y;
+            });
+            S.itp[t] = two;
+            // a figure run starts at each side's first point after a Close: the forward side
+            // always (after the previous sub-stroke's Close, or first), the reverse side when
+            // the sub-stroke is joined (stroker.rs:255-260)
+            const bool rev = u > sr.len, joined = sr.joined != 0;
+            const int j = rev ? u - sr.len - 1 : u;
+            starts = (!rev && ((!joined && j == 0) || (joined && j == 1))) || (rev && joined && j == 1);
         }
         int tot;
         const int off = block_excl_sum(n, tmp, tot);
-        if (t < n_items) S.itoff[t] = off;
+        if (t < n_items) S.itoff[t] = make_int2(off, n | (starts ? INT_MIN : 0));
         if (tid == 0) S.itc[c] = tot;
     }
     if (depth_hit) atomicMax(&P.status[0], FT_ERR_DEPTH);
@@ -3910,24 +3929,26 @@ __global__ void __launch_bounds__(BLOCK) k_go_emit(KParams P) {
     const float4* spts = reinterpret_cast<const float4*>(P.scratch + P.L.spts);
     const SubRec* subs = reinterpret_cast<const SubRec*>(P.scratch + P.L.subs);
     for (int t = blockIdx.x * BLOCK + tid; t < n_items; t += gridDim.x * BLOCK) {
-        int u;
-        const SubRec sr = go_item(S, subs, nsub, t, u);
-        const int off = S.itc[t / BLOCK] + S.itoff[t];
-        // a figure run starts at each side's first point after a Close: the forward side
-        // always (after the previous sub-stroke's Close, or first), the reverse side when
-        // the sub-stroke is joined (stroker.rs:255-260)
-        const bool rev = u > sr.len, joined = sr.joined != 0;
-        const int j = rev ? u - sr.len - 1 : u;
-        const int rsk = ((!rev && ((!joined && j == 0) || (joined && j == 1))) || (rev && joined && j == 1)) ? 0 : -1;
-        int dh = 0;
-        const int n = outline_item(P, spts, sr, u, 0, INT_MAX, &dh, [&](int k, P2 q) {
+        const int2 it = S.itoff[t];
+        const int off = S.itc[t / BLOCK] + it.x, n = it.y & INT_MAX;
+        const bool starts = it.y < 0;
+        auto put = [&](int k, P2 q) {
             const P2 tq = xform(P.xf, q);  // the outline is transformed again (F9)
             if (ck(off + k < cap, 16) && off + k < cap) {
                 G.raw[off + k] = make_int2(f2fx(tq.x), f2fx(tq.y));
-                G.fl[off + k] = k == rsk ? (unsigned char)1 : (unsigned char)0;
+                G.fl[off + k] = k == 0 && starts ? (unsigned char)1 : (unsigned char)0;
             }
-        });
-        if (rsk == 0 && n > 0 && off < cap) atomicMax(&G.tr[off / GB_TILE], off);
+        };
+        if (n <= 2) {  // kept by k_go_count
+            const float4 two = S.itp[t];
+            if (n > 0) put(0, p2(two.x, two.y));
+            if (n > 1) put(1, p2(two.z, two.w));
+        } else {  // an arc: again
+            int u, dh = 0;
+            const SubRec sr = go_item(S, subs, nsub, t, u);
+            outline_item(P, spts, sr, u, 0, INT_MAX, &dh, put);
+        }
+        if (starts && n > 0 && off < cap) atomicMax(&G.tr[off / GB_TILE], off);
     }
     if (!gb_last_block(&G.done[2])) return;
     gb_scan_tr(G, n_raw, tmp, s_c);

@@ -140,14 +140,15 @@ struct GridStrokeBufs {
     int* sopi;           // per raw point: its op
     int2* stile;         // per tile of raw points: kept, sub-stroke starts
     int* subt;           // per 256 sub-strokes: outline items
-    int* itoff;          // per outline item: raw offset in its 256
+    int2* itoff;         // per outline item: raw offset in its 256; raw vertices, the top bit when it starts a run
+    float4* itp;         // per outline item: its first two points
     int* itc;            // per 256 outline items: raw vertices
     int* final_flag;     // nullable: set when the 65,535-point cap is reached (the points are complete)
     const int* skip;     // nullable: the stroke point kernels do nothing when *skip is set
 };
 struct GbLayout {
     size_t state, opa, opw, opn, opi, opl, raw, fl, kp, rk, tr, tr2, tp, top;
-    size_t raw4, sfl, sopi, stile, subt, itoff, itc, bytes;
+    size_t raw4, sfl, sopi, stile, subt, itoff, itc, itp, bytes;
 };
 constexpr GbLayout gb_layout(size_t n_ops, size_t raw_cap, size_t sraw_cap = 0) {
     GbLayout g{};
@@ -176,8 +177,9 @@ constexpr GbLayout gb_layout(size_t n_ops, size_t raw_cap, size_t sraw_cap = 0) 
     g.stile = align256(g.sopi + sraw_cap * 4);
     g.subt = align256(g.stile + sraw_cap / GB_TILE * 8);
     g.itoff = align256(g.subt + (sraw_cap ? (size_t)(PT_CAP / BLOCK + 1) * 4 : 0));
-    g.itc = align256(g.itoff + (sraw_cap ? (size_t)GS_ITEMS_CAP * 4 : 0));
-    g.bytes = align256(g.itc + (sraw_cap ? (size_t)(GS_ITEMS_CAP / BLOCK + 1) * 4 : 0));
+    g.itc = align256(g.itoff + (sraw_cap ? (size_t)GS_ITEMS_CAP * 8 : 0));
+    g.itp = align256(g.itc + (sraw_cap ? (size_t)(GS_ITEMS_CAP / BLOCK + 1) * 4 : 0));
+    g.bytes = align256(g.itp + (sraw_cap ? (size_t)GS_ITEMS_CAP * 16 : 0));
     return g;
 }
 
