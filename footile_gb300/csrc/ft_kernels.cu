@@ -2897,7 +2897,7 @@ cudaError_t launch_figure_bins(const KParams& p, int grid, cudaStream_t s) {
 // to the range's beginning, mp: largest exclusive prefix in the range); mp finds the
 // first tile that reaches the cap.  Kernels, in stream order (each scan is run by the
 // last CTA of its kernel to finish):
-//   k_gb_ops    per 256 ops: the last Move/Line/Quad/Cubic/Close op and the last PenWidth op
+//   k_gb_ops    resets; per 256 ops: the last Move/Line/Quad/Cubic/Close op and the last PenWidth op
 //   k_gb_count  every op's pen (the end point of the last such op before it) and raw
 //               vertex count (the count walk, 2^d0 lanes per op); scan of the counts
 //   k_gb_emit   every op's raw vertices at its offset (the emit walk); per tile of 1,024
@@ -3099,6 +3099,15 @@ __global__ void __launch_bounds__(BLOCK) k_gb_ops(KParams P) {
     __shared__ int s_tot[3];
     const GridBuildBufs& G = P.gb;
     const int tid = threadIdx.x, i = blockIdx.x * BLOCK + tid;
+    // what the kernels behind this one count in
+    for (int k = i; k < G.n_tr; k += gridDim.x * BLOCK) G.tr_all[k] = -1;
+    for (int k = i; k < P.n_bands; k += gridDim.x * BLOCK) P.bin_hist[k] = 0;
+    if (i < 64) P.queue[i] = 0;
+    if (i == 0) {
+        P.status[0] = 0;
+        *P.pool_used = 0;
+        P.fig_state[0] = make_int4(0, 0, 0, 0);
+    }
     const int kind = i < G.n_ops ? __ldg(&G.ops[i].kind) : -1;
     int mpc, lpc;
     block_max_scan((kind >= FT_OP_CLOSE && kind <= FT_OP_CUBIC) ? i : -1, tmp, mpc, lpc);

@@ -119,6 +119,8 @@ struct GridBuildBufs {
     unsigned char* fl;  // per raw vertex: 1 = starts a sub-figure
     unsigned char* kp;  // per raw vertex: 1 = kept, 2 = pops its sub-figure's first vertex
     int* rk;            // per raw vertex: the first raw vertex of its sub-figure
+    int* tr_all;        // the tile starts of both builds, n_tr of them: k_gb_ops resets them
+    int n_tr;
     int* tr;            // per tile: last sub-figure start
     int4* tp;           // per tile: position aggregate (kept - popped, runs, max prefix)
     int4* top;          // per CTA of the top-vertex search: min (y, x, id)
