@@ -2011,8 +2011,7 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) {
 // false when it did not complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, unsigned parity) {
     const unsigned a = smem_u32(mbar);
-    unsigned long long t0;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    unsigned long long t0 = 0;
     for (int it = 0; it < (1 << 22); it++) {
         unsigned done;
         asm volatile(
@@ -2024,6 +2023,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, unsigned parity) {
         if ((it & 255) == 255) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            if (!t0) t0 = t;
             if (t - t0 > 200000000ull) break;
         }
     }
@@ -2486,13 +2486,10 @@ constexpr int SO_SMEM = SO_STAGES * SO_STAGE_BYTES + 128 + 1024;  // stages, mba
 
 // ch8_mul(d, b) of the four channels of d, b's 12-bit expansion (b << 4 | b >> 4) given
 __device__ __forceinline__ unsigned ch8_mul4(unsigned d, unsigned bx) {
-    unsigned out = 0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const unsigned dc = (d >> (8 * c)) & 0xFFu;
-        out |= ((((dc << 4) | (dc >> 4)) * bx) >> 16) << (8 * c);
-    }
-    return out;
+    const unsigned e = d & 0x00FF00FFu, o = (d >> 8) & 0x00FF00FFu;  // two channels per word
+    const unsigned le = (e << 4) | ((e >> 4) & 0x000F000Fu), lo = (o << 4) | ((o >> 4) & 0x000F000Fu);
+    return __byte_perm((le & 0xFFFFu) * bx, (le >> 16) * bx, 0x7632) |
+           (__byte_perm((lo & 0xFFFFu) * bx, (lo >> 16) * bx, 0x7632) << 8);
 }
 
 // Warps 0..7 composite; warp 8 moves the tiles (one lane issues every TMA operation):
@@ -2585,23 +2582,16 @@ __global__ void __launch_bounds__(SO_THREADS, 6) k_srcover_mask(const __grid_con
             const unsigned m4 = mk[i];
             const uint4 d = reinterpret_cast<const uint4*>(cv)[i];
             unsigned dv[4] = {d.x, d.y, d.z, d.w};
-            // alpha 0 changes only channels in 1..15 (nonzero bytes whose high nibble is zero)
-            auto low = [](unsigned v) {
-                const unsigned nz = (((v & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | v) & 0x80808080u;
-                const unsigned hi = (((v & 0x70707070u) + 0x70707070u) | v) & 0x80808080u;
-                return nz & ~hi;
-            };
-            if (!m4 && !(low(dv[0]) | low(dv[1]) | low(dv[2]) | low(dv[3]))) continue;  // four pixels unchanged
+            // alpha 0 changes only channels in 1..15: four pixels unchanged
+            if (!m4 && !(low_channels(dv[0]) | low_channels(dv[1]) | low_channels(dv[2]) | low_channels(dv[3]))) continue;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const unsigned av = (m4 >> (8 * j)) & 0xFFu;
-                const unsigned v = dv[j];
-                if (!av && !low(v)) continue;
-                // pix SrcOver: clr * a + d * (255 - clr_alpha * a), channel by channel; an opaque
-                // source (inverse alpha 0) replaces the pixel
-                const unsigned s4 = src[av];
+                // pix SrcOver: clr * a + d * (255 - clr_alpha * a), channel by channel.  Of pixels that
+                // change and that do not alike: with branches the lanes went through it in turns
+                // (4096 x 4096 stroke, 40.7 us; all four pixels, and channels by pairs, 31.1 us)
+                const unsigned s4 = src[(m4 >> (8 * j)) & 0xFFu];
                 const unsigned inv = 255u - (s4 >> 24);
-                dv[j] = inv ? __vaddus4(s4, ch8_mul4(v, (inv << 4) | (inv >> 4))) : s4;
+                dv[j] = __vaddus4(s4, ch8_mul4(dv[j], (inv << 4) | (inv >> 4)));
             }
             reinterpret_cast<uint4*>(cv)[i] = make_uint4(dv[0], dv[1], dv[2], dv[3]);
         }
