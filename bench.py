@@ -363,7 +363,7 @@ def measured_peak_hbm():
 
 def profiled(key):
     """A per-launch figure of the rasteriser from the committed ncu summary."""
-    p = os.path.join(ROOT, "profiles", "k_raster_warp_glyphs_65536.txt")
+    p = os.path.join(ROOT, "profiles", "k_tile_glyphs_65536.txt")
     try:
         for line in open(p):
             if line.startswith(key + ":"):
@@ -386,7 +386,7 @@ def accumulation(kernel_ms):
             "warp_instructions_per_launch": profiled("shared_atomic_warp_insts_per_launch"),
             "achieved": wf / (kernel_ms * 1e-3) / 1e9, "unit": "G atomic wavefronts/s",
             "utilisation_pct_of_peak": profiled("shared_atomic_pipe_pct_of_peak"),
-            "source": "profiles/k_raster_warp_glyphs_65536.txt"}
+            "source": "profiles/k_tile_glyphs_65536.txt"}
 
 
 def cpu_baseline(ops, paths, nbytes, seconds, threads, gpu_masks=None):
@@ -881,7 +881,7 @@ def run_ours(args):
                                   "d2h_bytes_per_step": int(nbytes)}},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": profiled_traffic() if args.n_paths == 65536 else None, "peak_kind": peak_kind,
-                     "kernel": "ftk::k_raster_warp<false> + ftk::k_raster<false> (graph: 2 memsets, warp rasteriser, CTA rasteriser)", "kernel_ms": kmean,
+                     "kernel": "ftk::k_tile<128> + ftk::k_raster<false> (graph: 2 memsets, tile rasteriser, CTA rasteriser)", "kernel_ms": kmean,
                      "algorithmic_bytes_per_launch": int(alg_bytes)},
         # the cell accumulation's bound: shared-memory atomics (data-path wavefronts of one
         # launch from the ncu summary, over this run's kernel time; the atomic data path's
