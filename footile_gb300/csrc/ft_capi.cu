@@ -1198,9 +1198,6 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
                                     c->sm_count * ftk::composite_build_blocks_per_sm(smem_a, stroke != 0)));
     if (uncapped) grid = (int)std::max<size_t>(1, std::min<size_t>((size_t)grid, (8ull << 30) / L.bytes));
     FT_CU(c->scratch.ensure(L.bytes * (size_t)grid), "alloc scratch");
-    if (n_paths)
-        FT_CU(cudaMemcpyAsync(c->paths.p, paths, sizeof(ft_path_desc) * n_paths, cudaMemcpyHostToDevice, c->stream),
-              "upload paths");
     // one fill path: its figure is built over the whole GPU (the grid build, whose raw
     // vertex arrays grow until the path's raw vertices fit) or by one CTA of k_cbuild
     const int fig_build = c->tuned ? c->tune.fig_build : 0;
@@ -1218,6 +1215,12 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
     // first pool size in edges (it grows on demand)
     const bool penv = c->tuned && c->tune.pool_edges > 0;
     uint64_t want = penv ? (uint64_t)c->tune.pool_edges : std::max<uint64_t>((uint64_t)n_ops_total * 64, 1u << 20);
+    // descriptors on the device: for k_cbuild and the tile compositor, and for the pen width of a
+    // call that has none of its own there
+    bool paths_up = false;
+    auto need_paths = [&](bool grid) {
+        return n_paths > 0 && !(grid && sw_in && (fmt == FT_MATTE8 || mask_route));
+    };
     for (int attempt = 0; attempt < 4; attempt++) {
         if (!penv || attempt > 0) want = std::max<uint64_t>(want, c->pool.cap / sizeof(ftk::EdgeRec));
         if (penv && attempt == 0 && c->pool.cap > want * sizeof(ftk::EdgeRec)) c->pool.release();
@@ -1342,6 +1345,21 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
                 g.skip = q.final_flag;
             }
         }
+        // Read-back in page-locked memory: up to five copies to pageable memory each waited for
+        // themselves.  With the resets left to k_gb_ops, 4096 x 4096 scene 170 / 138 us, its stroke
+        // 269 / 219 us, poster of 1531 x 1117 115 / 89 us; written by the kernels instead of three
+        // copies behind them 138 / 125, 217 / 204 and 90 / 83 us.
+        if (!c->h_sum) FT_CU(cudaHostAlloc(&c->h_sum, 2 * ftk::GB_STATE, cudaHostAllocMapped), "alloc summary");
+        unsigned char* sum = static_cast<unsigned char*>(c->h_sum);
+        memset(sum, 0, 2 * ftk::GB_STATE);
+        void* sum_d = nullptr;
+        FT_CU(cudaHostGetDevicePointer(&sum_d, c->h_sum, 0), "map summary");
+        p.summary = pp.summary = static_cast<unsigned char*>(sum_d);
+        if (need_paths(grid_build) && !paths_up) {
+            FT_CU(cudaMemcpyAsync(c->paths.p, paths, sizeof(ft_path_desc) * n_paths, cudaMemcpyHostToDevice, c->stream),
+                  "upload paths");
+            paths_up = true;
+        }
         c->comp_timed = false;
         FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
         if (n_paths) {
@@ -1364,21 +1382,10 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
                 c->launches += 3;
             }
         }
-        // what the host decides on, in page-locked memory: up to five copies to pageable memory each
-        // waited for themselves.  With the resets left to k_gb_ops, 4096 x 4096 scene 170 / 138 us,
-        // its stroke 269 / 219 us, poster of 1531 x 1117 115 / 89 us.
-        if (!c->h_sum) FT_CU(cudaHostAlloc(&c->h_sum, 1024, cudaHostAllocDefault), "alloc summary");
-        const unsigned char* sum = static_cast<const unsigned char*>(c->h_sum);
-        memset(c->h_sum, 0, 1024);
-        FT_CU(cudaMemcpyAsync(c->h_sum, c->pool_used.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream),
-              "pool size");
-        if (n_paths == 1)
-            FT_CU(cudaMemcpyAsync(static_cast<char*>(c->h_sum) + 16, c->crec.p, sizeof(int4), cudaMemcpyDeviceToHost,
-                                  c->stream),
-                  "path record");
-        if (grid_build)
-            FT_CU(cudaMemcpyAsync(static_cast<char*>(c->h_sum) + 512, c->gbuf.p, 512, cudaMemcpyDeviceToHost, c->stream),
-                  "build counts");
+        // a single call's last build kernels write what the host decides on into its memory
+        if (n_paths != 1)
+            FT_CU(cudaMemcpyAsync(sum, c->pool_used.p, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream),
+                  "pool size");
         FT_CU(cudaStreamSynchronize(c->stream), "synchronize");
         unsigned long long used;
         int4 cr0;  // a single call's first raster row, binned edges
@@ -1386,7 +1393,7 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
         memcpy(&cr0, sum + 16, sizeof(cr0));
         auto count_at = [&](const void* p) {
             long long v = 0;
-            if (p) memcpy(&v, sum + 512 + (static_cast<const unsigned char*>(p) - static_cast<const unsigned char*>(c->gbuf.p)), sizeof(v));
+            if (p) memcpy(&v, sum + ftk::GB_STATE + (static_cast<const unsigned char*>(p) - static_cast<const unsigned char*>(c->gbuf.p)), sizeof(v));
             return v;
         };
         long long n_raw = 0, n_raw_probe = 0, n_sraw = 0, n_sraw_probe = 0;

@@ -2284,7 +2284,7 @@ __global__ void __launch_bounds__(128, 5) k_ctile(KParams P, const __grid_consta
                     ((unsigned long long)(unsigned)cr.z | ((unsigned long long)(unsigned)cr.w << 32)) + (unsigned)o0;
                 unsigned my_clr = 0;
                 if (reach && any) my_clr = *reinterpret_cast<const unsigned*>(P.paths[i].clr);
-                if (has_out && ok) {  // room for this round's sums
+                if (has_out && ok) {  // room for the sums of these 32 calls
                     unsigned v;
                     ok = __all_sync(FULL, smem_wait(out + CT_CHAIN, v, [&](unsigned d) { return m - d <= CT_CHAIN - 32; }));
                 }
@@ -2755,6 +2755,14 @@ __global__ void __launch_bounds__(BLOCK) k_fig_bin_scan(KParams P) {
         P.fig_state[0].w = fits ? 1 : 0;
         if (!fits) atomicMax(&P.status[0], FT_ERR_CAP);  // the host grows the pool and runs again
     }
+    // what the host decides on, straight into its memory
+    if (tid == 0) {
+        *reinterpret_cast<unsigned long long*>(P.summary) = base + (unsigned long long)carry;
+        *reinterpret_cast<int4*>(P.summary + 16) = P.crec[0];
+    }
+    if (P.gb.done && tid < GB_STATE / 8)
+        reinterpret_cast<unsigned long long*>(P.summary + GB_STATE)[tid] =
+            reinterpret_cast<const unsigned long long*>(P.gb.done)[tid];
 }
 
 // (edge, band) pairs of 256 edges at a time spread over the CTA (run-length item map):
@@ -3145,15 +3153,15 @@ __global__ void __launch_bounds__(BLOCK) k_gb_ops(KParams P) {
     }
 }
 
-// Op i of a CTA of k_gb_count / k_gb_emit (2^d0 lanes each) and its pen.
+// A lane's op of block `blk` of the walks (2^d0 lanes an op) and its pen.
 struct GbOp {
     int i, lane, kind, lpc, rs;
     float px, py;
     ft_op op;
 };
-__device__ __forceinline__ GbOp gb_op_of(const GridBuildBufs& G, int& flags) {
+__device__ __forceinline__ GbOp gb_op_of(const GridBuildBufs& G, int blk, int& flags) {
     GbOp o;
-    o.i = (int)((blockIdx.x * BLOCK + threadIdx.x) >> G.d0);
+    o.i = (int)(((unsigned)blk * BLOCK + threadIdx.x) >> G.d0);
     o.lane = (int)(threadIdx.x & ((1u << G.d0) - 1u));
     o.kind = -1;
     o.lpc = -1;
@@ -3182,29 +3190,31 @@ __global__ void __launch_bounds__(BLOCK) k_gb_count(KParams P) {
     if (G.skip && *G.skip) return;  // a probe over a prefix of the ops completed the figure
     const int tid = threadIdx.x;
     int flags = 0;
-    const GbOp o = gb_op_of(G, flags);
-    int n = 0;
-    if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
-        n = gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [](int, int2) {});
+    for (int blk = blockIdx.x; blk < gb_ctas(G.n_ops); blk += gridDim.x) {
+        const GbOp o = gb_op_of(G, blk, flags);
+        int n = 0;
+        if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
+            n = gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [](int, int2) {});
+        // the lanes' offsets within the op, the ops' offsets within the CTA
+        int inc = n;
+        const int lanes = 1 << G.d0;
+        for (int d = 1; d < lanes; d <<= 1) {
+            const int t = __shfl_up_sync(FULL, inc, d, lanes);
+            if (o.lane >= d) inc += t;
+        }
+        const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
+        int tot;
+        const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
+        if (o.i < G.n_ops) {
+            G.opl[(o.i << G.d0) + o.lane] = inc - n;
+            if (o.lane == 0) G.opi[o.i].y = ex;
+        }
+        if (tid == 0) G.opn[blk] = tot;
+    }
     if (flags) atomicMax(&P.status[0], (flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
-    // the lanes' offsets within the op, the ops' offsets within the CTA
-    int inc = n;
-    const int lanes = 1 << G.d0;
-    for (int d = 1; d < lanes; d <<= 1) {
-        const int t = __shfl_up_sync(FULL, inc, d, lanes);
-        if (o.lane >= d) inc += t;
-    }
-    const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
-    int tot;
-    const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
-    if (o.i < G.n_ops) {
-        G.opl[(o.i << G.d0) + o.lane] = inc - n;
-        if (o.lane == 0) G.opi[o.i].y = ex;
-    }
-    if (tid == 0) G.opn[blockIdx.x] = tot;
     if (!gb_last_block(&G.done[1])) return;
-    // exclusive sum over the CTAs, in place; the total is the path's raw vertex count
-    const int nb = (int)gridDim.x;
+    // exclusive sum over the blocks, in place; the total is the path's raw vertex count
+    const int nb = gb_ctas(G.n_ops);
     long long carry = 0;
     for (int b0 = 0; b0 < nb; b0 += BLOCK) {
         const int b = b0 + tid;
@@ -3241,21 +3251,23 @@ __global__ void __launch_bounds__(BLOCK) k_gb_emit(KParams P) {
     const long long n_raw = *G.n_raw;
     if (n_raw > G.raw_cap) return;  // every CTA: the caller grows the arrays
     int flags = 0;
-    const GbOp o = gb_op_of(G, flags);
-    if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC) {
-        const long long off0 = G.opn[blockIdx.x] + G.opi[o.i].y;
-        const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
-        int2* raw = G.raw;
-        unsigned char* fl = G.fl;
-        const int cap = G.raw_cap;
-        const unsigned char rs0 = (o.lane == 0 && o.rs) ? 1 : 0;
-        gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [&](int k, int2 q) {
-            if (ck(off + k < cap, 13) && off + k < cap) {
-                raw[off + k] = q;
-                fl[off + k] = k == 0 ? rs0 : (unsigned char)0;
-            }
-        });
-        if (rs0 && ck(off < cap, 13) && off < cap) atomicMax(&G.tr[off / GB_TILE], off);
+    for (int blk = blockIdx.x; blk < gb_ctas(G.n_ops); blk += gridDim.x) {
+        const GbOp o = gb_op_of(G, blk, flags);
+        if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC) {
+            const long long off0 = G.opn[blk] + G.opi[o.i].y;
+            const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
+            int2* raw = G.raw;
+            unsigned char* fl = G.fl;
+            const int cap = G.raw_cap;
+            const unsigned char rs0 = (o.lane == 0 && o.rs) ? 1 : 0;
+            gb_walk(P, o.op, o.kind, o.px, o.py, o.lane, G.d0, flags, [&](int k, int2 q) {
+                if (ck(off + k < cap, 13) && off + k < cap) {
+                    raw[off + k] = q;
+                    fl[off + k] = k == 0 ? rs0 : (unsigned char)0;
+                }
+            });
+            if (rs0 && ck(off < cap, 13) && off < cap) atomicMax(&G.tr[off / GB_TILE], off);
+        }
     }
     if (!gb_last_block(&G.done[2])) return;
     gb_scan_tr(G, n_raw, tmp, s_c);
@@ -3487,7 +3499,7 @@ cudaError_t launch_grid_build(const KParams& p, int sm_count, cudaStream_t s, co
     if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens of every op (the probe's too) and the pen width after
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
-        const int nbw = gb_ctas(q->gb.n_ops);
+        const int nbw = std::min(gb_ctas(q->gb.n_ops), 8 * sm_count);  // all resident: a skipped build only launches these
         if ((e = launch_chain(k_gb_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gb_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gb_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;
@@ -3634,28 +3646,30 @@ __global__ void __launch_bounds__(BLOCK) k_gs_count(KParams P) {
     if (S.skip && *S.skip) return;  // a probe over a prefix of the ops completed the points
     const int tid = threadIdx.x;
     int flags = 0;
-    const GbOp o = gb_op_of(G, flags);
-    int n = 0;
-    if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
-        n = gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
-                    [](int, P2, float) {});
+    for (int blk = blockIdx.x; blk < gb_ctas(G.n_ops); blk += gridDim.x) {
+        const GbOp o = gb_op_of(G, blk, flags);
+        int n = 0;
+        if (o.kind >= FT_OP_MOVE && o.kind <= FT_OP_CUBIC)
+            n = gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
+                        [](int, P2, float) {});
+        int inc = n;
+        const int lanes = 1 << G.d0;
+        for (int d = 1; d < lanes; d <<= 1) {
+            const int t = __shfl_up_sync(FULL, inc, d, lanes);
+            if (o.lane >= d) inc += t;
+        }
+        const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
+        int tot;
+        const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
+        if (o.i < G.n_ops) {
+            G.opl[(o.i << G.d0) + o.lane] = inc - n;
+            if (o.lane == 0) G.opi[o.i].y = ex;
+        }
+        if (tid == 0) G.opn[blk] = tot;
+    }
     if (flags) atomicMax(&P.status[0], (flags & 1) ? FT_ERR_DEPTH : FT_ERR_ARG);
-    int inc = n;
-    const int lanes = 1 << G.d0;
-    for (int d = 1; d < lanes; d <<= 1) {
-        const int t = __shfl_up_sync(FULL, inc, d, lanes);
-        if (o.lane >= d) inc += t;
-    }
-    const int n_op = __shfl_sync(FULL, inc, lanes - 1, lanes);
-    int tot;
-    const int ex = block_excl_sum(o.lane == 0 ? n_op : 0, tmp, tot);
-    if (o.i < G.n_ops) {
-        G.opl[(o.i << G.d0) + o.lane] = inc - n;
-        if (o.lane == 0) G.opi[o.i].y = ex;
-    }
-    if (tid == 0) G.opn[blockIdx.x] = tot;
     if (!gb_last_block(&S.done[0])) return;
-    const int nb = (int)gridDim.x;
+    const int nb = gb_ctas(G.n_ops);
     long long carry = 0;
     for (int b0 = 0; b0 < nb; b0 += BLOCK) {
         const int b = b0 + tid;
@@ -3674,26 +3688,28 @@ __global__ void __launch_bounds__(BLOCK) k_gs_emit(KParams P) {
     if (S.skip && *S.skip) return;  // a probe over a prefix of the ops completed the points
     if (gs_over(S)) return;  // every CTA: the caller grows the arrays
     int flags = 0;
-    const GbOp o = gb_op_of(G, flags);
-    if (o.kind < FT_OP_MOVE || o.kind > FT_OP_CUBIC) return;
-    const long long off0 = G.opn[blockIdx.x] + G.opi[o.i].y;
-    const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
-    const int cap = S.sraw_cap;
-    // a Move ends the sub-stroke before it open, a Close joined (stroker.rs:87-96)
-    const unsigned char f0 = (unsigned char)(((o.lane == 0 && o.rs) ? 1 : 0) | (o.kind != FT_OP_MOVE ? 2 : 0));
-    const unsigned char f1 = (unsigned char)(o.kind != FT_OP_MOVE ? 2 : 0);
-    float4* raw4 = S.raw4;
-    unsigned char* sfl = S.sfl;
-    int* sopi = S.sopi;
-    const int i = o.i;
-    gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
-            [&](int k, P2 q, float w) {
-                if (ck(off + k < cap, 13) && off + k < cap) {
-                    raw4[off + k] = make_float4(q.x, q.y, w, 0.f);
-                    sfl[off + k] = k == 0 ? f0 : f1;
-                    sopi[off + k] = i;
-                }
-            });
+    for (int blk = blockIdx.x; blk < gb_ctas(G.n_ops); blk += gridDim.x) {
+        const GbOp o = gb_op_of(G, blk, flags);
+        if (o.kind < FT_OP_MOVE || o.kind > FT_OP_CUBIC) continue;
+        const long long off0 = G.opn[blk] + G.opi[o.i].y;
+        const int off = (int)(off0 + G.opl[(o.i << G.d0) + o.lane]);
+        const int cap = S.sraw_cap;
+        // a Move ends the sub-stroke before it open, a Close joined (stroker.rs:87-96)
+        const unsigned char f0 = (unsigned char)(((o.lane == 0 && o.rs) ? 1 : 0) | (o.kind != FT_OP_MOVE ? 2 : 0));
+        const unsigned char f1 = (unsigned char)(o.kind != FT_OP_MOVE ? 2 : 0);
+        float4* raw4 = S.raw4;
+        unsigned char* sfl = S.sfl;
+        int* sopi = S.sopi;
+        const int i = o.i;
+        gs_walk(P, o.op, o.kind, o.px, o.py, gs_width(G, o.lpc), gs_width(G, o.i), o.lane, G.d0, flags,
+                [&](int k, P2 q, float w) {
+                    if (ck(off + k < cap, 13) && off + k < cap) {
+                        raw4[off + k] = make_float4(q.x, q.y, w, 0.f);
+                        sfl[off + k] = k == 0 ? f0 : f1;
+                        sopi[off + k] = i;
+                    }
+                });
+    }
 }
 
 // Kept raw stroke points and sub-stroke starts per tile, packed (kept << 32 | starts).
@@ -3970,7 +3986,7 @@ cudaError_t launch_grid_stroke(const KParams& p, int sm_count, cudaStream_t s, c
     if ((e = launch_chain(k_gb_ops, nbo, BLOCK, 0, s, p)) != cudaSuccess) return e;  // pens and widths of every op (the probe's too)
     for (const KParams* q : {probe, &p}) {
         if (!q) continue;
-        const int nbw = gb_ctas(q->gb.n_ops);
+        const int nbw = std::min(gb_ctas(q->gb.n_ops), 8 * sm_count);  // all resident: a skipped build only launches these
         if ((e = launch_chain(k_gs_count, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gs_emit, nbw, BLOCK, 0, s, *q)) != cudaSuccess) return e;
         if ((e = launch_chain(k_gs_keep, gt, BLOCK, 0, s, *q)) != cudaSuccess) return e;

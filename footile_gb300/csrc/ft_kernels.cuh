@@ -98,8 +98,9 @@ constexpr int GB_TOP_BLOCKS = 512;             // CTAs of the top-vertex search
 // complete a capped figure: 4096 x 4096 scene 188 / 178 / 168 us, its stroke 288 / 280 / 268;
 // on 3,780 ops, poster of 1531 x 1117 119 / 116 / 116 us.
 constexpr int GB_WIDE_OPS = 8192;
-constexpr int gb_d0(size_t n_ops) { return n_ops <= (size_t)GB_WIDE_OPS ? 5 : 3; }
-constexpr int gb_ctas(size_t n_ops) { return (int)(((n_ops << gb_d0(n_ops)) + BLOCK - 1) / BLOCK); }
+constexpr __host__ __device__ int gb_d0(size_t n_ops) { return n_ops <= (size_t)GB_WIDE_OPS ? 5 : 3; }
+constexpr __host__ __device__ int gb_ctas(size_t n_ops) { return (int)(((n_ops << gb_d0(n_ops)) + BLOCK - 1) / BLOCK); }
+constexpr int GB_STATE = 512;                  // bytes of counters at the front (gb_layout)
 constexpr long long GB_RAW_MAX = 1ll << 29;    // raw vertices the grid build takes at most
 struct GridBuildBufs {
     const ft_op* ops;   // the path's ops
@@ -112,8 +113,8 @@ struct GridBuildBufs {
     int4* opa;          // per 256 ops: last Move/Line/Quad/Cubic/Close op, last PenWidth op, last Close/Move op
     int* opw;           // per op: last PenWidth op at or before it in its 256 (strokes)
     int d0;             // gb_d0(n_ops)
-    long long* opn;     // per CTA of the walks: raw vertices
-    int2* opi;          // per op: last Move/Line/Quad/Cubic/Close op before it in its 256, raw offset in its CTA
+    long long* opn;     // per block of the walks: raw vertices
+    int2* opi;          // per op: last Move/Line/Quad/Cubic/Close op before it in its 256, raw offset in its block
     int* opl;           // per op and lane: the lane's raw offset in the op
     int2* raw;          // raw vertices, 16.16
     unsigned char* fl;  // per raw vertex: 1 = starts a sub-figure
@@ -160,7 +161,7 @@ constexpr GbLayout gb_layout(size_t n_ops, size_t raw_cap, size_t sraw_cap = 0) 
     // a stroke build's st[] at 128, n_sraw at 160, done[] at 192, its probe's n_sraw at 256,
     // done[] at 288, final at 320
     g.state = 0;
-    g.opa = 512;
+    g.opa = GB_STATE;
     g.opw = align256(g.opa + nbo * 16);
     g.opn = align256(g.opw + n_ops * 4);
     g.opi = align256(g.opn + nbw * 8);
@@ -235,6 +236,8 @@ struct KParams {
     int bin_segs;         // segments of seg_w pixels that a band's edges are binned by (1: not)
     int tile_batches;     // batches the calls are cut into (k_ctile)
     unsigned* tile_done;  // per tile: batches done
+    unsigned char* summary;  // a single call's page-locked read-back: edges binned, crec[0] at 16, the
+                             // grid build's counters at GB_STATE
     // one fill path built over the whole GPU (launch_grid_build) instead of by k_cbuild
     GridBuildBufs gb;
     GridStrokeBufs gs;  // and the stroker's part of one stroke path (launch_grid_stroke)
