@@ -205,8 +205,9 @@ FT_API void ft_batch_destroy(ft_batch* batch);
  * resident CTAs per SM of the persistent kernels (0 = occupancy maximum).
  * Ordered composites (ft_composite_batch, and single calls of at least split_px pixels):
  * `band_rows`, rows per band (1..8, 0 = built-in: 4 for Rgba8p, 8 for Matte8) — the
- * height of a compositor tile; `tile_w`, the width of an Rgba8p compositor tile in pixels
- * (128, 256, 512 or 1024, 0 = built-in: 1024, or the narrowest that needs no more tiles);
+ * height of a compositor tile or a multiple of it; `tile_w`, the pixels of a row that one warp
+ * of the Rgba8p compositor takes (128, 256, 512 or 1024, 0 = built-in: the row in equal parts of
+ * at most 1,024, up to four parts while their warps find room);
  * `tile_stage`, how an Rgba8p compositor tile reaches the canvas: 1 = staged in shared
  * memory by TMA (when the canvas base and row stride are 16-byte aligned), 2 = read and
  * written in place, 0 = built-in; `pool_edges`, the first size of the binned-edge pool in edges (it
