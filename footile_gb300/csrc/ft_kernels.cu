@@ -2047,17 +2047,18 @@ __device__ __forceinline__ bool smem_wait(const unsigned* word, unsigned& v, F d
     return false;
 }
 
-// Wait until a tile's `batch` batches are done; false after ten seconds.
+// Wait until a tile's `batch` batches are done; false after a hundred seconds (a batch of
+// very many heavy calls may take some).
 __device__ __forceinline__ bool tile_wait(const unsigned* done, unsigned batch) {
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    for (int it = 0; it < (1 << 28); it++) {
+    for (int it = 0; it < (1 << 30); it++) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
         if (v >= batch) return true;
         __nanosleep(200);
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (t - t0 > 10000000000ull) break;
+        if (t - t0 > 100000000000ull) break;
     }
     return false;
 }
