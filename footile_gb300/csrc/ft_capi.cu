@@ -1173,10 +1173,12 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
     const int tile_w = composite_tile_w(c, w, h);
     const int stage = (c->tuned && c->tune.tile_stage > 0) ? c->tune.tile_stage : 1;
     // The segments of a row that fit in one tile have their edges binned by segment, while the
-    // build's counters of all bins fit in the shared memory it runs with.
+    // build's counters of all bins fit in the shared memory it runs with and the bins' offsets of
+    // all calls in 16 GB (by bands alone they are as many times fewer as there are segments).
     const int n_segs = (int)((w + tile_w - 1) / tile_w);
     const bool by_segs = fmt == FT_RGBA8P && n_paths > 1 && n_segs <= ftk::CT_MAX_SEGS &&
-                         ((size_t)n_bands * n_segs + 1) * sizeof(int) <= (size_t)build_smem(c, 0);
+                         ((size_t)n_bands * n_segs + 1) * sizeof(int) <= (size_t)build_smem(c, 0) &&
+                         ((size_t)n_bands * n_segs + 1) * sizeof(int) * n_paths <= (16ull << 30);
     const int bin_segs = by_segs ? std::max(n_segs, 1) : 1;
     const int smem_b = fmt == FT_MATTE8 ? ftk::composite_bands_smem(R, (int)w)
                                         : ftk::composite_tile_smem(R, bin_segs, tile_w, stage == 1);
