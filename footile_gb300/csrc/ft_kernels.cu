@@ -2298,8 +2298,11 @@ __global__ void __launch_bounds__(128, 5) k_ctile(KParams P, const __grid_consta
                     const int y = r + __shfl_sync(FULL, cr.y, j);
                     const int4* E = reinterpret_cast<const int4*>(P.pool + first);
                     if (dmask) {  // the next call's first edges, on their way meanwhile
-                        const unsigned long long nf = __shfl_sync(FULL, my_first, __ffs(dmask) - 1);
-                        asm volatile("prefetch.global.L1 [%0];" ::"l"(P.pool + nf + lane));
+                        const int nj = __ffs(dmask) - 1;
+                        const unsigned long long nf = __shfl_sync(FULL, my_first, nj);
+                        const int nn = ct_ahead(__shfl_sync(FULL, o1 - o0, nj));
+                        if (lane < nn && ck(nf + lane < P.pool_cap, 17))
+                            asm volatile("prefetch.global.L1 [%0];" ::"l"(P.pool + nf + lane));
                     }
                     unsigned base = 0;  // the running sum entering the segment
                     for (int e = lane; e < ne; e += 32) {

@@ -303,6 +303,9 @@ cudaError_t launch_composite_bands(const KParams& p, int smem_bytes, cudaStream_
 cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_count, cudaStream_t s);
 int composite_tiles(const KParams& p);
 constexpr int CT_MAX_SEGS = 4;  // segments of a row in one tile
+// Edges of a run of `n` that a warp asks L1 for ahead, one a lane.  A call may have none in a
+// warp's bin, and the last run of the pool ends where the pool may end: never past the run.
+constexpr __host__ __device__ int ct_ahead(int n) { return n < 32 ? n : 32; }
 int composite_tile_smem(int band_rows, int bin_segs, int seg_w, bool staged);
 int composite_tile_rows(int band_rows, int bin_segs);  // rows of a tile (and of its tensor-map boxes)
 // SrcOver of one call's colour onto the canvas rows r0.. from its Matte8 coverage `mask`
