@@ -1803,13 +1803,17 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
 }  // namespace
 
 // The backward reads g at each piece's own cell and needs no shared band.
+cudaError_t setup_adjoint() {
+    return cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                BAND_FLOATS * (int)sizeof(float));
+}
+
 int adjoint_blocks_per_sm(bool backward) {
     const int smem = BAND_FLOATS * (int)sizeof(float);
     int n = 0;
     if (backward) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adjoint<true>, ABLOCK, (int)sizeof(SlotBuf));
     } else {
-        cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_adjoint<false>, ABLOCK, smem);
     }
     return n > 0 ? n : 1;
@@ -1820,7 +1824,6 @@ cudaError_t launch_adjoint(bool backward, const AParams& p, int grid, cudaStream
     if (backward) {
         k_adjoint<true><<<grid, ABLOCK, sizeof(SlotBuf), s>>>(p);
     } else {
-        cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         k_adjoint<false><<<grid, ABLOCK, smem, s>>>(p);
     }
     return cudaGetLastError();

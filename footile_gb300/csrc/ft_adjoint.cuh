@@ -71,5 +71,6 @@ struct AParams {
 
 cudaError_t launch_adjoint(bool backward, const AParams& p, int grid, cudaStream_t s);
 int adjoint_blocks_per_sm(bool backward);
+cudaError_t setup_adjoint();  // as ftk::setup_kernels
 
 }  // namespace fta

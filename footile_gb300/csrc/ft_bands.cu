@@ -139,8 +139,6 @@ __global__ void __launch_bounds__(256) k_srcover_rows(uint8_t* canvas, unsigned 
 template <int NT>
 cudaError_t launch_band(const KParams& p, cudaStream_t s) {
     const int smem = band_smem(NT, p.band_rows, (int)p.canvas_w);
-    cudaError_t e = cudaFuncSetAttribute(k_band_single<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     k_band_single<NT><<<p.n_bands, NT, smem, s>>>(p);
     return cudaGetLastError();
 }
@@ -160,6 +158,12 @@ cudaError_t launch_srcover_rows(uint8_t* canvas, uint32_t stride, const uint8_t*
     const int nseg = (W + 256 * SR_PX - 1) / (256 * SR_PX);
     k_srcover_rows<<<(H - r0) * nseg, 256, 0, s>>>(canvas, stride, mask, mstride, W, r0, nseg, clr);
     return cudaGetLastError();
+}
+
+cudaError_t setup_bands() {
+    cudaError_t e = allow_smem((const void*)k_band_single<256>);
+    if (e == cudaSuccess) e = allow_smem((const void*)k_band_single<512>);
+    return e == cudaSuccess ? allow_smem((const void*)k_band_single<1024>) : e;
 }
 
 int band_single_smem(int band_rows, int width) { return band_smem(256, band_rows, width); }

@@ -17,6 +17,10 @@
 #include "ft_adjoint.cuh"
 #include "ft_kernels.cuh"
 
+namespace ftc {
+cudaError_t setup_convert();  // as ftk::setup_kernels
+}
+
 namespace {
 
 struct DevBuf {
@@ -647,7 +651,7 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
     b->params.queue = static_cast<uint32_t*>(b->queue.p);
     b->params.status = static_cast<int32_t*>(b->status.p);
     b->params.scratch = static_cast<unsigned char*>(b->scratch.p);
-    ftk::raster_blocks_per_sm(b->smem, stroke != 0);  // sets the kernels' shared-memory attributes outside capture
+    ftk::raster_blocks_per_sm(b->smem, stroke != 0);  // sets the kernel's shared-memory carveout outside capture
     *out = b;
     return FT_OK;
 }
@@ -762,6 +766,11 @@ FT_API int ft_ctx_create(int device, ft_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
     if (e == cudaSuccess) e = cudaEventCreate(&c->ev_comp);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = ftk::setup_kernels();
+    if (e == cudaSuccess) e = ftk::setup_tile();
+    if (e == cudaSuccess) e = ftk::setup_bands();
+    if (e == cudaSuccess) e = fta::setup_adjoint();
+    if (e == cudaSuccess) e = ftc::setup_convert();
     if (e != cudaSuccess) {
         delete c;
         return FT_ERR_CUDA;

@@ -101,11 +101,13 @@ __global__ void __launch_bounds__(CBLOCK, 2) k_convert(const uint8_t* src, uint3
     }
 }
 
+cudaError_t setup_convert() {
+    return cudaFuncSetAttribute(k_convert<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, convert_smem(true));
+}
 int convert_block() { return CBLOCK; }
 int convert_blocks_per_sm(int src_fmt) {
     const bool rgba = src_fmt == FT_RGBA8P;
     auto kern = rgba ? k_convert<true> : k_convert<false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, convert_smem(rgba));
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, CBLOCK, convert_smem(rgba)) != cudaSuccess) return 1;
     return n > 0 ? n : 1;

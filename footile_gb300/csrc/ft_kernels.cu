@@ -1651,8 +1651,6 @@ cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream
     auto kern = p.stroke ? k_raster<true> : k_raster<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                          few_ctas ? FEW_CTAS_CARVEOUT : (int)cudaSharedmemCarveoutDefault);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
     if (chained) return launch_chain(kern, grid, BLOCK, smem_bytes, s, p);
     kern<<<grid, BLOCK, smem_bytes, s>>>(p);
     return cudaGetLastError();
@@ -1665,7 +1663,6 @@ cudaError_t launch_raster(const KParams& p, int grid, int smem_bytes, cudaStream
 int raster_blocks_per_sm(int smem_bytes, bool stroke) {
     auto kern = stroke ? k_raster<true> : k_raster<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutDefault);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, BLOCK, smem_bytes) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
@@ -2613,8 +2610,6 @@ __global__ void __launch_bounds__(SO_THREADS, 6) k_srcover_mask(const __grid_con
 
 cudaError_t launch_srcover_mask(const CUtensorMap& canvas, const CUtensorMap& mask, int W, int H, int r0,
                                 unsigned clr, int32_t* status, int sm_count, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_srcover_mask, cudaFuncAttributeMaxDynamicSharedMemorySize, SO_SMEM);
-    if (e != cudaSuccess) return e;
     const int ntiles = ((W + SO_COLS - 1) / SO_COLS) * ((H - r0 + SO_ROWS - 1) / SO_ROWS);
     if (ntiles <= 0) return cudaSuccess;
     const int grid = std::max(1, std::min(ntiles, 6 * sm_count));
@@ -2638,11 +2633,10 @@ cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_co
     const int smem = ctile_layout(t, p.seg_w, staged).bytes;
     auto kern = staged ? (odd ? k_ctile<true, FT_EVENODD> : k_ctile<true, FT_NONZERO>)
                        : (odd ? k_ctile<false, FT_EVENODD> : k_ctile<false, FT_NONZERO>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     const int threads = 32 * t.rows * t.segs;
     int per_sm = 0;
+    cudaError_t e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem)) != cudaSuccess) return e;
     const int tiles = composite_tiles(p), slots = std::max(1, per_sm) * sm_count;
     // A tile beyond the resident ones would be composited alone, from the first call to the last
@@ -2870,12 +2864,7 @@ cudaError_t launch_figure_bins(const KParams& p, int grid, cudaStream_t s) {
     const bool local = p.n_bands <= BIN_SMEM_BANDS;
     const int sm_e = local ? (p.n_bands + 1) * (int)sizeof(int) : 0;
     const int sm_f = local ? ((2 * p.n_bands + 1 + 3) & ~3) * (int)sizeof(int) + (int)sizeof(BinStage) : 0;
-    cudaError_t e = cudaFuncSetAttribute(k_fig_bin_fill, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         ((2 * BIN_SMEM_BANDS + 1 + 3) & ~3) * (int)sizeof(int) + (int)sizeof(BinStage));
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_fig_edges, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (BIN_SMEM_BANDS + 1) * (int)sizeof(int));
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
     if ((e = launch_chain(k_fig_edges, grid, BLOCK, sm_e, s, p)) != cudaSuccess) return e;
     if ((e = launch_chain(k_fig_bin_scan, 1, BLOCK, 0, s, p)) != cudaSuccess) return e;
     return launch_chain(k_fig_bin_fill, grid, BLOCK, sm_f, s, p);
@@ -4009,8 +3998,6 @@ cudaError_t launch_composite_build(const KParams& p, int grid, int smem_bytes, c
     auto kern = p.stroke ? k_cbuild<true> : k_cbuild<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
                          few_ctas ? FEW_CTAS_CARVEOUT : (int)cudaSharedmemCarveoutDefault);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
     kern<<<grid, BLOCK, smem_bytes, s>>>(p);
     return cudaGetLastError();
 }
@@ -4019,17 +4006,38 @@ cudaError_t launch_composite_build(const KParams& p, int grid, int smem_bytes, c
 int composite_build_blocks_per_sm(int smem_bytes, bool stroke) {
     auto kern = stroke ? k_cbuild<true> : k_cbuild<false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutDefault);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, BLOCK, smem_bytes) != cudaSuccess) return 1;
     return n > 0 ? n : 1;
 }
 
 cudaError_t launch_composite_bands(const KParams& p, int smem_bytes, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_cbands, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-    if (e != cudaSuccess) return e;
     k_cbands<<<p.n_bands, 32 * p.band_rows, smem_bytes, s>>>(p);
     return cudaGetLastError();
+}
+
+cudaError_t allow_smem(const void* kern) {
+    int dev = 0, most = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+    return e;
+}
+cudaError_t setup_kernels() {
+    const void* kernels[] = {(const void*)k_raster<false>,  (const void*)k_raster<true>,
+                             (const void*)k_cbuild<false>,  (const void*)k_cbuild<true>,
+                             (const void*)k_cbands,         (const void*)k_srcover_mask,
+                             (const void*)k_fig_edges,      (const void*)k_fig_bin_fill,
+                             (const void*)k_ctile<true, FT_NONZERO>,  (const void*)k_ctile<true, FT_EVENODD>,
+                             (const void*)k_ctile<false, FT_NONZERO>, (const void*)k_ctile<false, FT_EVENODD>};
+    for (const void* k : kernels) {
+        const cudaError_t e = allow_smem(k);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace ftk

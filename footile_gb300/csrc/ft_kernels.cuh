@@ -360,4 +360,13 @@ int raster_blocks_per_sm(int smem_bytes, bool stroke);
 // Maximum dynamic shared memory the kernel may be configured for.
 int raster_max_smem();
 
+// Let the kernels take as much dynamic shared memory as the current device has.  The limit belongs
+// to a kernel and device, not to a context: it is set to the same value whenever a context is
+// created and by no launch (a launch that set it to its own size took it away from another
+// context's thread between that one's setting and launch).
+cudaError_t allow_smem(const void* kern);
+cudaError_t setup_kernels();
+cudaError_t setup_tile();
+cudaError_t setup_bands();
+
 }  // namespace ftk

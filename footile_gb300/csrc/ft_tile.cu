@@ -653,21 +653,18 @@ int tile_smem(int threads, int area_ints, bool staged) {
 
 int tile_blocks_per_sm(int threads, int smem) {
     int n = 0;
-    cudaError_t e;
-    if (threads == 128) {
-        cudaFuncSetAttribute(k_tile<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<128>, 128, smem);
-    } else {
-        cudaFuncSetAttribute(k_tile<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<512>, 512, smem);
-    }
+    const cudaError_t e =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, threads == 128 ? k_tile<128> : k_tile<512>, threads, smem);
     return e == cudaSuccess && n > 0 ? n : 1;
+}
+
+cudaError_t setup_tile() {
+    const cudaError_t e = allow_smem((const void*)k_tile<128>);
+    return e == cudaSuccess ? allow_smem((const void*)k_tile<512>) : e;
 }
 
 cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cudaStream_t s) {
     auto kern = threads == 128 ? k_tile<128> : k_tile<512>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
     kern<<<grid, threads, smem, s>>>(p);
     return cudaGetLastError();
 }
