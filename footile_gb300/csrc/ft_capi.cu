@@ -23,9 +23,14 @@ cudaError_t setup_convert();  // as ftk::setup_kernels
 
 namespace {
 
+// Device memory that grows; given back with the object that holds it.
 struct DevBuf {
     void* p = nullptr;
     size_t cap = 0;
+    DevBuf() = default;
+    DevBuf(const DevBuf&) = delete;
+    DevBuf& operator=(const DevBuf&) = delete;
+    ~DevBuf() { release(); }
     cudaError_t ensure(size_t bytes) {
         if (bytes <= cap) return cudaSuccess;
         if (p) {
@@ -60,10 +65,6 @@ struct PlanSlot {
     ftk::TilePlan tile;
     int smem = -1, stroke = -1, wside = -1;
     uint64_t split = 0;
-    void release() {
-        items.release();
-        items_w.release();
-    }
 };
 }  // namespace
 
@@ -567,16 +568,8 @@ struct ft_batch {
     void* g_ras = nullptr;
     cudaStream_t g_stream = nullptr;
     cudaGraphExec_t exec = nullptr;
-    void release() {
+    ~ft_batch() {
         if (exec) cudaGraphExecDestroy(exec);
-        exec = nullptr;
-        paths.release();
-        items.release();
-        items_w.release();
-        overflow.release();
-        status.release();
-        queue.release();
-        scratch.release();
     }
 };
 
@@ -637,7 +630,6 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
                             cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
-        b->release();
         delete b;
         return cuda_fail(c, e, "batch setup");
     }
@@ -720,8 +712,6 @@ FT_API int ft_batch_launch_status(ft_ctx* c, ft_batch* b, int32_t* status, uint3
 }
 
 FT_API void ft_batch_destroy(ft_batch* b) {
-    if (!b) return;
-    b->release();
     delete b;
 }
 
@@ -785,16 +775,9 @@ FT_API void ft_ctx_destroy(ft_ctx* c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    c->plan.release();
-    for (auto& sl : c->chunk_plans) sl->release();
     for (cudaEvent_t e : c->ev_chunk) cudaEventDestroy(e);
     if (c->s_in) cudaStreamDestroy(c->s_in);
     if (c->s_out) cudaStreamDestroy(c->s_out);
-    DevBuf* bufs[] = {&c->ops,     &c->paths,   &c->overflow,
-                      &c->status,  &c->sw_out,  &c->rasters, &c->queue,   &c->scratch,
-                      &c->sw_chain, &c->pool,   &c->pool_used, &c->bandoff, &c->crec,
-                      &c->srgb_lut, &c->conv_src, &c->conv_dst, &c->figbins, &c->mask, &c->tile_done};
-    for (DevBuf* b : bufs) b->release();
     if (c->h_sum) cudaFreeHost(c->h_sum);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev_comp) cudaEventDestroy(c->ev_comp);
@@ -1829,8 +1812,6 @@ FT_API void ft_adjoint_destroy(ft_adjoint* a) {
         cudaSetDevice(a->ctx->device);
         if (a->ctx->stream) cudaStreamSynchronize(a->ctx->stream);
     }
-    DevBuf* bufs[] = {&a->ops, &a->paths, &a->area, &a->status, &a->scratch, &a->cov, &a->gcov, &a->gops, &a->gwidth};
-    for (DevBuf* b : bufs) b->release();
     delete a;
 }
 
@@ -2149,8 +2130,6 @@ FT_API void ft_stroke_composite_destroy(ft_composite_adjoint* s) {
         if (s->ctx->stream) cudaStreamSynchronize(s->ctx->stream);
     }
     ft_adjoint_destroy(s->adj);
-    DevBuf* bufs[] = {&s->ops, &s->clr, &s->prefix, &s->cov, &s->gcov, &s->gbuf, &s->status, &s->gops, &s->gwidth};
-    for (DevBuf* b : bufs) b->release();
     delete s;
 }
 
