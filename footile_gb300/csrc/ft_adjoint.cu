@@ -815,7 +815,9 @@ __device__ void edge_integrals(int W, int H, int V, const float2* vpos, const in
                 const float cl = floorf(xl), cr = floorf(xr);
                 const bool one = cl == cr || xr == xl;  // one cell
                 const int first = cl < 0.0f ? 0 : (cl < (float)W ? (int)cl : W);  // cells from the raster's left on
-                const int end = one ? (cl < 0.0f ? -1 : first) : (int)fminf(cr, (float)(W - 1));
+                // the last cell with some of the edge in it: one that the edge only touches from the left is
+                // not read, whose gradient need not be finite
+                const int end = one ? (cl < 0.0f ? -1 : first) : (int)fminf(xr > cr ? cr : __fsub_rn(cr, 1.0f), (float)(W - 1));
                 // the edge's parameter along x: u(x) = ut or ub at xl, du / span per pixel
                 const float dy = __fsub_rn(b.y, a.y);
                 const float ut = __fdiv_rn(__fsub_rn(yt, a.y), dy), ub = __fdiv_rn(__fsub_rn(yb, a.y), dy);
