@@ -21,16 +21,19 @@ constexpr size_t AS_POS = 0;                                              // flo
 constexpr size_t AS_SUB = a_align(AS_POS + (size_t)VCAP * 8);             // int[VCAP]
 constexpr size_t AS_GRAD = a_align(AS_SUB + (size_t)VCAP * 4);            // float2[VCAP]
 constexpr size_t AS_FLAG = a_align(AS_GRAD + (size_t)VCAP * 8);           // int[VCAP]
-constexpr size_t VPROV_BYTES = 16;
-constexpr size_t AS_PROV = a_align(AS_FLAG + (size_t)VCAP * 4);           // where each vertex came from (backward)
 // Edges binned by row band, built once per path: band k's edges are
 // blist[boff[k] .. boff[k + 1]).  Paths with more bands or (edge, band) pairs scan
 // every edge for every band instead.
 constexpr int NB_CAP = BAND_FLOATS - 1;     // bands (the shared band buffer is the histogram)
 constexpr int PAIR_CAP = 1 << 18;           // (edge, band) pairs
-constexpr size_t AS_BOFF = a_align(AS_PROV + (size_t)VCAP * VPROV_BYTES);  // int[NB_CAP + 1]
+constexpr size_t AS_BOFF = a_align(AS_FLAG + (size_t)VCAP * 4);          // int[NB_CAP + 1]
 constexpr size_t AS_BLIST = a_align(AS_BOFF + (size_t)(NB_CAP + 1) * 4);  // int[PAIR_CAP]
 constexpr size_t A_SCRATCH_PER_CTA = a_align(AS_BLIST + (size_t)PAIR_CAP * 4);
+// Where each vertex came from, in the place of the bins: the forward alone bins edges, the
+// backward alone chains vertices (1 MB of 3.7 for each of some 450 CTAs of every Adjoint).
+constexpr size_t VPROV_BYTES = 16;
+constexpr size_t AS_PROV = AS_BLIST;
+static_assert(AS_PROV + (size_t)VCAP * VPROV_BYTES <= A_SCRATCH_PER_CTA, "provenance fits the bins");
 
 // Strokes add, after the fill arrays: the node of each outline vertex, stroke points,
 // sub-strokes, outline nodes (offset points, miter intersections, arc points) and
