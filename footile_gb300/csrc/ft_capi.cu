@@ -41,7 +41,10 @@ struct DevBuf {
         cap = 0;
         size_t want = std::max(bytes, (size_t)256);
         cudaError_t e = cudaMalloc(&p, want);
-        if (e == cudaSuccess) cap = want;
+        if (e == cudaSuccess)
+            cap = want;
+        else
+            cudaGetLastError();  // reported here: the next launch's check must not find it
         return e;
     }
     void release() {
@@ -1121,9 +1124,12 @@ FT_API int ft_composite_batch(ft_ctx* c, int32_t stroke, int32_t rule, const ft_
 
 }  // extern "C"
 
-static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* ops, uint32_t n_ops_total,
-                          const ft_path_desc* paths, uint32_t n_paths, int32_t fmt, uint8_t* raster, uint32_t w,
-                          uint32_t h, uint32_t stride, int32_t where, float* sw_out, const float* sw_in) {
+// One composite; `segs`: its edges may be binned by segment, and whether they were.
+static int composite_run(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* ops, uint32_t n_ops_total,
+                         const ft_path_desc* paths, uint32_t n_paths, int32_t fmt, uint8_t* raster, uint32_t w,
+                         uint32_t h, uint32_t stride, int32_t where, float* sw_out, const float* sw_in, bool& segs) {
+    const bool may_segs = segs;
+    segs = false;
     if (!c) return FT_ERR_ARG;
     if ((rule != FT_NONZERO && rule != FT_EVENODD) || (fmt != FT_MATTE8 && fmt != FT_RGBA8P) ||
         (where != FT_HOST && where != FT_DEVICE))
@@ -1168,7 +1174,7 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
     // build's counters of all bins fit in the shared memory it runs with and the bins' offsets of
     // all calls in 16 GB (by bands alone they are as many times fewer as there are segments).
     const int n_segs = (int)((w + tile_w - 1) / tile_w);
-    const bool by_segs = fmt == FT_RGBA8P && n_paths > 1 && n_segs <= ftk::CT_MAX_SEGS &&
+    const bool by_segs = segs = may_segs && fmt == FT_RGBA8P && n_paths > 1 && n_segs <= ftk::CT_MAX_SEGS &&
                          ((size_t)n_bands * n_segs + 1) * sizeof(int) <= (size_t)build_smem(c, 0) &&
                          ((size_t)n_bands * n_segs + 1) * sizeof(int) * n_paths <= (16ull << 30);
     const int bin_segs = by_segs ? std::max(n_segs, 1) : 1;
@@ -1490,6 +1496,24 @@ static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* 
         return FT_OK;
     }
     return fail(c, FT_ERR_NOMEM, "edge pool did not converge");
+}
+
+// Bins by segment take up to CT_MAX_SEGS times the memory (offsets, and edges that reach several
+// segments): where it cannot be had, nothing is drawn yet and the edges are binned by band alone.
+static int composite_impl(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* ops, uint32_t n_ops_total,
+                          const ft_path_desc* paths, uint32_t n_paths, int32_t fmt, uint8_t* raster, uint32_t w,
+                          uint32_t h, uint32_t stride, int32_t where, float* sw_out, const float* sw_in) {
+    bool segs = true;
+    int st = composite_run(c, stroke, rule, ops, n_ops_total, paths, n_paths, fmt, raster, w, h, stride, where, sw_out,
+                           sw_in, segs);
+    if (st == FT_ERR_NOMEM && segs) {
+        segs = false;
+        c->bandoff.release();
+        c->pool.release();
+        st = composite_run(c, stroke, rule, ops, n_ops_total, paths, n_paths, fmt, raster, w, h, stride, where, sw_out,
+                           sw_in, segs);
+    }
+    return st;
 }
 
 // ---------------------------------------------------------------- conversion
