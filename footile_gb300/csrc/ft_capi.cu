@@ -1477,7 +1477,7 @@ static int composite_run(ft_ctx* c, int32_t stroke, int32_t rule, const ft_op* o
                                 ? 1
                                 : 0;
                 FT_CU(cudaEventRecord(c->ev_comp, c->stream), "event");
-                FT_CU(c->tile_done.ensure(sizeof(unsigned) * (size_t)ftk::composite_tiles(p)), "alloc tile counters");
+                FT_CU(c->tile_done.ensure(2 * sizeof(unsigned) * (size_t)ftk::composite_tiles(p)), "alloc tile counters");
                 p.tile_done = static_cast<unsigned*>(c->tile_done.p);
                 FT_CU(ftk::launch_composite_tiles(p, tm, c->sm_count, c->stream), "launch tile compositor");
                 c->comp_timed = true;

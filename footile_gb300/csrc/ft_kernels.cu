@@ -2027,36 +2027,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, unsigned parity) {
     return false;
 }
 
-// Wait until `done(word)` of a word in shared memory that another warp writes; false after ten
-// seconds.
+// Wait until `done(word)` of a word in shared memory that another warp writes; false when it gives
+// up (CT_POLLS_SMEM).
 template <class F>
 __device__ __forceinline__ bool smem_wait(const unsigned* word, unsigned& v, F done) {
-    unsigned long long t0 = 0, t;
-    for (int it = 0; it < (1 << 30); it++) {
+    Patience p;
+    do {
         v = *reinterpret_cast<const volatile unsigned*>(word);
         if (done(v)) return true;
-        if ((it & 255) == 255) {
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (!t0) t0 = t;
-            if (t - t0 > 10000000000ull) break;
-        }
-    }
+    } while (!p.ends(v, CT_POLLS_SMEM));
     return false;
 }
 
-// Wait until a tile's `batch` batches are done; false after a hundred seconds (a batch of
-// very many heavy calls may take some).
-__device__ __forceinline__ bool tile_wait(const unsigned* done, unsigned batch) {
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    for (int it = 0; it < (1 << 30); it++) {
-        unsigned v;
+// Wait until a tile's `batch` batches are done; false when it gives up (CT_POLLS_TILE).
+__device__ __forceinline__ bool tile_wait(const unsigned* done, const unsigned* rounds, unsigned batch) {
+    Patience p;
+    unsigned v, r;
+    do {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(done) : "memory");
         if (v >= batch) return true;
         __nanosleep(200);
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        if (t - t0 > 100000000000ull) break;
-    }
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(r) : "l"(rounds) : "memory");
+    } while (!p.ends(r, CT_POLLS_TILE));
     return false;
 }
 
@@ -2203,7 +2195,7 @@ __global__ void __launch_bounds__(128, 5) k_ctile(KParams P, const __grid_consta
             const int u = (int)atomicAdd(&P.queue[3], 1u);
             s_unit = u;
             if (u >= n_tiles && u < n_tiles * P.tile_batches &&
-                !tile_wait(P.tile_done + u % n_tiles, (unsigned)(u / n_tiles)))
+                !tile_wait(P.tile_done + u % n_tiles, P.tile_done + n_tiles + u % n_tiles, (unsigned)(u / n_tiles)))
                 ok = false;
         }
         ok = __syncthreads_and(ok) != 0;
@@ -2423,6 +2415,7 @@ __global__ void __launch_bounds__(128, 5) k_ctile(KParams P, const __grid_consta
                 }
                 __syncwarp();
                 if (has_in && lane == 0) *reinterpret_cast<volatile unsigned*>(in + CT_CHAIN) = m;
+                if (P.tile_batches > 1 && lane == 0) atomicAdd(P.tile_done + n_tiles + tix, 1u);
                 const int G0 = G;
                 G += __popc(rmask);
                 if ((G0 >> 6) != (G >> 6)) {
@@ -2647,7 +2640,7 @@ cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_co
     if (tiles > slots)
         for (int nb = 2; nb <= 16 && (int)p.n_items >= 32 * nb; nb++)
             if (rounds(nb) < 0.97 * rounds(p.tile_batches)) p.tile_batches = nb;
-    if (p.tile_batches > 1 && (e = cudaMemsetAsync(p.tile_done, 0, sizeof(unsigned) * tiles, s)) != cudaSuccess) return e;
+    if (p.tile_batches > 1 && (e = cudaMemsetAsync(p.tile_done, 0, 2 * sizeof(unsigned) * tiles, s)) != cudaSuccess) return e;
     kern<<<(int)std::min<long long>((long long)tiles * p.tile_batches, slots), threads, smem, s>>>(p, tmap);
     return cudaGetLastError();
 }

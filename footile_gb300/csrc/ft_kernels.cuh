@@ -235,7 +235,7 @@ struct KParams {
     int use_tma;
     int bin_segs;         // segments of seg_w pixels that a band's edges are binned by (1: not)
     int tile_batches;     // batches the calls are cut into (k_ctile)
-    unsigned* tile_done;  // per tile: batches done
+    unsigned* tile_done;  // per tile: batches done, then per tile: rounds of 32 calls that warps are through with
     unsigned char* summary;  // a single call's page-locked read-back: edges binned, crec[0] at 16, the
                              // grid build's counters at GB_STATE
     // one fill path built over the whole GPU (launch_grid_build) instead of by k_cbuild
@@ -299,9 +299,25 @@ cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cu
 cudaError_t launch_composite_build(const KParams& p, int grid, int smem_bytes, cudaStream_t s, bool few_ctas);
 cudaError_t launch_composite_bands(const KParams& p, int smem_bytes, cudaStream_t s);
 // Rgba8p: tiles of band_rows x seg_w pixels, canvas staged through `tmap` when use_tma.
-// p.tile_done: composite_tiles(p) words, p.queue[3] zero.
+// p.tile_done: 2 * composite_tiles(p) words, p.queue[3] zero.
 cudaError_t launch_composite_tiles(KParams p, const CUtensorMap& tmap, int sm_count, cudaStream_t s);
 int composite_tiles(const KParams& p);
+// Waits of the tile compositor end after this many polls in which the work waited for has not moved
+// (64 s and more of polling).  Polls and not the clock: neither calls that take long nor a GPU
+// given to others meanwhile may fail a composite.
+constexpr unsigned CT_POLLS_TILE = 1u << 27;  // of half a microsecond and more
+constexpr unsigned CT_POLLS_SMEM = 1u << 31;  // of some 60 cycles
+struct Patience {
+    unsigned seen = 0, polls = 0;
+    // after a poll that found `moved`, any word that the work waited for changes as it goes on
+    __host__ __device__ bool ends(unsigned moved, unsigned limit) {
+        if (moved != seen) {
+            seen = moved;
+            polls = 0;
+        }
+        return ++polls > limit;
+    }
+};
 constexpr int CT_MAX_SEGS = 4;  // segments of a row in one tile
 // Edges of a run of `n` that a warp asks L1 for ahead, one a lane.  A call may have none in a
 // warp's bin, and the last run of the pool ends where the pool may end: never past the run.
