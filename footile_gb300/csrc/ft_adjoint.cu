@@ -268,7 +268,7 @@ __device__ int list_slots(ASmem& sm, SlotBuf& Q, int slots, P2 A, P2 B, P2 C, P2
         if (k < wp) pre += v;
         sum += v;
     }
-    if (slots) {
+    if (slots && ftk::ck((pre + inc - own) >> 22 < (unsigned)ABLOCK, 31)) {
         const unsigned ex = pre + inc - own;
         const int at = (int)(ex >> 22);
         Q.g0[at] = make_float4(A.x, A.y, B.x, B.y);
@@ -749,6 +749,7 @@ __device__ void band_areas(ASmem& sm, float* band, int W, int b0, int nb, int V,
                 const int r = r0 + (it - sm.off[slot]);
                 float* row = band + (size_t)(r - b0) * W;
                 row_cells(E, r, W, [&](int c, float h, float xm) {
+                    if (!ftk::ck(r >= b0 && r < b0 + nb && c < W && nb * W <= BAND_FLOATS, 30)) return;
                     const float dh = __fmul_rn(E.dir, h);
                     if (c < 0) {
                         atomicAdd(row, dh);
@@ -1805,6 +1806,8 @@ __global__ void __launch_bounds__(ABLOCK, 3) k_adjoint(AParams p) {
 }  // namespace
 
 // The backward reads g at each piece's own cell and needs no shared band.
+cudaError_t take_check_adjoint(ftk::CheckState* s, bool reached) { return ftk::take_check(s, reached); }
+
 cudaError_t setup_adjoint() {
     return cudaFuncSetAttribute(k_adjoint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 BAND_FLOATS * (int)sizeof(float));

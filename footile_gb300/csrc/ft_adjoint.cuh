@@ -7,6 +7,10 @@
 
 #include "../../include/footile_gpu.h"
 
+namespace ftk {
+struct CheckState;
+}
+
 namespace fta {
 
 constexpr int ABLOCK = 256;                 // threads per CTA (one CTA per path at a time)
@@ -75,5 +79,6 @@ struct AParams {
 cudaError_t launch_adjoint(bool backward, const AParams& p, int grid, cudaStream_t s);
 int adjoint_blocks_per_sm(bool backward);
 cudaError_t setup_adjoint();  // as ftk::setup_kernels
+cudaError_t take_check_adjoint(ftk::CheckState* s, bool reached);  // as ftk::take_check_tile
 
 }  // namespace fta

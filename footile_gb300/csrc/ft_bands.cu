@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(NT, 1) k_band_single(KParams P) {
         SegRec s;
         s.n_items = 0;
         s.ra = s.rb = make_int4(0, 0, 0, 0);
-        if (lane < per_warp && g + lane < ne) {
+        if (lane < per_warp && g + lane < ne &&
+            ck((unsigned long long)(reinterpret_cast<const EdgeRec*>(edges) - P.pool) + g + lane < P.pool_cap, 27)) {
             const int4 a = edges[2 * (g + lane)], c = edges[2 * (g + lane) + 1];
             const EdgeRec E{a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
             const int fu = fxfract(E.y_upper);
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(NT, 1) k_band_single(KParams P) {
                 s = seg_items(wsub(E.x_bot0, fxmul(E.inv_slope, FX_ONE - fu)), fu, fxfract(E.y_lower), E.start_row,
                               E.end_row, E.inv_slope, E.step_pix > 0 ? E.step_pix : FX_ONE, E.ed < 0, yb0, yb1, pitch);
         }
-        run_items(rec, s, area, pitch, W);
+        run_items(rec, s, area, R * pitch, pitch, W);
     }
     __syncthreads();
     const int parts = NW / R;  // warps per row (R <= 8 <= NW)
@@ -98,10 +99,10 @@ __global__ void __launch_bounds__(NT, 1) k_band_single(KParams P) {
                    (unsigned)v.z + (unsigned)v.w;
         }
         sum = __reduce_add_sync(ALL, sum);
-        if (lane == 0) part[warp] = (int)sum;
+        if (lane == 0 && ck(q * pitch + x1 <= R * pitch, 26)) part[warp] = (int)sum;
     }
     __syncthreads();
-    if (q >= nr) return;
+    if (q >= nr || !ck(q * pitch + min((x1 + 7) & ~7, pitch) <= R * pitch && r0 + q < H, 26)) return;
     const int al = ((reinterpret_cast<uintptr_t>(P.rasters) | P.canvas_stride) & 7) == 0
                        ? 8
                        : ((reinterpret_cast<uintptr_t>(P.rasters) | P.canvas_stride) & 3) == 0 ? 4 : 1;
@@ -159,6 +160,8 @@ cudaError_t launch_srcover_rows(uint8_t* canvas, uint32_t stride, const uint8_t*
     k_srcover_rows<<<(H - r0) * nseg, 256, 0, s>>>(canvas, stride, mask, mstride, W, r0, nseg, clr);
     return cudaGetLastError();
 }
+
+cudaError_t take_check_bands(CheckState* s, bool reached) { return take_check(s, reached); }
 
 cudaError_t setup_bands() {
     cudaError_t e = allow_smem((const void*)k_band_single<256>);

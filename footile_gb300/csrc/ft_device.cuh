@@ -105,6 +105,37 @@ __device__ __forceinline__ bool pline_x(P2 a0, P2 a1, P2 b0, P2 b1, P2* out) {
     return true;
 }
 
+// Bounds checks of the check build (nvcc -DFT_CHECK=1, see _build.build_variant): a failed
+// check keeps the first failing site's number and skips the access; no trap.  Every source
+// file has a state of its own (take_check), which also knows the sites that were reached.
+// In the shipped build every check folds to true.
+#ifndef FT_CHECK
+#define FT_CHECK 0
+#endif
+struct CheckState {
+    int failed = 0;
+    unsigned long long reached = 0;  // a bit per site
+};
+static __device__ int g_check = 0;
+static __device__ unsigned long long g_reached = 0;
+__device__ __forceinline__ bool ck(bool ok, int site) {
+    if (FT_CHECK) {
+        if (!((*(volatile unsigned long long*)&g_reached >> site) & 1)) atomicOr(&g_reached, 1ull << site);
+        if (!ok) atomicCAS(&g_check, 0, site);
+    }
+    return !FT_CHECK || ok;
+}
+// This file's failed site, or (`reached`) the sites reached, since the last call.
+[[maybe_unused]] static cudaError_t take_check(CheckState* s, bool reached) {
+    const CheckState zero;
+    if (reached) {
+        const cudaError_t e = cudaMemcpyFromSymbol(&s->reached, g_reached, sizeof(s->reached));
+        return e != cudaSuccess ? e : cudaMemcpyToSymbol(g_reached, &zero.reached, sizeof(zero.reached));
+    }
+    const cudaError_t e = cudaMemcpyFromSymbol(&s->failed, g_check, sizeof(s->failed));
+    return e != cudaSuccess ? e : cudaMemcpyToSymbol(g_check, &zero.failed, sizeof(zero.failed));
+}
+
 // min (y, x, id)
 __device__ __forceinline__ bool top_less(int ay, int ax, int ai, int by, int bx, int bi) {
     return ay < by || (ay == by && (ax < bx || (ax == bx && ai < bi)));

@@ -76,8 +76,9 @@ __device__ __forceinline__ SegRec seg_items(int ux, int fu, int fl, int start, i
 // One lane works out a segment; the (segment, row) items are then spread over the lanes, an
 // item that walks many cells as several lanes of CELLS cells each, so that a window of 32
 // costs the same whatever the slopes in it: the walk is closed (x_cov after j cells is
-// first + j * step), so any lane can start in the middle of it.  rec: 64 records of the warp.
-__device__ __forceinline__ void run_items(int4* rec, SegRec s, int* area, int pitch, int W) {
+// first + j * step), so any lane can start in the middle of it.  rec: 64 records of the warp;
+// cells: those that `area` holds.
+__device__ __forceinline__ void run_items(int4* rec, SegRec s, int* area, int cells, int pitch, int W) {
     const int lane = threadIdx.x & 31;
     int inc = s.n_items;
 #pragma unroll
@@ -104,6 +105,7 @@ __device__ __forceinline__ void run_items(int4* rec, SegRec s, int* area, int pi
         const int item = w0 + lane;
         if (item >= tot) continue;
         const int j = before + __popc(at & (ALL >> (31 - lane))) - 1;
+        if (!ck(j >= 0 && j < 32, 19)) continue;
         const int4 A = rec[2 * j], C = rec[2 * j + 1];
         const int ls = C.y >> 20, step = C.y & 0xFFFFF;
         const int k = (item - C.x) >> ls, c0 = ((item - C.x) & ((1 << ls) - 1)) * CELLS;
@@ -137,7 +139,7 @@ __device__ __forceinline__ void run_items(int4* rec, SegRec s, int* area, int pi
 #pragma unroll
         for (int u = 0; u < CELLS; u++) {
             const int v = min((int)(xc >> 8), cov);
-            if (v != prev) atomicAdd(cell + u, (v - prev) * sgn);
+            if (v != prev && ck((unsigned)(cell + u - area) < (unsigned)cells, 18)) atomicAdd(cell + u, (v - prev) * sgn);
             prev = v;
             xc += (unsigned)step;
         }

@@ -36,6 +36,7 @@
 
 #include <cuda.h>
 
+#include "ft_adjoint.cuh"
 #include "ft_device.cuh"
 #include "ft_items.cuh"
 #include "ft_kernels.cuh"
@@ -45,17 +46,6 @@ namespace ftk {
 
 constexpr unsigned FULL = 0xFFFFFFFFu;
 
-// Bounds checks of the check build (nvcc -DFT_CHECK=1, see _build.build_variant): a failed
-// check keeps the first failing site's number in g_check and skips the access; no trap.
-// In the shipped build every check folds to true.
-#ifndef FT_CHECK
-#define FT_CHECK 0
-#endif
-static __device__ int g_check = 0;
-__device__ __forceinline__ bool ck(bool ok, int site) {
-    if (FT_CHECK && !ok) atomicCAS(&g_check, 0, site);
-    return !FT_CHECK || ok;
-}
 // Curve leaves of an op kept (in local memory) from the count pass for the emit pass;
 // ops with more leaves are walked again.
 constexpr int LEAF_CACHE_CTA = 256;
@@ -994,7 +984,7 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
                 sum += v;
             }
             const int listed = (int)(sum >> 22), total = (int)(sum & ((1u << 22) - 1));
-            if (slots) {
+            if (slots && ck((pre + inc - own) >> 22 < (unsigned)N, 20)) {
                 const unsigned ex = pre + inc - own;
                 const int at = (int)(ex >> 22);
                 const bool curve = (kind == FT_OP_QUAD || kind == FT_OP_CUBIC) && !nonfinite;
@@ -1057,7 +1047,7 @@ __device__ void build_fill(const KParams& P, const ft_path_desc& d, float sw0, B
                 }
                 int m;
                 const int pos = block_excl_sum(at >= 0 ? 1 : 0, B.scan, m);
-                if (at >= 0) {
+                if (at >= 0 && ck(pos < N, 28)) {
                     Q.rs[pos] = (unsigned char)(idx == 0 ? (info >> 10) & 1 : 0);
                     if (STROKE) {
                         Q.raw[pos] = make_float4(z.x, z.y, zw, 0.f);
@@ -4200,10 +4190,25 @@ extern "C" FT_API int ft_fill_noalloc(int32_t rule, const ft_op* ops, uint32_t n
 extern "C" FT_API int ft_check_failures(int32_t* site, int32_t* compiled_in) {
     if (compiled_in) *compiled_in = FT_CHECK;
     if (!site) return FT_OK;
-    int v = 0;
-    if (cudaMemcpyFromSymbol(&v, ftk::g_check, sizeof(int)) != cudaSuccess) return FT_ERR_CUDA;
-    *site = v;
-    const int zero = 0;
-    if (cudaMemcpyToSymbol(ftk::g_check, &zero, sizeof(int)) != cudaSuccess) return FT_ERR_CUDA;
+    ftk::CheckState s;
+    for (auto take : {ftk::take_check, ftk::take_check_tile, ftk::take_check_bands, fta::take_check_adjoint}) {
+        ftk::CheckState t;
+        if (take(&t, false) != cudaSuccess) return FT_ERR_CUDA;
+        if (!s.failed) s.failed = t.failed;
+    }
+    *site = s.failed;
     return FT_OK;
 }
+
+#if FT_CHECK
+// The check build alone: the sites whose checks ran since the last call, a bit each.
+extern "C" FT_API int ft_check_reached(unsigned long long* sites) {
+    *sites = 0;
+    for (auto take : {ftk::take_check, ftk::take_check_tile, ftk::take_check_bands, fta::take_check_adjoint}) {
+        ftk::CheckState t;
+        if (take(&t, true) != cudaSuccess) return FT_ERR_CUDA;
+        *sites |= t.reached;
+    }
+    return FT_OK;
+}
+#endif

@@ -384,5 +384,9 @@ cudaError_t allow_smem(const void* kern);
 cudaError_t setup_kernels();
 cudaError_t setup_tile();
 cudaError_t setup_bands();
+// The check build's state of the other source files (ft_device.cuh, take_check).
+struct CheckState;
+cudaError_t take_check_tile(CheckState* s, bool reached);
+cudaError_t take_check_bands(CheckState* s, bool reached);
 
 }  // namespace ftk

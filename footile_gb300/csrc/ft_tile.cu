@@ -238,7 +238,7 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
         const int listed = (int)(sum >> 22), total = (int)(sum & ((1u << 22) - 1));
         const unsigned excl = pre + inc - mine;
         const int off = (int)(excl & ((1u << 22) - 1));
-        if (slots) {
+        if (slots && ck(excl >> 22 < (unsigned)NT, 20)) {
             const int at = (int)(excl >> 22);
             B.g0[at] = ga;
             B.g1[at] = gb;
@@ -253,7 +253,7 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
             const P2 l = xform(P.xf, lvo >= 0 ? p2(B.endp[lvo].x, B.endp[lvo].y) : op_end(tile_op(ops, S.c_vo)));
             const P2 f = first_vertex(P, ops, lrs_op);
             const int4 e = make_int4(to_fx(l.x), to_fx(l.y), to_fx(f.x), to_fx(f.y));
-            E[base + off] = e;
+            if (ck(base + off < P.cap, 21)) E[base + off] = e;
             consider(e, base + off);
         }
         __syncthreads();
@@ -297,7 +297,7 @@ __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& 
             }
             const unsigned cm = __ballot_sync(ALL, close_slot);
             if (lane == 0) ends[(base + s) >> 5] = cm;
-            if (!close_slot) E[base + s] = e;
+            if (!close_slot && ck(base + s < P.cap, 22)) E[base + s] = e;
             consider(e, base + s);
         }
         base += padded;
@@ -367,7 +367,7 @@ __device__ __noinline__ int tile_dir(const int4* E, const unsigned* ends, int n_
 
 // ------------------------------------------------------------------- raster
 // Items of the first m segments in Q.q (all reach rows [yb0, yb1)) into `area`.
-__device__ __forceinline__ void tile_items(TileWarp& Q, int m, int yb0, int yb1, int* area, int pitch, int W) {
+__device__ __forceinline__ void tile_items(TileWarp& Q, int m, int yb0, int yb1, int* area, int cells, int pitch, int W) {
     const int lane = threadIdx.x & 31;
     SegRec s;
     s.n_items = 0;
@@ -388,7 +388,7 @@ __device__ __forceinline__ void tile_items(TileWarp& Q, int m, int yb0, int yb1,
         if (step <= 0) step = FX_ONE;  // step_cov(ONE) (fig.rs:315-321)
         s = seg_items(ux, fxfract(uy), fxfract(ly), uy >> 16, ly >> 16, fx_div(dx, dy), step, !down, yb0, yb1, pitch);
     }
-    run_items(Q.rec, s, area, pitch, W);
+    run_items(Q.rec, s, area, cells, pitch, W);
 }
 
 struct TileOut {  // where a band's rows go (in shared memory: it would only hold registers)
@@ -397,6 +397,7 @@ struct TileOut {  // where a band's rows go (in shared memory: it would only hol
     int W, pitch, rule, fmt;
     int neg;         // the figure runs in reverse: cell sums change sign
     int lprl;        // log2 of the lanes per row, eight pixels each
+    int cells;       // of the area; the staged bytes are as many and 256 more
     bool host;       // mapped host memory: Matte8 rows leave as aligned words
     unsigned char* stg;
 };
@@ -419,7 +420,7 @@ __device__ __noinline__ void tile_rows_matte(const TileOut& T, int* area, int r0
     int* ap = area + first * T.pitch + 8 * l;
     uint8_t* dp = T.base + (size_t)(r0 + first) * T.stride + 8 * l;
     for (int q = warp * rpw; q < nr; q += NW * rpw) {
-        const bool in = nb > 0 && q + (lane >> T.lprl) < nr;
+        const bool in = nb > 0 && q + (lane >> T.lprl) < nr && ck(ap + 8 - area <= T.cells, 25);
         unsigned s[8], inc;
         take8(ap, in, l, s, inc);
         const uint2 px = pixels8<RULE>(s, inc - s[7], sg);
@@ -450,7 +451,7 @@ __device__ __noinline__ void tile_rows(const TileOut& T, int* area, int r0, int 
         unsigned carry = 0;
         for (int x0 = 0; x0 < W; x0 += lpr * 8) {
             const int x = x0 + l * 8, nb = min(W - x, 8);
-            const bool in = valid && nb > 0;
+            const bool in = valid && nb > 0 && ck(arow + x + 8 - area <= T.cells, 25);
             unsigned s[8], inc;
             take8(arow + x, in, l, s, inc);
             const uint2 px = pixels8<RULE>(s, inc - s[7] + carry, T.neg ? -1 : 1);
@@ -458,11 +459,11 @@ __device__ __noinline__ void tile_rows(const TileOut& T, int* area, int r0, int 
             if (!in) continue;
             if (contig) {
                 unsigned char* sp = T.stg + o0 + rr * W + x;
-                for (int k = 0; k < nb; k++) sp[k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
+                if (ck(o0 + rr * W + x + nb <= T.cells + 256, 24)) for (int k = 0; k < nb; k++) sp[k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
             } else if (T.fmt == FT_MATTE8 && !T.host) {
                 for (int k = 0; k < nb; k++) drow[x + k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
             } else {
-                *reinterpret_cast<uint2*>(T.stg + rr * T.pitch + x) = px;
+                if (ck(rr * T.pitch + x + 8 <= T.cells + 256, 24)) *reinterpret_cast<uint2*>(T.stg + rr * T.pitch + x) = px;
             }
         }
         if (contig || (T.fmt == FT_MATTE8 && !T.host)) continue;
@@ -561,6 +562,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
                         ((unsigned)d.clr[3] << 24);
                 T.W = W;
                 T.pitch = pitch;
+                T.cells = P.area_ints;
                 T.rule = P.rule;
                 T.fmt = P.fmt;
                 T.host = host;
@@ -592,12 +594,13 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
                             const int y0 = min(e.y, e.w), y1 = max(e.y, e.w);
                             const bool on = y0 != y1 && (y0 >> 16) < yb1 && ((y1 - 1) >> 16) >= yb0;
                             const unsigned m = __ballot_sync(ALL, on);
-                            if (on) Q.q[cnt + __popc(m & ((1u << lane) - 1u))] = e;
+                            const int at = cnt + __popc(m & ((1u << lane) - 1u));
+                            if (on && ck(at < 64, 23)) Q.q[at] = e;
                             cnt += __popc(m);
                             __syncwarp();
                         }
                         if (cnt >= 32 || (!more && cnt > 0)) {
-                            tile_items(Q, min(cnt, 32), yb0, yb1, area, pitch, W);
+                            tile_items(Q, min(cnt, 32), yb0, yb1, area, P.area_ints, pitch, W);
                             cnt -= 32;
                             if (lane < cnt) Q.q[lane] = Q.q[32 + lane];
                             __syncwarp();
@@ -618,7 +621,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
                     if (contig) {
                         const bool last = r0 + nr >= hi;
                         const int fill = o0 + nr * W, lines = last ? (fill + 127) >> 7 : fill >> 7;
-                        for (int x = tid * 16; x < lines * 128; x += NT * 16) {
+                        for (int x = tid * 16; x < lines * 128 && ck(x + 16 <= P.area_ints + 256, 24); x += NT * 16) {
                             uint8_t* a = L0 + x;
                             const uint4 v = *reinterpret_cast<const uint4*>(T.stg + x);
                             if (a >= g0 && a + 16 <= g1) {
@@ -657,6 +660,8 @@ int tile_blocks_per_sm(int threads, int smem) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, threads == 128 ? k_tile<128> : k_tile<512>, threads, smem);
     return e == cudaSuccess && n > 0 ? n : 1;
 }
+
+cudaError_t take_check_tile(CheckState* s, bool reached) { return take_check(s, reached); }
 
 cudaError_t setup_tile() {
     const cudaError_t e = allow_smem((const void*)k_tile<128>);

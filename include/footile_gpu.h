@@ -406,9 +406,9 @@ FT_API int ft_last_composite_ms(ft_ctx* ctx, float* ms);
 
 /* Bounds-check build (the library compiled with -DFT_CHECK=1) — no counterpart in
  * footile; it stands in for a memory checker.  Device code checks the indices of its
- * shared-memory cell buffers, edge pool, compositor queues and the grid-wide
- * figure build's raw vertices and figure writes; a failed check
- * skips the access and keeps the first failing site's number.  `site` (may be NULL)
+ * shared-memory cell buffers and item records, the lists and scratch of segments, the staged
+ * rows, the edge pool, the compositor's queues and the grid-wide figure build's raw vertices and
+ * figure writes; a failed check skips the access and keeps the first failing site's number.  `site` (may be NULL)
  * receives that number since the last call (0: none) and is reset; `compiled_in` (may be
  * NULL) is 1 in the check build and 0 in the shipped build, whose checks fold away. */
 FT_API int ft_check_failures(int32_t* site, int32_t* compiled_in);
