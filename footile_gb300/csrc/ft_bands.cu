@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(NT, 1) k_band_single(KParams P) {
             // x_bot0 is the x it starts at, moved to the bottom of its first row (fig.rs:187-199)
             if (E.ed)
                 s = seg_items(wsub(E.x_bot0, fxmul(E.inv_slope, FX_ONE - fu)), fu, fxfract(E.y_lower), E.start_row,
-                              E.end_row, E.inv_slope, E.step_pix > 0 ? E.step_pix : FX_ONE, E.ed < 0, yb0, yb1, pitch);
+                              E.end_row, E.inv_slope, E.step_pix > 0 ? E.step_pix : FX_ONE, E.ed < 0, yb0, yb1, pitch, W);
         }
         run_items(rec, s, area, R * pitch, pitch, W);
     }

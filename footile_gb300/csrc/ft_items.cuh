@@ -44,11 +44,10 @@ struct SegRec {
     int n_items;
     int4 ra, rb;
 };
-constexpr int CELLS = 4;  // cells a lane walks
 // Items of a segment that reaches rows [yb0, yb1): its rows there, each as 2^ls lanes of CELLS
-// cells.  (ux, fu): where it starts and the y fraction there, fl: the fraction where it ends.
+// cells (item_shift; the raster is W pixels wide).  (ux, fu): where it starts and the y fraction there, fl: the fraction where it ends.
 __device__ __forceinline__ SegRec seg_items(int ux, int fu, int fl, int start, int end, int inv, int step, bool neg,
-                                            int yb0, int yb1, int pitch) {
+                                            int yb0, int yb1, int pitch, int W) {
     SegRec s;
     const int pu = (fu + 128) >> 8, pl = (fl + 128) >> 8;  // pixel_cov of the fractions
     const int ya = max(start, yb0), yl = min(fl ? end : end - 1, yb1 - 1);
@@ -56,7 +55,7 @@ __device__ __forceinline__ SegRec seg_items(int ux, int fu, int fl, int start, i
     // the longest walk of its rows: cov * 256 / step cells and one, rounded up
     const int most = start == end ? pl - pu : (end - start > 1 ? 256 : max(256 - pu, pl));
     const int cells = (int)__fdividef((float)max(most, 0) * 256.0256f, (float)step) + 2;
-    const int ls = cells <= CELLS ? 0 : 32 - __clz((cells - 1) / CELLS);
+    const int ls = item_shift(cells, W);
     s.n_items = nrow > 0 ? nrow << ls : 0;
     s.ra.x = wadd(wadd(ux, fxmul(inv, FX_ONE - fu)), wmul(ya - start, inv));
     s.ra.y = inv;

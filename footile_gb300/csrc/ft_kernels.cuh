@@ -276,6 +276,21 @@ struct TileParams {
     float xf[6];
     float tol, tol_sq;
 };
+// A row of a segment goes to 2^item_shift lanes of CELLS cells each.  `cells`: the row's longest
+// walk; of a raster W pixels wide it needs no more than W (cells right of the raster are dropped,
+// those left of it are one): 3,000 canvases of 64 x 64 under flat segments of 32,000 pixels 3,440 us
+// by the walk alone, 255 us this way, 270 us with one lane a row.
+constexpr int CELLS = 4;
+inline __host__ __device__ int item_shift(int cells, int W) {
+    const int more = ((cells < W ? cells : W) - 1) / CELLS;
+#ifdef __CUDA_ARCH__
+    return 32 - __clz(more);
+#else
+    int s = 0;
+    while (more >> s) s++;
+    return s;
+#endif
+}
 int tile_smem(int threads, int area_ints, bool staged);
 // What one launch of the tile rasteriser runs with.
 struct TilePlan {

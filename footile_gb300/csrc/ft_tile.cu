@@ -386,7 +386,7 @@ __device__ __forceinline__ void tile_items(TileWarp& Q, int m, int yb0, int yb1,
             step = min(fxabs(fx_div(dy, dx)), FX_ONE);
         }
         if (step <= 0) step = FX_ONE;  // step_cov(ONE) (fig.rs:315-321)
-        s = seg_items(ux, fxfract(uy), fxfract(ly), uy >> 16, ly >> 16, fx_div(dx, dy), step, !down, yb0, yb1, pitch);
+        s = seg_items(ux, fxfract(uy), fxfract(ly), uy >> 16, ly >> 16, fx_div(dx, dy), step, !down, yb0, yb1, pitch, W);
     }
     run_items(Q.rec, s, area, cells, pitch, W);
 }
