@@ -249,6 +249,14 @@ constexpr int TILE_THREADS = 128, TILE_THREADS_FEW = 512;
 constexpr int TILE_MAX_SIDE = 512;                      // canvases up to this width and height (batches)
 constexpr int TILE_CAP = 32768, TILE_CAP_FEW = 65504;   // segment slots per CTA (at most the vertex cap)
 static_assert(TILE_CAP % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");
+// Whether a path is handed to k_raster after the ops [0, done) of its n that have `slots` slots: it
+// has too many, or will have at this rate.  A path built to the end of its scratch and then built
+// again by k_raster cost more than k_raster alone (one of 30,000 curves on 500 x 2000: 2,780 us, handed
+// over after its first ops 2,550); one handed over that would have fitted is drawn as well, by the
+// slower kernel.
+inline __host__ __device__ bool tile_overflows(int slots, int done, int n, int cap) {
+    return slots > cap || (done < n && (long long)slots * n > (long long)cap * done);
+}
 // Cells from one row of a band to the next: three spare cells (a walk of four cells may run
 // past the raster's last), a multiple of eight.
 __host__ __device__ constexpr int tile_pitch(int w) { return (w + 3 + 7) & ~7; }

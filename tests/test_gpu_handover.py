@@ -1,0 +1,34 @@
+"""Paths that the tile rasteriser hands over early: uneven ones (dense ops first, or last) are drawn
+bit-exactly whichever kernel takes them."""
+import numpy as np
+import pytest
+
+import oracle
+from footile_gb300 import _abi, workloads
+from footile_gb300.plotter import fill_batch, pack_batch
+from helpers import assert_same, gpu_vs_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def uneven(seed, side, big, small, dense_first):
+    """`big` long curves and `small` short lines, one after the other."""
+    rng = np.random.default_rng(seed)
+    curves = workloads.random_path(rng, side, big, n_sub=1)
+    lines = workloads.random_path(rng, side, small, n_sub=1)
+    lines["kind"] = np.where((lines["kind"] == _abi.OP_QUAD) | (lines["kind"] == _abi.OP_CUBIC), _abi.OP_LINE, lines["kind"])
+    return np.concatenate([curves, lines] if dense_first else [lines, curves])
+
+
+@pytest.mark.parametrize("dense_first", [True, False])
+@pytest.mark.parametrize("big,small", [(600, 3000), (130, 4000), (2000, 600)])
+def test_uneven_paths(ctx, big, small, dense_first):
+    parts = [uneven(k, 200, big, small, dense_first) for k in range(3)]
+    for n in (3, 330):  # row ranges, and paths whole
+        ops, paths, size = pack_batch([parts[k % 3] for k in range(n)], [200] * n)
+        want, got = np.zeros(size, np.uint8), np.zeros(size, np.uint8)
+        oracle.fill_batch(0, _abi.NONZERO, ops, paths, 0, want, n_threads=8)
+        fill_batch(ctx, ops, paths, 0, got)
+        assert_same(got, want, f"{n} paths")
+    got, want, *_ = gpu_vs_oracle(ctx, parts[0], 200, 170, rule=_abi.EVENODD, fmt=_abi.RGBA8P, clr=(9, 8, 7, 99), init=37)
+    assert_same(got, want, "single call")
