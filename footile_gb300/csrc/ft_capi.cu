@@ -300,6 +300,16 @@ int grid_for(ft_ctx* c, int smem, uint32_t n_items, bool stroke) {
     return std::max(1, std::min(grid, (int)std::max(n_items, 1u)));
 }
 
+// Grid of the CTA rasteriser beside `n_items_w` items of the tile rasteriser.  Of few paths any may
+// be handed over, all at once when they are large: CTAs as for items of its own (300 paths of 3,000
+// curves on 512 x 512, all handed over: one CTA per SM 26.2 ms, this way 14.0 ms).  A batch hands
+// over a path here and there.
+int grid_behind_tile(ft_ctx* c, int smem, const ftk::TilePlan& t, uint32_t n_items, uint32_t n_items_w, bool stroke) {
+    if (!n_items_w) return grid_for(c, smem, n_items, stroke);
+    if (t.threads == ftk::TILE_THREADS_FEW) return grid_for(c, smem, n_items + n_items_w, stroke);
+    return std::max(grid_for(c, smem, n_items, stroke), c->sm_count);
+}
+
 // Grid of the tile rasteriser.
 int grid_for_tile(ft_ctx* c, const ftk::TilePlan& t, uint32_t n_items_w, int tile_smem) {
     const int grid = grid_cap(c, ftk::tile_blocks_per_sm(t.threads, tile_smem));
@@ -378,8 +388,7 @@ int run_plan(ft_ctx* c, PlanSlot& slot, int stroke, int rule, const ft_op* ops_d
     }
     FT_CU(c->overflow.ensure(sizeof(uint32_t) * std::max(n_items_w, 1u)), "alloc overflow list");
     FT_CU(c->queue.ensure(256), "alloc queue");
-    const int grid = n_items_w ? std::max(grid_for(c, smem, n_items, stroke), c->sm_count)
-                               : grid_for(c, smem, n_items, stroke);
+    const int grid = grid_behind_tile(c, smem, slot.tile, n_items, n_items_w, stroke != 0);
     const int grid_w = grid_for_tile(c, slot.tile, n_items_w, slot.tile.smem(fmt, host_rasters));
     FT_CU(c->scratch.ensure(raster_scratch(slot.tile, grid, grid_w, n_items_w)), "alloc scratch");
     FT_CU(cudaMemcpyAsync(c->paths.p, paths, sizeof(ft_path_desc) * n_paths, cudaMemcpyHostToDevice, c->stream),
@@ -612,8 +621,7 @@ FT_API int ft_batch_create(ft_ctx* c, int32_t stroke, int32_t rule, const ft_pat
     plan_items(c, paths, n_paths, b->smem, items, items_w, b->tile, stroke != 0);
     b->n_items = (uint32_t)items.size();
     b->n_items_w = (uint32_t)items_w.size();
-    b->grid = b->n_items_w ? std::max(grid_for(c, b->smem, b->n_items, stroke), c->sm_count)
-                           : grid_for(c, b->smem, b->n_items, stroke);
+    b->grid = grid_behind_tile(c, b->smem, b->tile, b->n_items, b->n_items_w, stroke != 0);
     b->grid_w = grid_for_tile(c, b->tile, b->n_items_w, b->tile.smem(fmt, false));
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = b->paths.ensure(sizeof(ft_path_desc) * std::max(n_paths, 1u));

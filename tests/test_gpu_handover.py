@@ -32,3 +32,28 @@ def test_uneven_paths(ctx, big, small, dense_first):
         assert_same(got, want, f"{n} paths")
     got, want, *_ = gpu_vs_oracle(ctx, parts[0], 200, 170, rule=_abi.EVENODD, fmt=_abi.RGBA8P, clr=(9, 8, 7, 99), init=37)
     assert_same(got, want, "single call")
+
+
+def test_handed_over_paths_take_their_kernels_time(ctx):
+    """Few large paths, all handed over, against the same batch sent to the CTA rasteriser outright:
+    the hand-over may not double the time (1.84 times it with one CTA per SM behind the tile
+    rasteriser, 0.97 now)."""
+    import torch
+    from footile_gb300.plotter import PreparedBatch
+
+    rng = np.random.default_rng(2)
+    ops, paths, size = pack_batch([workloads.random_path(rng, 512, 3000)] * 300, [512] * 300)
+    dev = torch.from_numpy(ops.view(np.uint8)).cuda()
+    ras = torch.zeros(size, dtype=torch.uint8, device="cuda")
+
+    def ms(side):
+        ctx.tune(warp_max_side=side)
+        batch, took = PreparedBatch(ctx, paths), []
+        for _ in range(7):
+            batch.launch(dev, ras)
+            took.append(ctx.last_ms())
+        batch.close()
+        return sorted(took)[3]
+
+    by_cta, handed_over = ms(0), ms(512)
+    assert handed_over < 1.4 * by_cta, (handed_over, by_cta)
