@@ -450,13 +450,12 @@ int run(ft_ctx* c, int stroke, int rule, const ft_op* ops_d, const ft_path_desc*
 // uploaded or reset, and k_raster is set up while k_tile runs.  Every CTA rebuilds the figure,
 // which bounds how low the ranges go.  256 x 256 fill / 97 x 61 stroke, us: planned, uploaded
 // and drawn from the queue in ranges of 16 rows 29.6 / 33.4; this way in ranges of 16 rows
-// 21.4 / 27.8, 8 rows 20.5 / 26.6, 4 rows 20.8 / 29.1.
+// 21.4 / 27.8, 8 rows 20.5 / 26.6, 4 rows 20.8 / 29.1 (single_rows).
 int run_single(ft_ctx* c, int stroke, int rule, const ft_op* ops_d, const ft_path_desc& d, int fmt, uint8_t* ras_d,
                const float* sw_in, float* sw_next) {
     const int smem = choose_smem(c, std::max(d.width, 1u));
     const bool tiled = !stroke && tile_max_side(c) > 0;
-    const int parts = std::max(1, grid_cap(c, 2)), h = (int)std::max(d.height, 1u);
-    const int rows = std::max(8, (h + parts - 1) / parts), n = (h + rows - 1) / rows;
+    const int h = (int)std::max(d.height, 1u), rows = ftk::single_rows(h, grid_cap(c, 1)), n = (h + rows - 1) / rows;
     ftk::TilePlan t{ftk::TILE_THREADS_FEW, ftk::TILE_CAP_FEW, few_area((int)d.width, std::min(rows, h))};
     FT_CU(c->status.ensure(sizeof(int32_t)), "alloc status");
     FT_CU(c->overflow.ensure(sizeof(uint32_t) * n), "alloc overflow list");

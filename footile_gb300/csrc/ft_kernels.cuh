@@ -249,6 +249,13 @@ constexpr int TILE_THREADS = 128, TILE_THREADS_FEW = 512;
 constexpr int TILE_MAX_SIDE = 512;                      // canvases up to this width and height (batches)
 constexpr int TILE_CAP = 32768, TILE_CAP_FEW = 65504;   // segment slots per CTA (at most the vertex cap)
 static_assert(TILE_CAP % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");
+// Rows of a single call's ranges, a CTA each: 8, and no more ranges than SMs.  Two builds on one SM
+// take longer than one with twice the rows to draw: 30,000 curves on 500 x 2000 in 250 / 143 ranges
+// on 152 SMs 2,533 / 1,814 us, 500 curves on 64 x 16000 in 302 / 151 2,034 / 1,413 us.
+inline __host__ __device__ int single_rows(int h, int sms) {
+    const int even = (h + (sms > 1 ? sms : 1) - 1) / (sms > 1 ? sms : 1);
+    return even > 8 ? even : 8;
+}
 // Whether a path is handed to k_raster after the ops [0, done) of its n that have `slots` slots: it
 // has too many, or will have at this rate.  A path built to the end of its scratch and then built
 // again by k_raster cost more than k_raster alone (one of 30,000 curves on 500 x 2000: 2,780 us, handed
