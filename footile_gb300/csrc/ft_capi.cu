@@ -190,8 +190,11 @@ int grid_cap(const ft_ctx* c, int per_sm) {
     return c->sm_count * per_sm;
 }
 
-// Most cells of a tile band when there are few paths (96 KB: a row range is one band).
-constexpr int TILE_AREA_FEW = 24576;
+// Most cells of a tile band when there are few paths: 96 KB, a row range is one band, while every
+// range has an SM to itself; else what leaves room for a second CTA (k_tile<512>: 32 KB of queues
+// and 5 bytes a cell where rows are staged, of 113 KB).  300 paths of 900 x 900 Rgba8p with 24,576
+// cells, so in two rounds, and one pixel under way per lane 2,560 us, this way 1,100 (by k_raster 1,270).
+constexpr int TILE_AREA_FEW = 24576, TILE_AREA_PAIR = 16000;
 
 // Cells of a band for row ranges of `rows` rows: the whole range up to TILE_AREA_FEW, a row at
 // least.
@@ -214,6 +217,7 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
     const bool few = n_paths < (uint32_t)std::max(2 * c->sm_count, 1);
     const uint32_t wside = stroke ? 0u : (uint32_t)tile_max_side(c);  // strokes use the CTA kernel
     tile = ftk::TilePlan{few ? ftk::TILE_THREADS_FEW : ftk::TILE_THREADS, few ? ftk::TILE_CAP_FEW : ftk::TILE_CAP, 8};
+    int widest = 8;
     for (uint32_t i = 0; i < n_paths; i++) {
         const ft_path_desc& d = paths[i];
         const uint32_t wp = (d.width + 3) & ~3u;
@@ -234,11 +238,14 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
             rows_per_item = std::max(16u, (d.height + parts - 1) / parts);
         }
         const bool tiled = few && !big && wside > 0;
-        if (tiled)
+        if (tiled) {
+            widest = std::max(widest, ftk::tile_pitch((int)d.width));
             tile.few_area = std::max(tile.few_area, few_area((int)d.width, (int)std::min(rows_per_item, std::max(d.height, 1u))));
+        }
         for (uint32_t r = 0; r < std::max(d.height, 1u); r += rows_per_item)
             (tiled ? out_w : out).push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
     }
+    if (few && (int)out_w.size() > c->sm_count) tile.few_area = std::max(widest, std::min(tile.few_area, TILE_AREA_PAIR));
     // Longest first, to a quarter of a power of two, which is all the order the queue needs:
     // a counting sort over 256 classes.  A call on 3,000 / 16,384 paths with a comparison
     // sort here and with this one: 313 / 227 us, 3.6 / 2.7 ms.

@@ -399,14 +399,9 @@ struct TileOut {  // where a band's rows go (in shared memory: it would only hol
     int lprl;        // log2 of the lanes per row, eight pixels each
     int cells;       // of the area; the staged bytes are as many and 256 more
     bool host;       // mapped host memory: Matte8 rows leave as aligned words
+    bool words;      // rows on 4-byte boundaries
     unsigned char* stg;
 };
-
-// SrcOver of one pixel, skipped when it changes nothing
-__device__ __forceinline__ void tile_px(unsigned* p, unsigned clr, unsigned av) {
-    const unsigned v = *p;
-    if (av || low_channels(v)) *p = srcover_rgba(v, clr, av);
-}
 
 // Resolve rows r0 .. r0 + nr - 1 (imgbuf.rs:38-199) from `area`, clearing it, and write them
 // (fig.rs:621-665).  Matte8 in device memory, rows of at most 256 pixels on 4-byte
@@ -460,6 +455,12 @@ __device__ __noinline__ void tile_rows(const TileOut& T, int* area, int r0, int 
             if (contig) {
                 unsigned char* sp = T.stg + o0 + rr * W + x;
                 if (ck(o0 + rr * W + x + nb <= T.cells + 256, 24)) for (int k = 0; k < nb; k++) sp[k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
+            } else if (T.fmt == FT_MATTE8 && !T.host && T.words) {
+                if (nb >= 4) __stcs(reinterpret_cast<unsigned*>(drow + x), px.x);
+                if (nb >= 8)
+                    __stcs(reinterpret_cast<unsigned*>(drow + x + 4), px.y);
+                else if (nb & 3)
+                    store_tail(drow + x + (nb & 4), nb < 4 ? px.x : px.y, nb & 3);
             } else if (T.fmt == FT_MATTE8 && !T.host) {
                 for (int k = 0; k < nb; k++) drow[x + k] = (uint8_t)((k < 4 ? px.x : px.y) >> (8 * (k & 3)));
             } else {
@@ -472,7 +473,18 @@ __device__ __noinline__ void tile_rows(const TileOut& T, int* area, int r0, int 
             const unsigned char* sp = T.stg + rr * T.pitch;
             if (T.fmt == FT_RGBA8P) {
                 unsigned* dp = reinterpret_cast<unsigned*>(drow);
-                for (int x = l; x < W; x += lpr) tile_px(dp + x, T.clr, sp[x]);
+                for (int x = l; x < W; x += 4 * lpr) {  // four loads in flight per lane
+                    unsigned v[4], av[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int at = x + k * lpr;
+                        v[k] = at < W ? dp[at] : 0u;  // a pixel of 0 under no coverage stays
+                        av[k] = at < W ? sp[at] : 0u;
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (av[k] || low_channels(v[k])) dp[x + k * lpr] = srcover_rgba(v[k], T.clr, av[k]);
+                }
             } else {  // aligned words of a host row, its ends byte by byte
                 const int mis = (int)(reinterpret_cast<uintptr_t>(drow) & 3);
                 for (int x = 4 * l - mis; x < W; x += 4 * lpr) {
@@ -569,8 +581,9 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
                 T.stg = smem + TileLayout<NT>::warps + P.area_ints * 4;
                 T.lprl = W <= 8 ? 0 : min(32 - __clz((W - 1) >> 3), 5);
             }
-            const bool quick = P.fmt == FT_MATTE8 && !host && W <= 256 &&
-                               (((unsigned)reinterpret_cast<uintptr_t>(base) | d.stride) & 3) == 0;
+            const bool words = (((unsigned)reinterpret_cast<uintptr_t>(base) | d.stride) & 3) == 0;
+            const bool quick = P.fmt == FT_MATTE8 && !host && W <= 256 && words;
+            if (tid == 0) T.words = words;
             // contiguous host rows: whole 128-byte lines leave from the staging bytes
             const bool contig = host && P.fmt == FT_MATTE8 && d.stride == d.width;
             uint8_t* const g0 = base + (size_t)lo * d.stride;
