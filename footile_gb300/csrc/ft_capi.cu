@@ -217,6 +217,7 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
     const bool few = n_paths < (uint32_t)std::max(2 * c->sm_count, 1);
     const uint32_t wside = stroke ? 0u : (uint32_t)tile_max_side(c);  // strokes use the CTA kernel
     tile = ftk::TilePlan{few ? ftk::TILE_THREADS_FEW : ftk::TILE_THREADS, few ? ftk::TILE_CAP_FEW : ftk::TILE_CAP, 8};
+    bool tiny = !few;
     int widest = 8;
     for (uint32_t i = 0; i < n_paths; i++) {
         const ft_path_desc& d = paths[i];
@@ -227,6 +228,7 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
         uint32_t rows_per_item = std::max(d.height, 1u);
         if (!few && d.width <= wside && d.height <= wside) {
             out_w.push_back(ftk::WorkItem{i, 0, d.height, R});
+            tiny = tiny && std::max(d.width, d.height) <= ftk::TILE_TINY_SIDE && d.n_ops <= ftk::TILE_TINY_OPS;
             continue;
         }
         if (big && c->sm_count > 0) {
@@ -245,6 +247,7 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
         for (uint32_t r = 0; r < std::max(d.height, 1u); r += rows_per_item)
             (tiled ? out_w : out).push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
     }
+    if (tiny) tile = ftk::TilePlan{ftk::TILE_THREADS_TINY, ftk::TILE_CAP_TINY, 8};
     if (few && (int)out_w.size() > c->sm_count) tile.few_area = std::max(widest, std::min(tile.few_area, TILE_AREA_PAIR));
     // Longest first, to a quarter of a power of two, which is all the order the queue needs:
     // a counting sort over 256 classes.  A call on 3,000 / 16,384 paths with a comparison

@@ -244,11 +244,17 @@ struct KParams {
 };
 
 // The tile rasteriser (ft_tile.cu): fills of small canvases, one CTA of TILE_THREADS per
-// path, or of TILE_THREADS_FEW per row range of a path when there are few paths.
-constexpr int TILE_THREADS = 128, TILE_THREADS_FEW = 512;
+// path, of TILE_THREADS_TINY where all of a batch's are tiny, or of TILE_THREADS_FEW per row range
+// of a path when there are few paths.
+constexpr int TILE_THREADS = 128, TILE_THREADS_TINY = 32, TILE_THREADS_FEW = 512;
+// Tiny: canvases up to TILE_TINY_SIDE a side under TILE_TINY_OPS ops at most, where four warps wait
+// for one another more than they share.  Four warps / one a path: 65,536 canvases of 8 x 8 under 3
+// lines 389 / 144 us, of 24 x 24 under 60 curves 1,295 / 1,095; 3,000 of 24 x 24 under 60 curves
+// 85 / 87, of 48 x 48 under 24 curves 98 / 120 us.
+constexpr int TILE_TINY_SIDE = 24, TILE_TINY_OPS = 64;
 constexpr int TILE_MAX_SIDE = 512;                      // canvases up to this width and height (batches)
-constexpr int TILE_CAP = 32768, TILE_CAP_FEW = 65504;   // segment slots per CTA (at most the vertex cap)
-static_assert(TILE_CAP % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");
+constexpr int TILE_CAP = 32768, TILE_CAP_TINY = 8192, TILE_CAP_FEW = 65504;  // segment slots per CTA (at most the vertex cap)
+static_assert(TILE_CAP % 32 == 0 && TILE_CAP_TINY % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");
 // Rows of a single call's ranges, a CTA each: 8, and no more ranges than SMs.  Two builds on one SM
 // take longer than one with twice the rows to draw: 30,000 curves on 500 x 2000 in 250 / 143 ranges
 // on 152 SMs 2,533 / 1,814 us, 500 curves on 64 x 16000 in 302 / 151 2,034 / 1,413 us.
@@ -315,7 +321,9 @@ struct TilePlan {
     static bool staged(int fmt, bool host) { return host || fmt == FT_RGBA8P; }
     // Batches: the cells that leave room for eight CTAs per SM.  65,536 glyphs with 2,560 /
     // 3,328 / 4,096 / 4,992 cells (the last seven CTAs): 4.75 / 4.46 / 4.29 / 4.34 ms.
+    // Tiny: 32 CTAs per SM.
     int area(int fmt, bool host) const {
+        if (threads == TILE_THREADS_TINY) return staged(fmt, host) ? 768 : 1000;
         return threads == TILE_THREADS_FEW ? few_area : (staged(fmt, host) ? 3712 : 4736);
     }
     int smem(int fmt, bool host) const { return tile_smem(threads, area(fmt, host), staged(fmt, host)); }

@@ -513,7 +513,7 @@ struct TileLayout {
 };
 
 template <int NT>
-__global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
+__global__ void __launch_bounds__(NT, NT == 32 ? 32 : NT == 128 ? 8 : 2) k_tile(TileParams P) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileState<NT> S;
     __shared__ TileOut T;
@@ -663,26 +663,28 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 8 : 2) k_tile(TileParams P) {
 
 }  // namespace
 
+static_assert(TILE_THREADS_TINY == 32 && TILE_THREADS == 128 && TILE_THREADS_FEW == 512, "the kernels there are");
 int tile_smem(int threads, int area_ints, bool staged) {
+    if (threads == 32) return TileLayout<32>::bytes(area_ints, staged);
     return threads == 128 ? TileLayout<128>::bytes(area_ints, staged) : TileLayout<512>::bytes(area_ints, staged);
 }
 
 int tile_blocks_per_sm(int threads, int smem) {
     int n = 0;
-    const cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, threads == 128 ? k_tile<128> : k_tile<512>, threads, smem);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &n, threads == 32 ? k_tile<32> : threads == 128 ? k_tile<128> : k_tile<512>, threads, smem);
     return e == cudaSuccess && n > 0 ? n : 1;
 }
 
 cudaError_t take_check_tile(CheckState* s, bool reached) { return take_check(s, reached); }
 
 cudaError_t setup_tile() {
-    const cudaError_t e = allow_smem((const void*)k_tile<128>);
+    const cudaError_t e = allow_smem((const void*)k_tile<128>);  // (k_tile<32> stays within 48 KB)
     return e == cudaSuccess ? allow_smem((const void*)k_tile<512>) : e;
 }
 
 cudaError_t launch_tile(const TileParams& p, int threads, int grid, int smem, cudaStream_t s) {
-    auto kern = threads == 128 ? k_tile<128> : k_tile<512>;
+    auto kern = threads == 32 ? k_tile<32> : threads == 128 ? k_tile<128> : k_tile<512>;
     kern<<<grid, threads, smem, s>>>(p);
     return cudaGetLastError();
 }
