@@ -1539,10 +1539,9 @@ cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride,
                            uint32_t w, uint32_t h, const uint8_t* lut, int grid, cudaStream_t s);
 int convert_block();
 int convert_blocks_per_sm(int src_fmt);
-int srcover_block();
 cudaError_t launch_srcover(bool backward, const float* cov, uint32_t n_layers, uint64_t plane, const float4* clr,
                            const float4* init, float4* out, const float4* grad_out, float* grad_cov,
-                           float4* grad_init, uint32_t n_px, int grid, cudaStream_t s, bool partial = false);
+                           float4* grad_init, uint32_t n_px, int sm_count, cudaStream_t s, bool partial = false);
 }
 
 // lut[a * 256 + c]: the straight channel c / a (clamped to 1; 0 when a = 0) through
@@ -1917,14 +1916,12 @@ static int srcover_call(ft_ctx* c, bool backward, const float* cov, uint32_t n_l
                          reinterpret_cast<uintptr_t>(grad_init);
     if (v4 & 15) return fail(c, FT_ERR_ARG, "colour and canvas buffers need 16-byte alignment");
     FT_CU(cudaSetDevice(c->device), "set device");
-    const int sob = ftc::srcover_block();
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     FT_CU(ftc::launch_srcover(backward, cov, n_layers, plane, reinterpret_cast<const float4*>(clr),
                               reinterpret_cast<const float4*>(init), reinterpret_cast<float4*>(out),
                               reinterpret_cast<const float4*>(grad_out), grad_cov, reinterpret_cast<float4*>(grad_init),
-                              n_px, grid, c->stream),
+                              n_px, c->sm_count, c->stream),
           "launch SrcOver");
     FT_CU(cudaEventRecord(c->ev1, c->stream), "event");
     c->timed = true;
@@ -2059,8 +2056,6 @@ FT_API int ft_stroke_composite_forward(ft_ctx* c, const ft_op* ops, uint32_t n_o
         FT_CU(cudaMemcpyAsync(s->prefix.p, init, 16ull * n_px, in, c->stream), "copy initial canvas");
     else
         FT_CU(cudaMemsetAsync(s->prefix.p, 0, 16ull * n_px, c->stream), "clear initial canvas");
-    const int sob = ftc::srcover_block();
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     for (uint32_t ch = 0; ch < s->n_chunks; ch++) {
@@ -2072,7 +2067,7 @@ FT_API int ft_stroke_composite_forward(ft_ctx* c, const ft_op* ops, uint32_t n_o
               "copy status");
         FT_CU(ftc::launch_srcover(false, static_cast<const float*>(s->cov.p), k, plane / 4,
                                   static_cast<const float4*>(s->clr.p) + b, s->prefix_at(ch), s->prefix_at(ch + 1),
-                                  nullptr, nullptr, nullptr, (uint32_t)n_px, grid, c->stream),
+                                  nullptr, nullptr, nullptr, (uint32_t)n_px, c->sm_count, c->stream),
               "launch SrcOver");
         c->launches++;
     }
@@ -2121,8 +2116,6 @@ FT_API int ft_stroke_composite_backward(ft_ctx* c, ft_composite_adjoint* s, cons
           "copy canvas gradient");
     if (gops_bytes) FT_CU(cudaMemsetAsync(gops_d, 0, gops_bytes, c->stream), "reset op gradient");
     if (s->n_paths) FT_CU(cudaMemsetAsync(gw_d, 0, 4ull * s->n_paths, c->stream), "reset width gradient");
-    const int sob = ftc::srcover_block();
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(((uint64_t)n_px + sob - 1) / sob, (uint64_t)c->sm_count * 16));
     c->comp_timed = false;
     FT_CU(cudaEventRecord(c->ev0, c->stream), "event");
     for (uint32_t ch = s->n_chunks; ch-- > 0;) {
@@ -2133,7 +2126,7 @@ FT_API int ft_stroke_composite_backward(ft_ctx* c, ft_composite_adjoint* s, cons
         const uint32_t b = s->chunk_begin(ch), k = s->chunk_size(ch);
         FT_CU(ftc::launch_srcover(true, static_cast<const float*>(s->cov.p), k, plane / 4,
                                   static_cast<const float4*>(s->clr.p) + b, s->prefix_at(ch), nullptr, g_cur,
-                                  static_cast<float*>(s->gcov.p), g_next, (uint32_t)n_px, grid, c->stream, true),
+                                  static_cast<float*>(s->gcov.p), g_next, (uint32_t)n_px, c->sm_count, c->stream, true),
               "launch SrcOver adjoint");
         c->launches++;
         int st = adjoint_backward_dev(c, s->adj, static_cast<const float*>(s->gcov.p), gops_d, gw_d + b, false);

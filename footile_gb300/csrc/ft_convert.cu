@@ -132,18 +132,19 @@ cudaError_t launch_convert(int src_fmt, const uint8_t* src, uint32_t src_stride,
 // one pass forward for E (recomputed, nothing kept from the forward call), written
 // into the gradient planes, then one pass backward for P.  No division, so opaque
 // layers (factor 0) are exact.  One thread per pixel; planes are n_layers x n_px floats.
-// Bound by the planes' stream from memory: the recurrence goes SB layers at a time, the
-// loads of the next SB in flight meanwhile, in CTAs of 128 threads (400 layers of 480 x 360
-// are 5 CTAs of 256 on some SMs and 4 on the others).  400 layers, 276 MB, forward / backward:
-// loads and recurrence in turn 114 / 268 us, next loads in flight 69 / 274 us (4 layers at a
-// time 93 / 234 us), in CTAs of 128 64 / 277 us, nine of the backward's per SM instead of eight
-// (all 1,350 resident; ten, with fewer registers, 234 us) 64 / 194 us.
+// Bound by the planes' stream from memory, and below some 300,000 pixels by the latency of a pixel's
+// chain: the recurrence goes SB layers at a time, the loads of the next SB in flight meanwhile.  A
+// thread takes one pixel, a CTA SO_BLOCK of them; how many fit a round of resident CTAs chooses the
+// shape (launch_srcover).  400 layers of mostly empty coverage, forward / backward of some / of all:
+// 100,000 pixels 53 / 131 / 147 us, 180,000 67 / 196 / 300, 260,000 96 / 266 / 375, 1,000,000
+// 289 / 893 / 1,370; loads and recurrence in turn 111 / 131 / 153, 112 / 225 / 313, 120 / 273 / 385,
+// 447 / 944 / 1,415.
 constexpr int SB = 8;
 constexpr int SO_BLOCK = 128;
 
 // `step(k, v)` for k = 0 .. n - 1 in turn, v[u] = the SB coverages from layer(k) on (layer(k) +
 // dir * u), loaded a step ahead
-template <class Step>
+template <int SB, class Step>
 __device__ __forceinline__ void stream_layers(const float* cov, uint64_t plane, uint32_t n, uint32_t first, int dir,
                                               Step step) {
     const float* at = cov + (uint64_t)first * plane;
@@ -166,6 +167,8 @@ __device__ __forceinline__ void stream_layers(const float* cov, uint64_t plane, 
     }
 }
 
+// A step of SB layers: 8 take 40 registers, 12 CTAs per SM; 4 take 32 and 16.
+template <int SB>
 __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
                               const float4* __restrict__ clr, const float4* __restrict__ init,
                               float4* __restrict__ out, uint32_t n_px) {
@@ -178,7 +181,7 @@ __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, 
             const float f = 1.0f - k.w * v;
             c = make_float4(k.x * v + c.x * f, k.y * v + c.y * f, k.z * v + c.z * f, k.w * v + c.w * f);
         };
-        stream_layers(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
+        stream_layers<SB>(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
 #pragma unroll
             for (int u = 0; u < SB; u++) layer(k * SB + u, v[u]);
         });
@@ -189,8 +192,8 @@ __global__ void k_srcover_fwd(const float* __restrict__ cov, uint32_t n_layers, 
 
 // PARTIAL: dLoss/dcov only where 0 < cov < 1 (elsewhere the plane is neither read nor
 // written) — all a NonZero coverage adjoint needs, since dcov/dS is 0 at cov 0 and 1.
-template <bool PARTIAL>
-__global__ void __launch_bounds__(SO_BLOCK, 9) k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
+template <bool PARTIAL, int PER_SM>
+__global__ void __launch_bounds__(SO_BLOCK, PER_SM) k_srcover_bwd(const float* __restrict__ cov, uint32_t n_layers, uint64_t plane,
                               const float4* __restrict__ clr, const float4* __restrict__ init,
                               const float4* __restrict__ grad_out, float* __restrict__ grad_cov,
                               float4* __restrict__ grad_init, uint32_t n_px) {
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(SO_BLOCK, 9) k_srcover_bwd(const float* __rest
             const float4 k = clr[n];
             e = (g.x * k.x + g.y * k.y + g.z * k.z + g.w * k.w) * v + e * (1.0f - k.w * v);
         };
-        stream_layers(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
+        stream_layers<SB>(cov + p, plane, n_layers / SB, 0, 1, [&](uint32_t k, const float* v) {
 #pragma unroll
             for (int u = 0; u < SB; u++) up(k * SB + u, v[u]);
         });
@@ -219,7 +222,7 @@ __global__ void __launch_bounds__(SO_BLOCK, 9) k_srcover_bwd(const float* __rest
             if (keep(v)) grad_cov[(uint64_t)n * plane + p] = P * ((g.x * k.x + g.y * k.y + g.z * k.z + g.w * k.w) - k.w * en);
             P *= 1.0f - k.w * v;
         };
-        stream_layers(cov + p, plane, n_layers / SB, n_layers - 1, -1, [&](uint32_t k, const float* v) {
+        stream_layers<SB>(cov + p, plane, n_layers / SB, n_layers - 1, -1, [&](uint32_t k, const float* v) {
             const uint32_t m = n_layers - k * SB;
             float en[SB];
 #pragma unroll
@@ -235,17 +238,30 @@ __global__ void __launch_bounds__(SO_BLOCK, 9) k_srcover_bwd(const float* __rest
     }
 }
 
-int srcover_block() { return SO_BLOCK; }
-
 cudaError_t launch_srcover(bool backward, const float* cov, uint32_t n_layers, uint64_t plane, const float4* clr,
                            const float4* init, float4* out, const float4* grad_out, float* grad_cov,
-                           float4* grad_init, uint32_t n_px, int grid, cudaStream_t s, bool partial) {
-    if (backward && partial)
-        k_srcover_bwd<true><<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
-    else if (backward)
-        k_srcover_bwd<false><<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
-    else
-        k_srcover_fwd<<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, out, n_px);
+                           float4* grad_init, uint32_t n_px, int sm_count, cudaStream_t s, bool partial) {
+    // CTAs that a canvas needs, and that a round takes with `per_sm` on an SM
+    const unsigned ctas = (unsigned)(((uint64_t)n_px + SO_BLOCK - 1) / SO_BLOCK);
+    auto round = [&](unsigned per_sm) { return per_sm * (unsigned)sm_count; };
+    // under few layers a pixel costs less than a CTA's launch: some take several
+    const unsigned grid = n_layers < SB && ctas > round(32) ? round(32) : ctas;
+    if (backward) {
+        // 8 per SM with 64 registers; 9 with 56, spilled, where the ninth completes the one round.  172,800
+        // pixels, 9 / 8 on 152 SMs: coverage of some 191 / 196 us, of all 239 / 295; elsewhere 8 are
+        // faster (100,000 158 / 147, 220,000 352 / 330, 180,000 of some 213 / 196)
+        const bool nine = ctas > round(8) && ctas <= round(9);
+        auto kern = partial ? (nine ? k_srcover_bwd<true, 9> : k_srcover_bwd<true, 8>)
+                            : (nine ? k_srcover_bwd<false, 9> : k_srcover_bwd<false, 8>);
+        kern<<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, grad_out, grad_cov, grad_init, n_px);
+    } else {
+        // steps of 4 layers with 16 CTAs per SM where that is one round and 12 are not (260,000 pixels, 4 / 8
+        // layers a step 96 / 108 us; 220,000, one round either way, 83 / 81; 1,000,000, the rest among
+        // several rounds, 309 / 289), and under fewer layers than a step of 8
+        const bool four = n_layers < SB || (ctas > round(12) && ctas <= round(16));
+        auto kern = four ? k_srcover_fwd<4> : k_srcover_fwd<SB>;
+        kern<<<grid, SO_BLOCK, 0, s>>>(cov, n_layers, plane, clr, init, out, n_px);
+    }
     return cudaGetLastError();
 }
 
