@@ -1390,9 +1390,8 @@ __device__ void build_edges(const CState& S, const int2* pts, const int* ss, Edg
 // `area` (the band row of width W).  The edge on this row: x_bot where it leaves the
 // row, its inverse slope, whether the row is its first (st) or last (en), the 16.16
 // fractions of its upper and lower y, the cell step (1 .. ONE) and its direction ed.
-// With `spans`, the 128-pixel spans holding the touched cells are marked too.
 __device__ __forceinline__ void scan_row(int x_bot, int inv, bool st, bool en, int fu, int fl, int step, int ed,
-                                         int* area, int W, unsigned* spans) {
+                                         int* area, int W) {
     const int ccov = en ? pixel_cov(fl) : 256;
     const int cov = st ? ccov - pixel_cov(fu) : ccov;
     if (cov <= 0) return;
@@ -1410,8 +1409,6 @@ __device__ __forceinline__ void scan_row(int x_bot, int inv, bool st, bool en, i
     // gets the growth of min(pixel_cov(x_cov), cov) until it reaches cov
     const int jmax = W - 1 - minp;  // the loop also stops at the raster's last cell
     int j, prev, x_cov;
-    const int cell0 = max(minp, 0);
-    int cell1 = cell0;
     if (minp < 0) {
         // cells left of the raster all land in cell 0 (fig.rs:295): their sum telescopes
         j = -minp;
@@ -1432,23 +1429,20 @@ __device__ __forceinline__ void scan_row(int x_bot, int inv, bool st, bool en, i
             const int p = v - prev;
             prev = v;
             if (p && ck(minp + j >= 0 && minp + j < W, 2)) atomicAdd(&area[minp + j], ed * p);
-            cell1 = minp + j;
             if (v >= cov) break;
             x_cov = min(x_cov + step, FX_ONE);
         }
     }
-    if (spans)
-        for (int sp = cell0 >> 7; sp <= (cell1 >> 7); sp++) atomicOr(&spans[sp >> 5], 1u << (sp & 31));
 }
 
 // The cell step of an edge, step_cov(ONE) (fig.rs:315-321): step_pix when positive,
 // else ONE; first_cov's r * step equals step_cov(r) for both.
 __device__ __forceinline__ int cell_step(const EdgeRec& E) { return E.step_pix > 0 ? E.step_pix : FX_ONE; }
 
-__device__ __forceinline__ void scan_item(const EdgeRec& E, int y, int* area, int W, unsigned* spans = nullptr) {
+__device__ __forceinline__ void scan_item(const EdgeRec& E, int y, int* area, int W) {
     const int x_bot = wadd(E.x_bot0, wmul(y - E.start_row, E.inv_slope));
     scan_row(x_bot, E.inv_slope, y == E.start_row, y == E.end_row, fxfract(E.y_upper), fxfract(E.y_lower),
-             cell_step(E), E.ed, area, W, spans);
+             cell_step(E), E.ed, area, W);
 }
 
 // Resolve one band row and write it (fig.rs:621-665, imgbuf.rs:38-199).
@@ -1869,33 +1863,28 @@ __global__ void __launch_bounds__(BLOCK, 4) k_cbuild(KParams P) {
 }
 
 // Per-warp shared memory of the Matte8 band compositor for rows of `width` pixels: the
-// row's i32 cell areas and its touched-span marks.
-__host__ __device__ constexpr int row_smem_bytes(int width) {
-    return (int)align256((size_t)((width + 3) & ~3) * 4 + (size_t)(((width + 127) / 128 + 31) / 32) * 4);
-}
+// row's i32 cell areas.
+__host__ __device__ constexpr int row_smem_bytes(int width) { return (int)align256((size_t)((width + 3) & ~3) * 4); }
 
 // Accumulate the cells of the `ne` band edges that cross scan row y into `row`
-// (one warp; each lane takes edges), marking the touched 128-pixel spans.
-__device__ __forceinline__ void row_items(const EdgeRec* edges, int ne, int y, int* row, int W, unsigned* spans) {
+// (one warp; each lane takes edges).
+__device__ __forceinline__ void row_items(const EdgeRec* edges, int ne, int y, int* row, int W) {
     const int lane = threadIdx.x & 31;
     for (int e = lane; e < ne; e += 32) {
         const EdgeRec E = edges[e];
-        if (E.start_row <= y && y <= E.end_row) scan_item(E, y, row, W, spans);
+        if (E.start_row <= y && y <= E.end_row) scan_item(E, y, row, W);
     }
 }
 
 // Resolve one Matte8 row (imgbuf.rs:38-199) and overwrite every pixel of it
-// (fig.rs:629-636).  Clears the row buffer and the span marks.
-__device__ __forceinline__ void matte_row(int* row, unsigned* spans, int W, int Wp, uint8_t* drow, int rule) {
+// (fig.rs:629-636).
+__device__ __forceinline__ void matte_row(const int* row, int W, int Wp, uint8_t* drow, int rule) {
     const int lane = threadIdx.x & 31;
     unsigned carry = 0;
     for (int x0 = 0; x0 < W; x0 += 128) {
         const int x = x0 + lane * 4;
         int4 a = make_int4(0, 0, 0, 0);
-        if (x < Wp) {
-            a = *reinterpret_cast<const int4*>(row + x);
-            *reinterpret_cast<int4*>(row + x) = make_int4(0, 0, 0, 0);
-        }
+        if (x < Wp) a = *reinterpret_cast<const int4*>(row + x);
         const unsigned s0 = (unsigned)a.x, s1 = s0 + (unsigned)a.y, s2 = s1 + (unsigned)a.z, s3 = s2 + (unsigned)a.w;
         const unsigned inc = warp_incl_sum_u(s3);
         const unsigned ex = inc - s3 + carry;
@@ -1906,10 +1895,6 @@ __device__ __forceinline__ void matte_row(int* row, unsigned* spans, int W, int 
         for (int c = 0; c < 4; c++)
             if (x + c < W) drow[x + c] = (uint8_t)av[c];
     }
-    __syncwarp();
-    const int n_words = ((W + 127) / 128 + 31) / 32;
-    for (int k = lane; k < n_words; k += 32) spans[k] = 0;
-    __syncwarp();
 }
 
 // Matte8 ordered composite: every call overwrites its rows from its top row down
@@ -1923,12 +1908,8 @@ __global__ void __launch_bounds__(BLOCK) k_cbands(KParams P) {
     const int R = P.band_rows, b = blockIdx.x;
     const int r = b * R + warp;  // this warp's raster row
     if (warp >= R || r >= H) return;
-    unsigned char* mine = smem + (size_t)warp * row_smem_bytes(W);
-    int* row = reinterpret_cast<int*>(mine);
-    unsigned* spans = reinterpret_cast<unsigned*>(row + Wp);
-    const int n_words = ((W + 127) / 128 + 31) / 32;
+    int* row = reinterpret_cast<int*>(smem + (size_t)warp * row_smem_bytes(W));
     for (int x = lane * 4; x < Wp; x += 128) *reinterpret_cast<int4*>(row + x) = make_int4(0, 0, 0, 0);
-    for (int k = lane; k < n_words; k += 32) spans[k] = 0;
     __syncwarp();
     uint8_t* drow = P.rasters + (size_t)r * P.canvas_stride;
     const int n = (int)P.n_items;
@@ -1943,9 +1924,9 @@ __global__ void __launch_bounds__(BLOCK) k_cbands(KParams P) {
     const int4 cr = P.crec[found];
     const int o0 = P.bandoff[(size_t)b * n + found], o1 = P.bandoff[(size_t)(b + 1) * n + found];
     const unsigned long long first = ((unsigned long long)(unsigned)cr.z | ((unsigned long long)(unsigned)cr.w << 32)) + o0;
-    row_items(P.pool + first, o1 - o0, r + cr.y, row, W, nullptr);
+    row_items(P.pool + first, o1 - o0, r + cr.y, row, W);
     __syncwarp();
-    matte_row(row, spans, W, Wp, drow, P.rule);
+    matte_row(row, W, Wp, drow, P.rule);
 }
 
 // ===========================================================================

@@ -129,7 +129,7 @@ __device__ __forceinline__ unsigned long long top_key(int x, int y) {
 // 32, or -1: the path is not for this kernel.  S.top and S.top_slot are set.
 template <int NT>
 __device__ __noinline__ int tile_build(const TileParams& P, const ft_path_desc& d, TileState<NT>& S, TileBuild<NT>& B, int4* E,
-                          unsigned* ends, float sw0) {
+                          unsigned* ends) {
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const ft_op* ops = P.ops + d.op_begin;
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(NT, NT == 32 ? 32 : NT == 128 ? 8 : 2) k_tile(
             d = P.paths[wi.path];
         }
         const float sw0 = P.sw_chain ? *P.sw_chain : d.s_width;
-        const int n_slots = tile_build<NT>(P, d, S, B, E, ends, sw0);
+        const int n_slots = tile_build<NT>(P, d, S, B, E, ends);
         if (P.single && tid == 0) P.overflow[it] = n_slots < 0;
         if (n_slots < 0) {  // these rows go to k_raster
             if (!P.single && tid == 0) P.overflow[atomicAdd(&P.queue[2], 1u)] = (uint32_t)it;
