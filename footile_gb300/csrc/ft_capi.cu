@@ -514,7 +514,7 @@ int single(ft_ctx* c, int stroke, int32_t rule, const ft_op* ops, uint32_t n_ops
     d.op_begin = 0;
     d.n_ops = n_ops;
     d.width = w;
-    d.height = h;
+    d.height = w ? h : 0;  // of no columns there may be any number of rows, more than an int holds
     d.raster_offset = 0;
     d.stride = stride;
     d.s_width = c->s_width;
