@@ -969,9 +969,10 @@ static int run_pipelined(ft_ctx* c, int stroke, int rule, const ft_op* ops, uint
     return FT_OK;
 }
 
-// Chunks of a host batch: the tuning's host_chunks, else 2 from 64 MB of rasters.  More
-// chunks lose: every chunk's persistent launch ends on its slowest paths (65,536 glyphs
-// in 1 / 2 / 4 chunks: 16.3 / 15.7 / 21.6 ms end to end).
+// Chunks of a host batch: the tuning's host_chunks, else 2 from 64 MB of rasters.  Every
+// chunk's persistent launch ends on its slowest paths, so what more chunks overlap they
+// lose again: 65,536 glyphs in 1 / 2 / 3 / 4 / 6 / 8 chunks 13.1 / 11.4 / 11.0 / 10.5 / 10.5 /
+// 11.3 ms end to end.
 static int host_chunks(const ft_ctx* c, uint64_t raster_bytes, uint32_t n_paths) {
     int k = (c->tuned && c->tune.host_chunks > 0) ? c->tune.host_chunks : (raster_bytes >= (64ull << 20) ? 2 : 1);
     k = std::max(1, std::min(k, 16));

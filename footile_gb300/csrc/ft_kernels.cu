@@ -1671,12 +1671,13 @@ namespace ftk {
 // Plotter::fill / Plotter::stroke calls on one Plotter (plotter.rs:339-365).
 //
 // k_cbuild: one CTA per path builds its figure and edges as k_raster does, then
-// bins the edges by raster band into a device pool.  k_cbands: one CTA per band
-// walks the paths in call order; for each it accumulates the band's cell areas,
-// resolves its rows and composites.  Every call of footile composites every pixel
-// from its top row down, alpha 0 included, and SrcOver with alpha 0 maps each
-// premultiplied channel d to ch8_mul(d, 255), which changes only d in 1..15 and
-// is the identity after 15 applications.  So a tile keeps, per row, the number of
+// bins the edges by raster band into a device pool.  k_cbands (Matte8) draws of each
+// row the last call that reaches it.  k_ctile (Rgba8p) walks the paths in call order;
+// for each it accumulates the tile's cell areas, resolves its rows and composites.
+// Every call of footile composites every pixel from its top row down, alpha 0
+// included, and SrcOver with alpha 0 maps each premultiplied channel d to
+// ch8_mul(d, 255), which changes only d in 1..15 and is the identity after 15
+// applications.  So a tile keeps, per row, the number of
 // calls so far and, per four pixels, the call count at their last visit: covered
 // pixels first take the alpha-0 maps they missed in one step, uncovered pixels are
 // not touched, and the tile ends with one pending flush.

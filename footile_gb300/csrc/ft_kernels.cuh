@@ -229,8 +229,9 @@ struct KParams {
     int split_bin;
     int4* fig_state;             // count, direction, top row, edges fit the pool
     int* bin_hist;               // n_bands counts, then n_bands fill cursors
-    // Rgba8p tile compositor (k_ctile): tile width in pixels (128, 256, 512 or 1024) and
-    // whether the canvas is staged by TMA through the tensor map passed beside these
+    // Rgba8p tile compositor (k_ctile): segment width in pixels (128 or a multiple of
+    // 256, at most 1,024) and whether the canvas is staged by TMA through the tensor map passed
+    // beside these
     int seg_w;
     int use_tma;
     int bin_segs;         // segments of seg_w pixels that a band's edges are binned by (1: not)
@@ -375,9 +376,10 @@ cudaError_t launch_figure_bins(const KParams& p, int grid, cudaStream_t s);
 // The figure of one fill path (p.gb's ops) over the whole GPU, in place of k_cbuild with
 // split_bin: vertices and sub-figure starts into CTA 0's scratch, fig_state[0], the pen
 // width after the path and the path's status.  p.gb's state (done, n_raw, count) must be
-// zero and tr all -1 (bytes 0xFF) before the launch.  When the path has more raw
-// vertices than p.gb.raw_cap, *n_raw says how many and nothing else is written but a
-// figure of no vertices; the caller grows the arrays and builds again.  `probe`
+// zero before the launch; k_gb_ops resets tr, the queue, the path's status, the pool
+// counter and the bins.  When the path has more raw vertices than p.gb.raw_cap, *n_raw
+// says how many and nothing else is written but a figure of no vertices; the caller grows
+// the arrays and builds again.  `probe`
 // (nullable): the same build over a prefix of the ops first (its own state and tr, its
 // final_flag the full build's skip): when the cap is reached within the prefix the figure
 // is complete and the full build does nothing.
