@@ -263,14 +263,6 @@ inline __host__ __device__ int single_rows(int h, int sms) {
     const int even = (h + (sms > 1 ? sms : 1) - 1) / (sms > 1 ? sms : 1);
     return even > 8 ? even : 8;
 }
-// Whether a path is handed to k_raster after the ops [0, done) of its n that have `slots` slots: it
-// has too many, or will have at this rate.  A path built to the end of its scratch and then built
-// again by k_raster cost more than k_raster alone (one of 30,000 curves on 500 x 2000: 2,780 us, handed
-// over after its first ops 2,550); one handed over that would have fitted is drawn as well, by the
-// slower kernel.
-inline __host__ __device__ bool tile_overflows(int slots, int done, int n, int cap) {
-    return slots > cap || (done < n && (long long)slots * n > (long long)cap * done);
-}
 // Cells from one row of a band to the next: three spare cells (a walk of four cells may run
 // past the raster's last), a multiple of eight.
 __host__ __device__ constexpr int tile_pitch(int w) { return (w + 3 + 7) & ~7; }
