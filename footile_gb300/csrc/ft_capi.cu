@@ -217,7 +217,7 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
     const bool few = n_paths < (uint32_t)std::max(2 * c->sm_count, 1);
     const uint32_t wside = stroke ? 0u : (uint32_t)tile_max_side(c);  // strokes use the CTA kernel
     tile = ftk::TilePlan{few ? ftk::TILE_THREADS_FEW : ftk::TILE_THREADS, few ? ftk::TILE_CAP_FEW : ftk::TILE_CAP, 8};
-    bool tiny = !few;
+    bool tiny = !few && n_paths >= (uint32_t)(ftk::TILE_TINY_PATHS * c->sm_count);
     int widest = 8;
     for (uint32_t i = 0; i < n_paths; i++) {
         const ft_path_desc& d = paths[i];

@@ -248,11 +248,14 @@ struct KParams {
 // path, of TILE_THREADS_TINY where all of a batch's are tiny, or of TILE_THREADS_FEW per row range
 // of a path when there are few paths.
 constexpr int TILE_THREADS = 128, TILE_THREADS_TINY = 32, TILE_THREADS_FEW = 512;
-// Tiny: canvases up to TILE_TINY_SIDE a side under TILE_TINY_OPS ops at most, where four warps wait
-// for one another more than they share.  Four warps / one a path: 65,536 canvases of 8 x 8 under 3
-// lines 389 / 144 us, of 24 x 24 under 60 curves 1,295 / 1,095; 3,000 of 24 x 24 under 60 curves
-// 85 / 87, of 48 x 48 under 24 curves 98 / 120 us.
-constexpr int TILE_TINY_SIDE = 24, TILE_TINY_OPS = 64;
+// Tiny: TILE_TINY_PATHS canvases per SM and more, up to TILE_TINY_SIDE a side under TILE_TINY_OPS ops
+// at most, where four warps wait for one another more than they share.  Four warps / one a path,
+// 65,536 canvases of 8 x 8 under 3 lines 389 / 144 us, of 24 x 24 under 14 curves 700 / 434, zoomed in
+// 1,000 times 5,764 / 5,560.  Of fewer canvases each path's chain sets the time, longer by one warp:
+// 20,000 of the same 223 / 146, zoomed in 1,807 / 1,847, 8,000 98 / 68, 763 / 841, 1,200 25 / 29, 156 / 262;
+// of more ops the scratch of so many CTAs holds too little: 65,536 under 30 curves 956 / 742,
+// zoomed in 12,031 / 70,407 (handed over).
+constexpr int TILE_TINY_SIDE = 24, TILE_TINY_OPS = 16, TILE_TINY_PATHS = 128;
 constexpr int TILE_MAX_SIDE = 512;                      // canvases up to this width and height (batches)
 constexpr int TILE_CAP = 32768, TILE_CAP_TINY = 8192, TILE_CAP_FEW = 65504;  // segment slots per CTA (at most the vertex cap)
 static_assert(TILE_CAP % 32 == 0 && TILE_CAP_TINY % 32 == 0 && TILE_CAP_FEW % 32 == 0 && TILE_CAP_FEW <= PT_CAP, "a tile figure never reaches the cap");

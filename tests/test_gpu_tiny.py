@@ -66,3 +66,44 @@ def test_one_large_path_among_tiny_ones(ctx):
     rng = np.random.default_rng(4)
     sides = [12] * 399 + [200]
     run(ctx, [workloads.random_path(rng, s, 9) for s in sides], sides, _abi.MATTE8, _abi.NONZERO)
+
+
+@pytest.mark.parametrize("fmt,rule,pad", [(0, 0, 0), (0, 1, 1), (1, 0, 0), (1, 1, 3)])
+@pytest.mark.parametrize("top,n_ops,less", [(8, 3, 0), (24, 16, 0), (24, 17, 0), (25, 16, 0), (24, 16, 1)])
+def test_as_many_as_one_warp_a_path_takes(ctx, fmt, rule, pad, top, n_ops, less):
+    """128 canvases per SM, and one less; sides and ops at their limits and above."""
+    import torch
+
+    n = 128 * torch.cuda.get_device_properties(0).multi_processor_count - less
+    rng = np.random.default_rng(top + n_ops)
+    some = [workloads.random_path(rng, top, int(rng.integers(1, n_ops - 1))) for _ in range(200)]
+    for k in range(0, 200, 5):  # zoomed in: up to the scratch's last slot, and curves too deep for slots
+        some[k]["v"] = (some[k]["v"] - top / 2) * (100 if k % 10 else 4000)
+    some[1] = workloads.random_path(rng, top, n_ops - 2)
+    assert len(some[1]) == n_ops
+    sides = rng.integers(1, top + 1, (n, 2))
+    sides[1] = top
+    run(ctx, [some[k % 200] for k in range(n)], [tuple(int(v) for v in s) for s in sides],
+        _abi.RGBA8P if fmt else _abi.MATTE8, rule, pad)
+
+
+def test_zoomed_in_batches_keep_four_warps(ctx):
+    """Curves far larger than 3,000 tiny canvases: a path's chain sets the time, by one warp a path five
+    times that of four."""
+    import torch
+    from footile_gb300.plotter import PreparedBatch
+
+    rng = np.random.default_rng(4)
+    parts = [workloads.random_path(rng, 16000, 62, probs=(0, .5, .5)) for _ in range(64)]
+    took = []
+    for side in (24, 25):  # 25: not tiny
+        ops, paths, size = pack_batch([parts[k % 64] for k in range(3000)], [side] * 3000)
+        dev = torch.from_numpy(ops.view(np.uint8)).cuda()
+        ras = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        batch, ms = PreparedBatch(ctx, paths), []
+        for _ in range(7):
+            batch.launch(dev, ras)
+            ms.append(ctx.last_ms())
+        batch.close()
+        took.append(sorted(ms)[3])
+    assert took[0] < 2 * took[1], took
