@@ -192,9 +192,10 @@ int grid_cap(const ft_ctx* c, int per_sm) {
 
 // Most cells of a tile band when there are few paths: 96 KB, a row range is one band, while every
 // range has an SM to itself; else what leaves room for a second CTA (k_tile<512>: 32 KB of queues
-// and 5 bytes a cell where rows are staged, of 113 KB).  300 paths of 900 x 900 Rgba8p with 24,576
-// cells, so in two rounds, and one pixel under way per lane 2,560 us, this way 1,100 (by k_raster 1,270).
-constexpr int TILE_AREA_FEW = 24576, TILE_AREA_PAIR = 16000;
+// and 4 bytes a cell, 5 where rows are staged, of 112 KB).  300 paths of 900 x 900 Rgba8p with
+// 24,576 cells, so in two rounds, and one pixel under way per lane 2,560 us, this way 1,100 (by
+// k_raster 1,270); of 128 x 128 Matte8 with 16,000 cells, so in two bands, 50.6, with 20,400 48.4 us.
+constexpr int TILE_AREA_FEW = 24576, TILE_AREA_PAIR = 20400, TILE_AREA_PAIR_STAGED = 16000;
 
 // Cells of a band for row ranges of `rows` rows: the whole range up to TILE_AREA_FEW, a row at
 // least.
@@ -248,7 +249,11 @@ void plan_items(ft_ctx* c, const ft_path_desc* paths, uint32_t n_paths, int smem
             (tiled ? out_w : out).push_back(ftk::WorkItem{i, r, std::min(d.height, r + rows_per_item), R});
     }
     if (tiny) tile = ftk::TilePlan{ftk::TILE_THREADS_TINY, ftk::TILE_CAP_TINY, 8};
-    if (few && (int)out_w.size() > c->sm_count) tile.few_area = std::max(widest, std::min(tile.few_area, TILE_AREA_PAIR));
+    tile.few_staged = tile.few_area;
+    if (few && (int)out_w.size() > c->sm_count) {
+        tile.few_area = std::max(widest, std::min(tile.few_area, TILE_AREA_PAIR));
+        tile.few_staged = std::max(widest, std::min(tile.few_staged, TILE_AREA_PAIR_STAGED));
+    }
     // Longest first, to a quarter of a power of two, which is all the order the queue needs:
     // a counting sort over 256 classes.  A call on 3,000 / 16,384 paths with a comparison
     // sort here and with this one: 313 / 227 us, 3.6 / 2.7 ms.
@@ -466,7 +471,8 @@ int run_single(ft_ctx* c, int stroke, int rule, const ft_op* ops_d, const ft_pat
     const int smem = choose_smem(c, std::max(d.width, 1u));
     const bool tiled = !stroke && tile_max_side(c) > 0;
     const int h = (int)std::max(d.height, 1u), rows = ftk::single_rows(h, grid_cap(c, 1)), n = (h + rows - 1) / rows;
-    ftk::TilePlan t{ftk::TILE_THREADS_FEW, ftk::TILE_CAP_FEW, few_area((int)d.width, std::min(rows, h))};
+    const int area = few_area((int)d.width, std::min(rows, h));
+    ftk::TilePlan t{ftk::TILE_THREADS_FEW, ftk::TILE_CAP_FEW, area, area};
     FT_CU(c->status.ensure(sizeof(int32_t)), "alloc status");
     FT_CU(c->overflow.ensure(sizeof(uint32_t) * n), "alloc overflow list");
     FT_CU(c->scratch.ensure(std::max(ftk::SCRATCH_BYTES_PER_CTA * (size_t)n,

@@ -312,7 +312,8 @@ int tile_smem(int threads, int area_ints, bool staged);
 // What one launch of the tile rasteriser runs with.
 struct TilePlan {
     int threads = TILE_THREADS, cap = TILE_CAP;
-    int few_area = 8;  // with TILE_THREADS_FEW: the largest item's cells, up to 96 KB
+    int few_area = 8;    // with TILE_THREADS_FEW: the largest item's cells, up to 96 KB
+    int few_staged = 8;  // the same where rows are staged
     // Rgba8p and host rows are staged as bytes
     static bool staged(int fmt, bool host) { return host || fmt == FT_RGBA8P; }
     // Batches: the cells that leave room for eight CTAs per SM.  65,536 glyphs with 2,560 /
@@ -320,7 +321,8 @@ struct TilePlan {
     // Tiny: 32 CTAs per SM.
     int area(int fmt, bool host) const {
         if (threads == TILE_THREADS_TINY) return staged(fmt, host) ? 768 : 1000;
-        return threads == TILE_THREADS_FEW ? few_area : (staged(fmt, host) ? 3712 : 4736);
+        if (threads == TILE_THREADS_FEW) return staged(fmt, host) ? few_staged : few_area;
+        return staged(fmt, host) ? 3712 : 4736;
     }
     int smem(int fmt, bool host) const { return tile_smem(threads, area(fmt, host), staged(fmt, host)); }
 };

@@ -65,3 +65,11 @@ def test_no_slower_than_the_cta_rasteriser(ctx, n):
 
     by_cta, tiled = ms(0), ms(512)
     assert tiled < 1.3 * by_cta, (tiled, by_cta)
+
+
+@pytest.mark.parametrize("w,h", [(128, 128), (149, 134), (149, 135), (117, 133), (117, 134)])
+@pytest.mark.parametrize("fmt", [_abi.MATTE8, _abi.RGBA8P])
+def test_bands_of_two_ctas(ctx, w, h, fmt):
+    """A path in one band of its cells, in two: on both sides of what two CTAs per SM leave room for,
+    20,400 cells, 16,000 where rows are staged."""
+    test_row_ranges(ctx, 200, w, h, fmt)
